@@ -54,9 +54,15 @@ enum sfq_op {
   SFQ_OP_PROPAGATE = 3,
   SFQ_OP_ORTHOGONALIZE = 4,
   SFQ_OP_ENERGY = 5,
-  SFQ_OP_INVERSE_LOGDET = 6
+  SFQ_OP_INVERSE_LOGDET = 6,
+  SFQ_OP_VBIAS = 7,         /* sfq_vbias_ws, real Lnak */
+  SFQ_OP_VHS = 8,           /* sfq_vhs_ws */
+  SFQ_OP_VBIAS_COMPLEX = 9  /* sfq_vbias_ws, complex Lnak */
 };
-/* device bytes of scratch the op needs for these sizes */
+/* device bytes of scratch the op needs for these sizes.  SFQ_OP_PROPAGATE and the two _ws operations
+ * also run in less: the size returned is what their int8 tensor-core path takes, and with a smaller
+ * workspace they run on the FP64 tensor pipe (propagate: in 3 * (16 nwalk nmo nel, rounded up to 256)
+ * bytes at least, the _ws operations in none). */
 size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol);
 
 /* det_ops::MixedDensityMatrix(A, B, C, ovlp, compact, herm=true)
@@ -115,6 +121,15 @@ int sfq_vbias(const void* G, const void* Lnak, int lnak_complex, void* v, int nw
  * vHS[w,i,k] = sqrt(dt) * sum_n Likn[i,k,n] X[w,n];  Likn (nmo, nmo, nchol) real; X (nwalk, nchol) complex;
  * vHS (nwalk, nmo, nmo) complex */
 int sfq_vhs(const double* Likn, const void* X, void* vHS, int nwalk, int nmo, int nchol, double dt, void* stream);
+
+/* the same two with a workspace of sfq_workspace_size(SFQ_OP_VBIAS / _VBIAS_COMPLEX / SFQ_OP_VHS, ...)
+ * bytes, in which large products run on the int8 tensor cores: FP64 operands scaled per row to
+ * 58-bit integers, multiplied exactly modulo 15 coprime moduli and reconstructed (Ozaki scheme II),
+ * at least as accurate as the FP64 tensor pipe relative to the operand rows' norms. */
+int sfq_vbias_ws(const void* G, const void* Lnak, int lnak_complex, void* v, int nwalk, int nel, int nmo, int nchol,
+                 double dt, int closed, void* ws, size_t ws_bytes, void* stream);
+int sfq_vhs_ws(const double* Likn, const void* X, void* vHS, int nwalk, int nmo, int nchol, double dt, void* ws,
+               size_t ws_bytes, void* stream);
 
 /* energy(E, G, idet=0, addH1, addEJ, addEXX)   Real3IndexFactorization.hpp:138-174, energy_impl :476-590
  * E (nwalk, 3) complex out [E1, EXX, EJ]; G (nwalk, nel*nmo); haj (nel, nmo) complex; Lnak as in vbias;
@@ -202,7 +217,11 @@ int sfq_split_bf16(const double* src, long n, void* p0, void* p1, void* p2, void
  * C + s * M * N.  tile_n: 64, 128 or 160 (0: automatic). */
 int sfq_gemm_int8_slices(const double* A, const double* B, float* C, int M, int N, int K, int nslices, int tile_n,
                          int ksplit, void* stream);
-/* the Taylor term's product in the same arithmetic: C[c][w][a][j] = part c of sum_i A[w][a][i] V[w][j][i]
+/* C = A B^T (M x N, FP64) of device doubles A (M x K), B (N x K) by the modular int8 products of
+ * sfq_vhs_ws; operands it cannot hold (an Inf, a NaN, a row norm outside 1e+-150) go through the FP64
+ * tensor pipe instead.  M <= 65535, K <= 90000. */
+int sfq_gemm_f64_modular(const double* A, const double* B, double* C, int M, int N, int K, void* stream);
+/* the Taylor term's product in the same arithmetic (the int8 slices'): C[c][w][a][j] = part c of sum_i A[w][a][i] V[w][j][i]
  * (A (W, N, M), V (W, M, M) complex doubles, taken through FP32 as the engine holds them; C planar
  * FP32 (2, W, N, M)); half: 32, 64 or 80 orbitals per tile. */
 int sfq_gemm_int8_cplx_b(const void* A, const void* V, float* C, int W, int M, int N, int nslices, int half,

@@ -110,7 +110,9 @@ def vbias(G, Lnak, dt, closed=True):
     W = G.shape[0]
     Nc, N, M = Lnak.shape
     v = torch.empty((W, Nc), dtype=torch.complex128, device="cuda")
-    check(lib().sfq_vbias(ptr(G), ptr(Lnak), int(_is_cplx(Lnak)), ptr(v), W, N, M, Nc, dt, int(closed), _stream()))
+    ws = _ws(capi.OP_VBIAS_COMPLEX if _is_cplx(Lnak) else capi.OP_VBIAS, W, M, N, Nc)
+    check(lib().sfq_vbias_ws(ptr(G), ptr(Lnak), int(_is_cplx(Lnak)), ptr(v), W, N, M, Nc, dt, int(closed), ptr(ws),
+                             ws.numel(), _stream()))
     return v
 
 
@@ -120,7 +122,8 @@ def vHS(Likn, X, dt):
     M, _, Nc = Likn.shape
     W = X.shape[0]
     V = torch.empty((W, M, M), dtype=torch.complex128, device="cuda")
-    check(lib().sfq_vhs(ptr(Likn), ptr(X), ptr(V), W, M, Nc, dt, _stream()))
+    ws = _ws(capi.OP_VHS, W, M, 0, Nc)
+    check(lib().sfq_vhs_ws(ptr(Likn), ptr(X), ptr(V), W, M, Nc, dt, ptr(ws), ws.numel(), _stream()))
     return V
 
 

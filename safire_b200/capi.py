@@ -13,6 +13,7 @@ SFQ_OK = 0
 ERRORS = {1: "SHAPE", 2: "ARG", 3: "UNSUPPORTED", 4: "CUDA", 5: "OOM", 6: "WEIGHT_COLLAPSE", 7: "NONFINITE",
           8: "TIMEOUT", 9: "WORKSPACE", 10: "INTERNAL", 11: "RANK"}
 OP_MIXED_DENSITY_MATRIX, OP_LOG_OVERLAP, OP_PROPAGATE, OP_ORTHOGONALIZE, OP_ENERGY, OP_INVERSE_LOGDET = 1, 2, 3, 4, 5, 6
+OP_VBIAS, OP_VHS, OP_VBIAS_COMPLEX = 7, 8, 9
 
 # walker property columns, in the order the engine stores them (WalkerConfig.hpp:28-48 names)
 PROPS = ("WEIGHT", "PHASE", "PSEUDO_ELOC_", "E1_", "EXX_", "EJ_", "OVLP", "THETA")
@@ -93,6 +94,8 @@ _SIGS = {
     "sfq_orthogonalize": ([_VP, _VP, _I, _I, _I, _VP, _SZ, _VP], _I),
     "sfq_vbias": ([_VP, _VP, _I, _VP, _I, _I, _I, _I, _D, _I, _VP], _I),
     "sfq_vhs": ([_VP, _VP, _VP, _I, _I, _I, _D, _VP], _I),
+    "sfq_vbias_ws": ([_VP, _VP, _I, _VP, _I, _I, _I, _I, _D, _I, _VP, _SZ, _VP], _I),
+    "sfq_vhs_ws": ([_VP, _VP, _VP, _I, _I, _I, _D, _VP, _SZ, _VP], _I),
     "sfq_energy": ([_VP, _VP, _VP, _VP, _I, _D, _I, _I, _I, _I, _I, _I, _I, _VP, _SZ, _VP], _I),
     "sfq_assemble_x": ([_VP, _VP, _VP, _VP, _VP, _U64, _U64, _I, _I, _D, _I, _VP], _I),
     "sfq_comb": ([_VP, _D, _I, _VP, _VP], _I),
@@ -103,6 +106,7 @@ _SIGS = {
     "sfq_gemm_bf16_planes": ([ctypes.POINTER(_VP), ctypes.POINTER(_VP), _I, _VP, _I, _I, _I, _I, ctypes.c_long,
                               ctypes.c_long, ctypes.c_float, ctypes.c_float, _I, _VP], _I),
     "sfq_split_bf16": ([_VP, ctypes.c_long, _VP, _VP, _VP, _VP], _I),
+    "sfq_gemm_f64_modular": ([_VP, _VP, _VP, _I, _I, _I, _VP], _I),
     "sfq_gemm_int8_slices": ([_VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP], _I),
     "sfq_engine_copy_walker": ([_VP, _I, _I], _I),
     "sfq_engine_walker_row_elems": ([_VP], ctypes.c_long),

@@ -1,0 +1,176 @@
+// FP64 products on the int8 tensor cores by modular arithmetic (Ozaki scheme II: K. Ozaki,
+// Y. Uchino, T. Imamura, "Ozaki Scheme II: A GEMM-oriented emulation of floating-point matrix
+// multiplication using an integer modular technique", 2025).
+//
+// Every operand row is scaled by a power of two and rounded to integers a' with a 2-norm below
+// 2^58; a product C' = sum_k a'_k b'_k is then an integer with |C'| < 2^116 < P/2 (Cauchy-Schwarz),
+// P = prod p_i over 15 pairwise coprime moduli p_i <= 256 (log2 P = 117.78).  C' is known from its
+// residues, and each residue is one exact int8 product with int32 accumulation (tcgen05
+// kind::i8) of the operands' residues.  The only rounding is that of the operands, 2^-59 of their
+// row's norm, and of the result to FP64: with K random terms the relative error of a result is
+// about 2^-58 sqrt(K), against 2^-55 sqrt(K) of an FP64 chain of K additions.
+//
+// Rows that the scheme cannot hold (an Inf or a NaN, a norm outside 2^+-500) raise a flag in
+// device memory; the FP64 tensor-pipe product (gemm_f64), launched behind it with
+// GemmDesc::only_if, then computes the result.
+#pragma once
+#include "common.cuh"
+
+namespace sfq {
+namespace crt {
+
+constexpr int NMOD = 15;
+constexpr int kNormBits = 58;        // operand rows are scaled to a 2-norm below 2^kNormBits
+constexpr long kMaxK = 90000;        // |sum of K residue products| <= K 2^14 < 2^30.5
+
+typedef unsigned __int128 u128;
+
+struct Tables {
+  unsigned mod[16];        // p_i; the 16th is a placeholder (never used)
+  // residue of u = a' + 2^60 (8 bytes): t = sum_j byte_j (256^j mod p) + init, centred afterwards
+  unsigned clo[16], chi[16], init[16];
+  unsigned m32[16];        // ceil(2^32 / p): floor(t / p) of t < 2^20
+  unsigned m39[16];        // ceil(2^39 / p): floor(u / p) of u < 2^28 as umulhi(u, m39) >> 7
+  unsigned big27[16];      // the smallest multiple of p >= 2^27
+  unsigned big30[16];      // the smallest multiple of p >= 3 * 2^29
+  unsigned r16[16];        // 2^16 mod p
+  // C'/P mod 1 = sum_i r_i G_i mod 1 with G_i = ((P / p_i)^-1 mod p_i) / p_i, in 80-bit fixed point;
+  // byte j of the G_i of moduli 4q .. 4q+3 in g[j][q]
+  unsigned g[10][4];
+  double P;                // P rounded to double
+};
+
+constexpr unsigned kModuli[15] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
+
+constexpr Tables make_tables() {
+  Tables t{};
+  double P = 1.0;
+  for (int i = 0; i < 15; ++i) P *= double(kModuli[i]);
+  t.P = P;
+  for (int i = 0; i < 15; ++i) {
+    const unsigned p = kModuli[i];
+    t.mod[i] = p;
+    unsigned pw = 1 % p;
+    for (int j = 0; j < 8; ++j) {
+      if (j < 4) t.clo[i] |= pw << (8 * j);
+      else t.chi[i] |= pw << (8 * (j - 4));
+      pw = pw * 256 % p;
+    }
+    unsigned off = 1;
+    for (int j = 0; j < 60; ++j) off = off * 2 % p;
+    t.init[i] = (p - off) % p;
+    t.m32[i] = unsigned(((1ull << 32) + p - 1) / p);
+    t.m39[i] = unsigned(((1ull << 39) + p - 1) / p);
+    t.big27[i] = unsigned(((1ull << 27) + p - 1) / p * p);
+    t.big30[i] = unsigned(((3ull << 29) + p - 1) / p * p);
+    t.r16[i] = 65536u % p;
+    unsigned rest = 1;  // P / p_i mod p_i
+    for (int j = 0; j < 15; ++j)
+      if (j != i) rest = rest * (kModuli[j] % p) % p;
+    unsigned inv = 0;
+    for (unsigned x = 1; x < p; ++x)
+      if (rest * x % p == 1) inv = x;
+    const u128 G = ((u128(inv) << 80) + p / 2) / p;
+    for (int j = 0; j < 10; ++j) t.g[j][i / 4] |= unsigned(G >> (8 * j) & 255) << (8 * (i % 4));
+  }
+  t.mod[15] = 1;
+  return t;
+}
+
+// ---- operands ---------------------------------------------------------------------------------
+// NMOD residue planes of an operand: plane i at q + i * plane, rows of ld bytes (a multiple of 16),
+// the row's scale exponent in e: x = a' 2^e
+struct Planes {
+  int8_t* q = nullptr;
+  int* e = nullptr;
+  long rows = 0, ld = 0, plane = 0;
+};
+inline long ld_of(long K) { return (K + 63) / 64 * 64; }
+inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
+inline size_t planes_bytes(long rows, long K) { return align256((size_t)rows * ld_of(K)) * NMOD; }
+inline size_t exps_bytes(long rows) { return align256(sizeof(int) * (size_t)rows); }
+// lays the planes of rows x K out at *at and advances it (e_rows exponents behind them)
+inline Planes lay_out(char*& at, long rows, long K, long e_rows) {
+  Planes p;
+  p.rows = rows;
+  p.ld = ld_of(K);
+  p.plane = (long)align256((size_t)rows * p.ld);
+  p.q = reinterpret_cast<int8_t*>(at);
+  at += planes_bytes(rows, K);
+  p.e = reinterpret_cast<int*>(at);
+  at += exps_bytes(e_rows);
+  return p;
+}
+
+// ---- the product of residues: C_i = A_i B_i^T mod p_i for every modulus ------------------------
+// Output row ((part * batch + b) * M + m), column n, at C + i * c_plane + row * ldc + n (bytes).
+// A rows a_off[part][seg] + b * a_bs + m, B rows b_off[seg] + b * b_bs + n, summed over the segments
+// (a complex product: parts re, im; segments against Re B and Im B).
+struct Gemm {
+  Planes A, B;
+  int M = 0, N = 0, K = 0, batch = 1, parts = 1, segs = 1;
+  long a_bs = 0, b_bs = 0;
+  long a_off[2][2] = {{0, 0}, {0, 0}};
+  long b_off[2] = {0, 0};
+  uint8_t* C = nullptr;
+  long ldc = 0, c_plane = 0;
+  int* flag = nullptr;  // set when a bounded wait expires
+};
+int gemm(const Gemm& g, cudaStream_t st);
+
+// The same for products whose left rows are a walker's: [re; im] rows (w, a) of A's blocks (re, im, -im at
+// block strides a_blk; row w N + a) against cols rows of B (row w b_bs + n; segs = 2: complex B, its
+// imaginary rows b_off1 further).  Output row c c_part + w N + a.
+struct WalkerGemm {
+  Planes A, B;
+  int N = 0, cols = 0, K = 0, batch = 1, segs = 1;
+  long a_blk = 0, b_bs = 0, b_off1 = 0;
+  uint8_t* C = nullptr;
+  long ldc = 0, c_plane = 0, c_part = 0;
+  int* flag = nullptr;
+};
+bool walker_gemm_fits(int N, int cols, int K, int segs);
+int walker_gemm(const WalkerGemm& g, cudaStream_t st);
+
+// the output of a product: NMOD planes of rows x ldc bytes
+struct Out {
+  uint8_t* q = nullptr;
+  long ldc = 0, plane = 0;
+};
+inline long ldc_of(long N) { return (N + 15) / 16 * 16; }
+inline size_t out_bytes(long rows, long N) { return align256((size_t)rows * ldc_of(N)) * NMOD; }
+inline Out lay_out_c(char*& at, long rows, long N) {
+  Out o;
+  o.q = reinterpret_cast<uint8_t*>(at);
+  o.ldc = ldc_of(N);
+  o.plane = (long)align256((size_t)rows * o.ldc);
+  at += out_bytes(rows, N);
+  return o;
+}
+
+// ---- operands to residues -----------------------------------------------------------------------
+// real rows (row r of `rows` at src + r * stride, K doubles) -> planes row r
+int rows_real(const double* src, long rows, long K, long stride, const Planes& out, int* flag, cudaStream_t st);
+// complex rows (K complex each) -> blocks re, im (nb = 2) or re, im, -im (nb = 3): row r's block k at
+// plane row k * blk_stride + (r / inner) * outer + r % inner, one exponent per complex row (e[r])
+int rows_cplx(const cplx* src, long rows, long K, long stride, int nb, long blk_stride, long inner, long outer,
+              const Planes& out, int* flag, cudaStream_t st);
+// walkers (W, M, N) complex -> rows (w, a) over the M orbitals, blocks re, im: plane row k * W N + w N + a
+int walkers_in(const cplx* SM, int W, int M, int N, const Planes& out, int* flag, cudaStream_t st);
+
+// ---- residues to FP64 ---------------------------------------------------------------------------
+// out[m][n] = alpha (C_re + i C_im) for parts = 2 products with M rows; exponents eA[m], eB[n]
+int out_cplx(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, cplx* out, long ldo,
+             const int* skip_if, cudaStream_t st);
+int out_real(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, double* out, long ldo,
+             const int* skip_if, cudaStream_t st);
+// one Taylor term: T = (i / k) C (k = 0: T = C), S (2, W, N, M) += T (k = 0: S = T), and the residues of T,
+// blocks re, im, -im (last: of S, blocks re, im) -> `next`.  C rows (part, w, a), columns j.
+int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int* eA, const int* eB, int eB_per_w,
+                  double* S, const Planes& next, int* flag, cudaStream_t st);
+// SM[w][j][a] = C_re + i C_im of rows (part, w, a), columns j
+int walkers_out(const Out& c, int W, int M, int N, const int* eA, const int* eB, cplx* SM, const int* skip_if,
+                cudaStream_t st);
+
+}  // namespace crt
+}  // namespace sfq

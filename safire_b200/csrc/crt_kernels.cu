@@ -1,0 +1,386 @@
+// Residues of FP64 operands and FP64 values of residue products (see crt.cuh).
+#include "crt.cuh"
+#include "crt_dev.cuh"
+
+namespace sfq {
+namespace crt {
+
+namespace {
+
+// the loads of four consecutive elements from k on, zeros past K
+__device__ __forceinline__ void load4(const double* row, long k, long K, bool vec, double x[4]) {
+  if (vec && k + 3 < K) {
+    const double2 a = *reinterpret_cast<const double2*>(row + k), b = *reinterpret_cast<const double2*>(row + k + 2);
+    x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = k + j < K ? row[k + j] : 0.0;
+  }
+}
+
+// sum over the TPR threads of a row (TPR = 32: a warp; else the whole block)
+template <int TPR>
+__device__ __forceinline__ double row_sum(double v, double* sh) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (TPR == 32) return v;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = 0.0;
+#pragma unroll
+  for (int w = 0; w < TPR / 32; ++w) s += sh[w];
+  return s;
+}
+
+// Real rows.  Two passes over a row: its norm, then its residues (the second read comes from L1 or
+// L2: a row is at most a few hundred KB).  One warp per row below 1024 elements, one block above.
+template <int TPR>
+__global__ void __launch_bounds__(256) rows_real_kernel(const double* src, long rows, long K, long stride, int8_t* q,
+                                                        long ld, long plane, int* e, int* flag, int vec) {
+  __shared__ double sh[8];
+  const long r = TPR == 32 ? (long)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;
+  const int t = TPR == 32 ? (threadIdx.x & 31) : threadIdx.x;
+  if (r >= rows) return;  // TPR = 32: whole warps
+  const double* row = src + r * stride;
+  double n2 = 0.0, nz = 0.0;
+  for (long k = 4 * t; k < K; k += 4 * TPR) {
+    double x[4];
+    load4(row, k, K, vec, x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      n2 = fma(x[j], x[j], n2);
+      nz = fmax(nz, fabs(x[j]));
+    }
+  }
+  n2 = row_sum<TPR>(n2, sh);
+  // a row of zeros has the norm 0; one whose squares all vanish does not
+  const bool any = TPR == 32 ? __any_sync(0xffffffffu, nz != 0.0) : __syncthreads_or(nz != 0.0) != 0;
+  const int ex = row_exponent(n2, any, t == 0 ? flag : nullptr);
+  if (t == 0) e[r] = ex;
+  const double sc = pow2(-ex);
+  int8_t* qr = q + r * ld;
+  for (long k = 4 * t; k < K; k += 4 * TPR) {
+    double x[4];
+    load4(row, k, K, vec, x);
+    Quad qd;
+    qd.set(x, sc);
+    qd.store(qr + k, plane);
+  }
+}
+
+// Complex rows: the same, both parts with one exponent; blocks re, im (, -im)
+template <int TPR, int NB>
+__global__ void __launch_bounds__(256) rows_cplx_kernel(const cplx* src, long rows, long K, long stride,
+                                                        long blk_stride, long inner, long outer, int8_t* q, long ld,
+                                                        long plane, int* e, int* flag) {
+  __shared__ double sh[8];
+  const long r = TPR == 32 ? (long)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;
+  const int t = TPR == 32 ? (threadIdx.x & 31) : threadIdx.x;
+  if (r >= rows) return;
+  const cplx* row = src + r * stride;
+  double n2 = 0.0, nz = 0.0;
+  for (long k = t; k < K; k += TPR) {
+    const cplx z = row[k];
+    n2 = fma(z.x, z.x, fma(z.y, z.y, n2));
+    nz = fmax(nz, fmax(fabs(z.x), fabs(z.y)));
+  }
+  n2 = row_sum<TPR>(n2, sh);
+  const bool any = TPR == 32 ? __any_sync(0xffffffffu, nz != 0.0) : __syncthreads_or(nz != 0.0) != 0;
+  const int ex = row_exponent(n2, any, t == 0 ? flag : nullptr);
+  if (t == 0) e[r] = ex;
+  const double sc = pow2(-ex);
+  int8_t* qr = q + ((r / inner) * outer + r % inner) * ld;
+  for (long k = 4 * t; k < K; k += 4 * TPR) {
+    double x[4], y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const cplx z = k + j < K ? row[k + j] : mk(0.0, 0.0);
+      x[j] = z.x;
+      y[j] = z.y;
+    }
+    Quad a;
+    a.set(x, sc);
+    a.store(qr + k, plane);
+    a.set(y, sc);
+    if (NB == 3) a.store2(qr + blk_stride * ld + k, qr + 2 * blk_stride * ld + k, plane);
+    else a.store(qr + blk_stride * ld + k, plane);
+  }
+}
+
+// Walkers (W, M, N) -> rows (w, a) over the orbitals: a block takes 16 columns of one walker, their
+// norms first, then 64 orbitals at a time through shared memory (the transpose).
+__global__ void __launch_bounds__(256) walkers_in_kernel(const cplx* SM, int W, int M, int N, int8_t* q, long ld,
+                                                         long plane, int* e, int* flag) {
+  __shared__ cplx tile[64][17];
+  __shared__ double sh[16][17];
+  __shared__ double scs[16];
+  __shared__ int nz[16];
+  const int w = blockIdx.y, a0 = blockIdx.x * 16;
+  const int ca = threadIdx.x & 15, ri = threadIdx.x >> 4;
+  const cplx* S = SM + (long)w * M * N;
+  double n2 = 0.0, mx = 0.0;
+  if (threadIdx.x < 16) nz[threadIdx.x] = 0;
+  __syncthreads();
+  if (a0 + ca < N) {
+    for (int i = ri; i < M; i += 16) {
+      const cplx z = S[(long)i * N + a0 + ca];
+      n2 = fma(z.x, z.x, fma(z.y, z.y, n2));
+      mx = fmax(mx, fmax(fabs(z.x), fabs(z.y)));
+    }
+  }
+  sh[ri][ca] = n2;
+  if (mx != 0.0) nz[ca] = 1;
+  __syncthreads();
+  if (threadIdx.x < 16 && a0 + ca < N) {
+    double s = 0.0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) s += sh[j][ca];
+    const int ex = row_exponent(s, nz[ca] != 0, flag);
+    e[(long)w * N + a0 + ca] = ex;
+    scs[ca] = pow2(-ex);
+  }
+  const long WN = (long)W * N;
+  for (int i0 = 0; i0 < M; i0 += 64) {
+    __syncthreads();
+    for (int s = ri; s < 64; s += 16) {
+      const int i = i0 + s;
+      tile[s][ca] = i < M && a0 + ca < N ? S[(long)i * N + a0 + ca] : mk(0.0, 0.0);
+    }
+    __syncthreads();
+    const int a = threadIdx.x >> 4, i4 = 4 * (threadIdx.x & 15);  // 16 rows x 16 groups of four orbitals
+    if (a0 + a < N && i0 + i4 < M) {
+      double x[4], y[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        x[j] = tile[i4 + j][a].x;
+        y[j] = tile[i4 + j][a].y;
+      }
+      int8_t* qr = q + ((long)w * N + a0 + a) * ld + i0 + i4;
+      Quad d;
+      d.set(x, scs[a]);
+      d.store(qr, plane);
+      d.set(y, scs[a]);
+      d.store(qr + WN * ld, plane);
+    }
+  }
+}
+
+// four columns of one output row from its residue planes
+struct Vals {
+  double v[4];
+};
+__device__ __forceinline__ Vals values4(const uint8_t* c, long plane, int ea, const int eb[4], double s) {
+  long long X[4];
+  reconstruct4(c, plane, X);
+  Vals o;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) o.v[j] = double(X[j]) * (s * pow2(ea + eb[j]));
+  return o;
+}
+
+__device__ __forceinline__ void load_e4(const int* e, long n, long N, int eb[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) eb[j] = n + j < N ? e[n + j] : 0;
+}
+
+// complex output, 4 columns per thread, 128 per warp; the warp's values go through shared memory so that
+// its stores are whole 512-byte rows
+__global__ void __launch_bounds__(256) out_cplx_kernel(const uint8_t* c, long ldc, long plane, long M, long N,
+                                                       const int* eA, const int* eB, double alpha, cplx* out,
+                                                       long ldo, const int* skip_if) {
+  __shared__ cplx sh[8][130];
+  if (skip_if && *skip_if) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const long m = blockIdx.y, nw = ((long)blockIdx.x * 8 + warp) * 128;
+  if (nw >= N) return;
+  const long n = nw + 4 * lane;
+  if (n < N) {
+    int eb[4];
+    load_e4(eB, n, N, eb);
+    const double s = alpha * kTwoM64P;
+    const Vals re = values4(c + m * ldc + n, plane, eA[m], eb, s);
+    const Vals im = values4(c + (M + m) * ldc + n, plane, eA[m], eb, s);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sh[warp][4 * lane + j] = mk(re.v[j], im.v[j]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int t = 32 * j + lane;
+    if (nw + t < N) out[m * ldo + nw + t] = sh[warp][t];
+  }
+}
+
+__global__ void __launch_bounds__(256) out_real_kernel(const uint8_t* c, long ldc, long plane, long M, long N,
+                                                       const int* eA, const int* eB, double alpha, double* out,
+                                                       long ldo, const int* skip_if) {
+  if (skip_if && *skip_if) return;
+  const long m = blockIdx.y, n = 4 * ((long)blockIdx.x * 256 + threadIdx.x);
+  if (n >= N) return;
+  int eb[4];
+  load_e4(eB, n, N, eb);
+  const Vals re = values4(c + m * ldc + n, plane, eA[m], eb, alpha * kTwoM64P);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (n + j < N) out[m * ldo + n + j] = re.v[j];
+}
+
+// One Taylor term of one row (w, a): see taylor_update.  Memory bound (15 residues in, S in and out,
+// 45 residues out per complex element); the row's T waits in shared memory for its norm.
+template <bool FIRST, bool LAST>
+__global__ void __launch_bounds__(128) taylor_kernel(const uint8_t* c, long ldc, long plane, long WN, int N, int M,
+                                                     double inv_k, const int* eA, const int* eB, int eB_per_w,
+                                                     double* S, int8_t* q, long ld, long qplane, int* e, int* flag) {
+  extern __shared__ double row[];  // T (or S when LAST), re then im, M4 each
+  __shared__ double sh[4];
+  const long r = blockIdx.x;
+  const int w = int(r / N);
+  const int M4 = (M + 3) / 4 * 4;
+  const int* eb0 = eB + (eB_per_w ? (long)w * M : 0);
+  const int ea = eA[r];
+  double* Sr = S + r * M;
+  double* Si = S + (WN + r) * M;
+  double n2 = 0.0, nz = 0.0;
+  for (int j0 = 4 * threadIdx.x; j0 < M; j0 += 512) {
+    int eb[4];
+    load_e4(eb0, j0, M, eb);
+    const Vals re = values4(c + r * ldc + j0, plane, ea, eb, kTwoM64P * inv_k);
+    const Vals im = values4(c + (WN + r) * ldc + j0, plane, ea, eb, kTwoM64P * inv_k);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      double x = 0.0, y = 0.0;
+      if (j0 + j < M) {
+        x = FIRST ? re.v[j] : -im.v[j];  // T = (i / k) C
+        y = FIRST ? im.v[j] : re.v[j];
+        if (FIRST) {
+          Sr[j0 + j] = x;
+          Si[j0 + j] = y;
+        } else {
+          const double sx = Sr[j0 + j] + x, sy = Si[j0 + j] + y;
+          if (LAST) {
+            x = sx;
+            y = sy;
+          } else {
+            Sr[j0 + j] = sx;
+            Si[j0 + j] = sy;
+          }
+        }
+      }
+      n2 = fma(x, x, fma(y, y, n2));
+      nz = fmax(nz, fmax(fabs(x), fabs(y)));
+      row[j0 + j] = x;
+      row[M4 + j0 + j] = y;
+    }
+  }
+  n2 = row_sum<128>(n2, sh);
+  const bool any = __syncthreads_or(nz != 0.0) != 0;
+  const int ex = row_exponent(n2, any, threadIdx.x == 0 ? flag : nullptr);
+  if (threadIdx.x == 0) e[r] = ex;
+  const double sc = pow2(-ex);
+  int8_t* qr = q + r * ld;
+  for (int j0 = 4 * threadIdx.x; j0 < M; j0 += 512) {  // this thread's own entries of the row
+    Quad d;
+    d.set(row + j0, sc);
+    d.store(qr + j0, qplane);
+    d.set(row + M4 + j0, sc);
+    if (LAST) d.store(qr + WN * ld + j0, qplane);
+    else d.store2(qr + WN * ld + j0, qr + 2 * WN * ld + j0, qplane);
+  }
+}
+
+// SM[w][j][a] from rows (part, w, a), columns j: 32 x 32 tiles transposed through shared memory
+__global__ void __launch_bounds__(256) walkers_out_kernel(const uint8_t* c, long ldc, long plane, long WN, int M,
+                                                          int N, const int* eA, const int* eB, cplx* SM,
+                                                          const int* skip_if) {
+  __shared__ cplx tile[32][33];
+  if (skip_if && *skip_if) return;
+  const int w = blockIdx.z, j0 = blockIdx.x * 32, a0 = blockIdx.y * 32;
+  {
+    const int a = threadIdx.x >> 3, j4 = 4 * (threadIdx.x & 7);
+    if (a0 + a < N && j0 + j4 < M) {
+      const long r = (long)w * N + a0 + a;
+      int eb[4];
+      load_e4(eB, j0 + j4, M, eb);
+      const Vals re = values4(c + r * ldc + j0 + j4, plane, eA[r], eb, kTwoM64P);
+      const Vals im = values4(c + (WN + r) * ldc + j0 + j4, plane, eA[r], eb, kTwoM64P);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) tile[j4 + j][a] = mk(re.v[j], im.v[j]);
+    }
+  }
+  __syncthreads();
+  const int a = threadIdx.x & 31;
+  for (int j = threadIdx.x >> 5; j < 32; j += 8)
+    if (j0 + j < M && a0 + a < N) SM[((long)w * M + j0 + j) * N + a0 + a] = tile[j][a];
+}
+
+}  // namespace
+
+int rows_real(const double* src, long rows, long K, long stride, const Planes& o, int* flag, cudaStream_t st) {
+  if (rows <= 0 || K <= 0) return SFQ_OK;
+  const int vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && stride % 2 == 0;
+  if (K < 1024)
+    rows_real_kernel<32><<<ceil_div(rows, 8), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, flag, vec);
+  else
+    rows_real_kernel<256><<<unsigned(rows), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, flag, vec);
+  SFQ_LAUNCHED();
+  return SFQ_OK;
+}
+
+int rows_cplx(const cplx* src, long rows, long K, long stride, int nb, long blk, long inner, long outer,
+              const Planes& o, int* flag, cudaStream_t st) {
+  if (rows <= 0 || K <= 0) return SFQ_OK;
+  const bool wide = K >= 1024;
+  const unsigned grid = wide ? unsigned(rows) : unsigned(ceil_div(rows, 8));
+  auto k = wide ? (nb == 3 ? rows_cplx_kernel<256, 3> : rows_cplx_kernel<256, 2>)
+                : (nb == 3 ? rows_cplx_kernel<32, 3> : rows_cplx_kernel<32, 2>);
+  k<<<grid, 256, 0, st>>>(src, rows, K, stride, blk, inner, outer, o.q, o.ld, o.plane, o.e, flag);
+  SFQ_LAUNCHED();
+  return SFQ_OK;
+}
+
+int walkers_in(const cplx* SM, int W, int M, int N, const Planes& o, int* flag, cudaStream_t st) {
+  walkers_in_kernel<<<dim3((N + 15) / 16, W), 256, 0, st>>>(SM, W, M, N, o.q, o.ld, o.plane, o.e, flag);
+  SFQ_LAUNCHED();
+  return SFQ_OK;
+}
+
+int out_cplx(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, cplx* out, long ldo,
+             const int* skip_if, cudaStream_t st) {
+  out_cplx_kernel<<<dim3(ceil_div(N, 1024), unsigned(M)), 256, 0, st>>>(c.q, c.ldc, c.plane, M, N, eA, eB, alpha, out,
+                                                                        ldo, skip_if);
+  SFQ_LAUNCHED();
+  return SFQ_OK;
+}
+
+int out_real(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, double* out, long ldo,
+             const int* skip_if, cudaStream_t st) {
+  out_real_kernel<<<dim3(ceil_div(N, 1024), unsigned(M)), 256, 0, st>>>(c.q, c.ldc, c.plane, M, N, eA, eB, alpha, out,
+                                                                        ldo, skip_if);
+  SFQ_LAUNCHED();
+  return SFQ_OK;
+}
+
+int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int* eA, const int* eB, int eB_per_w,
+                  double* S, const Planes& o, int* flag, cudaStream_t st) {
+  const int M4 = (M + 3) / 4 * 4;
+  const size_t sm = sizeof(double) * 2 * M4;
+  const double ik = k > 0 ? 1.0 / double(k) : 1.0;
+  auto kern = k == 0 ? taylor_kernel<true, false> : last ? taylor_kernel<false, true> : taylor_kernel<false, false>;
+  if (sm > 48 * 1024) SFQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  kern<<<unsigned(W * N), 128, sm, st>>>(c.q, c.ldc, c.plane, (long)W * N, N, M, ik, eA, eB, eB_per_w, S, o.q, o.ld,
+                                         o.plane, o.e, flag);
+  SFQ_LAUNCHED();
+  return SFQ_OK;
+}
+
+int walkers_out(const Out& c, int W, int M, int N, const int* eA, const int* eB, cplx* SM, const int* skip_if,
+                cudaStream_t st) {
+  walkers_out_kernel<<<dim3((M + 31) / 32, (N + 31) / 32, W), 256, 0, st>>>(c.q, c.ldc, c.plane, (long)W * N, M, N, eA,
+                                                                           eB, SM, skip_if);
+  SFQ_LAUNCHED();
+  return SFQ_OK;
+}
+
+}  // namespace crt
+}  // namespace sfq

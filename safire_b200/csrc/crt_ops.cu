@@ -1,0 +1,242 @@
+// The FP64 path's large products on the int8 tensor cores (see crt.cuh): force bias, vHS and the
+// propagation.  Each raises a flag where the modular scheme cannot hold an operand, and launches the
+// FP64 tensor-pipe version behind it on that flag.
+#include "crt.cuh"
+#include "crt_ops.cuh"
+#include "ops.cuh"
+
+#include <algorithm>
+#include <cmath>
+
+namespace sfq {
+namespace ops {
+using namespace crt;
+
+namespace {
+constexpr size_t kFlagBytes = 256;
+// scratch of one chunk of a call's work: large enough to fill the GPU several times over
+constexpr size_t kChunkBytes = size_t(3) << 29;  // 1.5 GiB
+
+size_t vbias_row_bytes(long K, bool l_cplx, int W) {
+  return (size_t)NMOD * ((l_cplx ? 2 : 1) * (size_t)ld_of(K) + 2 * (size_t)W) + sizeof(int);
+}
+size_t vhs_row_bytes(int W, int Nc) { return (size_t)NMOD * ((size_t)ld_of(Nc) + 2 * (size_t)W) + sizeof(int); }
+// rows per chunk: the whole operand, or equal chunks of a multiple of 16 rows within kChunkBytes
+long chunk_rows(long rows, size_t row_bytes) {
+  const long most = std::max<long>(256, long(kChunkBytes / row_bytes));
+  const long n = (rows + most - 1) / most;
+  return n <= 1 ? rows : ((rows + n - 1) / n + 15) / 16 * 16;
+}
+size_t slack() { return 256 * (2 * NMOD + 4); }  // plane roundings
+}  // namespace
+
+// ---- force bias -----------------------------------------------------------------------------------
+size_t vbias_crt_bytes(int W, int N, int M, int Nc, bool l_cplx, bool prepared) {
+  const long K = (long)N * M;
+  const long nb = prepared ? Nc : chunk_rows(Nc, vbias_row_bytes(K, l_cplx, W));
+  size_t b = kFlagBytes + planes_bytes((l_cplx ? 3L : 2L) * W, K) + exps_bytes(W) + out_bytes(2L * W, nb);
+  if (!prepared) b += planes_bytes((l_cplx ? 2L : 1L) * nb, K) + exps_bytes(nb);
+  return b + slack();
+}
+
+// The FP64 tensor-pipe product walks K = N M in one chain per tile of few tiles (74 us at K = 576, 1.9 ms at
+// 16384, whatever the walkers); this path takes 29 us at K = 1024 and 402 us at 16384 with 256 walkers.
+// Below K = 300 its launches cost as much as the chain.
+bool vbias_crt_ok(int W, int N, int M, int Nc, bool l_cplx) {
+  const long K = (long)N * M;
+  return W >= 8 && W <= 65535 && Nc >= 64 && K >= 300 && K * (l_cplx ? 2 : 1) <= kMaxK;
+}
+
+int vbias_crt(const cplx* G, const void* Lnak, bool l_cplx, const Planes* Lq, cplx* v, int W, int N, int M, int Nc,
+              double a, char* ws, cudaStream_t st) {
+  const long K = (long)N * M;
+  const long nb = Lq ? Nc : chunk_rows(Nc, vbias_row_bytes(K, l_cplx, W));
+  int* flag = reinterpret_cast<int*>(ws);
+  char* at = ws + kFlagBytes;
+  int rc;
+  SFQ_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  Planes A = lay_out(at, (l_cplx ? 3L : 2L) * W, K, W);
+  Planes B = Lq ? *Lq : lay_out(at, (l_cplx ? 2L : 1L) * nb, K, nb);
+  Out C = lay_out_c(at, 2L * W, nb);
+  if ((rc = rows_cplx(G, W, K, K, l_cplx ? 3 : 2, W, W, W, A, flag, st))) return rc;
+  for (long n0 = 0; n0 < Nc; n0 += nb) {
+    const long n = std::min<long>(nb, Nc - n0);
+    if (!Lq) {
+      if (l_cplx) rc = rows_cplx((const cplx*)Lnak + n0 * K, n, K, K, 2, nb, n, n, B, flag, st);
+      else rc = rows_real((const double*)Lnak + n0 * K, n, K, K, B, flag, st);
+      if (rc) return rc;
+    }
+    crt::Gemm g;
+    g.A = A; g.B = B; g.K = int(K); g.N = int(n);
+    if (l_cplx) {
+      g.M = W; g.parts = g.segs = 2;
+      g.a_off[0][0] = 0; g.a_off[0][1] = 2L * W; g.a_off[1][0] = W; g.a_off[1][1] = 0;
+      g.b_off[1] = Lq ? Nc : nb;
+    } else {
+      g.M = 2 * W;
+    }
+    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.flag = flag;
+    Out c = C;
+    c.ldc = g.ldc;
+    if ((rc = crt::gemm(g, st))) return rc;
+    if ((rc = out_cplx(c, W, n, A.e, B.e, a, v + n0, Nc, nullptr, st))) return rc;
+  }
+  return vbias(G, Lnak, l_cplx, v, W, N, M, Nc, a, st, flag);
+}
+
+// ---- vHS --------------------------------------------------------------------------------------
+size_t vhs_crt_bytes(int W, long rows, int Nc, bool prepared) {
+  const long nb = chunk_rows(rows, vhs_row_bytes(W, Nc));
+  size_t b = kFlagBytes + planes_bytes(2L * W, Nc) + exps_bytes(W) + out_bytes(2L * W, nb);
+  if (!prepared) b += planes_bytes(nb, Nc) + exps_bytes(nb);
+  return b + slack();
+}
+
+// Converting L (M^2 Nc elements) costs what the FP64 product of about 64 walkers does: from 96 walkers on
+// the call gains (1.3x at M = 128 with 128 walkers, 2.5x at M = 256 and 400 with 256), at 64 it is even.  With
+// L's planes prepared the product alone counts.
+bool vhs_crt_ok(int W, long rows, int Nc, bool prepared) {
+  const double flops = 4.0 * W * double(rows) * Nc;
+  if (W > 65535 || Nc > kMaxK || Nc < 96) return false;
+  return prepared ? W >= 32 && flops >= 1e9 : W >= 96 && flops >= 4e9;
+}
+
+int vhs_crt(const double* L, long rows, const Planes* Lq, const cplx* X, cplx* V, int W, int Nc, double a, char* ws,
+            cudaStream_t st) {
+  const long nb = chunk_rows(rows, vhs_row_bytes(W, Nc));
+  int* flag = reinterpret_cast<int*>(ws);
+  char* at = ws + kFlagBytes;
+  int rc;
+  SFQ_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  Planes A = lay_out(at, 2L * W, Nc, W);
+  Planes B = Lq ? *Lq : lay_out(at, nb, Nc, nb);
+  Out C = lay_out_c(at, 2L * W, nb);
+  if ((rc = rows_cplx(X, W, Nc, Nc, 2, W, W, W, A, flag, st))) return rc;
+  for (long r0 = 0; r0 < rows; r0 += nb) {
+    const long n = std::min<long>(nb, rows - r0);
+    if (!Lq && (rc = rows_real(L + r0 * Nc, n, Nc, Nc, B, flag, st))) return rc;
+    crt::Gemm g;
+    g.A = A; g.B = B; g.M = 2 * W; g.N = int(n); g.K = Nc;
+    g.b_off[0] = Lq ? r0 : 0;
+    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.flag = flag;
+    Out c = C;
+    c.ldc = g.ldc;
+    if ((rc = crt::gemm(g, st))) return rc;
+    if ((rc = out_cplx(c, W, n, A.e, B.e + (Lq ? r0 : 0), a, V + r0, rows, nullptr, st))) return rc;
+  }
+  return vhs_rows(L, rows, X, V, W, Nc, a, st, 0, flag);
+}
+
+// ---- propagation --------------------------------------------------------------------------------
+namespace {
+size_t prop_walker_bytes(int M, int Nr) {  // Nr = npol * N rows per walker
+  return (size_t)NMOD * (3 * (size_t)Nr * ld_of(M) + 2 * (size_t)M * ld_of(M) + 2 * (size_t)Nr * ldc_of(M)) +
+         16 * (size_t)Nr * M + 4 * (size_t)(Nr + M);
+}
+int prop_chunk(int W, int M, int Nr) {
+  const long most = std::max<long>(1, long(kChunkBytes / prop_walker_bytes(M, Nr)));
+  const long n = (W + most - 1) / most;
+  return int((W + n - 1) / n);
+}
+}  // namespace
+
+size_t propagate_crt_bytes(int W, int M, int N, int npol, bool prepared) {
+  const int Nr = N * npol, wc = prop_chunk(W, M, Nr);
+  const long R = (long)wc * Nr;
+  size_t b = planes_bytes(3 * R, M) + exps_bytes(R) + planes_bytes(2L * wc * M, M) + exps_bytes((long)wc * M) +
+             out_bytes(2 * R, M) + align256(16 * (size_t)R * M);
+  b = std::max(b, 3 * align256(sizeof(cplx) * (size_t)R * M));  // the FP64 chain's buffers share the space
+  if (!prepared) b += planes_bytes(M, M) + exps_bytes(M);
+  return kFlagBytes + b + slack();
+}
+
+// The walkers' and V's conversions grow as M^2 and M N, the products as M^2 N: even at M = 192 (1.48 ms
+// both ways with 48 electrons, 256 walkers), 1.8x at M = 400 with 100 electrons.
+bool propagate_crt_ok(int W, int M, int N, int npol, bool p_cplx, int order) {
+  const double flops = 64.0 * W * M * double(M) * N * npol;
+  return !p_cplx && order >= 1 && W <= 30000 && M <= 4096 && N * npol >= 16 &&
+         (M >= 320 ? flops >= 5e9 : M >= 240 && flops >= 1.5e10) && walker_gemm_fits(N * npol, M, M, 2);
+}
+
+int propagate_crt(cplx* SM, const double* P1, const Planes* P1q, const cplx* V, int W, int M, int N, int npol,
+                  int order, char* ws, cudaStream_t st) {
+  const int Nr = N * npol, wc = prop_chunk(W, M, Nr);
+  int* flag = reinterpret_cast<int*>(ws);
+  char* at = ws + kFlagBytes;
+  int rc;
+  SFQ_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  Planes P = P1q ? *P1q : lay_out(at, M, M, M);
+  if (!P1q && (rc = rows_real(P1, M, M, M, P, flag, st))) return rc;
+  for (int w0 = 0; w0 < W; w0 += wc) {
+    const int w = std::min(wc, W - w0);
+    const long R = (long)w * Nr;
+    cplx* S0 = SM + (long)w0 * Nr * M;
+    const cplx* Vw = V + (long)w0 * M * M;
+    char* o = at;
+    Planes A = lay_out(o, 3 * R, M, R);
+    Planes B = lay_out(o, 2L * w * M, M, (long)w * M);
+    Out C = lay_out_c(o, 2 * R, M);
+    double* S = reinterpret_cast<double*>(o);
+    if ((rc = walkers_in(S0, w * npol, M, N, A, flag, st))) return rc;
+    if ((rc = rows_cplx(Vw, (long)w * M, M, M, 2, M, M, 2L * M, B, flag, st))) return rc;
+    crt::WalkerGemm p1;  // rows (part, w, a) of P1 SM
+    p1.A = A; p1.B = P; p1.N = Nr; p1.cols = M; p1.K = M; p1.batch = w; p1.segs = 1;
+    p1.a_blk = R; p1.C = C.q; p1.ldc = C.ldc; p1.c_plane = C.plane; p1.c_part = R; p1.flag = flag;
+    if ((rc = crt::walker_gemm(p1, st))) return rc;
+    if ((rc = taylor_update(C, w, Nr, M, 0, false, A.e, P.e, 0, S, A, flag, st))) return rc;
+    crt::WalkerGemm t = p1;  // C = V T: re = Vr Tr + Vi (-Ti), im = Vr Ti + Vi Tr
+    t.B = B; t.segs = 2; t.b_bs = 2L * M; t.b_off1 = M;
+    for (int k = 1; k <= order; ++k) {
+      if ((rc = crt::walker_gemm(t, st))) return rc;
+      if ((rc = taylor_update(C, w, Nr, M, k, k == order, A.e, B.e, 1, S, A, flag, st))) return rc;
+    }
+    if ((rc = crt::walker_gemm(p1, st))) return rc;
+    if ((rc = walkers_out(C, w * npol, M, N, A.e, P.e, S0, flag, st))) return rc;
+    const size_t blk = align256(sizeof(cplx) * (size_t)R * M);
+    if ((rc = propagate(S0, P1, false, Vw, w, M, N, order, (cplx*)at, (cplx*)(at + blk), (cplx*)(at + 2 * blk), st,
+                        npol, flag)))
+      return rc;
+  }
+  return SFQ_OK;
+}
+
+}  // namespace ops
+}  // namespace sfq
+
+extern "C" int sfq_gemm_f64_modular(const double* A, const double* B, double* C, int M, int N, int K, void* stream) {
+  using namespace sfq;
+  if (M < 0 || N < 0 || K < 0) return record_error(SFQ_ERR_SHAPE, "negative size");
+  if (!M || !N) return SFQ_OK;
+  if (!A || !B || !C) return record_error(SFQ_ERR_ARG, "null pointer");
+  if (K < 1 || K > crt::kMaxK || M > 65535)
+    return record_error(SFQ_ERR_SHAPE, "gemm_f64_modular: 1 <= K <= %ld, M <= 65535", crt::kMaxK);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  char* ws = nullptr;
+  const size_t bytes = 256 + crt::planes_bytes(M, K) + crt::exps_bytes(M) + crt::planes_bytes(N, K) +
+                       crt::exps_bytes(N) + crt::out_bytes(M, N);
+  SFQ_CUDA_TRY(cudaMallocAsync((void**)&ws, bytes, st));
+  int* flag = reinterpret_cast<int*>(ws);
+  char* at = ws + 256;
+  const crt::Planes a = crt::lay_out(at, M, K, M), b = crt::lay_out(at, N, K, N);
+  const crt::Out c = crt::lay_out_c(at, M, N);
+  int rc = SFQ_OK;
+  const cudaError_t ce = cudaMemsetAsync(flag, 0, sizeof(int), st);
+  if (ce != cudaSuccess) rc = record_cuda(ce, "gemm_f64_modular", __FILE__, __LINE__);
+  crt::Gemm g;
+  g.A = a; g.B = b; g.M = M; g.N = N; g.K = K; g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.flag = flag;
+  if (!rc) rc = crt::rows_real(A, M, K, K, a, flag, st);
+  if (!rc) rc = crt::rows_real(B, N, K, K, b, flag, st);
+  if (!rc) rc = crt::gemm(g, st);
+  if (!rc) rc = crt::out_real(c, M, N, a.e, b.e, 1.0, C, N, nullptr, st);
+  if (!rc) {
+    GemmDesc d;
+    d.M = M; d.N = N; d.K = K;
+    d.A = A; d.sAm = K; d.sAk = 1;
+    d.B = B; d.sBk = 1; d.sBn = K;
+    d.C = C; d.sCm = N; d.sCn = 1;
+    d.only_if = flag;
+    rc = gemm_f64(d, st);
+  }
+  cudaFreeAsync(ws, st);
+  return rc;
+}

@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "mixed.cuh"
+#include "crt_ops.cuh"
 #include "ops.cuh"
 #include "umma_gemm.cuh"
 #include "islice.cuh"
@@ -533,6 +534,13 @@ struct Engine {
   long P = 0;
   double* Lp = nullptr;  // (P, Nc), FP64 engines
   cplx* Vp = nullptr;    // (W, P), FP64 engines
+  // FP64 engines: residue planes of L (the packed rows when symmetric), Lnak and P1, made once at
+  // setup, and the scratch of the products on the int8 tensor cores (crt_ops.cuh); none where the
+  // sizes are too small for that path or the planes too large
+  crt::Planes L_m, Lnak_m, P1_m;
+  char* crt_buf = nullptr;
+  char* crt_ws = nullptr;
+  size_t crt_bytes = 0;
   // T holds the inverse overlap matrices (PsiT W)^-1 of the current walkers and inv_ov their log
   // overlaps whenever inv_cached is set: the log overlap taken after a propagation or an
   // orthogonalization factors exactly the matrix the next Green's function needs, so that step
@@ -1119,8 +1127,87 @@ struct Engine {
       if ((rc = fill_cplx(props + (long)P_PHASE * W, W, mk(1.0, 0.0), st))) return rc;
     }
     SFQ_CUDA_TRY(cudaMemsetAsync(stats, 0, sizeof(unsigned long long) * 8, st));
+    if (!mixed && (rc = setup_crt())) return rc;
     SFQ_CUDA_TRY(cudaStreamSynchronize(st));
     return SFQ_OK;
+  }
+
+  // FP64 engines: the residue planes of the resident operands and the products' scratch.  Planes take
+  // 15 bytes an element (FP64: 8); above 24 GB of them, or where the device has no room, the
+  // products stay on the FP64 tensor pipe, as they do below the sizes that gain.
+  int setup_crt() {
+    const long rows = sym ? P : (long)M * M;
+    const bool lc = !trial_real;
+    const bool vb = ndet == 1 && ops::vbias_crt_ok(W, N, Mr, Nc, lc);
+    const bool vh = ops::vhs_crt_ok(W, rows, Nc, true);
+    const bool pr = ops::propagate_crt_ok(W, M, N, npol, false, p.taylor_order);
+    if (!vb && !vh && !pr) return SFQ_OK;
+    const long K = (long)N * Mr;
+    size_t planes = 256, ws = 0;
+    if (vb) {
+      planes += crt::planes_bytes((lc ? 2L : 1L) * Nc, K) + crt::exps_bytes(Nc);
+      ws = std::max(ws, ops::vbias_crt_bytes(W, N, Mr, Nc, lc, true));
+    }
+    if (vh) {
+      planes += crt::planes_bytes(rows, Nc) + crt::exps_bytes(rows);
+      ws = std::max(ws, ops::vhs_crt_bytes(W, rows, Nc, true));
+    }
+    if (pr) {
+      planes += crt::planes_bytes(M, M) + crt::exps_bytes(M);
+      ws = std::max(ws, ops::propagate_crt_bytes(W, M, N, npol, true));
+    }
+    if (planes > (size_t(24) << 30)) return SFQ_OK;
+    if (cudaMalloc(&crt_buf, planes + ws) != cudaSuccess) {
+      cudaGetLastError();
+      crt_buf = nullptr;
+      return SFQ_OK;
+    }
+    crt_bytes = planes + ws;
+    crt_ws = crt_buf + planes;
+    int* flag = reinterpret_cast<int*>(crt_buf);
+    char* at = crt_buf + 256;
+    int rc;
+    SFQ_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    if (vb) {
+      Lnak_m = crt::lay_out(at, (lc ? 2L : 1L) * Nc, K, Nc);
+      rc = lc ? crt::rows_cplx((const cplx*)Lnak, Nc, K, K, 2, Nc, Nc, Nc, Lnak_m, flag, st)
+              : crt::rows_real((const double*)Lnak, Nc, K, K, Lnak_m, flag, st);
+      if (rc) return rc;
+    }
+    if (vh) {
+      L_m = crt::lay_out(at, rows, Nc, rows);
+      if ((rc = crt::rows_real(sym ? Lp : Likn, rows, Nc, Nc, L_m, flag, st))) return rc;
+    }
+    if (pr) {
+      P1_m = crt::lay_out(at, M, M, M);
+      if ((rc = crt::rows_real(P1, M, M, M, P1_m, flag, st))) return rc;
+    }
+    int bad = 0;
+    SFQ_CUDA_TRY(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SFQ_CUDA_TRY(cudaStreamSynchronize(st));
+    if (bad) {  // operands that the planes cannot hold
+      cudaFree(crt_buf);
+      crt_buf = crt_ws = nullptr;
+      crt_bytes = 0;
+      L_m = Lnak_m = P1_m = crt::Planes();
+    }
+    return SFQ_OK;
+  }
+  // the step's FP64 products, on the int8 tensor cores where their planes are there
+  int f64_vbias(cplx* out) {
+    if (Lnak_m.q) return ops::vbias_crt(G, Lnak, !trial_real, &Lnak_m, out, W, N, Mr, Nc, vb_scale(), crt_ws, st);
+    return ops::vbias(G, Lnak, !trial_real, out, W, N, Mr, Nc, vb_scale(), st);
+  }
+  int f64_vhs(const cplx* x) {  // -> Vp when symmetric, else V
+    const double* L = sym ? Lp : Likn;
+    const long rows = sym ? P : (long)M * M;
+    cplx* out = sym ? Vp : V;
+    if (L_m.q) return ops::vhs_crt(L, rows, &L_m, x, out, W, Nc, std::sqrt(p.dt), crt_ws, st);
+    return ops::vhs_rows(L, rows, x, out, W, Nc, std::sqrt(p.dt), st);
+  }
+  int f64_propagate(cplx* S) {
+    if (P1_m.q) return ops::propagate_crt(S, P1, &P1_m, V, W, M, N, npol, p.taylor_order, crt_ws, st);
+    return ops::propagate(S, P1, false, V, W, M, N, p.taylor_order, TMN, T1, T2, st, npol);
   }
 
   // the inverse overlap matrices (PsiT W)^-1 of the current walkers in T, their log overlaps in
@@ -1835,7 +1922,7 @@ struct Engine {
       if ((rc = density(nullptr))) return rc;                                        // 1. G
       ph_end(SFQ_PH_DENSITY);
       ph_begin(SFQ_PH_VBIAS);
-      if ((rc = ops::vbias(G, Lnak, !trial_real, X, W, N, Mr, Nc, vb_scale(), st))) return rc;
+      if ((rc = f64_vbias(X))) return rc;
       ph_end(SFQ_PH_VBIAS);
     }
     ph_begin(SFQ_PH_FIELDS);
@@ -1858,17 +1945,13 @@ struct Engine {
     ph_end(SFQ_PH_FIELDS);
     ph_begin(SFQ_PH_VHS);
     ph_begin(SFQ_PH_VHS_GEMM);
-    if (sym) {                                                                        // 3. vHS
-      if ((rc = ops::vhs_rows(Lp, P, X, Vp, W, Nc, std::sqrt(p.dt), st))) return rc;
-    } else {
-      if ((rc = ops::vhs(Likn, X, V, W, M, Nc, std::sqrt(p.dt), st))) return rc;
-    }
+    if ((rc = f64_vhs(X))) return rc;                                                 // 3. vHS
     ph_end(SFQ_PH_VHS_GEMM);
     if (sym && (rc = unpack_symmetric(Vp, W, M, V, st))) return rc;
     ph_end(SFQ_PH_VHS);
     ph_begin(SFQ_PH_PROPAGATE);
     inv_cached = false;
-    if ((rc = ops::propagate(SM, P1, false, V, W, M, N, p.taylor_order, TMN, T1, T2, st, npol))) return rc;  // 4.
+    if ((rc = f64_propagate(SM))) return rc;                                          // 4.
     ph_end(SFQ_PH_PROPAGATE);
     ph_begin(SFQ_PH_OVERLAP);
     if ((rc = ndet > 1 ? log_overlap_md(newov) : log_overlap(newov))) return rc;      // 5.
@@ -3553,6 +3636,7 @@ int sfq_engine_destroy(sfq_engine_t h) {
   if (e.arena) cudaFree(e.arena);
   if (e.Lp) cudaFree(e.Lp);
   if (e.Vp) cudaFree(e.Vp);
+  if (e.crt_buf) cudaFree(e.crt_buf);
   if (e.h_pinned) cudaFreeHost(e.h_pinned);
   if (e.rdm_buf) cudaFree(e.rdm_buf);
   for (void* q : {(void*)e.bp_SMN, (void*)e.bp_fields, (void*)e.bp_wfac, (void*)e.bp_refs, (void*)e.bp_ldet,
@@ -4007,7 +4091,8 @@ int sfq_engine_tiles(sfq_engine_t h, sfq_tiles_t* t) {
 int sfq_engine_footprint(sfq_engine_t h, size_t* bytes) {
   if (!h || !bytes) return record_error(SFQ_ERR_ARG, "null pointer");
   const Engine& e = h->e;
-  *bytes = e.arena_bytes + (e.Lp ? sizeof(double) * e.P * e.Nc : 0) + (e.Vp ? sizeof(cplx) * e.P * e.W : 0);
+  *bytes = e.arena_bytes + (e.Lp ? sizeof(double) * e.P * e.Nc : 0) + (e.Vp ? sizeof(cplx) * e.P * e.W : 0) +
+           e.crt_bytes;
   return SFQ_OK;
 }
 

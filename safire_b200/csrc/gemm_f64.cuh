@@ -30,6 +30,7 @@ struct GemmDesc {
   cplx alpha = {1.0, 0.0};
   cplx beta = {0.0, 0.0};
   const int* mask = nullptr;  // optional: batch b is computed only where mask[b] != 0
+  const int* only_if = nullptr;  // optional: nothing is computed unless *only_if != 0 when the kernel runs
   bool upper_only = false;    // C is needed on and above the diagonal only: tiles wholly below it are skipped
   bool b_upper = false;       // B is upper triangular: column n of C needs K <= n only
 };
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(WM* WN * 32)
   const int wm = warp / WN, wn = warp % WN;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const long bz = blockIdx.z;
+  if (d.only_if && !*d.only_if) return;
   if (d.mask && !d.mask[bz]) return;  // the whole CTA: batches left out by the mask
   if (d.upper_only && m0 >= n0 + BN) return;  // every row of the tile is below every column
 

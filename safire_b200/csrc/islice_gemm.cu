@@ -34,13 +34,11 @@ __host__ __device__ constexpr uint32_t idesc_i8(uint32_t n) {
 
 __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                         uint32_t accumulate) {
-  uint32_t mask0 = 0, mask1 = 0, mask2 = 0, mask3 = 0;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}\n"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(mask0), "r"(mask1), "r"(mask2),
-        "r"(mask3));
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
 // K-major operand tile, BK-byte swizzle (64 or 128): rows of BK bytes (one K slice), 8-row groups
@@ -387,17 +385,23 @@ __global__ void __launch_bounds__(kThreads, 1) islice_gemm_kernel(const __grid_c
         mbar_wait_for(&full[j % STAGES], (j / STAGES) & 1, kWaitNs);
     }
   } else if (warp == 1) {
-    if (lane == 0) {  // MMA issuer
-      uint32_t it = 0;
+    if (elect_one()) {  // MMA issuer
+      // The issue loop is short on purpose (descriptors advanced by additions, K steps unrolled, no lane
+      // masks): the tensor pipe takes 80 cycles for 128 x 160 x 32, and an MMA issued through descriptor
+      // arithmetic took 140 to 220.
+      uint64_t ad0[NS], bd0[NS];
+#pragma unroll
+      for (int q = 0; q < NS; ++q) {
+        ad0[q] = smem_desc_k<BK>(smem + q * L::A_BYTES);
+        bd0[q] = smem_desc_k<BK>(smem + NS * L::A_BYTES + q * L::B_BYTES);
+      }
+      uint32_t s = 0, ph = 0;
       int lt_n = 0;
       bool stop = false;
       for (long t = blockIdx.x; t < total && !stop; t += gridDim.x, ++lt_n) {
         const int b = BUFS == 2 ? (lt_n & 1) : 0;
         const uint32_t aph = BUFS == 2 ? ((uint32_t(lt_n) >> 1) & 1) : (uint32_t(lt_n) & 1);
-        if (*s_abort || !mbar_wait_for(&acc_empty[b], aph ^ 1, wait_ns)) {
-          *s_abort = 1;
-          break;
-        }
+        if (!mbar_wait_abort(&acc_empty[b], aph ^ 1, wait_ns, s_abort)) break;
         fence_after();
         const uint32_t d_tmem = tmem + uint32_t(b) * GCOLS;
         long lt;
@@ -409,35 +413,35 @@ __global__ void __launch_bounds__(kThreads, 1) islice_gemm_kernel(const __grid_c
         decode(p, lt, mt, nt, bz, ks);
         const int kb = k_begin<BK>(p.KT, p.KS, ks), ke = k_begin<BK>(p.KT, p.KS, ks + 1);
         const uint32_t idesc = idesc_i8(uint32_t(cb ? 2 * p.half : BN));
-        for (int kt = kb; kt < ke; ++kt, ++it) {
-          const int s = int(it % STAGES);
-          const uint32_t ph = (it / STAGES) & 1;
-          if (*s_abort || !mbar_wait_for(&full[s], ph, wait_ns)) {
-            *s_abort = 1;
+        for (int kt = kb; kt < ke; ++kt) {
+          if (!mbar_wait_abort(&full[s], ph, wait_ns, s_abort)) {
             stop = true;
             break;
           }
           fence_after();
-          unsigned char* stg = smem + s * L::STAGE;
-          uint64_t ad[NS], bd[NS];
-#pragma unroll
-          for (int q = 0; q < NS; ++q) {
-            ad[q] = smem_desc_k<BK>(stg + q * L::A_BYTES);
-            bd[q] = smem_desc_k<BK>(stg + NS * L::A_BYTES + q * L::B_BYTES);
-          }
+          const uint64_t so = uint64_t(s * uint32_t(L::STAGE >> 4));
           const int k0 = cb ? (kt >> 1) * BK : kt * BK;
           const int rem = Kv - k0;
-          const int nk = rem >= BK ? BK / KSTEP : (rem + KSTEP - 1) / KSTEP;  // K tail: skip all-zero steps
-          const bool first_slice = kt == kb;  // complex B: part 0 of the first K block initialises
-          for (int kk = 0; kk < nk; ++kk) {
-            const uint64_t off = uint64_t(kk * KSTEP) >> 4;  // 32 bytes along the swizzled row
+          const uint32_t later = kt != kb;  // complex B: part 0 of the first K block initialises
+          auto step = [&](int kk, uint32_t acc) {
+            const uint64_t off = so + uint64_t(kk * KSTEP >> 4);  // 32 bytes along the swizzled row
 #pragma unroll
-            for (int t2 = 0; t2 < NP; ++t2) {
-              const uint32_t accum = (first_slice && kk == 0 && pair_first(t2)) ? 0u : 1u;
-              umma_i8(d_tmem + uint32_t(pair_g(t2) * BN), ad[pair_a(t2)] + off, bd[pair_b(t2)] + off, idesc, accum);
-            }
+            for (int t2 = 0; t2 < NP; ++t2)
+              umma_i8(d_tmem + uint32_t(pair_g(t2) * BN), ad0[pair_a(t2)] + off, bd0[pair_b(t2)] + off, idesc,
+                      pair_first(t2) ? acc : 1u);
+          };
+          if (rem > BK - KSTEP) {
+#pragma unroll
+            for (int kk = 0; kk < BK / KSTEP; ++kk) step(kk, kk > 0 ? 1u : later);
+          } else {  // K tail: all-zero steps skipped
+            const int nk = (rem + KSTEP - 1) / KSTEP;
+            for (int kk = 0; kk < nk; ++kk) step(kk, kk > 0 ? 1u : later);
           }
           umma_commit(&empty[s]);
+          if (++s == uint32_t(STAGES)) {
+            s = 0;
+            ph ^= 1;
+          }
         }
         if (!stop) umma_commit(&acc_full[b]);
       }
@@ -445,6 +449,7 @@ __global__ void __launch_bounds__(kThreads, 1) islice_gemm_kernel(const __grid_c
       umma_commit(done);
       mbar_wait_for(done, 0, kWaitNs);
     }
+    __syncwarp();
   } else {  // epilogue warps 2..9 -> TMEM lane quarters 2,3,0,1 (a warp reaches only its quarter)
     const int q = warp & 3;
     const int row = q * 32 + lane;

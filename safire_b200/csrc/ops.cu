@@ -1,4 +1,5 @@
 // Composite device operations and the det_ops / HamOps C entry points.
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdarg>
@@ -6,6 +7,7 @@
 #include <cstring>
 #include <string>
 
+#include "crt_ops.cuh"
 #include "ops.cuh"
 #include <vector>
 #include "umma_gemm.cuh"
@@ -64,8 +66,9 @@ int green_full(const void* A, bool a_cplx, const cplx* Gc, cplx* C, int W, int M
 }
 
 int vbias(const cplx* G, const void* Lnak, bool l_cplx, cplx* v, int W, int N, int M, int Nc, double a,
-          cudaStream_t st) {
+          cudaStream_t st, const int* only_if) {
   GemmDesc d;
+  d.only_if = only_if;
   const long K = (long)N * M;
   d.M = W; d.N = Nc; d.K = int(K); d.batch = 1;
   d.A = G; d.sAm = K; d.sAk = 1; d.a_cplx = true;
@@ -75,12 +78,14 @@ int vbias(const cplx* G, const void* Lnak, bool l_cplx, cplx* v, int W, int N, i
   return gemm_f64(d, st);
 }
 
-int vhs_rows(const double* L, long rows, const cplx* X, cplx* V, int W, int Nc, double a, cudaStream_t st) {
+int vhs_rows(const double* L, long rows, const cplx* X, cplx* V, int W, int Nc, double a, cudaStream_t st,
+             long ldv, const int* only_if) {
   GemmDesc d;
+  d.only_if = only_if;
   d.M = W; d.N = int(rows); d.K = Nc; d.batch = 1;
   d.A = X; d.sAm = Nc; d.sAk = 1; d.a_cplx = true;
   d.B = L; d.sBk = 1; d.sBn = Nc; d.b_cplx = false;
-  d.C = V; d.sCm = rows; d.sCn = 1;
+  d.C = V; d.sCm = ldv ? ldv : rows; d.sCn = 1;
   d.alpha = mk(a, 0.0);
   return gemm_f64(d, st);
 }
@@ -89,8 +94,10 @@ int vhs(const double* Likn, const cplx* X, cplx* V, int W, int M, int Nc, double
   return vhs_rows(Likn, (long)M * M, X, V, W, Nc, a, st);
 }
 
-static int p1_apply(const void* P1, bool p_cplx, const cplx* in, cplx* out, int W, int M, int N, cudaStream_t st) {
+static int p1_apply(const void* P1, bool p_cplx, const cplx* in, cplx* out, int W, int M, int N, cudaStream_t st,
+                    const int* only_if) {
   GemmDesc d;
+  d.only_if = only_if;
   d.M = M; d.N = N; d.K = M; d.batch = W;
   d.A = P1; d.sAm = M; d.sAk = 1; d.sAb = 0; d.a_cplx = p_cplx;
   d.B = in; d.sBk = N; d.sBn = 1; d.sBb = (long)M * N; d.b_cplx = true;
@@ -98,22 +105,35 @@ static int p1_apply(const void* P1, bool p_cplx, const cplx* in, cplx* out, int 
   return gemm_f64(d, st);
 }
 
+namespace {
+__global__ void copy_if_kernel(cplx* dst, const cplx* src, long n, const int* flag) {
+  if (!*flag) return;
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) dst[t] = src[t];
+}
+}  // namespace
+
 int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M, int N, int order, cplx* TMN,
-              cplx* T1, cplx* T2, cudaStream_t st, int npol) {
+              cplx* T1, cplx* T2, cudaStream_t st, int npol, const int* only_if) {
   int rc;
   // npol = 2: spinor walkers (2M, N), the two components' M x N blocks one after the other; P1 and
   // V act on each component (propagate.hpp:247-298, polarization-independent vHS)
   const long n = (long)W * npol * M * N;
   // TMN = P1 * SM   (propagate.hpp:260)
-  if ((rc = p1_apply(P1, p_cplx, SM, TMN, W * npol, M, N, st))) return rc;
+  if ((rc = p1_apply(P1, p_cplx, SM, TMN, W * npol, M, N, st, only_if))) return rc;
   // apply_expM (propagate.hpp:45-70): T1 = S; T2 = (i/n) V T1; S += T2; swap
-  SFQ_CUDA_TRY(cudaMemcpyAsync(T1, TMN, n * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
+  if (only_if) {
+    copy_if_kernel<<<int(n / 256 < 1184 ? n / 256 + 1 : 1184), 256, 0, st>>>(T1, TMN, n, only_if);
+    SFQ_LAUNCHED();
+  } else {
+    SFQ_CUDA_TRY(cudaMemcpyAsync(T1, TMN, n * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
+  }
   cplx* a = T1;
   cplx* b = T2;
   const long MN = (long)M * N;
   for (int k = 1; k <= order; ++k) {
     for (int q = 0; q < npol; ++q) {
       GemmDesc d;
+      d.only_if = only_if;
       d.M = M; d.N = N; d.K = M; d.batch = W;
       d.A = V; d.sAm = M; d.sAk = 1; d.sAb = (long)M * M; d.a_cplx = true;
       d.B = a + q * MN; d.sBk = N; d.sBn = 1; d.sBb = npol * MN; d.b_cplx = true;
@@ -125,7 +145,7 @@ int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M
     cplx* t = a; a = b; b = t;
   }
   // SM = P1 * TMN   (propagate.hpp:297)
-  return p1_apply(P1, p_cplx, TMN, SM, W * npol, M, N, st);
+  return p1_apply(P1, p_cplx, TMN, SM, W * npol, M, N, st, only_if);
 }
 
 namespace {
@@ -300,6 +320,8 @@ using namespace sfq;
 namespace {
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 inline cudaStream_t S(void* p) { return reinterpret_cast<cudaStream_t>(p); }
+// scratch laid out on 256-byte boundaries inside a caller's workspace (whose size has 256 bytes to spare)
+inline char* aligned(void* ws) { return (char*)(((uintptr_t)ws + 255) & ~uintptr_t(255)); }
 constexpr long kEnergyChunkElems = 1L << 27;  // 2 GiB of complex T per chunk at most
 }  // namespace
 
@@ -335,8 +357,20 @@ size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol) {
       return align256(c * nwalk * nel * nel) + align256(c * nwalk * nel * nmo);
     case SFQ_OP_LOG_OVERLAP:
       return align256(c * nwalk * nel * nel);
-    case SFQ_OP_PROPAGATE:
-      return 3 * align256(c * (size_t)nwalk * nmo * nel);
+    case SFQ_OP_PROPAGATE: {
+      const size_t f64 = 3 * align256(c * (size_t)nwalk * nmo * nel);
+      if (nwalk <= 0 || nmo <= 0 || nel <= 0 || !ops::propagate_crt_ok(nwalk, nmo, nel, 1, false, 6)) return f64;
+      return std::max(f64, ops::propagate_crt_bytes(nwalk, nmo, nel, 1, false) + 256);
+    }
+    case SFQ_OP_VBIAS:
+    case SFQ_OP_VBIAS_COMPLEX: {
+      const bool lc = op == SFQ_OP_VBIAS_COMPLEX;
+      if (nwalk <= 0 || nmo <= 0 || nel <= 0 || nchol <= 0 || !ops::vbias_crt_ok(nwalk, nel, nmo, nchol, lc)) return 0;
+      return ops::vbias_crt_bytes(nwalk, nel, nmo, nchol, lc, false) + 256;
+    }
+    case SFQ_OP_VHS:
+      if (nwalk <= 0 || nmo <= 0 || nchol <= 0 || !ops::vhs_crt_ok(nwalk, (long)nmo * nmo, nchol, false)) return 0;
+      return ops::vhs_crt_bytes(nwalk, (long)nmo * nmo, nchol, false) + 256;
     case SFQ_OP_ORTHOGONALIZE:
       return align256(c * (size_t)nwalk * nmo * nel) + align256(c * nwalk * nel * nel) + align256(2 * sizeof(int) * nwalk);
     case SFQ_OP_ENERGY: {
@@ -398,9 +432,12 @@ int sfq_propagate(void* SM, const void* P1, int p1_complex, const void* V, int n
   if (nwalk < 0 || nmo < 0 || nel < 0 || order < 0) return record_error(SFQ_ERR_SHAPE, "negative size");
   if (nwalk == 0 || nel == 0 || nmo == 0) return SFQ_OK;
   if (!SM || !P1 || !V) return record_error(SFQ_ERR_ARG, "null pointer");
-  if (ws_bytes < sfq_workspace_size(SFQ_OP_PROPAGATE, nwalk, nmo, nel, 0))
-    return record_error(SFQ_ERR_WORKSPACE, "propagate: workspace too small");
   const size_t blk = align256(sizeof(cplx) * (size_t)nwalk * nmo * nel);
+  if (ws_bytes < 3 * blk) return record_error(SFQ_ERR_WORKSPACE, "propagate: workspace too small");
+  if (ops::propagate_crt_ok(nwalk, nmo, nel, 1, p1_complex != 0, order) &&
+      ws_bytes >= ops::propagate_crt_bytes(nwalk, nmo, nel, 1, false) + 256)
+    return ops::propagate_crt((cplx*)SM, (const double*)P1, nullptr, (const cplx*)V, nwalk, nmo, nel, 1, order,
+                              aligned(ws), S(stream));
   cplx* TMN = (cplx*)ws;
   cplx* T1 = (cplx*)((char*)ws + blk);
   cplx* T2 = (cplx*)((char*)ws + 2 * blk);
@@ -433,11 +470,32 @@ int sfq_vbias(const void* G, const void* Lnak, int lnak_complex, void* v, int nw
   return ops::vbias((const cplx*)G, Lnak, lnak_complex != 0, (cplx*)v, nwalk, nel, nmo, nchol, a, S(stream));
 }
 
+int sfq_vbias_ws(const void* G, const void* Lnak, int lnak_complex, void* v, int nwalk, int nel, int nmo, int nchol,
+                 double dt, int closed, void* ws, size_t ws_bytes, void* stream) {
+  const bool lc = lnak_complex != 0;
+  if (nwalk <= 0 || nel <= 0 || nmo <= 0 || nchol <= 0 || !G || !Lnak || !v || !ws ||
+      !ops::vbias_crt_ok(nwalk, nel, nmo, nchol, lc) ||
+      ws_bytes < ops::vbias_crt_bytes(nwalk, nel, nmo, nchol, lc, false) + 256)
+    return sfq_vbias(G, Lnak, lnak_complex, v, nwalk, nel, nmo, nchol, dt, closed, stream);
+  return ops::vbias_crt((const cplx*)G, Lnak, lc, nullptr, (cplx*)v, nwalk, nel, nmo, nchol,
+                        std::sqrt(dt) * (closed ? 2.0 : 1.0), aligned(ws), S(stream));
+}
+
 int sfq_vhs(const double* Likn, const void* X, void* vHS, int nwalk, int nmo, int nchol, double dt, void* stream) {
   if (nwalk < 0 || nmo < 0 || nchol < 0) return record_error(SFQ_ERR_SHAPE, "negative size");
   if (nwalk == 0 || nmo == 0) return SFQ_OK;
   if (!Likn || !X || !vHS) return record_error(SFQ_ERR_ARG, "null pointer");
   return ops::vhs(Likn, (const cplx*)X, (cplx*)vHS, nwalk, nmo, nchol, std::sqrt(dt), S(stream));
+}
+
+int sfq_vhs_ws(const double* Likn, const void* X, void* vHS, int nwalk, int nmo, int nchol, double dt, void* ws,
+               size_t ws_bytes, void* stream) {
+  const long rows = (long)nmo * nmo;
+  if (nwalk <= 0 || nmo <= 0 || nchol <= 0 || !Likn || !X || !vHS || !ws || !ops::vhs_crt_ok(nwalk, rows, nchol, false) ||
+      ws_bytes < ops::vhs_crt_bytes(nwalk, rows, nchol, false) + 256)
+    return sfq_vhs(Likn, X, vHS, nwalk, nmo, nchol, dt, stream);
+  return ops::vhs_crt(Likn, rows, nullptr, (const cplx*)X, (cplx*)vHS, nwalk, nchol, std::sqrt(dt), aligned(ws),
+                      S(stream));
 }
 
 int sfq_one_body_matrix(const double* hcore, const double* v0, const double* Likn, const double* vMF, int nmo,

@@ -14,13 +14,16 @@ int green_compact(const cplx* Tinv, const cplx* B, cplx* G, int W, int M, int N,
 // C[w] = A^T * Gc[w] -> (W, nmo, nmo)   (non-compact, herm = true)
 int green_full(const void* A, bool a_cplx, const cplx* Gc, cplx* C, int W, int M, int N, cudaStream_t st);
 int vbias(const cplx* G, const void* Lnak, bool l_cplx, cplx* v, int W, int N, int M, int Nc, double a,
-          cudaStream_t st);
+          cudaStream_t st, const int* only_if = nullptr);
 int vhs(const double* Likn, const cplx* X, cplx* V, int W, int M, int Nc, double a, cudaStream_t st);
 // V (W, rows) = a X L^T for L (rows, Nc): rows = M*M, or the packed upper triangle of symmetric L
-int vhs_rows(const double* L, long rows, const cplx* X, cplx* V, int W, int Nc, double a, cudaStream_t st);
+// (row stride ldv of V: 0 reads as rows)
+int vhs_rows(const double* L, long rows, const cplx* X, cplx* V, int W, int Nc, double a, cudaStream_t st,
+             long ldv = 0, const int* only_if = nullptr);
 // SM <- P1 * Taylor(iV) * P1 * SM with scratch TMN, T1, T2 (each W*M*N complex)
+// only_if: nothing happens unless *only_if != 0 when the kernels run
 int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M, int N, int order, cplx* TMN,
-              cplx* T1, cplx* T2, cudaStream_t st, int npol = 1);
+              cplx* T1, cplx* T2, cudaStream_t st, int npol = 1, const int* only_if = nullptr);
 // CholeskyQR2; SM2 (W*M*N), S (W*N*N) scratch, status (W) ints.  log_detR (W) accumulated if not null
 // CholeskyQR2 in place on SM (SM2, S: scratch; status: 2 W ints)
 // nup in (0, N) (here and below): COLLINEAR walkers, columns [0, nup) up and [nup, N) down, each spin

@@ -53,6 +53,22 @@ __device__ __forceinline__ bool mbar_wait_for(uint64_t* bar, uint32_t parity, un
   return true;
 }
 
+// the same; expired, or given up by another warp (looked at only while the phase is not there yet): raises
+// *abort and returns false
+__device__ __forceinline__ bool mbar_wait_abort(uint64_t* bar, uint32_t parity, unsigned long long limit_ns,
+                                                volatile int* abort) {
+  if (mbar_try_wait(bar, parity)) return true;
+  if (!*abort && mbar_wait_for(bar, parity, limit_ns)) return true;
+  *abort = 1;
+  return false;
+}
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"

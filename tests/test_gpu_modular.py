@@ -1,0 +1,150 @@
+"""FP64 products from int8 residues (crt.cuh): the tensor-core path of the large force-bias, vHS, propagation
+and energy calls against extended or plain FP64 references, at the edges of its tiles and ranges, and the
+operands that it hands to the FP64 tensor pipe."""
+import ctypes
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+def _stream():
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _modular(A, B):
+    from safire_b200.capi import check, lib, ptr
+    M, K = A.shape
+    N = B.shape[0]
+    C = torch.full((M, N), float("nan"), dtype=torch.float64, device="cuda")
+    check(lib().sfq_gemm_f64_modular(ptr(A), ptr(B), ptr(C), M, N, K, _stream()))
+    torch.cuda.synchronize()
+    return C
+
+
+def _rn(g, *shape):
+    return torch.randn(*shape, generator=g, device="cuda", dtype=torch.float64)
+
+
+def _cn(g, *shape):
+    return torch.complex(_rn(g, *shape), _rn(g, *shape))
+
+
+# K edges: one MMA step, the K slices' edges, both reductions of the int32 sums (K > 8192); M, N edges:
+# single rows, tile and column-tile edges, columns that divide by nothing
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (3, 17, 31), (128, 256, 32), (129, 257, 128), (127, 255, 129),
+                                   (64, 300, 400), (200, 513, 1023), (16, 33, 8192), (17, 30, 8193), (5, 40, 90000)])
+@pytest.mark.parametrize("spread", [0.0, 12.0])
+def test_product_against_extended_precision(M, N, K, spread):
+    """Error relative to the rows' norms: the operands' rounding is at most 2^-59 of their row's norm per
+    element, sqrt(K) / 2 of it per row in the 2-norm at most, plus the result's own roundings."""
+    g = torch.Generator(device="cuda").manual_seed(M * 7 + N * 3 + K)
+    A, B = _rn(g, M, K), _rn(g, N, K)
+    if spread:  # rows and columns over 24 decades, entries over 6
+        A = A * 10.0 ** (spread * (2 * torch.rand(M, 1, generator=g, device="cuda", dtype=torch.float64) - 1))
+        B = B * 10.0 ** (6 * (torch.rand(N, K, generator=g, device="cuda", dtype=torch.float64) - 0.5))
+    C = _modular(A, B).cpu().numpy().astype(np.longdouble)
+    a, b = A.cpu().numpy().astype(np.longdouble), B.cpu().numpy().astype(np.longdouble)
+    R = a @ b.T
+    norms = np.sqrt((a * a).sum(1))[:, None] * np.sqrt((b * b).sum(1))[None]
+    # two operands, each element off by at most half of 2^(1 - 58) of its norm; four roundings of the result
+    bound = 2.0 ** -57 * math.sqrt(K) * norms + 4 * 2.0 ** -53 * np.abs(R)
+    assert (np.abs(C - R) <= bound).all()
+
+
+def test_exact_on_integers_and_zeros():
+    g = torch.Generator(device="cuda").manual_seed(5)
+    A = torch.randint(-2**20, 2**20, (70, 333), generator=g, device="cuda").double()
+    B = torch.randint(-2**20, 2**20, (45, 333), generator=g, device="cuda").double()
+    A[3], B[7] = 0.0, 0.0
+    C = _modular(A, B)
+    R = A.cpu().numpy().astype(np.int64) @ B.cpu().numpy().astype(np.int64).T
+    # the operands are held exactly; the sum is rounded to 2^-64 of the residues' range P < 2^118, which is
+    # at most 2^(54 - 116) of the rows' scales 2^(e + 58) <= 2 |row| each: 2^-61 of the norms' product at
+    # most, then four roundings to FP64
+    norms = (A.norm(dim=1)[:, None] * B.norm(dim=1)[None]).cpu().numpy()
+    assert (np.abs(C.cpu().numpy() - R) <= 2.0 ** -61 * norms + 2.0 ** -51 * np.abs(R)).all()
+    assert (C[3] == 0).all() and (C[:, 7] == 0).all()
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 1e200, 1e-200])
+def test_operands_outside_the_range(value):
+    """Rows that the residues cannot hold: the result is the FP64 tensor pipe's."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    A, B = _rn(g, 40, 150), _rn(g, 50, 150)
+    A[5] = 0.0
+    A[5, 9] = value
+    C, R = _modular(A, B).cpu(), (A.cpu() @ B.cpu().T)
+    assert torch.equal(torch.isnan(C), torch.isnan(R)) and torch.equal(torch.isinf(C), torch.isinf(R))
+    ok = torch.isfinite(R)
+    # the FP64 chain's own bound
+    bound = 150 * 2.0 ** -53 * (A.cpu().abs().nan_to_num(0, 0, 0) @ B.cpu().abs().T)
+    assert ((C - R).abs()[ok] <= 2 * bound[ok]).all()
+
+
+def _workspace_path(op, *sizes):
+    from safire_b200.capi import lib
+    return lib().sfq_workspace_size(op, *sizes)
+
+
+@pytest.mark.parametrize("W,M,N", [(20, 331, 37),    # one row tile of [re; im], odd sizes
+                                   (12, 320, 64),    # [re; im] exactly 128 rows
+                                   (12, 321, 65),    # two row tiles
+                                   (6, 330, 128),    # the widest electron block
+                                   (6, 333, 129),    # two chunks of electrons
+                                   (2, 1030, 40),    # K slices that leave room for few electrons
+                                   (1, 900, 100)])   # fewer units than SMs: split columns
+@pytest.mark.parametrize("order", [1, 6])
+def test_propagate(W, M, N, order):
+    from safire_b200 import afqmc, capi
+    f64 = 3 * ((16 * W * M * N + 255) // 256 * 256)
+    assert _workspace_path(capi.OP_PROPAGATE, W, M, N, 0) > f64  # the int8 path runs
+    g = torch.Generator(device="cuda").manual_seed(W + M + N)
+    SM = _cn(g, W, M, N)
+    V = _cn(g, W, M, M) * (0.3 / math.sqrt(M))
+    P1 = torch.eye(M, device="cuda", dtype=torch.float64) + 1e-2 * _rn(g, M, M)
+    P = P1.to(torch.complex128)
+    T = P @ SM
+    S = T.clone()
+    for k in range(1, order + 1):
+        T = (V @ T) * (1j / k)
+        S += T
+    R = P @ S
+    out = afqmc.Propagate(SM.clone(), P1, V, order=order)
+    assert float((out - R).norm() / R.norm()) < 2e-15  # both within a few roundings of the exact chain
+    SM[0, 0, 0] = float("nan")  # a walker that the residues cannot hold: the FP64 tensor pipe's chain
+    bad = afqmc.Propagate(SM.clone(), P1, V, order=order)
+    assert torch.isnan(bad[0, :, 0].real).all() and not torch.isnan(bad[0, :, 1:].real).any()
+    assert W == 1 or float((bad[1:] - R[1:]).norm() / R[1:].norm()) < 1e-14
+
+
+@pytest.mark.parametrize("W,M,N,Nc,cplx", [(150, 100, 30, 1200, False), (8, 101, 23, 613, True),
+                                           (300, 90, 7, 65, False)])
+def test_vbias(W, M, N, Nc, cplx):
+    from safire_b200 import afqmc, capi
+    assert _workspace_path(capi.OP_VBIAS_COMPLEX if cplx else capi.OP_VBIAS, W, M, N, Nc) > 0
+    g = torch.Generator(device="cuda").manual_seed(W)
+    G, L = _cn(g, W, N, M), (_cn(g, Nc, N, M) if cplx else _rn(g, Nc, N, M))
+    R = 2 * math.sqrt(0.01) * (G.reshape(W, -1) @ L.to(torch.complex128).reshape(Nc, -1).T)
+    assert float((afqmc.vbias(G, L, 0.01) - R).norm() / R.norm()) < 1e-14
+    L[3, 2, 1] = float("inf")
+    bad = afqmc.vbias(G, L, 0.01)
+    assert not torch.isfinite(bad[:, 3].real).any() and torch.isfinite(bad[:, :3].real).all()
+
+
+@pytest.mark.parametrize("W,M,Nc", [(100, 160, 401), (200, 61, 1400), (97, 130, 700)])
+def test_vhs(W, M, Nc):
+    from safire_b200 import afqmc, capi
+    assert _workspace_path(capi.OP_VHS, W, M, 0, Nc) > 0
+    g = torch.Generator(device="cuda").manual_seed(W)
+    L, X = _rn(g, M, M, Nc), _cn(g, W, Nc)
+    R = 0.1 * (X @ L.to(torch.complex128).reshape(M * M, Nc).T).reshape(W, M, M)
+    V = afqmc.vHS(L, X, 0.01)
+    assert float((V - R).norm() / R.norm()) < 1e-14
+    X[1, 5] = float("nan")
+    bad = afqmc.vHS(L, X, 0.01)
+    assert torch.isnan(bad[1].real).all() and float((bad[2:] - R[2:]).norm() / R[2:].norm()) < 1e-14
