@@ -6,6 +6,7 @@ namespace sfq {
 using namespace gemm_detail;
 
 namespace {
+constexpr long kSMs = 148;
 
 template <bool AC, bool BC, bool CONJA, bool AK, bool BK, int BM, int BN, int WM, int WN, int STAGES>
 int launch(const GemmDesc& d, cudaStream_t st) {
@@ -27,7 +28,6 @@ int launch(const GemmDesc& d, cudaStream_t st) {
 template <bool AC, bool BC, bool CONJA, bool AK, bool BK>
 int pick_tile(const GemmDesc& d, cudaStream_t st) {
   if constexpr (AC || BC) {
-    if (d.N <= 32) return launch<AC, BC, CONJA, AK, BK, 128, 32, 4, 1, 3>(d, st);
     // per-walker products with 65-112 rows, a short K and many columns (the Green's function at
     // N = 100: 100 x 400 per walker, K = 100): one tile row of 104 or 112 pads 100 rows 1.04x or
     // 1.12x instead of the 1.28x of two 64-row tiles, 80 columns divide 400; one 8 x 40 warp
@@ -41,9 +41,33 @@ int pick_tile(const GemmDesc& d, cudaStream_t st) {
     // with 64 x 64 tiles; with a complex A (W^H W) they were slower
     if (!AC && d.batch > 1 && d.M > 64 && d.M <= 112 && d.N > 64 && d.N <= 112 && d.K >= 256)
       return launch<AC, BC, CONJA, AK, BK, 56, 56, 7, 1, 4>(d, st);
-    // per-walker products (overlaps, CholeskyQR, propagation, the Green's function): 8 warps per
-    // 64 x 64 tile hide more of the DMMA latency on their short K loops (measured 4-6 % faster at
-    // N = 100)
+    // The rest: the tile that leaves the busiest SM the fewest padded outputs, weighed by how near its tile
+    // shape comes to the FP64 pipe's rate (a tile's operand loads per DMMA).  Small matrices then fill
+    // 32 x 8 tiles instead of 128 x 32 (24 x 6 per walker: 10 us a product), few tiles spread over more
+    // SMs, and 33 to 48 rows or columns take 48 instead of 64.  All tiles add in the same order: same bits.
+    struct Shape { int bm, bn; double rate; };
+    static constexpr Shape shapes[] = {{64, 64, 1.0}, {128, 32, 0.95}, {48, 48, 0.95}, {32, 32, 0.85}, {32, 16, 0.7},
+                                       {32, 8, 0.5}};
+    int pick = 0;
+    double best = 0.0;
+    for (int i = 0; i < 6; ++i) {
+      const Shape& t = shapes[i];
+      const long ctas = (long)((d.M + t.bm - 1) / t.bm) * ((d.N + t.bn - 1) / t.bn) * d.batch;
+      const double cost = double((ctas + kSMs - 1) / kSMs) * t.bm * t.bn / t.rate;
+      if (i == 0 || (cost < best && (d.M + t.bm - 1) / t.bm <= 65535)) {
+        best = cost;
+        pick = i;
+      }
+    }
+    switch (pick) {
+      case 1: return launch<AC, BC, CONJA, AK, BK, 128, 32, 4, 1, 3>(d, st);
+      case 2: return launch<AC, BC, CONJA, AK, BK, 48, 48, 3, 2, 3>(d, st);
+      case 3: return launch<AC, BC, CONJA, AK, BK, 32, 32, 2, 2, 3>(d, st);
+      case 4: return launch<AC, BC, CONJA, AK, BK, 32, 16, 4, 1, 3>(d, st);
+      case 5: return launch<AC, BC, CONJA, AK, BK, 32, 8, 4, 1, 3>(d, st);
+    }
+    // 64 x 64: per-walker products (short K loops) with 8 warps, which hide more of the DMMA latency
+    // (measured 4-6 % faster at N = 100)
     if (d.batch > 1 && (d.N <= 128 || d.K <= 128)) return launch<AC, BC, CONJA, AK, BK, 64, 64, 4, 2, 3>(d, st);
     return launch<AC, BC, CONJA, AK, BK, 64, 64, 2, 2, 3>(d, st);
   } else {
