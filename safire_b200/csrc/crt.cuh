@@ -27,9 +27,7 @@ typedef unsigned __int128 u128;
 
 struct Tables {
   unsigned mod[16];        // p_i; the 16th is a placeholder (never used)
-  // residue of u = a' + 2^60 (8 bytes): t = sum_j byte_j (256^j mod p) + init, centred afterwards
-  unsigned clo[16], chi[16], init[16];
-  unsigned m32[16];        // ceil(2^32 / p): floor(t / p) of t < 2^20
+  int m32[16];             // ceil(2^32 / p): floor(x / p) of |x| <= 2^24 as mulhi(x, m32), or one less
   unsigned m39[16];        // ceil(2^39 / p): floor(u / p) of u < 2^28 as umulhi(u, m39) >> 7
   unsigned big27[16];      // the smallest multiple of p >= 2^27
   unsigned big30[16];      // the smallest multiple of p >= 3 * 2^29
@@ -50,16 +48,7 @@ constexpr Tables make_tables() {
   for (int i = 0; i < 15; ++i) {
     const unsigned p = kModuli[i];
     t.mod[i] = p;
-    unsigned pw = 1 % p;
-    for (int j = 0; j < 8; ++j) {
-      if (j < 4) t.clo[i] |= pw << (8 * j);
-      else t.chi[i] |= pw << (8 * (j - 4));
-      pw = pw * 256 % p;
-    }
-    unsigned off = 1;
-    for (int j = 0; j < 60; ++j) off = off * 2 % p;
-    t.init[i] = (p - off) % p;
-    t.m32[i] = unsigned(((1ull << 32) + p - 1) / p);
+    t.m32[i] = int(((1ull << 32) + p - 1) / p);
     t.m39[i] = unsigned(((1ull << 39) + p - 1) / p);
     t.big27[i] = unsigned(((1ull << 27) + p - 1) / p * p);
     t.big30[i] = unsigned(((3ull << 29) + p - 1) / p * p);
@@ -137,7 +126,7 @@ struct Out {
   uint8_t* q = nullptr;
   long ldc = 0, plane = 0;
 };
-inline long ldc_of(long N) { return (N + 15) / 16 * 16; }
+inline long ldc_of(long N) { return (N + 31) / 32 * 32; }  // rows of whole sectors
 inline size_t out_bytes(long rows, long N) { return align256((size_t)rows * ldc_of(N)) * NMOD; }
 inline Out lay_out_c(char*& at, long rows, long N) {
   Out o;
@@ -149,8 +138,10 @@ inline Out lay_out_c(char*& at, long rows, long N) {
 }
 
 // ---- operands to residues -----------------------------------------------------------------------
-// real rows (row r of `rows` at src + r * stride, K doubles) -> planes row r
-int rows_real(const double* src, long rows, long K, long stride, const Planes& out, int* flag, cudaStream_t st);
+// real rows (row r of `rows` at src + r * stride, K doubles) -> planes row (r / inner) * outer + r % inner
+// (inner 0: row r), exponent e[r]
+int rows_real(const double* src, long rows, long K, long stride, const Planes& out, int* flag, cudaStream_t st,
+              long inner = 0, long outer = 0);
 // complex rows (K complex each) -> blocks re, im (nb = 2) or re, im, -im (nb = 3): row r's block k at
 // plane row k * blk_stride + (r / inner) * outer + r % inner, one exponent per complex row (e[r])
 int rows_cplx(const cplx* src, long rows, long K, long stride, int nb, long blk_stride, long inner, long outer,
@@ -168,6 +159,11 @@ int out_real(const Out& c, long M, long N, const int* eA, const int* eB, double 
 // blocks re, im, -im (last: of S, blocks re, im) -> `next`.  C rows (part, w, a), columns j.
 int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int* eA, const int* eB, int eB_per_w,
                   double* S, const Planes& next, int* flag, cudaStream_t st);
+// exx[w, n0 + n] = sum_ab T[w,a,n,b] T[w,b,n,a] and kl[w, n0 + n] = sum_a T[w,a,n,a] of T[w,b,n,a] = rows
+// (part, w, b), columns n * N4 + a (exponents eB[n * N + a]); nup as in energy_exx_reduce
+constexpr int kExxMaxN = 116;  // a walker's N x N block of one n in shared memory
+int exx_reduce(const Out& c, int W, int N, int N4, int nv, int n0, int Nc, const int* eA, const int* eB, cplx* exxn,
+               cplx* kl, int nup, cudaStream_t st);
 // SM[w][j][a] = C_re + i C_im of rows (part, w, a), columns j
 int walkers_out(const Out& c, int W, int M, int N, const int* eA, const int* eB, cplx* SM, const int* skip_if,
                 cudaStream_t st);

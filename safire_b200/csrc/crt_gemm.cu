@@ -18,8 +18,10 @@ constexpr int BN = 256;       // widest tile: one of two accumulator buffers of 
 constexpr int BK = 128;       // K slice: one 128-byte swizzle row
 constexpr int KSTEP = 32;     // K of one kind::i8 MMA
 constexpr int STAGES = 4;
-constexpr int kThreads = 320;  // warps: 0 TMA producer, 1 TMEM owner + MMA issuer, 2-9 epilogue
-constexpr int kEpiThreads = 256;
+// warps: 0 TMA producer, 1 TMEM owner + MMA issuer, 2-17 epilogue (four per TMEM lane quarter: the reduction
+// of a tile with short K is what bounds it, and two warps a scheduler left half of its issue slots idle)
+constexpr int kThreads = 576;
+constexpr int kEpiThreads = 512;
 constexpr int A_BYTES = BM * BK, B_BYTES = BN * BK, STAGE = A_BYTES + B_BYTES;
 constexpr int BAR_OFF = STAGES * STAGE;
 constexpr int SMEM = BAR_OFF + (2 * STAGES + 5) * 8 + 16 + 1024;
@@ -36,7 +38,7 @@ struct KP {
   long a_bs, b_bs, a_off[2][2], b_off[2];
   uint8_t* C;
   long ldc, c_plane;
-  int wide;        // K sums that need the two-step reduction
+  int wide;        // reduce_kind of the K sums
   int* flag;
 };
 
@@ -72,21 +74,89 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
                : "memory");
 }
 
-// 32 int32 sums -> their residues mod p as bytes
-__device__ __forceinline__ void reduce32(const uint32_t* v, uint32_t* w, uint32_t p, uint32_t m39, uint32_t big,
-                                         uint32_t r16, int wide) {
+// 32 int32 sums -> their residues mod p as bytes (0 .. p: p, where a byte holds it, for 0 now and then).
+// kind 0: |sum| <= 2^24, q = mulhi(sum, ceil(2^32 / p)) is floor(sum / p) or, for a negative multiple of p, one
+// less; 1: |sum| <= 2^27; 2: |sum| < 3 2^29, folded at 16 bits first
+struct Mod {
+  uint32_t p, m39, big, r16;
+  int m32;
+};
+__device__ __forceinline__ Mod mod_of(int i, int kind) {
+  Mod m;
+  m.p = c_tab.mod[i];
+  m.m39 = c_tab.m39[i];
+  m.m32 = c_tab.m32[i];
+  m.big = kind == 2 ? c_tab.big30[i] : c_tab.big27[i];
+  m.r16 = c_tab.r16[i];
+  return m;
+}
+template <int KIND>
+__device__ __forceinline__ void reduce32_k(const uint32_t* v, uint32_t* w, const Mod& m) {
 #pragma unroll
   for (int g = 0; g < 8; ++g) {
     uint32_t r[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      uint32_t u = v[4 * g + j] + big;  // congruent and nonnegative
-      if (wide) u = (u >> 16) * r16 + (u & 0xffffu);
-      r[j] = u - (__umulhi(u, m39) >> 7) * p;
+      if (KIND == 0) {
+        r[j] = v[4 * g + j] - uint32_t(__mulhi(int(v[4 * g + j]), m.m32)) * m.p;
+      } else {
+        uint32_t u = v[4 * g + j] + m.big;  // congruent and nonnegative
+        if (KIND == 2) u = (u >> 16) * m.r16 + (u & 0xffffu);
+        r[j] = u - (__umulhi(u, m.m39) >> 7) * m.p;
+      }
     }
     w[g] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
   }
 }
+__device__ __forceinline__ void reduce32(const uint32_t* v, uint32_t* w, const Mod& m, int kind) {
+  if (kind == 0) reduce32_k<0>(v, w, m);
+  else if (kind == 1) reduce32_k<1>(v, w, m);
+  else reduce32_k<2>(v, w, m);
+}
+// A warp's 32 rows x 64 columns of accumulators at taddr -> bytes of C.  Each lane reduces its own row; four
+// lanes then trade 16-byte pieces so that a store instruction writes 64-byte pieces of eight rows (a lane's own
+// 16 bytes a row took 32 cache lines an instruction, and the stores bounded the tiles with short K).
+// rows[i]: C's row of the group's lane i at this block's first column, null where there is none; left: bytes
+// of the row from there on, a multiple of 16.
+__device__ __forceinline__ void drain64(uint32_t taddr, const Mod& m, int kind, uint8_t* const* rows, int left, int lane) {
+  uint32_t w[16];
+  {
+    uint32_t v[32];
+    tmem_ld32(taddr, v);
+    reduce32(v, w, m, kind);
+  }
+  if (left > 32) {  // the same for the whole warp
+    uint32_t v[32];
+    tmem_ld32(taddr + 32, v);
+    reduce32(v, w + 8, m, kind);
+  }
+  // 4 x 4 transpose of the pieces: after it piece i of this lane is piece (lane & 3) of the group's row i
+  const bool b1 = lane & 1, b2 = lane & 2;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // pieces 2 h and 2 h + 1 with lane ^ 1
+      uint32_t &lo = w[8 * h + i], &hi = w[8 * h + 4 + i];
+      const uint32_t x = __shfl_xor_sync(0xffffffffu, b1 ? lo : hi, 1);
+      if (b1) lo = x;
+      else hi = x;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // pieces h and h + 2 with lane ^ 2
+      uint32_t &lo = w[4 * h + i], &hi = w[8 + 4 * h + i];
+      const uint32_t x = __shfl_xor_sync(0xffffffffu, b2 ? lo : hi, 2);
+      if (b2) lo = x;
+      else hi = x;
+    }
+  }
+  const int at = 16 * (lane & 3);
+  if (at < left) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (rows[i]) *reinterpret_cast<uint4*>(rows[i] + at) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+  }
+}
+inline int reduce_kind(long K) { return K <= 1024 ? 0 : K <= 8192 ? 1 : 2; }
 
 struct Tile {
   int mt, part, nt, b, p;
@@ -220,10 +290,8 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
       mbar_wait_for(done, 0, kWaitNs);
     }
     __syncwarp();
-  } else {  // epilogue warps 2..9 -> TMEM lane quarters 2,3,0,1 (a warp reaches only its quarter)
+  } else {  // epilogue warps -> TMEM lane quarters 2,3,0,1 (a warp reaches only its quarter)
     const int q = warp & 3;
-    const int row = q * 32 + lane;
-    const int c0 = 32 * ((warp - 2) >> 2);  // the two warps of a quarter take alternate 32-column chunks
     uint32_t n = 0;
     for (long t = blockIdx.x; t < k.tiles; t += gridDim.x, ++n) {
       const uint32_t b = n & 1;
@@ -235,24 +303,17 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
       }
       fence_after();
       const Tile c = decode(k, t);
-      const int m = c.mt * BM + row;
-      const bool live = m < k.M;
-      const uint32_t p = c_tab.mod[c.p], m39 = c_tab.m39[c.p];
-      const uint32_t big = k.wide ? c_tab.big30[c.p] : c_tab.big27[c.p], r16 = c_tab.r16[c.p];
-      uint8_t* out = k.C + c.p * k.c_plane + (((long)c.part * k.batch + c.b) * k.M + m) * k.ldc;
+      const Mod md = mod_of(c.p, k.wide);
+      uint8_t* out = k.C + c.p * k.c_plane + ((long)c.part * k.batch + c.b) * k.M * k.ldc;
       const uint32_t taddr = tmem + (uint32_t(q * 32) << 16) + b * BN;
-      const int n0 = c.nt * k.bn;
-      for (int cc = c0; cc < k.bn; cc += 64) {
-        uint32_t v[32];
-        __syncwarp();
-        tmem_ld32(taddr + uint32_t(cc), v);  // columns past bn (bn a multiple of 16) are read and dropped
-        const int col = n0 + cc;
-        if (!live || col >= k.ldc) continue;
-        uint32_t w[8];
-        reduce32(v, w, p, m39, big, r16, k.wide);
-        *reinterpret_cast<uint4*>(out + col) = make_uint4(w[0], w[1], w[2], w[3]);
-        if (cc + 16 < k.bn && col + 16 < k.ldc)
-          *reinterpret_cast<uint4*>(out + col + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+      const int n0 = c.nt * k.bn, mg = c.mt * BM + q * 32 + (lane & ~3);
+      const int cc = 64 * ((warp - 2) >> 2);  // the quarter's four warps take 64 columns each
+      const int left = min(k.bn - cc, int(k.ldc) - n0 - cc);
+      if (left > 0) {
+        uint8_t* rows[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rows[i] = mg + i < k.M ? out + (mg + i) * k.ldc + n0 + cc : nullptr;
+        drain64(taddr + uint32_t(cc), md, k.wide, rows, left, lane);
       }
       fence_before();
       mbar_arrive(&acc_empty[b]);
@@ -479,20 +540,19 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
       mbar_wait_for(done, 0, kWaitNs);
     }
     __syncwarp();
-  } else {  // epilogue warps 2..9: one TMEM lane quarter each, and a row tile or alternate chunks
+  } else {  // epilogue warps: a TMEM lane quarter, a row tile and 64 columns
     const int q = warp & 3, h = (warp - 2) >> 2;
-    const int mt = MT == 2 ? h : 0;
-    const int r = mt * BM + q * 32 + lane;  // row of [re; im], Np each
-    const int part = r >= k.Np ? 1 : 0, a = r - part * k.Np;
-    const int c0 = MT == 2 ? 0 : 32 * h, cstep = MT == 2 ? 32 : 64;
+    const int mt = MT == 2 ? (h & 1) : 0;
+    const int rg = mt * BM + q * 32 + (lane & ~3);  // the lane group's first row of [re; im], Np each (Np % 8 == 0)
+    const int part = rg >= k.Np ? 1 : 0, ag = rg - part * k.Np;
+    const int cc = 64 * (MT == 2 ? h >> 1 : h);
     uint32_t n = 0;
     bool stop = false;
     for (long u = blockIdx.x; u < k.units && !stop; u += gridDim.x) {
       const RUnit c = unit_of(k, u);
-      const uint32_t p = c_tab.mod[c.p], m39 = c_tab.m39[c.p];
-      const uint32_t big = k.wide ? c_tab.big30[c.p] : c_tab.big27[c.p], r16 = c_tab.r16[c.p];
-      const bool live = a < k.Np && c.e0 + a < k.N && r < 2 * k.Np;
-      uint8_t* row = k.C + c.p * k.c_plane + (part * k.c_part + (long)c.w * k.N + c.e0 + a) * k.ldc;
+      const Mod md = mod_of(c.p, k.wide);
+      uint8_t* row = k.C + c.p * k.c_plane + (part * k.c_part + (long)c.w * k.N + c.e0 + ag) * k.ldc;
+      const int nrow = rg < 2 * k.Np ? k.N - c.e0 - ag : 0;  // rows of the group that exist (4 or more: all)
       for (int t = c.t0; t < c.t1; ++t, ++n) {
         const uint32_t b = n & 1;
         const bool ok = mbar_wait_for(&acc_full[b], (n >> 1) & 1, kWaitNs);
@@ -505,17 +565,12 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
         fence_after();
         const uint32_t taddr = tmem + (uint32_t(q * 32) << 16) + b * BN + uint32_t(mt * 128);
         const int bn = t == k.NT - 1 ? k.bn_last : k.bn, n0 = t * k.bn;
-        for (int cc = c0; cc < bn; cc += cstep) {
-          uint32_t v[32];
-          __syncwarp();
-          tmem_ld32(taddr + uint32_t(cc), v);
-          const int col = n0 + cc;
-          if (!live || col >= k.ldc) continue;
-          uint32_t w[8];
-          reduce32(v, w, p, m39, big, r16, k.wide);
-          *reinterpret_cast<uint4*>(row + col) = make_uint4(w[0], w[1], w[2], w[3]);
-          if (cc + 16 < bn && col + 16 < k.ldc)
-            *reinterpret_cast<uint4*>(row + col + 16) = make_uint4(w[4], w[5], w[6], w[7]);
+        const int left = min(bn - cc, int(k.ldc) - n0 - cc);
+        if (left > 0) {
+          uint8_t* rows[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) rows[i] = i < nrow ? row + i * k.ldc + n0 + cc : nullptr;
+          drain64(taddr + uint32_t(cc), md, k.wide, rows, left, lane);
         }
         fence_before();
         mbar_arrive(&acc_empty[b]);
@@ -567,7 +622,7 @@ int gemm(const Gemm& g, cudaStream_t st) {
     for (int s = 0; s < 2; ++s) k.a_off[p][s] = g.a_off[p][s];
   k.b_off[0] = g.b_off[0]; k.b_off[1] = g.b_off[1];
   k.C = g.C; k.ldc = g.ldc; k.c_plane = g.c_plane;
-  k.wide = (long)g.K * g.segs > 8192;  // sums at or above 2^27
+  k.wide = reduce_kind((long)g.K * g.segs);
   k.flag = g.flag;
   Maps maps;
   int rc;
@@ -613,7 +668,7 @@ bool plan_walker(const WalkerGemm& g, RKP* out) {
   k.cols = g.cols;
   k.a_blk = g.a_blk; k.b_bs = g.b_bs; k.b_off1 = g.b_off1;
   k.C = g.C; k.ldc = g.ldc; k.c_plane = g.c_plane; k.c_part = g.c_part;
-  k.wide = (long)g.K * g.segs > 8192;
+  k.wide = reduce_kind((long)g.K * g.segs);
   k.flag = g.flag;
   *out = k;
   return true;

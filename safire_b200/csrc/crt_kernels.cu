@@ -37,7 +37,8 @@ __device__ __forceinline__ double row_sum(double v, double* sh) {
 // L2: a row is at most a few hundred KB).  One warp per row below 1024 elements, one block above.
 template <int TPR>
 __global__ void __launch_bounds__(256) rows_real_kernel(const double* src, long rows, long K, long stride, int8_t* q,
-                                                        long ld, long plane, int* e, int* flag, int vec) {
+                                                        long ld, long plane, int* e, int* flag, int vec, long inner,
+                                                        long outer) {
   __shared__ double sh[8];
   const long r = TPR == 32 ? (long)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;
   const int t = TPR == 32 ? (threadIdx.x & 31) : threadIdx.x;
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(256) rows_real_kernel(const double* src, long 
   const int ex = row_exponent(n2, any, t == 0 ? flag : nullptr);
   if (t == 0) e[r] = ex;
   const double sc = pow2(-ex);
-  int8_t* qr = q + r * ld;
+  int8_t* qr = q + (inner ? (r / inner) * outer + r % inner : r) * ld;
   for (long k = 4 * t; k < K; k += 4 * TPR) {
     double x[4];
     load4(row, k, K, vec, x);
@@ -226,27 +227,33 @@ __global__ void __launch_bounds__(256) out_real_kernel(const uint8_t* c, long ld
     if (n + j < N) out[m * ldo + n + j] = re.v[j];
 }
 
-// One Taylor term of one row (w, a): see taylor_update.  Memory bound (15 residues in, S in and out,
-// 45 residues out per complex element); the row's T waits in shared memory for its norm.
+// One Taylor term (see taylor_update) of R rows (w, a): items of four columns, both parts, over the R rows
+// together, so that a block's threads stay busy whatever M is (100 items a row at M = 400: one row in a
+// block of 128 threads left a fifth of the lanes idle).  Each complex element: 30 residues in, S in and
+// out, 45 residues out; a row's T waits in shared memory for its norm.
 template <bool FIRST, bool LAST>
-__global__ void __launch_bounds__(128) taylor_kernel(const uint8_t* c, long ldc, long plane, long WN, int N, int M,
+__global__ void __launch_bounds__(256, 4) taylor_kernel(const uint8_t* c, long ldc, long plane, long WN, int N, int M,
                                                      double inv_k, const int* eA, const int* eB, int eB_per_w,
-                                                     double* S, int8_t* q, long ld, long qplane, int* e, int* flag) {
-  extern __shared__ double row[];  // T (or S when LAST), re then im, M4 each
-  __shared__ double sh[4];
-  const long r = blockIdx.x;
-  const int w = int(r / N);
-  const int M4 = (M + 3) / 4 * 4;
-  const int* eb0 = eB + (eB_per_w ? (long)w * M : 0);
-  const int ea = eA[r];
-  double* Sr = S + r * M;
-  double* Si = S + (WN + r) * M;
-  double n2 = 0.0, nz = 0.0;
-  for (int j0 = 4 * threadIdx.x; j0 < M; j0 += 512) {
+                                                     double* S, int8_t* q, long ld, long qplane, int* e, int* flag,
+                                                     int R) {
+  extern __shared__ double rows[];  // [R][2][M4] T (S when LAST), then [R * M4 / 4] squared norms, [R] scales
+  const int M4 = (M + 3) / 4 * 4, q4 = M4 / 4;
+  double* part = rows + 2 * R * M4;
+  double* scs = part + R * q4;
+  const long r0 = (long)blockIdx.x * R;
+  const int nr = int(WN - r0 < R ? WN - r0 : R), items = nr * q4;
+  for (int it = threadIdx.x; it < items; it += 256) {
+    const int rr = it / q4, j0 = 4 * (it - rr * q4);
+    const long r = r0 + rr;
+    const int* eb0 = eB + (eB_per_w ? (r / N) * M : 0);
     int eb[4];
     load_e4(eb0, j0, M, eb);
+    const int ea = eA[r];
     const Vals re = values4(c + r * ldc + j0, plane, ea, eb, kTwoM64P * inv_k);
     const Vals im = values4(c + (WN + r) * ldc + j0, plane, ea, eb, kTwoM64P * inv_k);
+    double* Sr = S + r * M + j0;
+    double* Si = S + (WN + r) * M + j0;
+    double n2 = 0.0, nz = 0.0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       double x = 0.0, y = 0.0;
@@ -254,38 +261,96 @@ __global__ void __launch_bounds__(128) taylor_kernel(const uint8_t* c, long ldc,
         x = FIRST ? re.v[j] : -im.v[j];  // T = (i / k) C
         y = FIRST ? im.v[j] : re.v[j];
         if (FIRST) {
-          Sr[j0 + j] = x;
-          Si[j0 + j] = y;
+          Sr[j] = x;
+          Si[j] = y;
         } else {
-          const double sx = Sr[j0 + j] + x, sy = Si[j0 + j] + y;
+          const double sx = Sr[j] + x, sy = Si[j] + y;
           if (LAST) {
             x = sx;
             y = sy;
           } else {
-            Sr[j0 + j] = sx;
-            Si[j0 + j] = sy;
+            Sr[j] = sx;
+            Si[j] = sy;
           }
         }
       }
       n2 = fma(x, x, fma(y, y, n2));
       nz = fmax(nz, fmax(fabs(x), fabs(y)));
-      row[j0 + j] = x;
-      row[M4 + j0 + j] = y;
+      rows[(2 * rr) * M4 + j0 + j] = x;
+      rows[(2 * rr + 1) * M4 + j0 + j] = y;
+    }
+    part[it] = n2 == 0.0 && nz != 0.0 ? 1e-320 : n2;  // squares that vanish: not a row of zeros
+  }
+  __syncthreads();
+  for (int rr = threadIdx.x >> 5; rr < nr; rr += 8) {
+    double n2 = 0.0;
+    for (int i = threadIdx.x & 31; i < q4; i += 32) n2 += part[rr * q4 + i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+    if ((threadIdx.x & 31) == 0) {
+      const int ex = row_exponent(n2, n2 != 0.0, flag);
+      e[r0 + rr] = ex;
+      scs[rr] = pow2(-ex);
     }
   }
-  n2 = row_sum<128>(n2, sh);
-  const bool any = __syncthreads_or(nz != 0.0) != 0;
-  const int ex = row_exponent(n2, any, threadIdx.x == 0 ? flag : nullptr);
-  if (threadIdx.x == 0) e[r] = ex;
-  const double sc = pow2(-ex);
-  int8_t* qr = q + r * ld;
-  for (int j0 = 4 * threadIdx.x; j0 < M; j0 += 512) {  // this thread's own entries of the row
+  __syncthreads();
+  for (int it = threadIdx.x; it < items; it += 256) {  // this thread's own entries again
+    const int rr = it / q4, j0 = 4 * (it - rr * q4);
+    int8_t* qr = q + (r0 + rr) * ld + j0;
     Quad d;
-    d.set(row + j0, sc);
-    d.store(qr + j0, qplane);
-    d.set(row + M4 + j0, sc);
-    if (LAST) d.store(qr + WN * ld + j0, qplane);
-    else d.store2(qr + WN * ld + j0, qr + 2 * WN * ld + j0, qplane);
+    d.set(rows + (2 * rr) * M4 + j0, scs[rr]);
+    d.store(qr, qplane);
+    d.set(rows + (2 * rr + 1) * M4 + j0, scs[rr]);
+    if (LAST) d.store(qr + WN * ld, qplane);
+    else d.store2(qr + WN * ld, qr + 2 * WN * ld, qplane);
+  }
+}
+
+// One block per (n, w): the walker's T of this n, reconstructed once into shared memory, then its
+// exchange trace.  Bound by the reconstruction (two residue groups per complex element) and its reads.
+__global__ void __launch_bounds__(256) exx_kernel(const uint8_t* c, long ldc, long plane, long WN, int N, int N4,
+                                                  const int* eA, const int* eB, int n0, int Nc, cplx* exxn, cplx* kl,
+                                                  int nup) {
+  extern __shared__ cplx T[];  // T[b][a], rows of P
+  __shared__ cplx red[2][8];
+  const int n = blockIdx.x, w = blockIdx.y, P = N | 1, q4 = N4 / 4;
+  for (int it = threadIdx.x; it < N * q4; it += 256) {
+    const int b = it / q4, a = 4 * (it % q4);
+    const long r = (long)w * N + b, col = (long)n * N4 + a;
+    int eb[4];
+    load_e4(eB + (long)n * N, a, N, eb);
+    const Vals re = values4(c + r * ldc + col, plane, eA[r], eb, kTwoM64P);
+    const Vals im = values4(c + (WN + r) * ldc + col, plane, eA[r], eb, kTwoM64P);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (a + j < N) T[b * P + a + j] = mk(re.v[j], im.v[j]);
+  }
+  __syncthreads();
+  cplx acc = mk(0.0, 0.0), tr = mk(0.0, 0.0);
+  for (int e = threadIdx.x; e < N * N; e += 256) {
+    const int i = e / N, j = e % N;
+    if (j < i || (i < nup) != (j < nup)) continue;
+    const cplx x = T[i * P + j];
+    if (i == j) tr = cadd(tr, x);
+    const cplx p = cmul(x, T[j * P + i]);
+    acc = cadd(acc, i == j ? p : cscale(p, 2.0));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+    tr.x += __shfl_xor_sync(0xffffffffu, tr.x, o);
+    tr.y += __shfl_xor_sync(0xffffffffu, tr.y, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = acc;
+    red[1][threadIdx.x >> 5] = tr;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    cplx s = mk(0.0, 0.0);
+    for (int i = 0; i < 8; ++i) s = cadd(s, red[threadIdx.x][i]);
+    (threadIdx.x == 0 ? exxn : kl)[(long)w * Nc + n0 + n] = s;
   }
 }
 
@@ -316,13 +381,16 @@ __global__ void __launch_bounds__(256) walkers_out_kernel(const uint8_t* c, long
 
 }  // namespace
 
-int rows_real(const double* src, long rows, long K, long stride, const Planes& o, int* flag, cudaStream_t st) {
+int rows_real(const double* src, long rows, long K, long stride, const Planes& o, int* flag, cudaStream_t st,
+              long inner, long outer) {
   if (rows <= 0 || K <= 0) return SFQ_OK;
   const int vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && stride % 2 == 0;
   if (K < 1024)
-    rows_real_kernel<32><<<ceil_div(rows, 8), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, flag, vec);
+    rows_real_kernel<32><<<ceil_div(rows, 8), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, flag, vec,
+                                                            inner, outer);
   else
-    rows_real_kernel<256><<<unsigned(rows), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, flag, vec);
+    rows_real_kernel<256><<<unsigned(rows), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, flag, vec,
+                                                            inner, outer);
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
@@ -363,13 +431,35 @@ int out_real(const Out& c, long M, long N, const int* eA, const int* eB, double 
 
 int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int* eA, const int* eB, int eB_per_w,
                   double* S, const Planes& o, int* flag, cudaStream_t st) {
-  const int M4 = (M + 3) / 4 * 4;
-  const size_t sm = sizeof(double) * 2 * M4;
+  const int M4 = (M + 3) / 4 * 4, q4 = M4 / 4;
+  const long WN = (long)W * N;
+  // rows per block: the count up to 8 that wastes least of the last round of 256 items, in 48 KB of rows
+  int R = 1;
+  double best = 0.0;
+  for (int n = 1; n <= 8 && (n == 1 || 16L * n * M4 <= 40 * 1024); ++n) {
+    const double use = double(n) * q4 / ((n * q4 + 255) / 256 * 256);
+    if (use > best + 0.02) {
+      best = use;
+      R = n;
+    }
+  }
+  const size_t sm = sizeof(double) * (2L * R * M4 + (long)R * q4 + R);
   const double ik = k > 0 ? 1.0 / double(k) : 1.0;
   auto kern = k == 0 ? taylor_kernel<true, false> : last ? taylor_kernel<false, true> : taylor_kernel<false, false>;
   if (sm > 48 * 1024) SFQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-  kern<<<unsigned(W * N), 128, sm, st>>>(c.q, c.ldc, c.plane, (long)W * N, N, M, ik, eA, eB, eB_per_w, S, o.q, o.ld,
-                                         o.plane, o.e, flag);
+  kern<<<unsigned((WN + R - 1) / R), 256, sm, st>>>(c.q, c.ldc, c.plane, WN, N, M, ik, eA, eB, eB_per_w, S, o.q, o.ld,
+                                                    o.plane, o.e, flag, R);
+  SFQ_LAUNCHED();
+  return SFQ_OK;
+}
+
+int exx_reduce(const Out& c, int W, int N, int N4, int nv, int n0, int Nc, const int* eA, const int* eB, cplx* exxn,
+               cplx* kl, int nup, cudaStream_t st) {
+  const size_t sm = sizeof(cplx) * N * (N | 1);
+  if (N > kExxMaxN) return record_error(SFQ_ERR_SHAPE, "crt exx: N=%d above %d", N, kExxMaxN);
+  SFQ_CUDA_TRY(cudaFuncSetAttribute(exx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  exx_kernel<<<dim3(nv, W), 256, sm, st>>>(c.q, c.ldc, c.plane, (long)W * N, N, N4, eA, eB, n0, Nc, exxn, kl,
+                                           nup < 0 ? N : nup);
   SFQ_LAUNCHED();
   return SFQ_OK;
 }

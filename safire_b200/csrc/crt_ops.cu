@@ -200,6 +200,71 @@ int propagate_crt(cplx* SM, const double* P1, const Planes* P1q, const cplx* V, 
   return SFQ_OK;
 }
 
+// ---- local energy ---------------------------------------------------------------------------
+namespace {
+int n4_of(int N) { return (N + 3) / 4 * 4; }
+size_t energy_n_bytes(int W, int N, int M, bool l_cplx) {  // per Cholesky vector
+  return (size_t)NMOD * ((l_cplx ? 2 : 1) * (size_t)n4_of(N) * ld_of(M) + 2 * (size_t)W * N * n4_of(N)) +
+         sizeof(int) * N;
+}
+size_t energy_fixed_bytes(int W, int N, int M, bool l_cplx) {
+  const long R = (long)W * N;
+  return kFlagBytes + planes_bytes((l_cplx ? 3 : 2) * R, M) + exps_bytes(R) + slack();
+}
+int energy_nv(int W, int N, int M, int Nc, bool l_cplx) {
+  const long most = std::max<long>(1, long(kChunkBytes / energy_n_bytes(W, N, M, l_cplx)));
+  const long n = (Nc + most - 1) / most;
+  return int((Nc + n - 1) / n);
+}
+}  // namespace
+
+bool energy_crt_ok(int W, int N, int M, int Nc, bool l_cplx) {
+  return W <= 65535 && N >= 8 && N <= kExxMaxN && M >= 32 && 8.0 * W * N * double(N) * M * Nc >= 2e9 &&
+         energy_n_bytes(W, N, M, l_cplx) <= kChunkBytes && walker_gemm_fits(N, 16 * n4_of(N), M, l_cplx ? 2 : 1);
+}
+
+size_t energy_crt_bytes(int W, int N, int M, int Nc, bool l_cplx) {
+  const int nv = energy_nv(W, N, M, Nc, l_cplx), N4 = n4_of(N);
+  return energy_fixed_bytes(W, N, M, l_cplx) + planes_bytes((l_cplx ? 2L : 1L) * nv * N4, M) +
+         exps_bytes((long)nv * N) + out_bytes(2L * W * N, (long)nv * N4);
+}
+
+int energy_crt(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool l_cplx, double E0, int W, int N, int M,
+               int Nc, int addH1, int addEJ, char* scratch, cplx* Tchunk, long tchunk_elems, cplx* exxn, cplx* kl,
+               cudaStream_t st, int nup) {
+  int rc;
+  const double scl = nup < 0 ? 2.0 : 1.0;
+  const int nv = energy_nv(W, N, M, Nc, l_cplx), N4 = n4_of(N);
+  const long R = (long)W * N;
+  int* flag = reinterpret_cast<int*>(scratch);
+  char* at = scratch + kFlagBytes;
+  SFQ_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  if ((rc = energy_e1(G, haj, E3, W, N, M, E0, scl, addH1, st))) return rc;
+  const Planes A = lay_out(at, (l_cplx ? 3 : 2) * R, M, R);
+  const Planes B = lay_out(at, (l_cplx ? 2L : 1L) * nv * N4, M, (long)nv * N);
+  const Out C = lay_out_c(at, 2 * R, (long)nv * N4);
+  if ((rc = rows_cplx(G, R, M, M, l_cplx ? 3 : 2, R, R, R, A, flag, st))) return rc;
+  for (int n0 = 0; n0 < Nc; n0 += nv) {
+    const int n = std::min(nv, Nc - n0);
+    // rows (n, a) of Lnak on rows n N4 + a: the columns of a vector then start on words
+    const long off = (long)n0 * N * M;
+    if (l_cplx) rc = rows_cplx((const cplx*)Lnak + off, (long)n * N, M, M, 2, (long)nv * N4, N, N4, B, flag, st);
+    else rc = rows_real((const double*)Lnak + off, (long)n * N, M, M, B, flag, st, N, N4);
+    if (rc) return rc;
+    crt::WalkerGemm g;
+    g.A = A; g.B = B; g.N = N; g.cols = n * N4; g.K = M; g.batch = W; g.segs = l_cplx ? 2 : 1;
+    g.a_blk = R; g.b_off1 = (long)nv * N4;
+    g.C = C.q; g.ldc = ldc_of((long)n * N4); g.c_plane = C.plane; g.c_part = R; g.flag = flag;
+    Out c = C;
+    c.ldc = g.ldc;
+    if ((rc = crt::walker_gemm(g, st))) return rc;
+    if ((rc = exx_reduce(c, W, N, N4, n, n0, Nc, A.e, B.e, exxn, kl, nup, st))) return rc;
+  }
+  if ((rc = energy_exx_f64(G, Lnak, l_cplx, W, N, M, Nc, Tchunk, tchunk_elems, exxn, kl, st, nup, flag)))
+    return rc;
+  return energy_finish(exxn, kl, E3, W, Nc, scl, 1, addEJ, st);
+}
+
 }  // namespace ops
 }  // namespace sfq
 

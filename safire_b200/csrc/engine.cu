@@ -535,12 +535,13 @@ struct Engine {
   double* Lp = nullptr;  // (P, Nc), FP64 engines
   cplx* Vp = nullptr;    // (W, P), FP64 engines
   // FP64 engines: residue planes of L (the packed rows when symmetric), Lnak and P1, made once at
-  // setup, and the scratch of the products on the int8 tensor cores (crt_ops.cuh); none where the
-  // sizes are too small for that path or the planes too large
+  // setup (none where the sizes are too small for the int8 tensor cores, crt_ops.cuh, or the planes too
+  // large), and those products' scratch, which shares the energy chunk's buffer
   crt::Planes L_m, Lnak_m, P1_m;
   char* crt_buf = nullptr;
   char* crt_ws = nullptr;
   size_t crt_bytes = 0;
+  bool crt_energy = false;  // the energy's exchange product that way too
   // T holds the inverse overlap matrices (PsiT W)^-1 of the current walkers and inv_ov their log
   // overlaps whenever inv_cached is set: the log overlap taken after a propagation or an
   // orthogonalization factors exactly the matrix the next Green's function needs, so that step
@@ -718,7 +719,7 @@ struct Engine {
         {(void**)&newov, c * W},
         {(void**)&E3, c * 3 * W},
         {(void**)&ovtmp, c * W},
-        {(void**)&Tchunk, c * tchunk_elems},
+        {(void**)&crt_ws, std::max(c * (size_t)tchunk_elems + 512, crt_scratch_bytes())},
         {(void**)&exxn, c * (size_t)W * Nc},
         {(void**)&kl, c * (size_t)W * Nc},
         {(void**)&status, sizeof(int) * 2 * W},
@@ -819,7 +820,22 @@ struct Engine {
       off += a256(it.bytes);
     }
     SFQ_CUDA_TRY(cudaMemsetAsync(arena, 0, total, st));
+    Tchunk = reinterpret_cast<cplx*>(crt_ws + 256);
     return SFQ_OK;
+  }
+  // FP64 engines: the most that a product on the int8 tensor cores takes of the energy chunk's buffer, whether
+  // L turns out symmetric or not
+  size_t crt_scratch_bytes() const {
+    if (mixed) return 0;
+    const bool lc = !trial_real;
+    size_t ws = 0;
+    if (ndet == 1 && ops::vbias_crt_ok(W, N, Mr, Nc, lc)) ws = ops::vbias_crt_bytes(W, N, Mr, Nc, lc, true);
+    for (long rows : {(long)M * (M + 1) / 2, (long)M * M})
+      if (ops::vhs_crt_ok(W, rows, Nc, true)) ws = std::max(ws, ops::vhs_crt_bytes(W, rows, Nc, true));
+    if (ops::propagate_crt_ok(W, M, N, npol, false, p.taylor_order))
+      ws = std::max(ws, ops::propagate_crt_bytes(W, M, N, npol, true));
+    if (ndet == 1 && ops::energy_crt_ok(W, N, Mr, Nc, lc)) ws = std::max(ws, ops::energy_crt_bytes(W, N, Mr, Nc, lc));
+    return ws;
   }
 
   // --- setup: RealDenseHamiltonian::getHamiltonianOperations + NOMSD::vMF + generateP1 --------
@@ -1132,7 +1148,7 @@ struct Engine {
     return SFQ_OK;
   }
 
-  // FP64 engines: the residue planes of the resident operands and the products' scratch.  Planes take
+  // FP64 engines: the residue planes of the resident operands.  Planes take
   // 15 bytes an element (FP64: 8); above 24 GB of them, or where the device has no room, the
   // products stay on the FP64 tensor pipe, as they do below the sizes that gain.
   int setup_crt() {
@@ -1141,29 +1157,22 @@ struct Engine {
     const bool vb = ndet == 1 && ops::vbias_crt_ok(W, N, Mr, Nc, lc);
     const bool vh = ops::vhs_crt_ok(W, rows, Nc, true);
     const bool pr = ops::propagate_crt_ok(W, M, N, npol, false, p.taylor_order);
-    if (!vb && !vh && !pr) return SFQ_OK;
+    const bool en = ndet == 1 && ops::energy_crt_ok(W, N, Mr, Nc, lc);
+    if (!vb && !vh && !pr && !en) return SFQ_OK;
     const long K = (long)N * Mr;
-    size_t planes = 256, ws = 0;
-    if (vb) {
-      planes += crt::planes_bytes((lc ? 2L : 1L) * Nc, K) + crt::exps_bytes(Nc);
-      ws = std::max(ws, ops::vbias_crt_bytes(W, N, Mr, Nc, lc, true));
-    }
-    if (vh) {
-      planes += crt::planes_bytes(rows, Nc) + crt::exps_bytes(rows);
-      ws = std::max(ws, ops::vhs_crt_bytes(W, rows, Nc, true));
-    }
-    if (pr) {
-      planes += crt::planes_bytes(M, M) + crt::exps_bytes(M);
-      ws = std::max(ws, ops::propagate_crt_bytes(W, M, N, npol, true));
-    }
+    crt_energy = en;
+    if (!vb && !vh && !pr) return SFQ_OK;
+    size_t planes = 256;
+    if (vb) planes += crt::planes_bytes((lc ? 2L : 1L) * Nc, K) + crt::exps_bytes(Nc);
+    if (vh) planes += crt::planes_bytes(rows, Nc) + crt::exps_bytes(rows);
+    if (pr) planes += crt::planes_bytes(M, M) + crt::exps_bytes(M);
     if (planes > (size_t(24) << 30)) return SFQ_OK;
-    if (cudaMalloc(&crt_buf, planes + ws) != cudaSuccess) {
+    if (cudaMalloc(&crt_buf, planes) != cudaSuccess) {
       cudaGetLastError();
       crt_buf = nullptr;
       return SFQ_OK;
     }
-    crt_bytes = planes + ws;
-    crt_ws = crt_buf + planes;
+    crt_bytes = planes;
     int* flag = reinterpret_cast<int*>(crt_buf);
     char* at = crt_buf + 256;
     int rc;
@@ -1187,7 +1196,7 @@ struct Engine {
     SFQ_CUDA_TRY(cudaStreamSynchronize(st));
     if (bad) {  // operands that the planes cannot hold
       cudaFree(crt_buf);
-      crt_buf = crt_ws = nullptr;
+      crt_buf = nullptr;
       crt_bytes = 0;
       L_m = Lnak_m = P1_m = crt::Planes();
     }
@@ -2889,9 +2898,13 @@ struct Engine {
       return SFQ_OK;
     }
     if ((rc = density(ovtmp))) return rc;
-    if ((rc = ops::energy(E3, G, haj, Lnak, !trial_real, p.E0, W, N, Mr, Nc, 1, 1, 1, Tchunk, tchunk_elems, exxn, kl,
-                          st, spin_split())))
-      return rc;
+    if (crt_energy)
+      rc = ops::energy_crt(E3, G, haj, Lnak, !trial_real, p.E0, W, N, Mr, Nc, 1, 1, crt_ws, Tchunk, tchunk_elems, exxn,
+                           kl, st, spin_split());
+    else
+      rc = ops::energy(E3, G, haj, Lnak, !trial_real, p.E0, W, N, Mr, Nc, 1, 1, 1, Tchunk, tchunk_elems, exxn, kl, st,
+                       spin_split());
+    if (rc) return rc;
     ph_end(SFQ_PH_ENERGY);
     return SFQ_OK;
   }

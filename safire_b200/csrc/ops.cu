@@ -294,19 +294,27 @@ int energy(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool l_cp
   const double scl = nup < 0 ? 2.0 : 1.0;  // CLOSED counts each orbital twice (energy, :148-173)
   if ((rc = energy_e1(G, haj, E3, W, N, M, E0, scl, addH1, st))) return rc;
   if (!addEXX && !addEJ) return SFQ_OK;
+  if ((rc = energy_exx_f64(G, Lnak, l_cplx, W, N, M, Nc, Tchunk, tchunk_elems, exxn, kl, st, nup))) return rc;
+  return energy_finish(exxn, kl, E3, W, Nc, scl, addEXX, addEJ, st);
+}
+
+int energy_exx_f64(const cplx* G, const void* Lnak, bool l_cplx, int W, int N, int M, int Nc, cplx* Tchunk,
+                   long tchunk_elems, cplx* exxn, cplx* kl, cudaStream_t st, int nup, const int* only_if) {
+  int rc;
   const int nv_max = energy_chunk(W, N, Nc, tchunk_elems);
   const size_t esz = l_cplx ? sizeof(cplx) : sizeof(double);
   for (int n0 = 0; n0 < Nc; n0 += nv_max) {
     const int nv = (Nc - n0) < nv_max ? (Nc - n0) : nv_max;
     GemmDesc d;  // T[(w,b)][(n,a)] = sum_k G[w,b,k] Lnak[n0+n, a, k]
+    d.only_if = only_if;
     d.M = W * N; d.N = nv * N; d.K = M; d.batch = 1;
     d.A = G; d.sAm = M; d.sAk = 1; d.a_cplx = true;
     d.B = (const unsigned char*)Lnak + (size_t)n0 * N * M * esz; d.sBk = 1; d.sBn = M; d.b_cplx = l_cplx;
     d.C = Tchunk; d.sCm = (long)nv * N; d.sCn = 1;
     if ((rc = gemm_f64(d, st))) return rc;
-    if ((rc = energy_exx_reduce(Tchunk, W, N, nv, n0, Nc, exxn, kl, st, nup))) return rc;
+    if ((rc = energy_exx_reduce(Tchunk, W, N, nv, n0, Nc, exxn, kl, st, nup, only_if))) return rc;
   }
-  return energy_finish(exxn, kl, E3, W, Nc, scl, addEXX, addEJ, st);
+  return SFQ_OK;
 }
 
 }  // namespace ops
@@ -375,7 +383,13 @@ size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol) {
       return align256(c * (size_t)nwalk * nmo * nel) + align256(c * nwalk * nel * nel) + align256(2 * sizeof(int) * nwalk);
     case SFQ_OP_ENERGY: {
       long nv = ops::energy_chunk(nwalk, nel, nchol, kEnergyChunkElems);
-      return align256(c * (size_t)nwalk * nel * nv * nel) + 2 * align256(c * (size_t)nwalk * nchol);
+      const size_t tc = align256(c * (size_t)nwalk * nel * nv * nel), vec = 2 * align256(c * (size_t)nwalk * nchol);
+      size_t big = tc;  // the int8 path's scratch, sized for a complex Lnak, holds the chunk too
+      if (nwalk > 0 && nmo > 0 && nel > 0 && nchol > 0)
+        for (bool lc : {false, true})
+          if (ops::energy_crt_ok(nwalk, nel, nmo, nchol, lc))
+            big = std::max(big, std::max(ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc), tc + 256) + 256);
+      return big + vec;
     }
     case SFQ_OP_INVERSE_LOGDET:
       return 0;
@@ -539,11 +553,18 @@ int sfq_energy(void* E, const void* G, const void* haj, const void* Lnak, int ln
   if (nwalk == 0) return SFQ_OK;
   if (!E || !G || !haj || !Lnak) return record_error(SFQ_ERR_ARG, "null pointer");
   if (addEJ && !addEXX) return record_error(SFQ_ERR_UNSUPPORTED, "addEJ and not addEXX not yet implemented");
-  if (ws_bytes < sfq_workspace_size(SFQ_OP_ENERGY, nwalk, nmo, nel, nchol))
-    return record_error(SFQ_ERR_WORKSPACE, "energy: workspace too small");
   long nv = ops::energy_chunk(nwalk, nel, nchol, kEnergyChunkElems);
   const size_t bt = align256(sizeof(cplx) * (size_t)nwalk * nel * nv * nel);
   const size_t bk = align256(sizeof(cplx) * (size_t)nwalk * nchol);
+  if (ws_bytes < bt + 2 * bk) return record_error(SFQ_ERR_WORKSPACE, "energy: workspace too small");
+  const bool lc = lnak_complex != 0;
+  if (addEXX && nel > 0 && nmo > 0 && nchol > 0 && ops::energy_crt_ok(nwalk, nel, nmo, nchol, lc) &&
+      ws_bytes >= std::max(ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc), bt + 256) + 256 + 2 * bk) {
+    char* at = aligned(ws);
+    return ops::energy_crt((cplx*)E, (const cplx*)G, (const cplx*)haj, Lnak, lc, E0, nwalk, nel, nmo, nchol, addH1,
+                           addEJ, at + 2 * bk, (cplx*)(at + 2 * bk + 256), (long)nwalk * nel * nv * nel, (cplx*)at,
+                           (cplx*)(at + bk), S(stream), -1);
+  }
   cplx* Tc = (cplx*)ws;
   cplx* exxn = (cplx*)((char*)ws + bt);
   cplx* kl = (cplx*)((char*)ws + bt + bk);

@@ -47,6 +47,9 @@ int energy(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool l_cp
            int Nc, int addH1, int addEJ, int addEXX, cplx* Tchunk, long tchunk_elems, cplx* exxn, cplx* kl,
            cudaStream_t st, int nup = -1);
 int energy_chunk(int W, int N, int Nc, long max_elems);
+// its exchange part alone on the FP64 tensor pipe: exxn and kl (W, Nc); only_if as in propagate
+int energy_exx_f64(const cplx* G, const void* Lnak, bool l_cplx, int W, int N, int M, int Nc, cplx* Tchunk,
+                   long tchunk_elems, cplx* exxn, cplx* kl, cudaStream_t st, int nup, const int* only_if = nullptr);
 
 }  // namespace ops
 }  // namespace sfq

@@ -288,8 +288,9 @@ __global__ void __launch_bounds__(RT) energy_e1_kernel(const cplx* G, const cplx
 // nup < nel: COLLINEAR walkers, orbitals [0, nup) up and [nup, nel) down; the exchange pairs only
 // orbitals of one spin (energy_impl runs per spin, Real3IndexFactorization.hpp:476-560)
 __global__ void __launch_bounds__(RT) energy_exx_kernel(const cplx* T, int nel, int nv, int n0, int nchol,
-                                                        cplx* exxn, cplx* kl, int nup) {
+                                                        cplx* exxn, cplx* kl, int nup, const int* only_if) {
   __shared__ cplx red[RT / 32];
+  if (only_if && !*only_if) return;
   const int n = blockIdx.x, w = blockIdx.y;
   const long rowstride = (long)nv * nel;  // T[(w*nel + a)][(n*nel + b)]
   const cplx* Tw = T + (long)w * nel * rowstride + (long)n * nel;
@@ -612,10 +613,10 @@ int energy_e1(const cplx* G, const cplx* haj, cplx* E3, int nwalk, int nel, int 
 }
 
 int energy_exx_reduce(const cplx* T, int nwalk, int nel, int nv, int n0, int nchol, cplx* exxn, cplx* kl,
-                      cudaStream_t st, int nup) {
+                      cudaStream_t st, int nup, const int* only_if) {
   if (nwalk <= 0 || nv <= 0) return SFQ_OK;
   dim3 grid(nv, nwalk);
-  energy_exx_kernel<<<grid, RT, 0, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup);
+  energy_exx_kernel<<<grid, RT, 0, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, only_if);
   SFQ_LAUNCHED();
   return SFQ_OK;
 }

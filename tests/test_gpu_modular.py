@@ -148,3 +148,28 @@ def test_vhs(W, M, Nc):
     X[1, 5] = float("nan")
     bad = afqmc.vHS(L, X, 0.01)
     assert torch.isnan(bad[1].real).all() and float((bad[2:] - R[2:]).norm() / R[2:].norm()) < 1e-14
+
+
+@pytest.mark.parametrize("W,M,N,Nc,cplx", [(20, 80, 21, 400, False),    # padded columns of a vector
+                                           (12, 90, 70, 150, True),     # complex Lnak, two row tiles
+                                           (3, 130, 116, 90, False)])   # the largest block in shared memory
+def test_energy(W, M, N, Nc, cplx):
+    from safire_b200 import afqmc
+    g = torch.Generator(device="cuda").manual_seed(N)
+    G, haj = _cn(g, W, N, M), _cn(g, N, M)
+    L = _cn(g, Nc, N, M) if cplx else _rn(g, Nc, N, M)
+    Lc = L.to(torch.complex128)
+    R = torch.zeros(W, 3, device="cuda", dtype=torch.complex128)
+    R[:, 0] = 0.25 + 2.0 * torch.einsum("waj,aj->w", G, haj)
+    K = torch.empty(W, Nc, device="cuda", dtype=torch.complex128)
+    for n in range(Nc):
+        T = G @ Lc[n].T  # (W, b, a)
+        R[:, 1] -= (T * T.transpose(1, 2)).sum((1, 2))
+        K[:, n] = torch.diagonal(T, dim1=1, dim2=2).sum(1)
+    R[:, 2] = 2.0 * (K * K).sum(1)
+    scale = R.abs().max(dim=0).values
+    E = afqmc.energy(G, haj, L, E0=0.25)
+    assert float(((E - R).abs() / scale).max()) < 1e-12
+    L[5, 2, 3] = float("nan")  # the FP64 tensor pipe's sums
+    bad = afqmc.energy(G, haj, L, E0=0.25)
+    assert torch.isnan(bad[:, 1].real).all() and float((bad[:, 0] - R[:, 0]).abs().max()) < 1e-9
