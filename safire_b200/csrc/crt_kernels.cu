@@ -327,13 +327,15 @@ __global__ void __launch_bounds__(256) exx_kernel(const uint8_t* c, long ldc, lo
   }
   __syncthreads();
   cplx acc = mk(0.0, 0.0), tr = mk(0.0, 0.0);
-  for (int e = threadIdx.x; e < N * N; e += 256) {
-    const int i = e / N, j = e % N;
-    if (j < i || (i < nup) != (j < nup)) continue;
-    const cplx x = T[i * P + j];
-    if (i == j) tr = cadd(tr, x);
-    const cplx p = cmul(x, T[j * P + i]);
-    acc = cadd(acc, i == j ? p : cscale(p, 2.0));
+  const int lane = threadIdx.x & 31;
+  for (int i = threadIdx.x >> 5; i < N; i += 8) {
+    const int j0 = i < nup ? 0 : nup, j1 = i < nup ? nup : N;  // orbitals of i's spin
+    for (int j = j0 + lane; j < j1; j += 32) {
+      const cplx x = T[i * P + j], y = T[j * P + i];
+      acc.x = fma(x.x, y.x, fma(-x.y, y.y, acc.x));
+      acc.y = fma(x.x, y.y, fma(x.y, y.x, acc.y));
+    }
+    if (lane == 0) tr = cadd(tr, T[i * P + i]);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {

@@ -82,7 +82,6 @@ struct IsliceGroupPlan {
   std::vector<char> image;
   size_t start_off = 0;  // byte offset of the nprob + 1 tile offsets in the image
   int nprob = 0, nslices = 0;
-  int bk = 64;  // K slice width of the launch
   long tiles = 0;
   unsigned long long wait_ns = 0;
 };

@@ -10,14 +10,18 @@ namespace islice {
 using namespace tc;
 
 constexpr int BM = 128;                  // MMA M: accumulator rows = TMEM lanes
-// int8 elements per K slice (BK, a template parameter): 64 (one 64-byte swizzle row) for products
-// whose tiles run over short K ranges, 128 (one 128-byte swizzle row, half the stages) for long ones
+// int8 elements per K slice: one 64-byte swizzle row, four stages of 54 KB at 160 columns.  Two stages of
+// 128-byte rows were no better for long K once the MMA issue loop was short (vHS and force bias, 2400 and
+// 40000 K: the step 1.5 % slower)
+constexpr int BK = 64;
 constexpr int KSTEP = 32;                // K of one kind::i8 MMA
-// warps: 0 TMA producer, 1 TMEM owner + MMA issuer, 2-9 epilogue (two per TMEM lane quarter, taking
-// alternate 16-column chunks of the tile)
-constexpr int kWarps = 10;
+// warps: 0 TMA producer, 1 TMEM owner + MMA issuer, 2-17 epilogue (four per TMEM lane quarter, taking
+// every fourth 16-column chunk of the tile: a 160-wide tile's epilogue does not overlap its MMAs, so its length
+// counts in full)
+constexpr int kWarps = 18;
 constexpr int kThreads = kWarps * 32;
-constexpr int kEpiThreads = 256;
+constexpr int kEpiThreads = 512;
+constexpr int kChunkStep = 64;  // columns between a warp's chunks
 constexpr unsigned long long kWaitNs = 2000000000ull;  // limit of one wait: 2 s without progress
 
 // slice pairs kept for NS slices, listed by group: g0 (0,0) | g1 (0,1) (1,0) | g2 (0,2) (1,1) (2,0)
@@ -41,18 +45,15 @@ __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t adesc, uint64_
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate));
 }
 
-// K-major operand tile, BK-byte swizzle (64 or 128): rows of BK bytes (one K slice), 8-row groups
-// 8 BK bytes apart
-template <int BK>
+// K-major operand tile, 64-byte swizzle: rows of 64 bytes (one K slice), 8-row groups 512 bytes apart
 __device__ __forceinline__ uint64_t smem_desc_k(const void* tile) {
-  static_assert(BK == 64 || BK == 128, "K slice width");
   const uint64_t addr = su32(tile);
   uint64_t d = 0;
   d |= (addr & 0x3FFFFull) >> 4;                  // start address
   d |= uint64_t(1) << 16;                         // leading byte offset (unused for swizzled K-major)
   d |= uint64_t((8 * BK) >> 4) << 32;             // stride byte offset: next 8-row group
   d |= uint64_t(1) << 46;                         // descriptor version (sm_100)
-  d |= uint64_t(BK == 128 ? 2 : 4) << 61;         // SWIZZLE_128B or SWIZZLE_64B
+  d |= uint64_t(4) << 61;                         // SWIZZLE_64B
   return d;
 }
 
@@ -60,7 +61,7 @@ __host__ __device__ constexpr uint32_t pow2_ceil(uint32_t x) {
   return x <= 32 ? 32 : x <= 64 ? 64 : x <= 128 ? 128 : x <= 256 ? 256 : 512;
 }
 
-template <int BN, int STAGES, int NS, int BK>
+template <int BN, int STAGES, int NS>
 struct Smem {
   static constexpr int A_BYTES = BM * BK;
   static constexpr int B_BYTES = BN * BK;
@@ -142,8 +143,7 @@ __device__ __forceinline__ void decode(const KParams& p, long t, int& mt, int& n
   ks = int(r / p.batch);
 }
 // first K slice of split s of KS over KT slices of BK elements: the boundaries fall on multiples of
-// 128 elements whatever BK, so a product's partial sums do not depend on the slice width
-template <int BK>
+// 128 elements
 __device__ __forceinline__ int k_begin(int KT, int KS, int s) {
   constexpr int per = 128 / BK;
   const int kt128 = (KT + per - 1) / per;
@@ -186,7 +186,7 @@ __device__ __forceinline__ int chunk_col0(const KParams& p, int nt, int c, int* 
   return nt * BN + c;
 }
 
-// the 16-column chunks c0, c0 + 32, ... of one tile's accumulator groups at taddr (group g at column
+// the 16-column chunks c0, c0 + 64, ... of one tile's accumulator groups at taddr (group g at column
 // g * BN) -> FP32 output, row `row`
 template <int BN, int NS>
 __device__ __forceinline__ void epilogue_tile(const KParams& p, uint32_t taddr, int row, int mt, int nt, int bz,
@@ -195,13 +195,13 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, uint32_t taddr, 
   const bool live = gm < p.M;
   const int width = p.half ? 2 * p.half : BN;  // complex B: the [re | im] halves may be narrower than BN
   const int lane = threadIdx.x & 31;
-  // the column exponents of all of this thread's chunks c0 + 32 j, loaded before the first one:
+  // the column exponents of all of this thread's chunks c0 + 64 j, loaded before the first one:
   // lanes 0-15 hold chunk 2m's 16 columns in eb2[m], lanes 16-31 chunk 2m + 1's
-  constexpr int NPAIR = ((BN + 31) / 32 + 1) / 2;
+  constexpr int NPAIR = ((BN + kChunkStep - 1) / kChunkStep + 1) / 2;
   int eb2[NPAIR];
 #pragma unroll
   for (int m = 0; m < NPAIR; ++m) {
-    const int c = c0 + 32 * (2 * m + (lane >> 4));
+    const int c = c0 + kChunkStep * (2 * m + (lane >> 4));
     int e = 0;
     if (c < width) {
       int part;
@@ -216,7 +216,7 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, uint32_t taddr, 
   const int ea = live ? p.ea[(long)bz * p.ea_bs + (p.ea_mod ? gm % p.ea_mod : gm)] : 0;
 #pragma unroll 1
   for (int j = 0;; ++j) {
-    const int c = c0 + 32 * j;
+    const int c = c0 + kChunkStep * j;
     if (c >= width) break;
     uint32_t acc[3][16];
     __syncwarp();
@@ -247,31 +247,57 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, uint32_t taddr, 
       if (NS > 2) sum += (long long)int(acc[2][jj]);
       v[jj] = __double2float_rn(double(sum) * pow2(ea + eb - 8 * (NS - 1)) * p.alpha);
     }
+    if (valid == 16 && (p.ldc & 3) == 0 && (obase & 3) == 0 && (p.sCc & 3) == 0) {
+      // Four lanes trade 16-byte pieces (a 4 x 4 transpose), so that a store instruction covers 64-byte pieces
+      // of eight rows; a lane's own 16 bytes of 32 rows took 32 cache lines each, and the stores the most of
+      // the epilogue.  The condition is the same for the warp: rows differ by multiples of ldc.
+      const bool b1 = lane & 1, b2 = lane & 2;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float &lo = v[8 * h + i], &hi = v[8 * h + 4 + i];
+          const float x = __shfl_xor_sync(0xffffffffu, b1 ? lo : hi, 1);
+          if (b1) lo = x;
+          else hi = x;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float &lo = v[4 * h + i], &hi = v[8 + 4 * h + i];
+          const float x = __shfl_xor_sync(0xffffffffu, b2 ? lo : hi, 2);
+          if (b2) lo = x;
+          else hi = x;
+        }
+      }
+      const int first = gm - (lane & 3);  // the group's first row
+      float* out = p.C + obase - (long)(lane & 3) * p.ldc + 4 * (lane & 3);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (first + i < p.M) {
+          float4* o = reinterpret_cast<float4*>(out + i * p.ldc);
+          float4 x = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          if (p.accumulate) {
+            const float4 c4 = *o;
+            x = make_float4(__fadd_rn(x.x, c4.x), __fadd_rn(x.y, c4.y), __fadd_rn(x.z, c4.z), __fadd_rn(x.w, c4.w));
+          }
+          *o = x;
+        }
+      }
+      continue;
+    }
     if (!live) continue;
     float* out = p.C + obase;
-    const bool vec = valid == 16 && (obase % 4) == 0;
-    if (p.accumulate) {
 #pragma unroll
-      for (int jj = 0; jj < 16; ++jj)
-        if (jj < valid) v[jj] = __fadd_rn(v[jj], out[jj]);
-    }
-    if (vec) {
-#pragma unroll
-      for (int jj = 0; jj < 4; ++jj)
-        reinterpret_cast<float4*>(out)[jj] = make_float4(v[4 * jj], v[4 * jj + 1], v[4 * jj + 2], v[4 * jj + 3]);
-    } else {
-#pragma unroll
-      for (int jj = 0; jj < 16; ++jj)
-        if (jj < valid) out[jj] = v[jj];
-    }
+    for (int jj = 0; jj < 16; ++jj)
+      if (jj < valid) out[jj] = p.accumulate ? __fadd_rn(v[jj], out[jj]) : v[jj];
   }
 }
 
-template <int BN, int STAGES, int NS, int BUFS, bool GROUP, int BK>
+template <int BN, int STAGES, int NS, int BUFS, bool GROUP>
 __global__ void __launch_bounds__(kThreads, 1) islice_gemm_kernel(const __grid_constant__ Maps maps0,
                                                                   const __grid_constant__ KParams p0,
                                                                   const __grid_constant__ GroupTab g) {
-  using L = Smem<BN, STAGES, NS, BK>;
+  using L = Smem<BN, STAGES, NS>;
   constexpr uint32_t GCOLS = uint32_t(NS * BN);               // columns of one tile's groups
   constexpr uint32_t ALLOC = pow2_ceil(GCOLS * BUFS);
   constexpr int NP = n_pairs(NS);
@@ -348,7 +374,7 @@ __global__ void __launch_bounds__(kThreads, 1) islice_gemm_kernel(const __grid_c
         decode(p, lt, mt, nt, bz, ks);
         const int m0 = mt * BM;
         const int ab = p.a_batched ? bz : 0, bb = p.b_batched ? bz : 0;
-        const int kb = k_begin<BK>(p.KT, p.KS, ks), ke = k_begin<BK>(p.KT, p.KS, ks + 1);
+        const int kb = k_begin(p.KT, p.KS, ks), ke = k_begin(p.KT, p.KS, ks + 1);
         for (int kt = kb; kt < ke; ++kt, ++it) {
           const int s = int(it % STAGES);
           const uint32_t ph = (it / STAGES) & 1;
@@ -392,8 +418,8 @@ __global__ void __launch_bounds__(kThreads, 1) islice_gemm_kernel(const __grid_c
       uint64_t ad0[NS], bd0[NS];
 #pragma unroll
       for (int q = 0; q < NS; ++q) {
-        ad0[q] = smem_desc_k<BK>(smem + q * L::A_BYTES);
-        bd0[q] = smem_desc_k<BK>(smem + NS * L::A_BYTES + q * L::B_BYTES);
+        ad0[q] = smem_desc_k(smem + q * L::A_BYTES);
+        bd0[q] = smem_desc_k(smem + NS * L::A_BYTES + q * L::B_BYTES);
       }
       uint32_t s = 0, ph = 0;
       int lt_n = 0;
@@ -411,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, 1) islice_gemm_kernel(const __grid_c
         const int Kv = cb ? p.N : p.K;  // valid K elements (complex B: the orbitals)
         int mt, nt, bz, ks;
         decode(p, lt, mt, nt, bz, ks);
-        const int kb = k_begin<BK>(p.KT, p.KS, ks), ke = k_begin<BK>(p.KT, p.KS, ks + 1);
+        const int kb = k_begin(p.KT, p.KS, ks), ke = k_begin(p.KT, p.KS, ks + 1);
         const uint32_t idesc = idesc_i8(uint32_t(cb ? 2 * p.half : BN));
         for (int kt = kb; kt < ke; ++kt) {
           if (!mbar_wait_abort(&full[s], ph, wait_ns, s_abort)) {
@@ -453,7 +479,7 @@ __global__ void __launch_bounds__(kThreads, 1) islice_gemm_kernel(const __grid_c
   } else {  // epilogue warps 2..9 -> TMEM lane quarters 2,3,0,1 (a warp reaches only its quarter)
     const int q = warp & 3;
     const int row = q * 32 + lane;
-    const int c0 = 16 * ((warp - 2) >> 2);  // the two warps of a quarter take alternate 16-column chunks
+    const int c0 = 16 * ((warp - 2) >> 2);  // the four warps of a quarter take every fourth 16-column chunk
     int lt_n = 0;
     for (long t = blockIdx.x; t < total; t += gridDim.x, ++lt_n) {
       const int b = BUFS == 2 ? (lt_n & 1) : 0;
@@ -492,8 +518,7 @@ __global__ void __launch_bounds__(kThreads, 1) islice_gemm_kernel(const __grid_c
 }
 
 // ---- host side -------------------------------------------------------------------------------
-int make_map_i8(CUtensorMap* m, const void* base, long rows, long K, long ld, long batch, long bstride, int box_rows,
-                int bk) {
+int make_map_i8(CUtensorMap* m, const void* base, long rows, long K, long ld, long batch, long bstride, int box_rows) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return record_error(SFQ_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
   if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld % 16) || ld < K)
@@ -506,10 +531,10 @@ int make_map_i8(CUtensorMap* m, const void* base, long rows, long K, long ld, lo
   }
   cuuint64_t dims[3] = {cuuint64_t(K), cuuint64_t(rows), cuuint64_t(batch)};
   cuuint64_t strides[2] = {cuuint64_t(ld), cuuint64_t(bstride)};
-  cuuint32_t box[3] = {cuuint32_t(bk), cuuint32_t(box_rows), 1};
+  cuuint32_t box[3] = {cuuint32_t(BK), cuuint32_t(box_rows), 1};
   cuuint32_t es[3] = {1, 1, 1};
   CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, es,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, bk == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return record_error(SFQ_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", int(r));
@@ -518,20 +543,19 @@ int make_map_i8(CUtensorMap* m, const void* base, long rows, long K, long ld, lo
 
 // the tensor maps and kernel parameters of one product; `group`: a member of a grouped launch of
 // tile width BN, whose complex-B products may use narrower halves
-template <int BN, int STAGES, int NS, int BK>
+template <int BN, int STAGES, int NS>
 int prepare(const IsliceGemmDesc& d, Maps* maps, KParams* kp_out, bool group) {
   const bool cb = d.cplx_half > 0;
   int rc;
   const long ab = d.A.batch_stride ? d.batch : 1, bb = d.B.batch_stride ? d.batch : 1;
   for (int q = 0; q < NS; ++q) {
     if (!d.A.q[q] || !d.B.q[q]) return record_error(SFQ_ERR_ARG, "islice_gemm: slice %d missing", q);
-    if ((rc = make_map_i8(&maps->a[q], d.A.q[q], d.A.rows, d.K, d.A.ld, ab, d.A.batch_stride, BM, BK))) return rc;
-    if ((rc = make_map_i8(&maps->b[q], d.B.q[q], d.B.rows, d.K, d.B.ld, bb, d.B.batch_stride, cb ? d.cplx_half : BN,
-                           BK)))
+    if ((rc = make_map_i8(&maps->a[q], d.A.q[q], d.A.rows, d.K, d.A.ld, ab, d.A.batch_stride, BM))) return rc;
+    if ((rc = make_map_i8(&maps->b[q], d.B.q[q], d.B.rows, d.K, d.B.ld, bb, d.B.batch_stride, cb ? d.cplx_half : BN)))
       return rc;
     if (cb) {
       if (!d.a_im[q]) return record_error(SFQ_ERR_ARG, "islice_gemm: complex B needs a_im");
-      if ((rc = make_map_i8(&maps->aim[q], d.a_im[q], d.A.rows, d.K, d.A.ld, ab, d.A.batch_stride, BM, BK))) return rc;
+      if ((rc = make_map_i8(&maps->aim[q], d.a_im[q], d.A.rows, d.K, d.A.ld, ab, d.A.batch_stride, BM))) return rc;
     } else {
       maps->aim[q] = maps->a[q];
     }
@@ -580,23 +604,23 @@ int prepare(const IsliceGemmDesc& d, Maps* maps, KParams* kp_out, bool group) {
   return SFQ_OK;
 }
 
-template <int BN, int STAGES, int NS, int BK>
+template <int BN, int STAGES, int NS>
 struct Config {
-  using L = Smem<BN, STAGES, NS, BK>;
+  using L = Smem<BN, STAGES, NS>;
   static_assert(BN % 16 == 0, "the epilogue drains whole 16-column chunks");
   static constexpr int BUFS = (2 * NS * BN <= 512) ? 2 : 1;
   static_assert(L::TOTAL <= 232448, "shared memory budget");
   static_assert(NS * BN * BUFS <= 512, "accumulator groups must fit in tensor memory");
 };
 
-template <int BN, int STAGES, int NS, int BK>
+template <int BN, int STAGES, int NS>
 int launch(const IsliceGemmDesc& d, cudaStream_t st) {
-  using C = Config<BN, STAGES, NS, BK>;
+  using C = Config<BN, STAGES, NS>;
   Maps maps;
   KParams kp;
   int rc;
-  if ((rc = prepare<BN, STAGES, NS, BK>(d, &maps, &kp, false))) return rc;
-  auto k = islice_gemm_kernel<BN, STAGES, NS, C::BUFS, false, BK>;
+  if ((rc = prepare<BN, STAGES, NS>(d, &maps, &kp, false))) return rc;
+  auto k = islice_gemm_kernel<BN, STAGES, NS, C::BUFS, false>;
   SFQ_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::L::TOTAL));
   const long grid = kp.tiles < sm_count() ? kp.tiles : sm_count();
   k<<<unsigned(grid), kThreads, C::L::TOTAL, st>>>(maps, kp, GroupTab{});
@@ -606,11 +630,11 @@ int launch(const IsliceGemmDesc& d, cudaStream_t st) {
 
 // the grouped launches' tile widths: every plain product of a group has tile width kGroupBN
 constexpr int kGroupBN = 160;
-constexpr int group_stages(int ns, int bk) { return (ns == 2 ? 6 : 4) * 64 / bk; }
+constexpr int group_stages(int ns) { return ns == 2 ? 6 : 4; }
 
-template <int NS, int BK>
+template <int NS>
 int group_plan(const IsliceGemmDesc* ds, int n, IsliceGroupPlan* out) {
-  constexpr int ST = group_stages(NS, BK);
+  constexpr int ST = group_stages(NS);
   std::vector<GroupProb> probs(static_cast<size_t>(n));
   std::vector<long> start(size_t(n) + 1, 0);
   int rc;
@@ -625,13 +649,12 @@ int group_plan(const IsliceGemmDesc* ds, int n, IsliceGroupPlan* out) {
     GroupProb* pr = probs.data() + i;
     Maps* mp = &pr->maps;
     KParams* kq = &pr->kp;
-    rc = prepare<kGroupBN, ST, NS, BK>(d, mp, kq, true);
+    rc = prepare<kGroupBN, ST, NS>(d, mp, kq, true);
     if (rc) return rc;
     start[size_t(i) + 1] = start[size_t(i)] + kq->tiles;
   }
   out->nprob = n;
   out->nslices = NS;
-  out->bk = BK;
   out->tiles = start[size_t(n)];
   out->wait_ns = n ? probs[0].kp.wait_ns : kWaitNs;
   out->start_off = sizeof(GroupProb) * size_t(n);
@@ -641,10 +664,10 @@ int group_plan(const IsliceGemmDesc* ds, int n, IsliceGroupPlan* out) {
   return SFQ_OK;
 }
 
-template <int NS, int BK>
+template <int NS>
 int group_launch(const void* table, const IsliceGroupPlan& plan, cudaStream_t st) {
-  constexpr int ST = group_stages(NS, BK);
-  using C = Config<kGroupBN, ST, NS, BK>;
+  constexpr int ST = group_stages(NS);
+  using C = Config<kGroupBN, ST, NS>;
   if (reinterpret_cast<uintptr_t>(table) & 127)
     return record_error(SFQ_ERR_ARG, "islice_gemm_group: the table needs 128-byte alignment");
   GroupTab g;
@@ -654,19 +677,12 @@ int group_launch(const void* table, const IsliceGroupPlan& plan, cudaStream_t st
   g.tiles = plan.tiles;
   KParams kp{};
   kp.wait_ns = plan.wait_ns;
-  auto k = islice_gemm_kernel<kGroupBN, ST, NS, C::BUFS, true, BK>;
+  auto k = islice_gemm_kernel<kGroupBN, ST, NS, C::BUFS, true>;
   SFQ_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::L::TOTAL));
   const long grid = plan.tiles < sm_count() ? plan.tiles : sm_count();
   k<<<unsigned(grid), kThreads, C::L::TOTAL, st>>>(Maps{}, kp, g);
   SFQ_LAUNCHED();
   return SFQ_OK;
-}
-
-// the K slice width for a product: 128 elements where its tiles run over 1024 or more K elements
-// (half as many stages, each twice as long), else 64
-inline int k_slice_width(const IsliceGemmDesc& d) {
-  const long k = d.cplx_half > 0 ? 2L * d.K : (d.K + (d.ksplit > 1 ? d.ksplit : 1) - 1) / (d.ksplit > 1 ? d.ksplit : 1);
-  return k >= 1024 ? 128 : 64;
 }
 
 }  // namespace islice
@@ -675,16 +691,15 @@ int islice_gemm(const IsliceGemmDesc& d, cudaStream_t st) {
   if (d.M <= 0 || d.N <= 0 || d.batch <= 0) return SFQ_OK;
   if (d.K <= 0) return record_error(SFQ_ERR_SHAPE, "islice_gemm: K must be positive");
   const int bn = d.cplx_half > 0 ? 2 * d.cplx_half : (d.bn ? d.bn : (d.N <= 64 ? 64 : 128));
-  const bool k128 = islice::k_slice_width(d) == 128;
   // stages: as many as about 216 KB of shared memory holds
   switch (d.nslices * 1000 + bn) {
-    case 2064: return k128 ? islice::launch<64, 4, 2, 128>(d, st) : islice::launch<64, 8, 2, 64>(d, st);
-    case 2128: return k128 ? islice::launch<128, 3, 2, 128>(d, st) : islice::launch<128, 6, 2, 64>(d, st);
-    case 2160: return k128 ? islice::launch<160, 3, 2, 128>(d, st) : islice::launch<160, 6, 2, 64>(d, st);
-    case 3064: return k128 ? islice::launch<64, 3, 3, 128>(d, st) : islice::launch<64, 6, 3, 64>(d, st);
-    case 3080: return k128 ? islice::launch<80, 2, 3, 128>(d, st) : islice::launch<80, 5, 3, 64>(d, st);
-    case 3128: return k128 ? islice::launch<128, 2, 3, 128>(d, st) : islice::launch<128, 4, 3, 64>(d, st);
-    case 3160: return k128 ? islice::launch<160, 2, 3, 128>(d, st) : islice::launch<160, 4, 3, 64>(d, st);
+    case 2064: return islice::launch<64, 8, 2>(d, st);
+    case 2128: return islice::launch<128, 6, 2>(d, st);
+    case 2160: return islice::launch<160, 6, 2>(d, st);
+    case 3064: return islice::launch<64, 6, 3>(d, st);
+    case 3080: return islice::launch<80, 5, 3>(d, st);
+    case 3128: return islice::launch<128, 4, 3>(d, st);
+    case 3160: return islice::launch<160, 4, 3>(d, st);
     default:
       return record_error(SFQ_ERR_ARG, "islice_gemm: %d slices with tile width %d not built", d.nslices, bn);
   }
@@ -692,22 +707,15 @@ int islice_gemm(const IsliceGemmDesc& d, cudaStream_t st) {
 
 int islice_gemm_group_plan(const IsliceGemmDesc* ds, int n, IsliceGroupPlan* out) {
   if (n <= 0 || !ds || !out) return record_error(SFQ_ERR_ARG, "islice_gemm_group: no members");
-  // one K slice width for the launch: the widest any member would take alone (the results do not
-  // depend on it)
-  bool k128 = false;
-  for (int i = 0; i < n; ++i) k128 = k128 || islice::k_slice_width(ds[i]) == 128;
-  if (ds[0].nslices == 2) return k128 ? islice::group_plan<2, 128>(ds, n, out) : islice::group_plan<2, 64>(ds, n, out);
-  if (ds[0].nslices == 3) return k128 ? islice::group_plan<3, 128>(ds, n, out) : islice::group_plan<3, 64>(ds, n, out);
+  if (ds[0].nslices == 2) return islice::group_plan<2>(ds, n, out);
+  if (ds[0].nslices == 3) return islice::group_plan<3>(ds, n, out);
   return record_error(SFQ_ERR_ARG, "islice_gemm_group: %d slices not built", ds[0].nslices);
 }
 
 int islice_gemm_group_launch(const void* table, const IsliceGroupPlan& plan, cudaStream_t st) {
   if (plan.nprob <= 0 || plan.tiles <= 0) return SFQ_OK;
-  const bool k128 = plan.bk == 128;
-  if (plan.nslices == 2)
-    return k128 ? islice::group_launch<2, 128>(table, plan, st) : islice::group_launch<2, 64>(table, plan, st);
-  if (plan.nslices == 3)
-    return k128 ? islice::group_launch<3, 128>(table, plan, st) : islice::group_launch<3, 64>(table, plan, st);
+  if (plan.nslices == 2) return islice::group_launch<2>(table, plan, st);
+  if (plan.nslices == 3) return islice::group_launch<3>(table, plan, st);
   return record_error(SFQ_ERR_ARG, "islice_gemm_group: %d slices not built", plan.nslices);
 }
 

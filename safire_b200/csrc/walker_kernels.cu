@@ -339,6 +339,62 @@ __global__ void __launch_bounds__(RT) energy_exx_f32_kernel(const float* C, int 
   }
 }
 
+// The same two sums with the walker's N x N block of one n in shared memory: each element is read once, in
+// rows; the kernels above read T[b][a] again down the columns of a chunk that does not fit in L2.
+// E: float2 (planar FP32 parts) or cplx.
+__device__ __forceinline__ cplx as_cplx(float2 v) { return mk(v.x, v.y); }
+__device__ __forceinline__ cplx as_cplx(cplx v) { return v; }
+template <typename E, typename LOAD>
+__device__ __forceinline__ void exx_block(LOAD&& load, int nel, int nup, cplx* exx, cplx* kl) {
+  extern __shared__ __align__(16) unsigned char exx_sm[];
+  __shared__ cplx red[RT / 32];
+  E* T = reinterpret_cast<E*>(exx_sm);
+  const int P = nel | 1;
+  // a warp to a row: an index division per element cost more than the sums
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int b = lane; b < nel; b += 32) {
+#pragma unroll 4
+    for (int a = warp; a < nel; a += RT / 32) T[a * P + b] = load(a, b);
+  }
+  __syncthreads();
+  cplx acc = mk(0.0, 0.0), tr = mk(0.0, 0.0);
+  for (int a = warp; a < nel; a += RT / 32) {
+    const int b0 = a < nup ? 0 : nup, b1 = a < nup ? nup : nel;  // orbitals of a's spin
+    for (int b = b0 + lane; b < b1; b += 32) {
+      const cplx x = as_cplx(T[a * P + b]), y = as_cplx(T[b * P + a]);
+      acc.x = fma(x.x, y.x, fma(-x.y, y.y, acc.x));
+      acc.y = fma(x.x, y.y, fma(x.y, y.x, acc.y));
+    }
+    if (lane == 0) tr = cadd(tr, as_cplx(T[a * P + a]));
+  }
+  const cplx s = block_sum<RT>(acc, red);
+  const cplx t = block_sum<RT>(tr, red);
+  if (threadIdx.x == 0) {
+    *exx = s;
+    *kl = t;
+  }
+}
+__global__ void __launch_bounds__(RT) energy_exx_sm_kernel(const cplx* T, int nel, int nv, int n0, int nchol,
+                                                           cplx* exxn, cplx* kl, int nup, const int* only_if) {
+  if (only_if && !*only_if) return;
+  const int n = blockIdx.x, w = blockIdx.y;
+  const long ld = (long)nv * nel, o = (long)w * nchol + n0 + n;
+  const cplx* Tw = T + (long)w * nel * ld + (long)n * nel;
+  exx_block<cplx>([&](int a, int b) { return Tw[a * ld + b]; }, nel, nup, exxn + o, kl + o);
+}
+__global__ void __launch_bounds__(RT) energy_exx_f32_sm_kernel(const float* C, int W, int nel, int nv, int n0, int nchol,
+                                                               long ldc, cplx* exxn, cplx* kl, int nup) {
+  const int n = blockIdx.x, w = blockIdx.y;
+  const float* Cr = C + (long)w * nel * ldc + (long)n * nel;
+  const float* Ci = Cr + (long)W * nel * ldc;
+  const long o = (long)w * nchol + n0 + n;
+  exx_block<float2>([&](int a, int b) { return make_float2(Cr[a * ldc + b], Ci[a * ldc + b]); }, nel, nup, exxn + o,
+                    kl + o);
+}
+constexpr size_t kExxSmem = 200 * 1024;  // a block's N x N in shared memory up to this, else through the caches
+template <typename E>
+size_t exx_smem(int nel) { return sizeof(E) * (size_t)nel * (nel | 1); }
+
 __global__ void __launch_bounds__(RT) energy_finish_kernel(const cplx* exxn, const cplx* kl, cplx* E3, int nchol,
                                                            double scl, int addEXX, int addEJ) {
   __shared__ cplx red[RT / 32];
@@ -616,7 +672,13 @@ int energy_exx_reduce(const cplx* T, int nwalk, int nel, int nv, int n0, int nch
                       cudaStream_t st, int nup, const int* only_if) {
   if (nwalk <= 0 || nv <= 0) return SFQ_OK;
   dim3 grid(nv, nwalk);
-  energy_exx_kernel<<<grid, RT, 0, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, only_if);
+  const size_t sm = exx_smem<cplx>(nel);
+  if (sm <= kExxSmem) {
+    SFQ_CUDA_TRY(cudaFuncSetAttribute(energy_exx_sm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    energy_exx_sm_kernel<<<grid, RT, sm, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, only_if);
+  } else {
+    energy_exx_kernel<<<grid, RT, 0, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, only_if);
+  }
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
@@ -625,7 +687,13 @@ int energy_exx_reduce_f32(const float* C, int nwalk, int nel, int nv, int n0, in
                           cplx* kl, cudaStream_t st, int nup) {
   if (nwalk <= 0 || nv <= 0) return SFQ_OK;
   dim3 grid(nv, nwalk);
-  energy_exx_f32_kernel<<<grid, RT, 0, st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
+  const size_t sm = exx_smem<float2>(nel);
+  if (sm <= kExxSmem) {
+    SFQ_CUDA_TRY(cudaFuncSetAttribute(energy_exx_f32_sm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    energy_exx_f32_sm_kernel<<<grid, RT, sm, st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
+  } else {
+    energy_exx_f32_kernel<<<grid, RT, 0, st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
+  }
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
