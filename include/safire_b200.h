@@ -218,7 +218,7 @@ int sfq_split_bf16(const double* src, long n, void* p0, void* p1, void* p2, void
 int sfq_gemm_int8_slices(const double* A, const double* B, float* C, int M, int N, int K, int nslices, int tile_n,
                          int ksplit, void* stream);
 /* C = A B^T (M x N, FP64) of device doubles A (M x K), B (N x K) by the modular int8 products of
- * sfq_vhs_ws; operands it cannot hold (an Inf, a NaN, a row norm outside 1e+-150) go through the FP64
+ * sfq_vhs_ws; operands it cannot hold (an Inf, a NaN, a row norm outside 1e+-120) go through the FP64
  * tensor pipe instead.  M <= 65535, K <= 90000. */
 int sfq_gemm_f64_modular(const double* A, const double* B, double* C, int M, int N, int K, void* stream);
 /* the Taylor term's product in the same arithmetic (the int8 slices'): C[c][w][a][j] = part c of sum_i A[w][a][i] V[w][j][i]

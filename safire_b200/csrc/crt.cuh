@@ -10,7 +10,7 @@
 // row's norm, and of the result to FP64: with K random terms the relative error of a result is
 // about 2^-58 sqrt(K), against 2^-55 sqrt(K) of an FP64 chain of K additions.
 //
-// Rows that the scheme cannot hold (an Inf or a NaN, a norm outside 2^+-500) raise a flag in
+// Rows that the scheme cannot hold (an Inf or a NaN, a norm outside 1e+-120) raise a flag in
 // device memory; the FP64 tensor-pipe product (gemm_f64), launched behind it with
 // GemmDesc::only_if, then computes the result.
 #pragma once
@@ -35,16 +35,24 @@ struct Tables {
   // C'/P mod 1 = sum_i r_i G_i mod 1 with G_i = ((P / p_i)^-1 mod p_i) / p_i, in 80-bit fixed point;
   // byte j of the G_i of moduli 4q .. 4q+3 in g[j][q]
   unsigned g[10][4];
-  double P;                // P rounded to double
+  double P_hi, P_lo;       // P 2^-64 as the sum of two doubles
 };
 
 constexpr unsigned kModuli[15] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
 
 constexpr Tables make_tables() {
   Tables t{};
-  double P = 1.0;
-  for (int i = 0; i < 15; ++i) P *= double(kModuli[i]);
-  t.P = P;
+  u128 P = 1;
+  for (int i = 0; i < 15; ++i) P *= kModuli[i];
+  // the top 53 bits of P and the rest, exactly
+  int sh = 0;
+  while ((P >> sh) >= (u128(1) << 53)) ++sh;
+  double w = 1.0;
+  for (int i = 0; i < sh; ++i) w *= 2.0;
+  t.P_hi = double((unsigned long long)(P >> sh)) * (w / 18446744073709551616.0);
+  const u128 rest = P - ((P >> sh) << sh);
+  t.P_lo = (double((unsigned long long)(rest >> 32)) * 4294967296.0 + double((unsigned long long)(rest & 0xffffffffu))) /
+           18446744073709551616.0;
   for (int i = 0; i < 15; ++i) {
     const unsigned p = kModuli[i];
     t.mod[i] = p;
@@ -148,6 +156,13 @@ int rows_cplx(const cplx* src, long rows, long K, long stride, int nb, long blk_
               const Planes& out, int* flag, cudaStream_t st);
 // walkers (W, M, N) complex -> rows (w, a) over the M orbitals, blocks re, im: plane row k * W N + w N + a
 int walkers_in(const cplx* SM, int W, int M, int N, const Planes& out, int* flag, cudaStream_t st);
+
+// alpha P 2^-64 as a sum of two doubles, so that values are rounded twice (as integers, as products) and not
+// pulled by a rounded constant as well
+struct Scale {
+  double hi, lo;
+};
+Scale scale_of(double alpha);
 
 // ---- residues to FP64 ---------------------------------------------------------------------------
 // out[m][n] = alpha (C_re + i C_im) for parts = 2 products with M rows; exponents eA[m], eB[n]

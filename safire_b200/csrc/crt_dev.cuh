@@ -7,17 +7,16 @@ namespace crt {
 
 static constexpr Tables kTabD = make_tables();
 static __constant__ Tables c_crt = kTabD;
-static constexpr double kTwoM64P = kTabD.P / 18446744073709551616.0;  // P 2^-64
 
 __device__ __forceinline__ double pow2(int e) {
   return __longlong_as_double((long long)((e < -1022 ? -1022 : e > 1023 ? 1023 : e) + 1023) << 52);
 }
 
 // the scale exponent of a row with squared norm n2: |row| 2^-e < 2^kNormBits.  Rows that cannot be held
-// (not finite, or so large or small that their squares leave the range) raise *flag.
+// (not finite, or a norm outside 1e+-120, beyond which two rows' scales could leave the exponent range) raise *flag.
 __device__ __forceinline__ int row_exponent(double n2, bool any, int* flag) {
   if (!any && n2 == 0.0) return 0;
-  if (!(n2 > 1e-300 && n2 < 1e300)) {
+  if (!(n2 > 1e-240 && n2 < 1e240)) {
     if (flag) *flag = 1;
     return 0;
   }

@@ -2,6 +2,8 @@
 #include "crt.cuh"
 #include "crt_dev.cuh"
 
+#include <cmath>
+
 namespace sfq {
 namespace crt {
 
@@ -171,12 +173,15 @@ __global__ void __launch_bounds__(256) walkers_in_kernel(const cplx* SM, int W, 
 struct Vals {
   double v[4];
 };
-__device__ __forceinline__ Vals values4(const uint8_t* c, long plane, int ea, const int eb[4], double s) {
+__device__ __forceinline__ Vals values4(const uint8_t* c, long plane, int ea, const int eb[4], Scale s) {
   long long X[4];
   reconstruct4(c, plane, X);
   Vals o;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) o.v[j] = double(X[j]) * (s * pow2(ea + eb[j]));
+  for (int j = 0; j < 4; ++j) {
+    const double x = double(X[j]), p = pow2(ea + eb[j]);
+    o.v[j] = fma(x, s.hi * p, x * (s.lo * p));
+  }
   return o;
 }
 
@@ -188,7 +193,7 @@ __device__ __forceinline__ void load_e4(const int* e, long n, long N, int eb[4])
 // complex output, 4 columns per thread, 128 per warp; the warp's values go through shared memory so that
 // its stores are whole 512-byte rows
 __global__ void __launch_bounds__(256) out_cplx_kernel(const uint8_t* c, long ldc, long plane, long M, long N,
-                                                       const int* eA, const int* eB, double alpha, cplx* out,
+                                                       const int* eA, const int* eB, Scale s, cplx* out,
                                                        long ldo, const int* skip_if) {
   __shared__ cplx sh[8][130];
   if (skip_if && *skip_if) return;
@@ -199,7 +204,6 @@ __global__ void __launch_bounds__(256) out_cplx_kernel(const uint8_t* c, long ld
   if (n < N) {
     int eb[4];
     load_e4(eB, n, N, eb);
-    const double s = alpha * kTwoM64P;
     const Vals re = values4(c + m * ldc + n, plane, eA[m], eb, s);
     const Vals im = values4(c + (M + m) * ldc + n, plane, eA[m], eb, s);
 #pragma unroll
@@ -214,14 +218,14 @@ __global__ void __launch_bounds__(256) out_cplx_kernel(const uint8_t* c, long ld
 }
 
 __global__ void __launch_bounds__(256) out_real_kernel(const uint8_t* c, long ldc, long plane, long M, long N,
-                                                       const int* eA, const int* eB, double alpha, double* out,
+                                                       const int* eA, const int* eB, Scale s, double* out,
                                                        long ldo, const int* skip_if) {
   if (skip_if && *skip_if) return;
   const long m = blockIdx.y, n = 4 * ((long)blockIdx.x * 256 + threadIdx.x);
   if (n >= N) return;
   int eb[4];
   load_e4(eB, n, N, eb);
-  const Vals re = values4(c + m * ldc + n, plane, eA[m], eb, alpha * kTwoM64P);
+  const Vals re = values4(c + m * ldc + n, plane, eA[m], eb, s);
 #pragma unroll
   for (int j = 0; j < 4; ++j)
     if (n + j < N) out[m * ldo + n + j] = re.v[j];
@@ -233,7 +237,7 @@ __global__ void __launch_bounds__(256) out_real_kernel(const uint8_t* c, long ld
 // out, 45 residues out; a row's T waits in shared memory for its norm.
 template <bool FIRST, bool LAST>
 __global__ void __launch_bounds__(256, 4) taylor_kernel(const uint8_t* c, long ldc, long plane, long WN, int N, int M,
-                                                     double inv_k, const int* eA, const int* eB, int eB_per_w,
+                                                     Scale sc, const int* eA, const int* eB, int eB_per_w,
                                                      double* S, int8_t* q, long ld, long qplane, int* e, int* flag,
                                                      int R) {
   extern __shared__ double rows[];  // [R][2][M4] T (S when LAST), then [R * M4 / 4] squared norms, [R] scales
@@ -249,8 +253,8 @@ __global__ void __launch_bounds__(256, 4) taylor_kernel(const uint8_t* c, long l
     int eb[4];
     load_e4(eb0, j0, M, eb);
     const int ea = eA[r];
-    const Vals re = values4(c + r * ldc + j0, plane, ea, eb, kTwoM64P * inv_k);
-    const Vals im = values4(c + (WN + r) * ldc + j0, plane, ea, eb, kTwoM64P * inv_k);
+    const Vals re = values4(c + r * ldc + j0, plane, ea, eb, sc);
+    const Vals im = values4(c + (WN + r) * ldc + j0, plane, ea, eb, sc);
     double* Sr = S + r * M + j0;
     double* Si = S + (WN + r) * M + j0;
     double n2 = 0.0, nz = 0.0;
@@ -310,7 +314,7 @@ __global__ void __launch_bounds__(256, 4) taylor_kernel(const uint8_t* c, long l
 // exchange trace.  Bound by the reconstruction (two residue groups per complex element) and its reads.
 __global__ void __launch_bounds__(256) exx_kernel(const uint8_t* c, long ldc, long plane, long WN, int N, int N4,
                                                   const int* eA, const int* eB, int n0, int Nc, cplx* exxn, cplx* kl,
-                                                  int nup) {
+                                                  int nup, Scale sc) {
   extern __shared__ cplx T[];  // T[b][a], rows of P
   __shared__ cplx red[2][8];
   const int n = blockIdx.x, w = blockIdx.y, P = N | 1, q4 = N4 / 4;
@@ -319,8 +323,8 @@ __global__ void __launch_bounds__(256) exx_kernel(const uint8_t* c, long ldc, lo
     const long r = (long)w * N + b, col = (long)n * N4 + a;
     int eb[4];
     load_e4(eB + (long)n * N, a, N, eb);
-    const Vals re = values4(c + r * ldc + col, plane, eA[r], eb, kTwoM64P);
-    const Vals im = values4(c + (WN + r) * ldc + col, plane, eA[r], eb, kTwoM64P);
+    const Vals re = values4(c + r * ldc + col, plane, eA[r], eb, sc);
+    const Vals im = values4(c + (WN + r) * ldc + col, plane, eA[r], eb, sc);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (a + j < N) T[b * P + a + j] = mk(re.v[j], im.v[j]);
@@ -359,7 +363,7 @@ __global__ void __launch_bounds__(256) exx_kernel(const uint8_t* c, long ldc, lo
 // SM[w][j][a] from rows (part, w, a), columns j: 32 x 32 tiles transposed through shared memory
 __global__ void __launch_bounds__(256) walkers_out_kernel(const uint8_t* c, long ldc, long plane, long WN, int M,
                                                           int N, const int* eA, const int* eB, cplx* SM,
-                                                          const int* skip_if) {
+                                                          const int* skip_if, Scale sc) {
   __shared__ cplx tile[32][33];
   if (skip_if && *skip_if) return;
   const int w = blockIdx.z, j0 = blockIdx.x * 32, a0 = blockIdx.y * 32;
@@ -369,8 +373,8 @@ __global__ void __launch_bounds__(256) walkers_out_kernel(const uint8_t* c, long
       const long r = (long)w * N + a0 + a;
       int eb[4];
       load_e4(eB, j0 + j4, M, eb);
-      const Vals re = values4(c + r * ldc + j0 + j4, plane, eA[r], eb, kTwoM64P);
-      const Vals im = values4(c + (WN + r) * ldc + j0 + j4, plane, eA[r], eb, kTwoM64P);
+      const Vals re = values4(c + r * ldc + j0 + j4, plane, eA[r], eb, sc);
+      const Vals im = values4(c + (WN + r) * ldc + j0 + j4, plane, eA[r], eb, sc);
 #pragma unroll
       for (int j = 0; j < 4; ++j) tile[j4 + j][a] = mk(re.v[j], im.v[j]);
     }
@@ -382,6 +386,14 @@ __global__ void __launch_bounds__(256) walkers_out_kernel(const uint8_t* c, long
 }
 
 }  // namespace
+
+Scale scale_of(double alpha) {
+  constexpr Tables t = make_tables();
+  Scale s;
+  s.hi = alpha * t.P_hi;
+  s.lo = std::fma(alpha, t.P_hi, -s.hi) + alpha * t.P_lo;
+  return s;
+}
 
 int rows_real(const double* src, long rows, long K, long stride, const Planes& o, int* flag, cudaStream_t st,
               long inner, long outer) {
@@ -417,7 +429,7 @@ int walkers_in(const cplx* SM, int W, int M, int N, const Planes& o, int* flag, 
 
 int out_cplx(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, cplx* out, long ldo,
              const int* skip_if, cudaStream_t st) {
-  out_cplx_kernel<<<dim3(ceil_div(N, 1024), unsigned(M)), 256, 0, st>>>(c.q, c.ldc, c.plane, M, N, eA, eB, alpha, out,
+  out_cplx_kernel<<<dim3(ceil_div(N, 1024), unsigned(M)), 256, 0, st>>>(c.q, c.ldc, c.plane, M, N, eA, eB, scale_of(alpha), out,
                                                                         ldo, skip_if);
   SFQ_LAUNCHED();
   return SFQ_OK;
@@ -425,7 +437,7 @@ int out_cplx(const Out& c, long M, long N, const int* eA, const int* eB, double 
 
 int out_real(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, double* out, long ldo,
              const int* skip_if, cudaStream_t st) {
-  out_real_kernel<<<dim3(ceil_div(N, 1024), unsigned(M)), 256, 0, st>>>(c.q, c.ldc, c.plane, M, N, eA, eB, alpha, out,
+  out_real_kernel<<<dim3(ceil_div(N, 1024), unsigned(M)), 256, 0, st>>>(c.q, c.ldc, c.plane, M, N, eA, eB, scale_of(alpha), out,
                                                                         ldo, skip_if);
   SFQ_LAUNCHED();
   return SFQ_OK;
@@ -449,7 +461,7 @@ int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int
   const double ik = k > 0 ? 1.0 / double(k) : 1.0;
   auto kern = k == 0 ? taylor_kernel<true, false> : last ? taylor_kernel<false, true> : taylor_kernel<false, false>;
   if (sm > 48 * 1024) SFQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
-  kern<<<unsigned((WN + R - 1) / R), 256, sm, st>>>(c.q, c.ldc, c.plane, WN, N, M, ik, eA, eB, eB_per_w, S, o.q, o.ld,
+  kern<<<unsigned((WN + R - 1) / R), 256, sm, st>>>(c.q, c.ldc, c.plane, WN, N, M, scale_of(ik), eA, eB, eB_per_w, S, o.q, o.ld,
                                                     o.plane, o.e, flag, R);
   SFQ_LAUNCHED();
   return SFQ_OK;
@@ -461,7 +473,7 @@ int exx_reduce(const Out& c, int W, int N, int N4, int nv, int n0, int Nc, const
   if (N > kExxMaxN) return record_error(SFQ_ERR_SHAPE, "crt exx: N=%d above %d", N, kExxMaxN);
   SFQ_CUDA_TRY(cudaFuncSetAttribute(exx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
   exx_kernel<<<dim3(nv, W), 256, sm, st>>>(c.q, c.ldc, c.plane, (long)W * N, N, N4, eA, eB, n0, Nc, exxn, kl,
-                                           nup < 0 ? N : nup);
+                                           nup < 0 ? N : nup, scale_of(1.0));
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
@@ -469,7 +481,7 @@ int exx_reduce(const Out& c, int W, int N, int N4, int nv, int n0, int Nc, const
 int walkers_out(const Out& c, int W, int M, int N, const int* eA, const int* eB, cplx* SM, const int* skip_if,
                 cudaStream_t st) {
   walkers_out_kernel<<<dim3((M + 31) / 32, (N + 31) / 32, W), 256, 0, st>>>(c.q, c.ldc, c.plane, (long)W * N, M, N, eA,
-                                                                           eB, SM, skip_if);
+                                                                           eB, SM, skip_if, scale_of(1.0));
   SFQ_LAUNCHED();
   return SFQ_OK;
 }

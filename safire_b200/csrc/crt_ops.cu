@@ -39,12 +39,11 @@ size_t vbias_crt_bytes(int W, int N, int M, int Nc, bool l_cplx, bool prepared) 
   return b + slack();
 }
 
-// The FP64 tensor-pipe product walks K = N M in one chain per tile of few tiles (74 us at K = 576, 1.9 ms at
-// 16384, whatever the walkers); this path takes 29 us at K = 1024 and 402 us at 16384 with 256 walkers.
-// Below K = 300 its launches cost as much as the chain.
+// The FP64 tensor-pipe product walks K = N M in one chain per tile of few tiles: 19 us at K = 576, 58 at 1024 and
+// 1.27 ms at 16384 with 256 walkers; this path, whose launches cost more, takes 38, 32 and 372 us.
 bool vbias_crt_ok(int W, int N, int M, int Nc, bool l_cplx) {
   const long K = (long)N * M;
-  return W >= 8 && W <= 65535 && Nc >= 64 && K >= 300 && K * (l_cplx ? 2 : 1) <= kMaxK;
+  return W >= 8 && W <= 65535 && Nc >= 64 && K >= 1024 && K * (l_cplx ? 2 : 1) <= kMaxK;
 }
 
 int vbias_crt(const cplx* G, const void* Lnak, bool l_cplx, const Planes* Lq, cplx* v, int W, int N, int M, int Nc,
@@ -93,7 +92,7 @@ size_t vhs_crt_bytes(int W, long rows, int Nc, bool prepared) {
 }
 
 // Converting L (M^2 Nc elements) costs what the FP64 product of about 64 walkers does: from 96 walkers on
-// the call gains (1.3x at M = 128 with 128 walkers, 2.5x at M = 256 and 400 with 256), at 64 it is even.  With
+// the call gains (1.4x at M = 128 with 128 walkers, 2.8x at M = 256 and 400 with 256), at 64 it is even.  With
 // L's planes prepared the product alone counts.
 bool vhs_crt_ok(int W, long rows, int Nc, bool prepared) {
   const double flops = 4.0 * W * double(rows) * Nc;
@@ -150,12 +149,13 @@ size_t propagate_crt_bytes(int W, int M, int N, int npol, bool prepared) {
   return kFlagBytes + b + slack();
 }
 
-// The walkers' and V's conversions grow as M^2 and M N, the products as M^2 N: even at M = 192 (1.48 ms
-// both ways with 48 electrons, 256 walkers), 1.8x at M = 400 with 100 electrons.
+// The conversions of V and of the Taylor terms grow as M^2 and M N, the products as M^2 N: 1.9x at M = 400 with
+// 100 electrons and 256 walkers, 1.1x at M = 256 with 64, slower with few electrons (0.8x at M = 256 with 32) and
+// even at M = 192; 16 walkers at M = 400 gain 1.3x with 100 electrons and nothing with 50.
 bool propagate_crt_ok(int W, int M, int N, int npol, bool p_cplx, int order) {
   const double flops = 64.0 * W * M * double(M) * N * npol;
-  return !p_cplx && order >= 1 && W <= 30000 && M <= 4096 && N * npol >= 16 &&
-         (M >= 320 ? flops >= 5e9 : M >= 240 && flops >= 1.5e10) && walker_gemm_fits(N * npol, M, M, 2);
+  return !p_cplx && order >= 1 && W <= 30000 && M >= 240 && M <= 4096 && N * npol >= 48 && flops >= 1.4e10 &&
+         walker_gemm_fits(N * npol, M, M, 2);
 }
 
 int propagate_crt(cplx* SM, const double* P1, const Planes* P1q, const cplx* V, int W, int M, int N, int npol,

@@ -86,18 +86,28 @@ def test_operands_outside_the_range(value):
     assert ((C - R).abs()[ok] <= 2 * bound[ok]).all()
 
 
+@pytest.mark.parametrize("fa,fb", [(1e118, 1e118), (1e-118, 1e-118), (1e118, 1e-118)])
+def test_edges_of_the_range(fa, fb):
+    """Rows whose norms are just inside the range: both scales at their largest or smallest."""
+    g = torch.Generator(device="cuda").manual_seed(8)
+    A, B = _rn(g, 20, 60) * fa, _rn(g, 30, 60) * fb
+    C = _modular(A, B).cpu().numpy().astype(np.longdouble)
+    R = A.cpu().numpy().astype(np.longdouble) @ B.cpu().numpy().astype(np.longdouble).T
+    assert float(np.abs(C - R).max() / np.abs(R).max()) < 4 * 2.0 ** -53
+
+
 def _workspace_path(op, *sizes):
     from safire_b200.capi import lib
     return lib().sfq_workspace_size(op, *sizes)
 
 
-@pytest.mark.parametrize("W,M,N", [(20, 331, 37),    # one row tile of [re; im], odd sizes
-                                   (12, 320, 64),    # [re; im] exactly 128 rows
-                                   (12, 321, 65),    # two row tiles
-                                   (6, 330, 128),    # the widest electron block
-                                   (6, 333, 129),    # two chunks of electrons
-                                   (2, 1030, 40),    # K slices that leave room for few electrons
-                                   (1, 900, 100)])   # fewer units than SMs: split columns
+@pytest.mark.parametrize("W,M,N", [(44, 331, 49),    # one row tile of [re; im], odd sizes
+                                   (36, 320, 64),    # [re; im] exactly 128 rows
+                                   (36, 321, 65),    # two row tiles
+                                   (18, 330, 128),   # the widest electron block
+                                   (17, 333, 129),   # two chunks of electrons
+                                   (5, 1030, 48),    # K slices that leave room for few electrons
+                                   (3, 900, 100)])   # fewer units than SMs: split columns
 @pytest.mark.parametrize("order", [1, 6])
 def test_propagate(W, M, N, order):
     from safire_b200 import afqmc, capi
@@ -123,7 +133,7 @@ def test_propagate(W, M, N, order):
 
 
 @pytest.mark.parametrize("W,M,N,Nc,cplx", [(150, 100, 30, 1200, False), (8, 101, 23, 613, True),
-                                           (300, 90, 7, 65, False)])
+                                           (300, 103, 10, 65, False)])
 def test_vbias(W, M, N, Nc, cplx):
     from safire_b200 import afqmc, capi
     assert _workspace_path(capi.OP_VBIAS_COMPLEX if cplx else capi.OP_VBIAS, W, M, N, Nc) > 0
