@@ -218,8 +218,11 @@ int energy_nv(int W, int N, int M, int Nc, bool l_cplx) {
 }
 }  // namespace
 
+// A walker's [re; im] rows fill 128-row tiles: with 50 electrons 112 of them (1.26x at M = 200, Nc = 1200, 128
+// walkers), with 32 half, where the product and the reconstruction together take what the FP64 product does.
+// Below 40 GFLOP (about a millisecond there) its launches count.
 bool energy_crt_ok(int W, int N, int M, int Nc, bool l_cplx) {
-  return W <= 65535 && N >= 8 && N <= kExxMaxN && M >= 32 && 8.0 * W * N * double(N) * M * Nc >= 2e9 &&
+  return W <= 65535 && N >= 40 && N <= kExxMaxN && M >= 32 && 8.0 * W * N * double(N) * M * Nc >= 4e10 &&
          energy_n_bytes(W, N, M, l_cplx) <= kChunkBytes && walker_gemm_fits(N, 16 * n4_of(N), M, l_cplx ? 2 : 1);
 }
 

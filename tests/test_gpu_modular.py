@@ -160,11 +160,13 @@ def test_vhs(W, M, Nc):
     assert torch.isnan(bad[1].real).all() and float((bad[2:] - R[2:]).norm() / R[2:].norm()) < 1e-14
 
 
-@pytest.mark.parametrize("W,M,N,Nc,cplx", [(20, 80, 21, 400, False),    # padded columns of a vector
-                                           (12, 90, 70, 150, True),     # complex Lnak, two row tiles
-                                           (3, 130, 116, 90, False)])   # the largest block in shared memory
+@pytest.mark.parametrize("W,M,N,Nc,cplx", [(20, 120, 45, 1100, False),   # padded columns of a vector
+                                           (16, 90, 70, 800, True),      # complex Lnak, two row tiles
+                                           (10, 130, 116, 300, False)])  # the largest block in shared memory
 def test_energy(W, M, N, Nc, cplx):
-    from safire_b200 import afqmc
+    from safire_b200 import afqmc, capi
+    nv = min(Nc, 2**27 // (W * N * N))
+    assert _workspace_path(capi.OP_ENERGY, W, M, N, Nc) > 16 * W * (N * nv * N + 2 * Nc) + 4096  # the int8 path's
     g = torch.Generator(device="cuda").manual_seed(N)
     G, haj = _cn(g, W, N, M), _cn(g, N, M)
     L = _cn(g, Nc, N, M) if cplx else _rn(g, Nc, N, M)
