@@ -59,6 +59,12 @@ void count_launch();
   } while (0)
 int record_error(int code, const char* fmt, ...);
 
+// A kernel's dynamic shared-memory limit belongs to the function, not to the launch: it is always set to the
+// kernel's largest, so that a call never lowers it between another host thread's setting and launch, nor below
+// what a captured graph's node needs.
+#define SFQ_MAX_SMEM(kernel, bytes) \
+  SFQ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)))
+
 inline int ceil_div(long a, long b) { return int((a + b - 1) / b); }
 
 }  // namespace sfq

@@ -443,6 +443,9 @@ int out_real(const Out& c, long M, long N, const int* eA, const int* eB, double 
   return SFQ_OK;
 }
 
+// of one row of 4096 orbitals, the most that the propagation takes this way
+constexpr size_t kTaylorSmem = sizeof(double) * (2 * 4096 + 4096 / 4 + 1);
+
 int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int* eA, const int* eB, int eB_per_w,
                   double* S, const Planes& o, int* flag, cudaStream_t st) {
   const int M4 = (M + 3) / 4 * 4, q4 = M4 / 4;
@@ -460,7 +463,8 @@ int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int
   const size_t sm = sizeof(double) * (2L * R * M4 + (long)R * q4 + R);
   const double ik = k > 0 ? 1.0 / double(k) : 1.0;
   auto kern = k == 0 ? taylor_kernel<true, false> : last ? taylor_kernel<false, true> : taylor_kernel<false, false>;
-  if (sm > 48 * 1024) SFQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  if (sm > kTaylorSmem) return record_error(SFQ_ERR_SHAPE, "crt taylor: M=%d too large", M);
+  SFQ_MAX_SMEM(kern, kTaylorSmem);
   kern<<<unsigned((WN + R - 1) / R), 256, sm, st>>>(c.q, c.ldc, c.plane, WN, N, M, scale_of(ik), eA, eB, eB_per_w, S, o.q, o.ld,
                                                     o.plane, o.e, flag, R);
   SFQ_LAUNCHED();
@@ -471,7 +475,7 @@ int exx_reduce(const Out& c, int W, int N, int N4, int nv, int n0, int Nc, const
                cplx* kl, int nup, cudaStream_t st) {
   const size_t sm = sizeof(cplx) * N * (N | 1);
   if (N > kExxMaxN) return record_error(SFQ_ERR_SHAPE, "crt exx: N=%d above %d", N, kExxMaxN);
-  SFQ_CUDA_TRY(cudaFuncSetAttribute(exx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  SFQ_MAX_SMEM(exx_kernel, sizeof(cplx) * kExxMaxN * (kExxMaxN | 1));
   exx_kernel<<<dim3(nv, W), 256, sm, st>>>(c.q, c.ldc, c.plane, (long)W * N, N, N4, eA, eB, n0, Nc, exxn, kl,
                                            nup < 0 ? N : nup, scale_of(1.0));
   SFQ_LAUNCHED();

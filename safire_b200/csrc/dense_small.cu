@@ -308,10 +308,10 @@ int lu_logdet(cplx* T, long sT, int nbatch, int N, cplx* ovlp, bool accumulate, 
   if (N <= kGjMaxLarge) return gj_logdet(T, sT, nbatch, N, ovlp, accumulate, post_scale, invert, st);
   const size_t sm = lu_smem_bytes(N);
   if (invert) {
-    SFQ_CUDA_TRY(cudaFuncSetAttribute(lu_logdet_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    SFQ_MAX_SMEM(lu_logdet_kernel<true>, lu_smem_bytes(kMaxSmallN));
     lu_logdet_kernel<true><<<nbatch, LU_THREADS, sm, st>>>(T, sT, N, ovlp, accumulate ? 1 : 0, post_scale);
   } else {
-    SFQ_CUDA_TRY(cudaFuncSetAttribute(lu_logdet_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    SFQ_MAX_SMEM(lu_logdet_kernel<false>, lu_smem_bytes(kMaxSmallN));
     lu_logdet_kernel<false><<<nbatch, LU_THREADS, sm, st>>>(T, sT, N, ovlp, accumulate ? 1 : 0, post_scale);
   }
   SFQ_LAUNCHED();
@@ -322,8 +322,9 @@ int chol_rinv(cplx* S, long sS, int nbatch, int N, int* status, int* again, cons
               cudaStream_t st, cplx* Rout) {
   if (nbatch <= 0 || N <= 0) return SFQ_OK;
   if (N > kMaxSmallN) return record_error(SFQ_ERR_UNSUPPORTED, "chol_rinv: N=%d exceeds %d", N, kMaxSmallN);
-  const size_t sm = size_t(N) * (N + 1) / 2 * sizeof(cplx) + size_t(N) * sizeof(cplx);  // packed R + work
-  SFQ_CUDA_TRY(cudaFuncSetAttribute(chol_rinv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+  auto smem = [](int n) { return size_t(n) * (n + 1) / 2 * sizeof(cplx) + size_t(n) * sizeof(cplx); };  // packed R + work
+  const size_t sm = smem(N);
+  SFQ_MAX_SMEM(chol_rinv_kernel, smem(kMaxSmallN));
   chol_rinv_kernel<<<nbatch, LU_THREADS, sm, st>>>(S, sS, N, status, again, active, kappa_max, Rout);
   SFQ_LAUNCHED();
   return SFQ_OK;

@@ -650,11 +650,12 @@ int islice_build_v(const float* Cv, int W, int M, bool packed, int nslices, int8
     // mirrored columns' stores spread over 8 banks)
     const int l4 = (M + 3) / 4;
     const int lds = 4 * (l4 | 1);
-    int rs = int((200L * 1024) / (2L * lds * sizeof(float)));
+    constexpr long kStrip = 200L * 1024;
+    int rs = int(kStrip / (2L * lds * sizeof(float)));
     if (rs > 32) rs = 32;
     if (rs < 1) return record_error(SFQ_ERR_SHAPE, "islice_build_v: nmo %d too large for a strip", M);
     const size_t smem = 2 * sizeof(float) * (size_t)rs * lds;
-    SFQ_CUDA_TRY(cudaFuncSetAttribute(v_strip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    SFQ_MAX_SMEM(v_strip_kernel, kStrip);
     v_strip_kernel<<<dim3(unsigned((M + rs - 1) / rs), unsigned(W)), 512, smem, st>>>(Cv, W, M, rs, lds, nslices,
                                                                                        qptrs(q), ld, e);
     SFQ_LAUNCHED();

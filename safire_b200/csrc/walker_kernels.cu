@@ -674,7 +674,7 @@ int energy_exx_reduce(const cplx* T, int nwalk, int nel, int nv, int n0, int nch
   dim3 grid(nv, nwalk);
   const size_t sm = exx_smem<cplx>(nel);
   if (sm <= kExxSmem) {
-    SFQ_CUDA_TRY(cudaFuncSetAttribute(energy_exx_sm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    SFQ_MAX_SMEM(energy_exx_sm_kernel, kExxSmem);
     energy_exx_sm_kernel<<<grid, RT, sm, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, only_if);
   } else {
     energy_exx_kernel<<<grid, RT, 0, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, only_if);
@@ -689,7 +689,7 @@ int energy_exx_reduce_f32(const float* C, int nwalk, int nel, int nv, int n0, in
   dim3 grid(nv, nwalk);
   const size_t sm = exx_smem<float2>(nel);
   if (sm <= kExxSmem) {
-    SFQ_CUDA_TRY(cudaFuncSetAttribute(energy_exx_f32_sm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sm)));
+    SFQ_MAX_SMEM(energy_exx_f32_sm_kernel, kExxSmem);
     energy_exx_f32_sm_kernel<<<grid, RT, sm, st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
   } else {
     energy_exx_f32_kernel<<<grid, RT, 0, st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
