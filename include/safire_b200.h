@@ -221,6 +221,14 @@ int sfq_gemm_int8_slices(const double* A, const double* B, float* C, int M, int 
  * sfq_vhs_ws; operands it cannot hold (an Inf, a NaN, a row norm outside 1e+-120) go through the FP64
  * tensor pipe instead.  M <= 65535, K <= 90000. */
 int sfq_gemm_f64_modular(const double* A, const double* B, double* C, int M, int N, int K, void* stream);
+/* launches of those products on the current device, since the process began, in which a bounded wait expired: the
+ * call's result was then computed on the FP64 tensor pipe, right but late.  Waits for the device. */
+int sfq_modular_expiries(unsigned long long* n);
+/* self-test of those products' bounded waits: C = A B^T (M even; walker != 0: by the per-walker kernel, K <= 4096)
+ * whose loads stop before their hold_at-th K slice, each wait limited to wait_ns (1 ns .. 1 s).  Returns
+ * SFQ_ERR_TIMEOUT, with C computed on the FP64 tensor pipe; SFQ_OK where there were no more than hold_at slices. */
+int sfq_selftest_modular_expiry(const double* A, const double* B, double* C, int M, int N, int K, int walker,
+                                int hold_at, unsigned long long wait_ns, void* stream);
 /* the Taylor term's product in the same arithmetic (the int8 slices'): C[c][w][a][j] = part c of sum_i A[w][a][i] V[w][j][i]
  * (A (W, N, M), V (W, M, M) complex doubles, taken through FP32 as the engine holds them; C planar
  * FP32 (2, W, N, M)); half: 32, 64 or 80 orbitals per tile. */

@@ -107,6 +107,8 @@ _SIGS = {
                               ctypes.c_long, ctypes.c_float, ctypes.c_float, _I, _VP], _I),
     "sfq_split_bf16": ([_VP, ctypes.c_long, _VP, _VP, _VP, _VP], _I),
     "sfq_gemm_f64_modular": ([_VP, _VP, _VP, _I, _I, _I, _VP], _I),
+    "sfq_modular_expiries": ([ctypes.POINTER(_U64)], _I),
+    "sfq_selftest_modular_expiry": ([_VP, _VP, _VP, _I, _I, _I, _I, _I, _U64, _VP], _I),
     "sfq_gemm_int8_slices": ([_VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP], _I),
     "sfq_engine_copy_walker": ([_VP, _I, _I], _I),
     "sfq_engine_walker_row_elems": ([_VP], ctypes.c_long),

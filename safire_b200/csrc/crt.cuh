@@ -112,6 +112,9 @@ struct Gemm {
   uint8_t* C = nullptr;
   long ldc = 0, c_plane = 0;
   int* flag = nullptr;  // set when a bounded wait expires
+  unsigned long long wait_ns = 0;  // limit of one wait without progress (0: 2 s)
+  const int* hold = nullptr;       // self-test: loads from the hold_at-th K slice on wait for *hold
+  unsigned hold_at = 0;
 };
 int gemm(const Gemm& g, cudaStream_t st);
 
@@ -125,9 +128,14 @@ struct WalkerGemm {
   uint8_t* C = nullptr;
   long ldc = 0, c_plane = 0, c_part = 0;
   int* flag = nullptr;
+  unsigned long long wait_ns = 0;  // as in Gemm
+  const int* hold = nullptr;
+  unsigned hold_at = 0;
 };
 bool walker_gemm_fits(int N, int cols, int K, int segs);
 int walker_gemm(const WalkerGemm& g, cudaStream_t st);
+// launches on this device since the process began in which a bounded wait expired
+int expiries(unsigned long long* n);
 
 // the output of a product: NMOD planes of rows x ldc bytes
 struct Out {

@@ -27,6 +27,24 @@ constexpr int BAR_OFF = STAGES * STAGE;
 constexpr int SMEM = BAR_OFF + (2 * STAGES + 5) * 8 + 16 + 1024;
 static_assert(SMEM <= 232448, "shared memory budget");
 constexpr unsigned long long kWaitNs = 2000000000ull;  // limit of one wait: 2 s without progress
+__device__ unsigned long long g_expiries;               // launches in which a bounded wait expired
+
+// A launch gave up: the call's flag (its FP64 product then replaces the result) and one count for the launch
+__device__ __forceinline__ void report_expiry(int* flag) {
+  if (!flag || atomicExch(flag, 1) == 0) atomicAdd(&g_expiries, 1ull);
+}
+// the self-test's hold: before its at-th slice the producer waits for *hold, which nothing sets
+__device__ __forceinline__ bool held_back(const int* hold, uint32_t at, uint32_t it, unsigned long long limit_ns,
+                                          volatile int* abort) {
+  if (!hold || it != at) return false;
+  const unsigned long long deadline = gtimer() + limit_ns;
+  while (*reinterpret_cast<const volatile int*>(hold) == 0)
+    if (gtimer() > deadline) {
+      *abort = 1;
+      return true;
+    }
+  return false;
+}
 
 struct Maps {
   CUtensorMap a, b;
@@ -40,6 +58,9 @@ struct KP {
   long ldc, c_plane;
   int wide;        // reduce_kind of the K sums
   int* flag;
+  unsigned long long wait_ns;
+  const int* hold;
+  uint32_t hold_at;
 };
 
 __device__ __forceinline__ uint32_t idesc_i8(uint32_t n) {
@@ -229,7 +250,8 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
           const int rb = int(k.b_off[sg] + c.b * k.b_bs) + c.nt * k.bn;
           for (int kt = 0; kt < k.KT; ++kt, ++it) {
             const int s = int(it % STAGES);
-            if (!mbar_wait_abort(&empty[s], ((it / STAGES) & 1) ^ 1, kWaitNs, s_abort)) {
+            if (held_back(k.hold, k.hold_at, it, k.wait_ns, s_abort) ||
+                !mbar_wait_abort(&empty[s], ((it / STAGES) & 1) ^ 1, k.wait_ns, s_abort)) {
               stop = true;
               break;
             }
@@ -258,12 +280,12 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
       bool stop = false;
       for (long t = blockIdx.x; t < k.tiles && !stop; t += gridDim.x, ++n) {
         const uint32_t b = n & 1;
-        if (!mbar_wait_abort(&acc_empty[b], ((n >> 1) & 1) ^ 1, kWaitNs, s_abort)) break;
+        if (!mbar_wait_abort(&acc_empty[b], ((n >> 1) & 1) ^ 1, k.wait_ns, s_abort)) break;
         fence_after();
         const uint32_t d = tmem + b * BN;
         int left = k.KT;
         for (int i = 0; i < slices; ++i) {
-          if (!mbar_wait_abort(&full[s], ph, kWaitNs, s_abort)) {
+          if (!mbar_wait_abort(&full[s], ph, k.wait_ns, s_abort)) {
             stop = true;
             break;
           }
@@ -295,7 +317,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
     uint32_t n = 0;
     for (long t = blockIdx.x; t < k.tiles; t += gridDim.x, ++n) {
       const uint32_t b = n & 1;
-      const bool ok = mbar_wait_for(&acc_full[b], (n >> 1) & 1, kWaitNs);
+      const bool ok = mbar_wait_for(&acc_full[b], (n >> 1) & 1, k.wait_ns);
       const bool go = __all_sync(0xffffffffu, ok) && !__any_sync(0xffffffffu, *s_abort != 0);
       if (!go) {
         *s_abort = 1;
@@ -321,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
   }
   fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *s_abort && k.flag) atomicExch(k.flag, 1);
+  if (threadIdx.x == 0 && *s_abort) report_expiry(k.flag);
   if (warp == 1) {
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -355,6 +377,9 @@ struct RKP {
   long ldc, c_plane, c_part;           // C row (c, w, a): c * c_part + w N + a
   int wide;
   int* flag;
+  unsigned long long wait_ns;
+  const int* hold;
+  uint32_t hold_at;
 };
 struct RUnit {
   int p, w, e0, t0, t1;
@@ -432,6 +457,8 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
     if (lane == 0) {  // TMA producer
       uint32_t it = 0, un = 0, s = 0, ph = 0;
       const uint32_t nst = uint32_t(k.stages);
+      uint32_t rows_un = 0;  // units whose rows were all issued, and the slices issued of the next one's
+      int rows_kt = 0;
       bool stop = false;
       for (long u = blockIdx.x; u < k.units && !stop; u += gridDim.x, ++un) {
         const RUnit c = unit_of(k, u);
@@ -440,8 +467,12 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
           const uint32_t bytes = uint32_t(k.segs * (last ? k.bn_last : k.bn) * RBK);
           const int rb = int(c.w * k.b_bs) + t * k.bn;
           for (int kt = 0; kt < k.KT; ++kt, ++it) {
+            if (held_back(k.hold, k.hold_at, it, k.wait_ns, s_abort)) {
+              stop = true;
+              break;
+            }
             if (t == c.t0) {  // the unit's own rows, slice by slice as the last unit's are done with
-              if (!mbar_wait_abort(&rempty[kt], (un & 1) ^ 1, kWaitNs, s_abort)) {
+              if (!mbar_wait_abort(&rempty[kt], (un & 1) ^ 1, k.wait_ns, s_abort)) {
                 stop = true;
                 break;
               }
@@ -453,8 +484,13 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
                 tma_load_3d(dst + j * blk_bytes, &maps.a, &rfull[kt], kt * RBK,
                             int(blk * k.a_blk) + c.w * k.N + c.e0, c.p);
               }
+              rows_kt = kt + 1;
+              if (rows_kt == k.KT) {
+                rows_kt = 0;
+                ++rows_un;
+              }
             }
-            if (!mbar_wait_abort(&empty[s], ph ^ 1, kWaitNs, s_abort)) {
+            if (!mbar_wait_abort(&empty[s], ph ^ 1, k.wait_ns, s_abort)) {
               stop = true;
               break;
             }
@@ -473,8 +509,10 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
       // every issued copy must have landed before the CTA may exit
       for (uint32_t j = (it > uint32_t(k.stages) ? it - k.stages : 0u); j < it; ++j)
         mbar_wait_for(&full[j % k.stages], (j / k.stages) & 1, kWaitNs);
-      if (stop) {  // a unit's rows may be on their way without their stage having been issued
-        for (int kt = 0; kt < k.KT; ++kt) mbar_wait_for(&rfull[kt], (un + 1) & 1, 1000000ull);
+      // (a slice of rows that an MMA took has landed; one issued by a unit that was given up may not have)
+      for (int kt = 0; kt < k.KT; ++kt) {
+        const uint32_t issued = rows_un + (kt < rows_kt ? 1u : 0u);
+        if (issued) mbar_wait_for(&rfull[kt], (issued - 1) & 1, kWaitNs);
       }
     }
   } else if (warp == 1) {
@@ -494,7 +532,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
         const RUnit c = unit_of(k, u);
         for (int t = c.t0; t < c.t1; ++t, ++n) {
           const uint32_t b = n & 1;
-          if (!mbar_wait_abort(&acc_empty[b], ((n >> 1) & 1) ^ 1, kWaitNs, s_abort)) {
+          if (!mbar_wait_abort(&acc_empty[b], ((n >> 1) & 1) ^ 1, k.wait_ns, s_abort)) {
             stop = true;
             break;
           }
@@ -503,7 +541,8 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
           const uint32_t idesc = t == k.NT - 1 ? id_last : id_full;
           const bool first = t == c.t0, last = t == c.t1 - 1;
           for (int kt = 0; kt < k.KT; ++kt) {
-            if ((first && !mbar_wait_abort(&rfull[kt], un & 1, kWaitNs, s_abort)) || !mbar_wait_abort(&full[s], ph, kWaitNs, s_abort)) {
+            if ((first && !mbar_wait_abort(&rfull[kt], un & 1, k.wait_ns, s_abort)) ||
+                !mbar_wait_abort(&full[s], ph, k.wait_ns, s_abort)) {
               stop = true;
               break;
             }
@@ -555,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
       const int nrow = rg < 2 * k.Np ? k.N - c.e0 - ag : 0;  // rows of the group that exist (4 or more: all)
       for (int t = c.t0; t < c.t1; ++t, ++n) {
         const uint32_t b = n & 1;
-        const bool ok = mbar_wait_for(&acc_full[b], (n >> 1) & 1, kWaitNs);
+        const bool ok = mbar_wait_for(&acc_full[b], (n >> 1) & 1, k.wait_ns);
         const bool go = __all_sync(0xffffffffu, ok) && !__any_sync(0xffffffffu, *s_abort != 0);
         if (!go) {
           *s_abort = 1;
@@ -579,7 +618,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
   }
   fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *s_abort && k.flag) atomicExch(k.flag, 1);
+  if (threadIdx.x == 0 && *s_abort) report_expiry(k.flag);
   if (warp == 1) {
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -635,6 +674,8 @@ int gemm(const Gemm& g, cudaStream_t st) {
   k.C = g.C; k.ldc = g.ldc; k.c_plane = g.c_plane;
   k.wide = reduce_kind((long)g.K * g.segs);
   k.flag = g.flag;
+  k.wait_ns = g.wait_ns ? g.wait_ns : kWaitNs;
+  k.hold = g.hold; k.hold_at = g.hold_at;
   Maps maps;
   int rc;
   if ((rc = make_map(&maps.a, g.A, g.K, BM)) || (rc = make_map(&maps.b, g.B, g.K, k.bn))) return rc;
@@ -681,6 +722,8 @@ bool plan_walker(const WalkerGemm& g, RKP* out) {
   k.C = g.C; k.ldc = g.ldc; k.c_plane = g.c_plane; k.c_part = g.c_part;
   k.wide = reduce_kind((long)g.K * g.segs);
   k.flag = g.flag;
+  k.wait_ns = g.wait_ns ? g.wait_ns : kWaitNs;
+  k.hold = g.hold; k.hold_at = g.hold_at;
   *out = k;
   return true;
 }
@@ -718,6 +761,11 @@ int walker_gemm(const WalkerGemm& g, cudaStream_t st) {
   const long grid = k.units < sm_count() ? k.units : sm_count();
   kern<<<unsigned(grid), kThreads, smem, st>>>(maps, k);
   SFQ_LAUNCHED();
+  return SFQ_OK;
+}
+
+int expiries(unsigned long long* n) {
+  SFQ_CUDA_TRY(cudaMemcpyFromSymbol(n, g_expiries, sizeof(*n)));
   return SFQ_OK;
 }
 

@@ -271,30 +271,37 @@ int energy_crt(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool 
 }  // namespace ops
 }  // namespace sfq
 
-extern "C" int sfq_gemm_f64_modular(const double* A, const double* B, double* C, int M, int N, int K, void* stream) {
-  using namespace sfq;
-  if (M < 0 || N < 0 || K < 0) return record_error(SFQ_ERR_SHAPE, "negative size");
-  if (!M || !N) return SFQ_OK;
-  if (!A || !B || !C) return record_error(SFQ_ERR_ARG, "null pointer");
-  if (K < 1 || K > crt::kMaxK || M > 65535)
-    return record_error(SFQ_ERR_SHAPE, "gemm_f64_modular: 1 <= K <= %ld, M <= 65535", crt::kMaxK);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
+namespace sfq {
+namespace {
+// C = A B^T by either kernel; the self-test's limit and hold, and whether a wait expired
+int modular_product(const double* A, const double* B, double* C, int M, int N, int K, bool walker, cudaStream_t st,
+                    unsigned long long wait_ns = 0, int hold_at = -1, int* expired = nullptr) {
   char* ws = nullptr;
   const size_t bytes = 256 + crt::planes_bytes(M, K) + crt::exps_bytes(M) + crt::planes_bytes(N, K) +
                        crt::exps_bytes(N) + crt::out_bytes(M, N);
   SFQ_CUDA_TRY(cudaMallocAsync((void**)&ws, bytes, st));
-  int* flag = reinterpret_cast<int*>(ws);
+  int* flag = reinterpret_cast<int*>(ws);  // [0] the call's flag, [1] the hold (0)
   char* at = ws + 256;
   const crt::Planes a = crt::lay_out(at, M, K, M), b = crt::lay_out(at, N, K, N);
   const crt::Out c = crt::lay_out_c(at, M, N);
+  const int* hold = hold_at < 0 ? nullptr : flag + 1;
   int rc = SFQ_OK;
-  const cudaError_t ce = cudaMemsetAsync(flag, 0, sizeof(int), st);
+  cudaError_t ce = cudaMemsetAsync(flag, 0, 2 * sizeof(int), st);
   if (ce != cudaSuccess) rc = record_cuda(ce, "gemm_f64_modular", __FILE__, __LINE__);
-  crt::Gemm g;
-  g.A = a; g.B = b; g.M = M; g.N = N; g.K = K; g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.flag = flag;
   if (!rc) rc = crt::rows_real(A, M, K, K, a, flag, st);
   if (!rc) rc = crt::rows_real(B, N, K, K, b, flag, st);
-  if (!rc) rc = crt::gemm(g, st);
+  if (!rc && walker) {  // the rows as the [re; im] of one walker
+    crt::WalkerGemm g;
+    g.A = a; g.B = b; g.N = M / 2; g.cols = N; g.K = K; g.a_blk = M / 2;
+    g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.c_part = M / 2; g.flag = flag;
+    g.wait_ns = wait_ns; g.hold = hold; g.hold_at = unsigned(hold_at);
+    rc = crt::walker_gemm(g, st);
+  } else if (!rc) {
+    crt::Gemm g;
+    g.A = a; g.B = b; g.M = M; g.N = N; g.K = K; g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.flag = flag;
+    g.wait_ns = wait_ns; g.hold = hold; g.hold_at = unsigned(hold_at);
+    rc = crt::gemm(g, st);
+  }
   if (!rc) rc = crt::out_real(c, M, N, a.e, b.e, 1.0, C, N, nullptr, st);
   if (!rc) {
     GemmDesc d;
@@ -305,6 +312,42 @@ extern "C" int sfq_gemm_f64_modular(const double* A, const double* B, double* C,
     d.only_if = flag;
     rc = gemm_f64(d, st);
   }
+  if (!rc && expired) {
+    ce = cudaMemcpyAsync(expired, flag, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+    if (ce != cudaSuccess) rc = record_cuda(ce, "gemm_f64_modular", __FILE__, __LINE__);
+  }
   cudaFreeAsync(ws, st);
   return rc;
+}
+}  // namespace
+}  // namespace sfq
+
+extern "C" int sfq_gemm_f64_modular(const double* A, const double* B, double* C, int M, int N, int K, void* stream) {
+  using namespace sfq;
+  if (M < 0 || N < 0 || K < 0) return record_error(SFQ_ERR_SHAPE, "negative size");
+  if (!M || !N) return SFQ_OK;
+  if (!A || !B || !C) return record_error(SFQ_ERR_ARG, "null pointer");
+  if (K < 1 || K > crt::kMaxK || M > 65535)
+    return record_error(SFQ_ERR_SHAPE, "gemm_f64_modular: 1 <= K <= %ld, M <= 65535", crt::kMaxK);
+  return modular_product(A, B, C, M, N, K, false, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int sfq_selftest_modular_expiry(const double* A, const double* B, double* C, int M, int N, int K, int walker,
+                                           int hold_at, unsigned long long wait_ns, void* stream) {
+  using namespace sfq;
+  if (wait_ns == 0 || wait_ns > 1000000000ull) return record_error(SFQ_ERR_ARG, "selftest: wait of 1 ns .. 1 s");
+  if (M < 2 || M > 65534 || M % 2 || N < 1 || K < 1 || K > 4096 || hold_at < 0)
+    return record_error(SFQ_ERR_SHAPE, "selftest: M even, K <= 4096");
+  if (!A || !B || !C) return record_error(SFQ_ERR_ARG, "null pointer");
+  int expired = 0;
+  const int rc = modular_product(A, B, C, M, N, K, walker != 0, static_cast<cudaStream_t>(stream), wait_ns, hold_at,
+                                 &expired);
+  return rc ? rc : expired ? SFQ_ERR_TIMEOUT : SFQ_OK;
+}
+
+extern "C" int sfq_modular_expiries(unsigned long long* n) {
+  using namespace sfq;
+  if (!n) return record_error(SFQ_ERR_ARG, "null pointer");
+  return crt::expiries(n);
 }

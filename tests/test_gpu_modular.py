@@ -185,3 +185,32 @@ def test_energy(W, M, N, Nc, cplx):
     L[5, 2, 3] = float("nan")  # the FP64 tensor pipe's sums
     bad = afqmc.energy(G, haj, L, E0=0.25)
     assert torch.isnan(bad[:, 1].real).all() and float((bad[:, 0] - R[:, 0]).abs().max()) < 1e-9
+
+
+# the loads stop before the first slice, within the first tile (or unit) and, in the walker kernel, after a tile
+# whose rows stay; K = 300 has three 128-byte slices a tile and five 64-byte ones
+@pytest.mark.parametrize("walker,hold_at,N", [(0, 0, 600), (0, 2, 600), (1, 0, 600), (1, 3, 600), (1, 5, 12000),
+                                              (1, 7, 12000)])  # 12000: two column tiles a unit
+def test_bounded_waits_expire(walker, hold_at, N):
+    """Every wait limited to 1 ms: the kernel gives up with nothing in flight, the expiry is counted, the FP64
+    product replaces the result, and the next product on the same context is right."""
+    from safire_b200.capi import check, lib, ptr
+    g = torch.Generator(device="cuda").manual_seed(hold_at)
+    M, K = 64, 300
+    A, B = _rn(g, M, K), _rn(g, N, K)
+    R = A @ B.T
+    n0, n1 = ctypes.c_ulonglong(), ctypes.c_ulonglong()
+    check(lib().sfq_modular_expiries(ctypes.byref(n0)))
+    C = torch.full((M, N), float("nan"), dtype=torch.float64, device="cuda")
+    assert lib().sfq_selftest_modular_expiry(ptr(A), ptr(B), ptr(C), M, N, K, walker, hold_at, 1_000_000,
+                                             _stream()) == 8  # SFQ_ERR_TIMEOUT
+    check(lib().sfq_modular_expiries(ctypes.byref(n1)))
+    assert n1.value == n0.value + 1
+    # two FP64 sums of K terms
+    bound = 2 * K * 2.0 ** -53 * (A.abs() @ B.abs().T)
+    assert ((C - R).abs() <= bound).all()
+    C.fill_(float("nan"))
+    assert lib().sfq_selftest_modular_expiry(ptr(A), ptr(B), ptr(C), M, N, K, walker, 10**6, 1_000_000_000,
+                                             _stream()) == 0
+    assert ((C - R).abs() <= bound).all()
+    assert ((_modular(A, B) - R).abs() <= bound).all()
