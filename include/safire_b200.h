@@ -221,7 +221,7 @@ int sfq_gemm_int8_slices(const double* A, const double* B, float* C, int M, int 
  * sfq_vhs_ws; operands it cannot hold (an Inf, a NaN, a row norm outside 1e+-120) go through the FP64
  * tensor pipe instead.  M <= 65535, K <= 90000. */
 int sfq_gemm_f64_modular(const double* A, const double* B, double* C, int M, int N, int K, void* stream);
-/* launches of those products on the current device, since the process began, in which a bounded wait expired: the
+/* calls on the current device, since the process began, in which a bounded wait of such a product expired: the
  * call's result was then computed on the FP64 tensor pipe, right but late.  Waits for the device. */
 int sfq_modular_expiries(unsigned long long* n);
 /* self-test of those products' bounded waits: C = A B^T (M even; walker != 0: by the per-walker kernel, K <= 4096)

@@ -65,6 +65,13 @@ int record_error(int code, const char* fmt, ...);
 #define SFQ_MAX_SMEM(kernel, bytes) \
   SFQ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)))
 
+// What a modular product (crt.cuh) could not hold and asks of the FP64 kernels launched behind it, in device memory:
+// call[0] (an operand that all walkers share) or call[1] (an expired wait): the whole call, row[w]: walker w
+struct Redo {
+  int* call = nullptr;
+  int* row = nullptr;
+};
+
 inline int ceil_div(long a, long b) { return int((a + b - 1) / b); }
 
 }  // namespace sfq

@@ -10,9 +10,9 @@
 // row's norm, and of the result to FP64: with K random terms the relative error of a result is
 // about 2^-58 sqrt(K), against 2^-55 sqrt(K) of an FP64 chain of K additions.
 //
-// Rows that the scheme cannot hold (an Inf or a NaN, a norm outside 1e+-120) raise a flag in
-// device memory; the FP64 tensor-pipe product (gemm_f64), launched behind it with
-// GemmDesc::only_if, then computes the result.
+// Rows that the scheme cannot hold (an Inf or a NaN, a norm outside 1e+-120) raise a flag in device memory, their
+// walker's or, for an operand that all walkers share, the call's (Redo); the FP64 tensor-pipe product (gemm_f64),
+// launched behind it, then computes what the flags ask for and leaves the other walkers' results as they are.
 #pragma once
 #include "common.cuh"
 
@@ -99,6 +99,16 @@ inline Planes lay_out(char*& at, long rows, long K, long e_rows) {
   return p;
 }
 
+// the flags of a call over W walkers, at *at, which advances
+inline size_t flag_bytes(long W) { return 256 + align256(sizeof(int) * (size_t)W); }
+inline Redo lay_out_flags(char*& at, long W) {
+  Redo r;
+  r.call = reinterpret_cast<int*>(at);
+  r.row = reinterpret_cast<int*>(at + 256);
+  at += flag_bytes(W);
+  return r;
+}
+
 // ---- the product of residues: C_i = A_i B_i^T mod p_i for every modulus ------------------------
 // Output row ((part * batch + b) * M + m), column n, at C + i * c_plane + row * ldc + n (bytes).
 // A rows a_off[part][seg] + b * a_bs + m, B rows b_off[seg] + b * b_bs + n, summed over the segments
@@ -111,7 +121,7 @@ struct Gemm {
   long b_off[2] = {0, 0};
   uint8_t* C = nullptr;
   long ldc = 0, c_plane = 0;
-  int* flag = nullptr;  // set when a bounded wait expires
+  int* expired = nullptr;          // set when a bounded wait expires
   unsigned long long wait_ns = 0;  // limit of one wait without progress (0: 2 s)
   const int* hold = nullptr;       // self-test: loads from the hold_at-th K slice on wait for *hold
   unsigned hold_at = 0;
@@ -127,14 +137,14 @@ struct WalkerGemm {
   long a_blk = 0, b_bs = 0, b_off1 = 0;
   uint8_t* C = nullptr;
   long ldc = 0, c_plane = 0, c_part = 0;
-  int* flag = nullptr;
+  int* expired = nullptr;
   unsigned long long wait_ns = 0;  // as in Gemm
   const int* hold = nullptr;
   unsigned hold_at = 0;
 };
 bool walker_gemm_fits(int N, int cols, int K, int segs);
 int walker_gemm(const WalkerGemm& g, cudaStream_t st);
-// launches on this device since the process began in which a bounded wait expired
+// calls on this device since the process began in which a bounded wait expired
 int expiries(unsigned long long* n);
 
 // the output of a product: NMOD planes of rows x ldc bytes
@@ -154,16 +164,18 @@ inline Out lay_out_c(char*& at, long rows, long N) {
 }
 
 // ---- operands to residues -----------------------------------------------------------------------
+// A row that cannot be held raises redo.call[0] (per_walker 0: the operand is all walkers') or the flag of
+// walker r / per_walker.
 // real rows (row r of `rows` at src + r * stride, K doubles) -> planes row (r / inner) * outer + r % inner
 // (inner 0: row r), exponent e[r]
-int rows_real(const double* src, long rows, long K, long stride, const Planes& out, int* flag, cudaStream_t st,
-              long inner = 0, long outer = 0);
+int rows_real(const double* src, long rows, long K, long stride, const Planes& out, Redo redo, long per_walker,
+              cudaStream_t st, long inner = 0, long outer = 0);
 // complex rows (K complex each) -> blocks re, im (nb = 2) or re, im, -im (nb = 3): row r's block k at
 // plane row k * blk_stride + (r / inner) * outer + r % inner, one exponent per complex row (e[r])
 int rows_cplx(const cplx* src, long rows, long K, long stride, int nb, long blk_stride, long inner, long outer,
-              const Planes& out, int* flag, cudaStream_t st);
-// walkers (W, M, N) complex -> rows (w, a) over the M orbitals, blocks re, im: plane row k * W N + w N + a
-int walkers_in(const cplx* SM, int W, int M, int N, const Planes& out, int* flag, cudaStream_t st);
+              const Planes& out, Redo redo, long per_walker, cudaStream_t st);
+// walkers (W npol, M, N) complex -> rows (w, q, a) over the M orbitals, blocks re, im: plane row k * W npol N + (w npol + q) N + a
+int walkers_in(const cplx* SM, int W, int npol, int M, int N, const Planes& out, Redo redo, cudaStream_t st);
 
 // alpha P 2^-64 as a sum of two doubles, so that values are rounded twice (as integers, as products) and not
 // pulled by a rounded constant as well
@@ -175,20 +187,20 @@ Scale scale_of(double alpha);
 // ---- residues to FP64 ---------------------------------------------------------------------------
 // out[m][n] = alpha (C_re + i C_im) for parts = 2 products with M rows; exponents eA[m], eB[n]
 int out_cplx(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, cplx* out, long ldo,
-             const int* skip_if, cudaStream_t st);
+             cudaStream_t st);
 int out_real(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, double* out, long ldo,
-             const int* skip_if, cudaStream_t st);
+             cudaStream_t st);
 // one Taylor term: T = (i / k) C (k = 0: T = C), S (2, W, N, M) += T (k = 0: S = T), and the residues of T,
 // blocks re, im, -im (last: of S, blocks re, im) -> `next`.  C rows (part, w, a), columns j.
 int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int* eA, const int* eB, int eB_per_w,
-                  double* S, const Planes& next, int* flag, cudaStream_t st);
+                  double* S, const Planes& next, Redo redo, cudaStream_t st);
 // exx[w, n0 + n] = sum_ab T[w,a,n,b] T[w,b,n,a] and kl[w, n0 + n] = sum_a T[w,a,n,a] of T[w,b,n,a] = rows
 // (part, w, b), columns n * N4 + a (exponents eB[n * N + a]); nup as in energy_exx_reduce
 constexpr int kExxMaxN = 116;  // a walker's N x N block of one n in shared memory
 int exx_reduce(const Out& c, int W, int N, int N4, int nv, int n0, int Nc, const int* eA, const int* eB, cplx* exxn,
                cplx* kl, int nup, cudaStream_t st);
-// SM[w][j][a] = C_re + i C_im of rows (part, w, a), columns j
-int walkers_out(const Out& c, int W, int M, int N, const int* eA, const int* eB, cplx* SM, const int* skip_if,
+// SM[w][q][j][a] = C_re + i C_im of rows (part, w, q, a), columns j; not of the walkers that redo asks for
+int walkers_out(const Out& c, int W, int npol, int M, int N, const int* eA, const int* eB, cplx* SM, Redo redo,
                 cudaStream_t st);
 
 }  // namespace crt

@@ -12,8 +12,17 @@ __device__ __forceinline__ double pow2(int e) {
   return __longlong_as_double((long long)((e < -1022 ? -1022 : e > 1023 ? 1023 : e) + 1023) << 52);
 }
 
+// the flag of row r (see rows_real)
+__device__ __forceinline__ int* flag_of(const Redo& redo, long r, long per_walker) {
+  return per_walker ? redo.row + r / per_walker : redo.call;
+}
+__device__ __forceinline__ bool asked_again(const Redo& redo, long w) {
+  return redo.call[0] || redo.call[1] || redo.row[w];
+}
+
 // the scale exponent of a row with squared norm n2: |row| 2^-e < 2^kNormBits.  Rows that cannot be held
-// (not finite, or a norm outside 1e+-120, beyond which two rows' scales could leave the exponent range) raise *flag.
+// (not finite, or a norm outside 1e+-120, beyond which two rows' scales could leave the exponent range) raise *flag
+// where there is one.
 __device__ __forceinline__ int row_exponent(double n2, bool any, int* flag) {
   if (!any && n2 == 0.0) return 0;
   if (!(n2 > 1e-240 && n2 < 1e240)) {

@@ -27,11 +27,11 @@ constexpr int BAR_OFF = STAGES * STAGE;
 constexpr int SMEM = BAR_OFF + (2 * STAGES + 5) * 8 + 16 + 1024;
 static_assert(SMEM <= 232448, "shared memory budget");
 constexpr unsigned long long kWaitNs = 2000000000ull;  // limit of one wait: 2 s without progress
-__device__ unsigned long long g_expiries;               // launches in which a bounded wait expired
+__device__ unsigned long long g_expiries;               // calls in which a bounded wait expired
 
-// A launch gave up: the call's flag (its FP64 product then replaces the result) and one count for the launch
-__device__ __forceinline__ void report_expiry(int* flag) {
-  if (!flag || atomicExch(flag, 1) == 0) atomicAdd(&g_expiries, 1ull);
+// A launch gave up: the call's flag (its FP64 product then replaces the result) and one count for the call
+__device__ __forceinline__ void report_expiry(int* expired) {
+  if (!expired || atomicExch(expired, 1) == 0) atomicAdd(&g_expiries, 1ull);
 }
 // the self-test's hold: before its at-th slice the producer waits for *hold, which nothing sets
 __device__ __forceinline__ bool held_back(const int* hold, uint32_t at, uint32_t it, unsigned long long limit_ns,
@@ -57,7 +57,7 @@ struct KP {
   uint8_t* C;
   long ldc, c_plane;
   int wide;        // reduce_kind of the K sums
-  int* flag;
+  int* expired;
   unsigned long long wait_ns;
   const int* hold;
   uint32_t hold_at;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
   }
   fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *s_abort) report_expiry(k.flag);
+  if (threadIdx.x == 0 && *s_abort) report_expiry(k.expired);
   if (warp == 1) {
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -376,7 +376,7 @@ struct RKP {
   uint8_t* C;
   long ldc, c_plane, c_part;           // C row (c, w, a): c * c_part + w N + a
   int wide;
-  int* flag;
+  int* expired;
   unsigned long long wait_ns;
   const int* hold;
   uint32_t hold_at;
@@ -618,7 +618,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
   }
   fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *s_abort) report_expiry(k.flag);
+  if (threadIdx.x == 0 && *s_abort) report_expiry(k.expired);
   if (warp == 1) {
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -673,7 +673,7 @@ int gemm(const Gemm& g, cudaStream_t st) {
   k.b_off[0] = g.b_off[0]; k.b_off[1] = g.b_off[1];
   k.C = g.C; k.ldc = g.ldc; k.c_plane = g.c_plane;
   k.wide = reduce_kind((long)g.K * g.segs);
-  k.flag = g.flag;
+  k.expired = g.expired;
   k.wait_ns = g.wait_ns ? g.wait_ns : kWaitNs;
   k.hold = g.hold; k.hold_at = g.hold_at;
   Maps maps;
@@ -721,7 +721,7 @@ bool plan_walker(const WalkerGemm& g, RKP* out) {
   k.a_blk = g.a_blk; k.b_bs = g.b_bs; k.b_off1 = g.b_off1;
   k.C = g.C; k.ldc = g.ldc; k.c_plane = g.c_plane; k.c_part = g.c_part;
   k.wide = reduce_kind((long)g.K * g.segs);
-  k.flag = g.flag;
+  k.expired = g.expired;
   k.wait_ns = g.wait_ns ? g.wait_ns : kWaitNs;
   k.hold = g.hold; k.hold_at = g.hold_at;
   *out = k;

@@ -39,8 +39,8 @@ __device__ __forceinline__ double row_sum(double v, double* sh) {
 // L2: a row is at most a few hundred KB).  One warp per row below 1024 elements, one block above.
 template <int TPR>
 __global__ void __launch_bounds__(256) rows_real_kernel(const double* src, long rows, long K, long stride, int8_t* q,
-                                                        long ld, long plane, int* e, int* flag, int vec, long inner,
-                                                        long outer) {
+                                                        long ld, long plane, int* e, Redo redo, long per_walker,
+                                                        int vec, long inner, long outer) {
   __shared__ double sh[8];
   const long r = TPR == 32 ? (long)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;
   const int t = TPR == 32 ? (threadIdx.x & 31) : threadIdx.x;
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256) rows_real_kernel(const double* src, long 
   n2 = row_sum<TPR>(n2, sh);
   // a row of zeros has the norm 0; one whose squares all vanish does not
   const bool any = TPR == 32 ? __any_sync(0xffffffffu, nz != 0.0) : __syncthreads_or(nz != 0.0) != 0;
-  const int ex = row_exponent(n2, any, t == 0 ? flag : nullptr);
+  const int ex = row_exponent(n2, any, t == 0 ? flag_of(redo, r, per_walker) : nullptr);
   if (t == 0) e[r] = ex;
   const double sc = pow2(-ex);
   int8_t* qr = q + (inner ? (r / inner) * outer + r % inner : r) * ld;
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) rows_real_kernel(const double* src, long 
 template <int TPR, int NB>
 __global__ void __launch_bounds__(256) rows_cplx_kernel(const cplx* src, long rows, long K, long stride,
                                                         long blk_stride, long inner, long outer, int8_t* q, long ld,
-                                                        long plane, int* e, int* flag) {
+                                                        long plane, int* e, Redo redo, long per_walker) {
   __shared__ double sh[8];
   const long r = TPR == 32 ? (long)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;
   const int t = TPR == 32 ? (threadIdx.x & 31) : threadIdx.x;
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(256) rows_cplx_kernel(const cplx* src, long ro
   }
   n2 = row_sum<TPR>(n2, sh);
   const bool any = TPR == 32 ? __any_sync(0xffffffffu, nz != 0.0) : __syncthreads_or(nz != 0.0) != 0;
-  const int ex = row_exponent(n2, any, t == 0 ? flag : nullptr);
+  const int ex = row_exponent(n2, any, t == 0 ? flag_of(redo, r, per_walker) : nullptr);
   if (t == 0) e[r] = ex;
   const double sc = pow2(-ex);
   int8_t* qr = q + ((r / inner) * outer + r % inner) * ld;
@@ -111,10 +111,10 @@ __global__ void __launch_bounds__(256) rows_cplx_kernel(const cplx* src, long ro
   }
 }
 
-// Walkers (W, M, N) -> rows (w, a) over the orbitals: a block takes 16 columns of one walker, their
+// Walkers' components (w, M, N), npol to a walker -> rows (w, a) over the orbitals: a block takes 16 columns of one, their
 // norms first, then 64 orbitals at a time through shared memory (the transpose).
-__global__ void __launch_bounds__(256) walkers_in_kernel(const cplx* SM, int W, int M, int N, int8_t* q, long ld,
-                                                         long plane, int* e, int* flag) {
+__global__ void __launch_bounds__(256) walkers_in_kernel(const cplx* SM, int W, int npol, int M, int N, int8_t* q,
+                                                         long ld, long plane, int* e, Redo redo) {
   __shared__ cplx tile[64][17];
   __shared__ double sh[16][17];
   __shared__ double scs[16];
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256) walkers_in_kernel(const cplx* SM, int W, 
     double s = 0.0;
 #pragma unroll
     for (int j = 0; j < 16; ++j) s += sh[j][ca];
-    const int ex = row_exponent(s, nz[ca] != 0, flag);
+    const int ex = row_exponent(s, nz[ca] != 0, redo.row + w / npol);
     e[(long)w * N + a0 + ca] = ex;
     scs[ca] = pow2(-ex);
   }
@@ -194,9 +194,8 @@ __device__ __forceinline__ void load_e4(const int* e, long n, long N, int eb[4])
 // its stores are whole 512-byte rows
 __global__ void __launch_bounds__(256) out_cplx_kernel(const uint8_t* c, long ldc, long plane, long M, long N,
                                                        const int* eA, const int* eB, Scale s, cplx* out,
-                                                       long ldo, const int* skip_if) {
+                                                       long ldo) {
   __shared__ cplx sh[8][130];
-  if (skip_if && *skip_if) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long m = blockIdx.y, nw = ((long)blockIdx.x * 8 + warp) * 128;
   if (nw >= N) return;
@@ -219,8 +218,7 @@ __global__ void __launch_bounds__(256) out_cplx_kernel(const uint8_t* c, long ld
 
 __global__ void __launch_bounds__(256) out_real_kernel(const uint8_t* c, long ldc, long plane, long M, long N,
                                                        const int* eA, const int* eB, Scale s, double* out,
-                                                       long ldo, const int* skip_if) {
-  if (skip_if && *skip_if) return;
+                                                       long ldo) {
   const long m = blockIdx.y, n = 4 * ((long)blockIdx.x * 256 + threadIdx.x);
   if (n >= N) return;
   int eb[4];
@@ -238,7 +236,7 @@ __global__ void __launch_bounds__(256) out_real_kernel(const uint8_t* c, long ld
 template <bool FIRST, bool LAST>
 __global__ void __launch_bounds__(256, 4) taylor_kernel(const uint8_t* c, long ldc, long plane, long WN, int N, int M,
                                                      Scale sc, const int* eA, const int* eB, int eB_per_w,
-                                                     double* S, int8_t* q, long ld, long qplane, int* e, int* flag,
+                                                     double* S, int8_t* q, long ld, long qplane, int* e, Redo redo,
                                                      int R) {
   extern __shared__ double rows[];  // [R][2][M4] T (S when LAST), then [R * M4 / 4] squared norms, [R] scales
   const int M4 = (M + 3) / 4 * 4, q4 = M4 / 4;
@@ -292,7 +290,7 @@ __global__ void __launch_bounds__(256, 4) taylor_kernel(const uint8_t* c, long l
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
     if ((threadIdx.x & 31) == 0) {
-      const int ex = row_exponent(n2, n2 != 0.0, flag);
+      const int ex = row_exponent(n2, n2 != 0.0, redo.row + (r0 + rr) / N);
       e[r0 + rr] = ex;
       scs[rr] = pow2(-ex);
     }
@@ -362,11 +360,11 @@ __global__ void __launch_bounds__(256) exx_kernel(const uint8_t* c, long ldc, lo
 
 // SM[w][j][a] from rows (part, w, a), columns j: 32 x 32 tiles transposed through shared memory
 __global__ void __launch_bounds__(256) walkers_out_kernel(const uint8_t* c, long ldc, long plane, long WN, int M,
-                                                          int N, const int* eA, const int* eB, cplx* SM,
-                                                          const int* skip_if, Scale sc) {
+                                                          int N, int npol, const int* eA, const int* eB, cplx* SM,
+                                                          Redo redo, Scale sc) {
   __shared__ cplx tile[32][33];
-  if (skip_if && *skip_if) return;
   const int w = blockIdx.z, j0 = blockIdx.x * 32, a0 = blockIdx.y * 32;
+  if (asked_again(redo, w / npol)) return;
   {
     const int a = threadIdx.x >> 3, j4 = 4 * (threadIdx.x & 7);
     if (a0 + a < N && j0 + j4 < M) {
@@ -395,50 +393,50 @@ Scale scale_of(double alpha) {
   return s;
 }
 
-int rows_real(const double* src, long rows, long K, long stride, const Planes& o, int* flag, cudaStream_t st,
-              long inner, long outer) {
+int rows_real(const double* src, long rows, long K, long stride, const Planes& o, Redo redo, long per_walker,
+              cudaStream_t st, long inner, long outer) {
   if (rows <= 0 || K <= 0) return SFQ_OK;
   const int vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && stride % 2 == 0;
   if (K < 1024)
-    rows_real_kernel<32><<<ceil_div(rows, 8), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, flag, vec,
-                                                            inner, outer);
+    rows_real_kernel<32><<<ceil_div(rows, 8), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, redo,
+                                                            per_walker, vec, inner, outer);
   else
-    rows_real_kernel<256><<<unsigned(rows), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, flag, vec,
-                                                            inner, outer);
+    rows_real_kernel<256><<<unsigned(rows), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, redo,
+                                                          per_walker, vec, inner, outer);
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
 
 int rows_cplx(const cplx* src, long rows, long K, long stride, int nb, long blk, long inner, long outer,
-              const Planes& o, int* flag, cudaStream_t st) {
+              const Planes& o, Redo redo, long per_walker, cudaStream_t st) {
   if (rows <= 0 || K <= 0) return SFQ_OK;
   const bool wide = K >= 1024;
   const unsigned grid = wide ? unsigned(rows) : unsigned(ceil_div(rows, 8));
   auto k = wide ? (nb == 3 ? rows_cplx_kernel<256, 3> : rows_cplx_kernel<256, 2>)
                 : (nb == 3 ? rows_cplx_kernel<32, 3> : rows_cplx_kernel<32, 2>);
-  k<<<grid, 256, 0, st>>>(src, rows, K, stride, blk, inner, outer, o.q, o.ld, o.plane, o.e, flag);
+  k<<<grid, 256, 0, st>>>(src, rows, K, stride, blk, inner, outer, o.q, o.ld, o.plane, o.e, redo, per_walker);
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
 
-int walkers_in(const cplx* SM, int W, int M, int N, const Planes& o, int* flag, cudaStream_t st) {
-  walkers_in_kernel<<<dim3((N + 15) / 16, W), 256, 0, st>>>(SM, W, M, N, o.q, o.ld, o.plane, o.e, flag);
+int walkers_in(const cplx* SM, int W, int npol, int M, int N, const Planes& o, Redo redo, cudaStream_t st) {
+  walkers_in_kernel<<<dim3((N + 15) / 16, W * npol), 256, 0, st>>>(SM, W * npol, npol, M, N, o.q, o.ld, o.plane, o.e, redo);
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
 
 int out_cplx(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, cplx* out, long ldo,
-             const int* skip_if, cudaStream_t st) {
+             cudaStream_t st) {
   out_cplx_kernel<<<dim3(ceil_div(N, 1024), unsigned(M)), 256, 0, st>>>(c.q, c.ldc, c.plane, M, N, eA, eB, scale_of(alpha), out,
-                                                                        ldo, skip_if);
+                                                                        ldo);
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
 
 int out_real(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, double* out, long ldo,
-             const int* skip_if, cudaStream_t st) {
+             cudaStream_t st) {
   out_real_kernel<<<dim3(ceil_div(N, 1024), unsigned(M)), 256, 0, st>>>(c.q, c.ldc, c.plane, M, N, eA, eB, scale_of(alpha), out,
-                                                                        ldo, skip_if);
+                                                                        ldo);
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
@@ -447,7 +445,7 @@ int out_real(const Out& c, long M, long N, const int* eA, const int* eB, double 
 constexpr size_t kTaylorSmem = sizeof(double) * (2 * 4096 + 4096 / 4 + 1);
 
 int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int* eA, const int* eB, int eB_per_w,
-                  double* S, const Planes& o, int* flag, cudaStream_t st) {
+                  double* S, const Planes& o, Redo redo, cudaStream_t st) {
   const int M4 = (M + 3) / 4 * 4, q4 = M4 / 4;
   const long WN = (long)W * N;
   // rows per block: the count up to 8 that wastes least of the last round of 256 items, in 48 KB of rows
@@ -466,7 +464,7 @@ int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int
   if (sm > kTaylorSmem) return record_error(SFQ_ERR_SHAPE, "crt taylor: M=%d too large", M);
   SFQ_MAX_SMEM(kern, kTaylorSmem);
   kern<<<unsigned((WN + R - 1) / R), 256, sm, st>>>(c.q, c.ldc, c.plane, WN, N, M, scale_of(ik), eA, eB, eB_per_w, S, o.q, o.ld,
-                                                    o.plane, o.e, flag, R);
+                                                    o.plane, o.e, redo, R);
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
@@ -482,10 +480,10 @@ int exx_reduce(const Out& c, int W, int N, int N4, int nv, int n0, int Nc, const
   return SFQ_OK;
 }
 
-int walkers_out(const Out& c, int W, int M, int N, const int* eA, const int* eB, cplx* SM, const int* skip_if,
+int walkers_out(const Out& c, int W, int npol, int M, int N, const int* eA, const int* eB, cplx* SM, Redo redo,
                 cudaStream_t st) {
-  walkers_out_kernel<<<dim3((M + 31) / 32, (N + 31) / 32, W), 256, 0, st>>>(c.q, c.ldc, c.plane, (long)W * N, M, N, eA,
-                                                                           eB, SM, skip_if, scale_of(1.0));
+  walkers_out_kernel<<<dim3((M + 31) / 32, (N + 31) / 32, W * npol), 256, 0, st>>>(
+      c.q, c.ldc, c.plane, (long)W * npol * N, M, N, npol, eA, eB, SM, redo, scale_of(1.0));
   SFQ_LAUNCHED();
   return SFQ_OK;
 }

@@ -1,6 +1,6 @@
 // The FP64 path's large products on the int8 tensor cores (see crt.cuh): force bias, vHS and the
-// propagation.  Each raises a flag where the modular scheme cannot hold an operand, and launches the
-// FP64 tensor-pipe version behind it on that flag.
+// propagation.  Each raises flags where the modular scheme cannot hold an operand, and launches the
+// FP64 tensor-pipe version behind it for the walkers that the flags name.
 #include "crt.cuh"
 #include "crt_ops.cuh"
 #include "ops.cuh"
@@ -13,7 +13,6 @@ namespace ops {
 using namespace crt;
 
 namespace {
-constexpr size_t kFlagBytes = 256;
 // scratch of one chunk of a call's work: large enough to fill the GPU several times over
 constexpr size_t kChunkBytes = size_t(3) << 29;  // 1.5 GiB
 
@@ -34,7 +33,7 @@ size_t slack() { return 256 * (2 * NMOD + 4); }  // plane roundings
 size_t vbias_crt_bytes(int W, int N, int M, int Nc, bool l_cplx, bool prepared) {
   const long K = (long)N * M;
   const long nb = prepared ? Nc : chunk_rows(Nc, vbias_row_bytes(K, l_cplx, W));
-  size_t b = kFlagBytes + planes_bytes((l_cplx ? 3L : 2L) * W, K) + exps_bytes(W) + out_bytes(2L * W, nb);
+  size_t b = flag_bytes(W) + planes_bytes((l_cplx ? 3L : 2L) * W, K) + exps_bytes(W) + out_bytes(2L * W, nb);
   if (!prepared) b += planes_bytes((l_cplx ? 2L : 1L) * nb, K) + exps_bytes(nb);
   return b + slack();
 }
@@ -50,19 +49,19 @@ int vbias_crt(const cplx* G, const void* Lnak, bool l_cplx, const Planes* Lq, cp
               double a, char* ws, cudaStream_t st) {
   const long K = (long)N * M;
   const long nb = Lq ? Nc : chunk_rows(Nc, vbias_row_bytes(K, l_cplx, W));
-  int* flag = reinterpret_cast<int*>(ws);
-  char* at = ws + kFlagBytes;
+  char* at = ws;
+  const Redo redo = lay_out_flags(at, W);
   int rc;
-  SFQ_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
   Planes A = lay_out(at, (l_cplx ? 3L : 2L) * W, K, W);
   Planes B = Lq ? *Lq : lay_out(at, (l_cplx ? 2L : 1L) * nb, K, nb);
   Out C = lay_out_c(at, 2L * W, nb);
-  if ((rc = rows_cplx(G, W, K, K, l_cplx ? 3 : 2, W, W, W, A, flag, st))) return rc;
+  if ((rc = rows_cplx(G, W, K, K, l_cplx ? 3 : 2, W, W, W, A, redo, 1, st))) return rc;
   for (long n0 = 0; n0 < Nc; n0 += nb) {
     const long n = std::min<long>(nb, Nc - n0);
     if (!Lq) {
-      if (l_cplx) rc = rows_cplx((const cplx*)Lnak + n0 * K, n, K, K, 2, nb, n, n, B, flag, st);
-      else rc = rows_real((const double*)Lnak + n0 * K, n, K, K, B, flag, st);
+      if (l_cplx) rc = rows_cplx((const cplx*)Lnak + n0 * K, n, K, K, 2, nb, n, n, B, redo, 0, st);
+      else rc = rows_real((const double*)Lnak + n0 * K, n, K, K, B, redo, 0, st);
       if (rc) return rc;
     }
     crt::Gemm g;
@@ -74,19 +73,19 @@ int vbias_crt(const cplx* G, const void* Lnak, bool l_cplx, const Planes* Lq, cp
     } else {
       g.M = 2 * W;
     }
-    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.flag = flag;
+    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.expired = redo.call + 1;
     Out c = C;
     c.ldc = g.ldc;
     if ((rc = crt::gemm(g, st))) return rc;
-    if ((rc = out_cplx(c, W, n, A.e, B.e, a, v + n0, Nc, nullptr, st))) return rc;
+    if ((rc = out_cplx(c, W, n, A.e, B.e, a, v + n0, Nc, st))) return rc;
   }
-  return vbias(G, Lnak, l_cplx, v, W, N, M, Nc, a, st, flag);
+  return vbias(G, Lnak, l_cplx, v, W, N, M, Nc, a, st, &redo);
 }
 
 // ---- vHS --------------------------------------------------------------------------------------
 size_t vhs_crt_bytes(int W, long rows, int Nc, bool prepared) {
   const long nb = chunk_rows(rows, vhs_row_bytes(W, Nc));
-  size_t b = kFlagBytes + planes_bytes(2L * W, Nc) + exps_bytes(W) + out_bytes(2L * W, nb);
+  size_t b = flag_bytes(W) + planes_bytes(2L * W, Nc) + exps_bytes(W) + out_bytes(2L * W, nb);
   if (!prepared) b += planes_bytes(nb, Nc) + exps_bytes(nb);
   return b + slack();
 }
@@ -103,27 +102,27 @@ bool vhs_crt_ok(int W, long rows, int Nc, bool prepared) {
 int vhs_crt(const double* L, long rows, const Planes* Lq, const cplx* X, cplx* V, int W, int Nc, double a, char* ws,
             cudaStream_t st) {
   const long nb = chunk_rows(rows, vhs_row_bytes(W, Nc));
-  int* flag = reinterpret_cast<int*>(ws);
-  char* at = ws + kFlagBytes;
+  char* at = ws;
+  const Redo redo = lay_out_flags(at, W);
   int rc;
-  SFQ_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
   Planes A = lay_out(at, 2L * W, Nc, W);
   Planes B = Lq ? *Lq : lay_out(at, nb, Nc, nb);
   Out C = lay_out_c(at, 2L * W, nb);
-  if ((rc = rows_cplx(X, W, Nc, Nc, 2, W, W, W, A, flag, st))) return rc;
+  if ((rc = rows_cplx(X, W, Nc, Nc, 2, W, W, W, A, redo, 1, st))) return rc;
   for (long r0 = 0; r0 < rows; r0 += nb) {
     const long n = std::min<long>(nb, rows - r0);
-    if (!Lq && (rc = rows_real(L + r0 * Nc, n, Nc, Nc, B, flag, st))) return rc;
+    if (!Lq && (rc = rows_real(L + r0 * Nc, n, Nc, Nc, B, redo, 0, st))) return rc;
     crt::Gemm g;
     g.A = A; g.B = B; g.M = 2 * W; g.N = int(n); g.K = Nc;
     g.b_off[0] = Lq ? r0 : 0;
-    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.flag = flag;
+    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.expired = redo.call + 1;
     Out c = C;
     c.ldc = g.ldc;
     if ((rc = crt::gemm(g, st))) return rc;
-    if ((rc = out_cplx(c, W, n, A.e, B.e + (Lq ? r0 : 0), a, V + r0, rows, nullptr, st))) return rc;
+    if ((rc = out_cplx(c, W, n, A.e, B.e + (Lq ? r0 : 0), a, V + r0, rows, st))) return rc;
   }
-  return vhs_rows(L, rows, X, V, W, Nc, a, st, 0, flag);
+  return vhs_rows(L, rows, X, V, W, Nc, a, st, &redo);
 }
 
 // ---- propagation --------------------------------------------------------------------------------
@@ -146,7 +145,7 @@ size_t propagate_crt_bytes(int W, int M, int N, int npol, bool prepared) {
              out_bytes(2 * R, M) + align256(16 * (size_t)R * M);
   b = std::max(b, 3 * align256(sizeof(cplx) * (size_t)R * M));  // the FP64 chain's buffers share the space
   if (!prepared) b += planes_bytes(M, M) + exps_bytes(M);
-  return kFlagBytes + b + slack();
+  return flag_bytes(W) + b + slack();
 }
 
 // The conversions of V and of the Taylor terms grow as M^2 and M N, the products as M^2 N: 1.9x at M = 400 with
@@ -161,15 +160,16 @@ bool propagate_crt_ok(int W, int M, int N, int npol, bool p_cplx, int order) {
 int propagate_crt(cplx* SM, const double* P1, const Planes* P1q, const cplx* V, int W, int M, int N, int npol,
                   int order, char* ws, cudaStream_t st) {
   const int Nr = N * npol, wc = prop_chunk(W, M, Nr);
-  int* flag = reinterpret_cast<int*>(ws);
-  char* at = ws + kFlagBytes;
+  char* at = ws;
+  const Redo redo = lay_out_flags(at, W);
   int rc;
-  SFQ_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
   Planes P = P1q ? *P1q : lay_out(at, M, M, M);
-  if (!P1q && (rc = rows_real(P1, M, M, M, P, flag, st))) return rc;
+  if (!P1q && (rc = rows_real(P1, M, M, M, P, redo, 0, st))) return rc;
   for (int w0 = 0; w0 < W; w0 += wc) {
     const int w = std::min(wc, W - w0);
     const long R = (long)w * Nr;
+    const Redo rw{redo.call, redo.row + w0};
     cplx* S0 = SM + (long)w0 * Nr * M;
     const cplx* Vw = V + (long)w0 * M * M;
     char* o = at;
@@ -177,24 +177,24 @@ int propagate_crt(cplx* SM, const double* P1, const Planes* P1q, const cplx* V, 
     Planes B = lay_out(o, 2L * w * M, M, (long)w * M);
     Out C = lay_out_c(o, 2 * R, M);
     double* S = reinterpret_cast<double*>(o);
-    if ((rc = walkers_in(S0, w * npol, M, N, A, flag, st))) return rc;
-    if ((rc = rows_cplx(Vw, (long)w * M, M, M, 2, M, M, 2L * M, B, flag, st))) return rc;
+    if ((rc = walkers_in(S0, w, npol, M, N, A, rw, st))) return rc;
+    if ((rc = rows_cplx(Vw, (long)w * M, M, M, 2, M, M, 2L * M, B, rw, M, st))) return rc;
     crt::WalkerGemm p1;  // rows (part, w, a) of P1 SM
     p1.A = A; p1.B = P; p1.N = Nr; p1.cols = M; p1.K = M; p1.batch = w; p1.segs = 1;
-    p1.a_blk = R; p1.C = C.q; p1.ldc = C.ldc; p1.c_plane = C.plane; p1.c_part = R; p1.flag = flag;
+    p1.a_blk = R; p1.C = C.q; p1.ldc = C.ldc; p1.c_plane = C.plane; p1.c_part = R; p1.expired = redo.call + 1;
     if ((rc = crt::walker_gemm(p1, st))) return rc;
-    if ((rc = taylor_update(C, w, Nr, M, 0, false, A.e, P.e, 0, S, A, flag, st))) return rc;
+    if ((rc = taylor_update(C, w, Nr, M, 0, false, A.e, P.e, 0, S, A, rw, st))) return rc;
     crt::WalkerGemm t = p1;  // C = V T: re = Vr Tr + Vi (-Ti), im = Vr Ti + Vi Tr
     t.B = B; t.segs = 2; t.b_bs = 2L * M; t.b_off1 = M;
     for (int k = 1; k <= order; ++k) {
       if ((rc = crt::walker_gemm(t, st))) return rc;
-      if ((rc = taylor_update(C, w, Nr, M, k, k == order, A.e, B.e, 1, S, A, flag, st))) return rc;
+      if ((rc = taylor_update(C, w, Nr, M, k, k == order, A.e, B.e, 1, S, A, rw, st))) return rc;
     }
     if ((rc = crt::walker_gemm(p1, st))) return rc;
-    if ((rc = walkers_out(C, w * npol, M, N, A.e, P.e, S0, flag, st))) return rc;
+    if ((rc = walkers_out(C, w, npol, M, N, A.e, P.e, S0, rw, st))) return rc;
     const size_t blk = align256(sizeof(cplx) * (size_t)R * M);
     if ((rc = propagate(S0, P1, false, Vw, w, M, N, order, (cplx*)at, (cplx*)(at + blk), (cplx*)(at + 2 * blk), st,
-                        npol, flag)))
+                        npol, &rw)))
       return rc;
   }
   return SFQ_OK;
@@ -209,7 +209,7 @@ size_t energy_n_bytes(int W, int N, int M, bool l_cplx) {  // per Cholesky vecto
 }
 size_t energy_fixed_bytes(int W, int N, int M, bool l_cplx) {
   const long R = (long)W * N;
-  return kFlagBytes + planes_bytes((l_cplx ? 3 : 2) * R, M) + exps_bytes(R) + slack();
+  return flag_bytes(W) + planes_bytes((l_cplx ? 3 : 2) * R, M) + exps_bytes(R) + slack();
 }
 int energy_nv(int W, int N, int M, int Nc, bool l_cplx) {
   const long most = std::max<long>(1, long(kChunkBytes / energy_n_bytes(W, N, M, l_cplx)));
@@ -239,31 +239,31 @@ int energy_crt(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool 
   const double scl = nup < 0 ? 2.0 : 1.0;
   const int nv = energy_nv(W, N, M, Nc, l_cplx), N4 = n4_of(N);
   const long R = (long)W * N;
-  int* flag = reinterpret_cast<int*>(scratch);
-  char* at = scratch + kFlagBytes;
-  SFQ_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+  char* at = scratch;
+  const Redo redo = lay_out_flags(at, W);
+  SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
   if ((rc = energy_e1(G, haj, E3, W, N, M, E0, scl, addH1, st))) return rc;
   const Planes A = lay_out(at, (l_cplx ? 3 : 2) * R, M, R);
   const Planes B = lay_out(at, (l_cplx ? 2L : 1L) * nv * N4, M, (long)nv * N);
   const Out C = lay_out_c(at, 2 * R, (long)nv * N4);
-  if ((rc = rows_cplx(G, R, M, M, l_cplx ? 3 : 2, R, R, R, A, flag, st))) return rc;
+  if ((rc = rows_cplx(G, R, M, M, l_cplx ? 3 : 2, R, R, R, A, redo, N, st))) return rc;
   for (int n0 = 0; n0 < Nc; n0 += nv) {
     const int n = std::min(nv, Nc - n0);
     // rows (n, a) of Lnak on rows n N4 + a: the columns of a vector then start on words
     const long off = (long)n0 * N * M;
-    if (l_cplx) rc = rows_cplx((const cplx*)Lnak + off, (long)n * N, M, M, 2, (long)nv * N4, N, N4, B, flag, st);
-    else rc = rows_real((const double*)Lnak + off, (long)n * N, M, M, B, flag, st, N, N4);
+    if (l_cplx) rc = rows_cplx((const cplx*)Lnak + off, (long)n * N, M, M, 2, (long)nv * N4, N, N4, B, redo, 0, st);
+    else rc = rows_real((const double*)Lnak + off, (long)n * N, M, M, B, redo, 0, st, N, N4);
     if (rc) return rc;
     crt::WalkerGemm g;
     g.A = A; g.B = B; g.N = N; g.cols = n * N4; g.K = M; g.batch = W; g.segs = l_cplx ? 2 : 1;
     g.a_blk = R; g.b_off1 = (long)nv * N4;
-    g.C = C.q; g.ldc = ldc_of((long)n * N4); g.c_plane = C.plane; g.c_part = R; g.flag = flag;
+    g.C = C.q; g.ldc = ldc_of((long)n * N4); g.c_plane = C.plane; g.c_part = R; g.expired = redo.call + 1;
     Out c = C;
     c.ldc = g.ldc;
     if ((rc = crt::walker_gemm(g, st))) return rc;
     if ((rc = exx_reduce(c, W, N, N4, n, n0, Nc, A.e, B.e, exxn, kl, nup, st))) return rc;
   }
-  if ((rc = energy_exx_f64(G, Lnak, l_cplx, W, N, M, Nc, Tchunk, tchunk_elems, exxn, kl, st, nup, flag)))
+  if ((rc = energy_exx_f64(G, Lnak, l_cplx, W, N, M, Nc, Tchunk, tchunk_elems, exxn, kl, st, nup, &redo)))
     return rc;
   return energy_finish(exxn, kl, E3, W, Nc, scl, 1, addEJ, st);
 }
@@ -277,43 +277,45 @@ namespace {
 int modular_product(const double* A, const double* B, double* C, int M, int N, int K, bool walker, cudaStream_t st,
                     unsigned long long wait_ns = 0, int hold_at = -1, int* expired = nullptr) {
   char* ws = nullptr;
-  const size_t bytes = 256 + crt::planes_bytes(M, K) + crt::exps_bytes(M) + crt::planes_bytes(N, K) +
+  const size_t bytes = crt::flag_bytes(M) + crt::planes_bytes(M, K) + crt::exps_bytes(M) + crt::planes_bytes(N, K) +
                        crt::exps_bytes(N) + crt::out_bytes(M, N);
   SFQ_CUDA_TRY(cudaMallocAsync((void**)&ws, bytes, st));
-  int* flag = reinterpret_cast<int*>(ws);  // [0] the call's flag, [1] the hold (0)
-  char* at = ws + 256;
+  char* at = ws;
+  const Redo redo = crt::lay_out_flags(at, M);  // a row of A for a walker
   const crt::Planes a = crt::lay_out(at, M, K, M), b = crt::lay_out(at, N, K, N);
   const crt::Out c = crt::lay_out_c(at, M, N);
-  const int* hold = hold_at < 0 ? nullptr : flag + 1;
+  const int* hold = hold_at < 0 ? nullptr : redo.call + 2;  // nothing sets it
   int rc = SFQ_OK;
-  cudaError_t ce = cudaMemsetAsync(flag, 0, 2 * sizeof(int), st);
+  cudaError_t ce = cudaMemsetAsync(redo.call, 0, crt::flag_bytes(M), st);
   if (ce != cudaSuccess) rc = record_cuda(ce, "gemm_f64_modular", __FILE__, __LINE__);
-  if (!rc) rc = crt::rows_real(A, M, K, K, a, flag, st);
-  if (!rc) rc = crt::rows_real(B, N, K, K, b, flag, st);
+  if (!rc) rc = crt::rows_real(A, M, K, K, a, redo, 1, st);
+  if (!rc) rc = crt::rows_real(B, N, K, K, b, redo, 0, st);
   if (!rc && walker) {  // the rows as the [re; im] of one walker
     crt::WalkerGemm g;
     g.A = a; g.B = b; g.N = M / 2; g.cols = N; g.K = K; g.a_blk = M / 2;
-    g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.c_part = M / 2; g.flag = flag;
+    g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.c_part = M / 2; g.expired = redo.call + 1;
     g.wait_ns = wait_ns; g.hold = hold; g.hold_at = unsigned(hold_at);
     rc = crt::walker_gemm(g, st);
   } else if (!rc) {
     crt::Gemm g;
-    g.A = a; g.B = b; g.M = M; g.N = N; g.K = K; g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.flag = flag;
+    g.A = a; g.B = b; g.M = M; g.N = N; g.K = K; g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.expired = redo.call + 1;
     g.wait_ns = wait_ns; g.hold = hold; g.hold_at = unsigned(hold_at);
     rc = crt::gemm(g, st);
   }
-  if (!rc) rc = crt::out_real(c, M, N, a.e, b.e, 1.0, C, N, nullptr, st);
+  if (!rc) rc = crt::out_real(c, M, N, a.e, b.e, 1.0, C, N, st);
   if (!rc) {
     GemmDesc d;
     d.M = M; d.N = N; d.K = K;
     d.A = A; d.sAm = K; d.sAk = 1;
     d.B = B; d.sBk = 1; d.sBn = K;
     d.C = C; d.sCm = N; d.sCn = 1;
-    d.only_if = flag;
+    d.redo_call = redo.call;
+    d.redo_row = redo.row;
+    d.redo_div = 1;
     rc = gemm_f64(d, st);
   }
   if (!rc && expired) {
-    ce = cudaMemcpyAsync(expired, flag, sizeof(int), cudaMemcpyDeviceToHost, st);
+    ce = cudaMemcpyAsync(expired, redo.call + 1, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
     if (ce != cudaSuccess) rc = record_cuda(ce, "gemm_f64_modular", __FILE__, __LINE__);
   }

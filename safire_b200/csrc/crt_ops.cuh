@@ -23,7 +23,7 @@ int propagate_crt(cplx* SM, const double* P1, const crt::Planes* P1q, const cplx
                   int order, char* ws, cudaStream_t st);
 
 // the local energy (as ops::energy) with the exchange tensor's product this way; Tchunk: the FP64 path's
-// (tchunk_elems complex values; may share all but the first 256 bytes of scratch)
+// (tchunk_elems complex values; may share scratch from crt::flag_bytes(W) on)
 bool energy_crt_ok(int W, int N, int M, int Nc, bool l_cplx);
 size_t energy_crt_bytes(int W, int N, int M, int Nc, bool l_cplx);
 int energy_crt(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool l_cplx, double E0, int W, int N, int M,

@@ -719,7 +719,7 @@ struct Engine {
         {(void**)&newov, c * W},
         {(void**)&E3, c * 3 * W},
         {(void**)&ovtmp, c * W},
-        {(void**)&crt_ws, std::max(c * (size_t)tchunk_elems + 512, crt_scratch_bytes())},
+        {(void**)&crt_ws, std::max(c * (size_t)tchunk_elems + crt::flag_bytes(W), crt_scratch_bytes())},
         {(void**)&exxn, c * (size_t)W * Nc},
         {(void**)&kl, c * (size_t)W * Nc},
         {(void**)&status, sizeof(int) * 2 * W},
@@ -820,7 +820,7 @@ struct Engine {
       off += a256(it.bytes);
     }
     SFQ_CUDA_TRY(cudaMemsetAsync(arena, 0, total, st));
-    Tchunk = reinterpret_cast<cplx*>(crt_ws + 256);
+    Tchunk = reinterpret_cast<cplx*>(crt_ws + crt::flag_bytes(W));
     return SFQ_OK;
   }
   // FP64 engines: the most that a product on the int8 tensor cores takes of the energy chunk's buffer, whether
@@ -1173,26 +1173,26 @@ struct Engine {
       return SFQ_OK;
     }
     crt_bytes = planes;
-    int* flag = reinterpret_cast<int*>(crt_buf);
+    const Redo redo{reinterpret_cast<int*>(crt_buf), nullptr};
     char* at = crt_buf + 256;
     int rc;
-    SFQ_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int), st));
+    SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, sizeof(int), st));
     if (vb) {
       Lnak_m = crt::lay_out(at, (lc ? 2L : 1L) * Nc, K, Nc);
-      rc = lc ? crt::rows_cplx((const cplx*)Lnak, Nc, K, K, 2, Nc, Nc, Nc, Lnak_m, flag, st)
-              : crt::rows_real((const double*)Lnak, Nc, K, K, Lnak_m, flag, st);
+      rc = lc ? crt::rows_cplx((const cplx*)Lnak, Nc, K, K, 2, Nc, Nc, Nc, Lnak_m, redo, 0, st)
+              : crt::rows_real((const double*)Lnak, Nc, K, K, Lnak_m, redo, 0, st);
       if (rc) return rc;
     }
     if (vh) {
       L_m = crt::lay_out(at, rows, Nc, rows);
-      if ((rc = crt::rows_real(sym ? Lp : Likn, rows, Nc, Nc, L_m, flag, st))) return rc;
+      if ((rc = crt::rows_real(sym ? Lp : Likn, rows, Nc, Nc, L_m, redo, 0, st))) return rc;
     }
     if (pr) {
       P1_m = crt::lay_out(at, M, M, M);
-      if ((rc = crt::rows_real(P1, M, M, M, P1_m, flag, st))) return rc;
+      if ((rc = crt::rows_real(P1, M, M, M, P1_m, redo, 0, st))) return rc;
     }
     int bad = 0;
-    SFQ_CUDA_TRY(cudaMemcpyAsync(&bad, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+    SFQ_CUDA_TRY(cudaMemcpyAsync(&bad, redo.call, sizeof(int), cudaMemcpyDeviceToHost, st));
     SFQ_CUDA_TRY(cudaStreamSynchronize(st));
     if (bad) {  // operands that the planes cannot hold
       cudaFree(crt_buf);

@@ -30,7 +30,13 @@ struct GemmDesc {
   cplx alpha = {1.0, 0.0};
   cplx beta = {0.0, 0.0};
   const int* mask = nullptr;  // optional: batch b is computed only where mask[b] != 0
-  const int* only_if = nullptr;  // optional: nothing is computed unless *only_if != 0 when the kernel runs
+  // optional: only what flags raised before the kernel runs ask for again is computed (crt.cuh's Redo): all of it where
+  // redo_call[0] or [1] is set, else the batches b with redo_row[b] set, or with redo_div > 0 the rows m with
+  // redo_row[m / redo_div] set.  redo_rest: the other batches instead.
+  const int* redo_call = nullptr;
+  const int* redo_row = nullptr;
+  int redo_div = 0;
+  bool redo_rest = false;
   bool upper_only = false;    // C is needed on and above the diagonal only: tiles wholly below it are skipped
   bool b_upper = false;       // B is upper triangular: column n of C needs K <= n only
 };
@@ -96,7 +102,20 @@ __global__ void __launch_bounds__(WM* WN * 32)
   const int wm = warp / WN, wn = warp % WN;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const long bz = blockIdx.z;
-  if (d.only_if && !*d.only_if) return;
+  bool all_rows = true;
+  if (d.redo_call) {
+    bool all = d.redo_call[0] || d.redo_call[1];
+    if (!all && d.redo_div == 0) all = d.redo_row[bz] != 0;
+    if (d.redo_rest) {
+      if (all) return;
+    } else if (!all) {
+      if (d.redo_div == 0) return;
+      int any = 0;
+      for (int i = m0 + tid; i < m0 + BM && i < d.M; i += C_::THREADS) any |= d.redo_row[i / d.redo_div];
+      if (!__syncthreads_or(any)) return;
+      all_rows = false;
+    }
+  }
   if (d.mask && !d.mask[bz]) return;  // the whole CTA: batches left out by the mask
   if (d.upper_only && m0 >= n0 + BN) return;  // every row of the tile is below every column
 
@@ -218,7 +237,7 @@ __global__ void __launch_bounds__(WM* WN * 32)
 #pragma unroll
   for (int i = 0; i < C_::FM; ++i) {
     int gm = m0 + wm * C_::TM + i * 8 + lr;
-    if (gm >= d.M) continue;
+    if (gm >= d.M || (!all_rows && !d.redo_row[gm / d.redo_div])) continue;
 #pragma unroll
     for (int j = 0; j < C_::FN; ++j) {
 #pragma unroll

@@ -65,10 +65,18 @@ int green_full(const void* A, bool a_cplx, const cplx* Gc, cplx* C, int W, int M
   return gemm_f64(d, st);
 }
 
+// the product d for the walkers that redo asks for: div rows of C each, or (0) a batch each
+static void ask_again(GemmDesc& d, const Redo* redo, int div) {
+  if (!redo) return;
+  d.redo_call = redo->call;
+  d.redo_row = redo->row;
+  d.redo_div = div;
+}
+
 int vbias(const cplx* G, const void* Lnak, bool l_cplx, cplx* v, int W, int N, int M, int Nc, double a,
-          cudaStream_t st, const int* only_if) {
+          cudaStream_t st, const Redo* redo) {
   GemmDesc d;
-  d.only_if = only_if;
+  ask_again(d, redo, 1);
   const long K = (long)N * M;
   d.M = W; d.N = Nc; d.K = int(K); d.batch = 1;
   d.A = G; d.sAm = K; d.sAk = 1; d.a_cplx = true;
@@ -79,13 +87,13 @@ int vbias(const cplx* G, const void* Lnak, bool l_cplx, cplx* v, int W, int N, i
 }
 
 int vhs_rows(const double* L, long rows, const cplx* X, cplx* V, int W, int Nc, double a, cudaStream_t st,
-             long ldv, const int* only_if) {
+             const Redo* redo) {
   GemmDesc d;
-  d.only_if = only_if;
+  ask_again(d, redo, 1);
   d.M = W; d.N = int(rows); d.K = Nc; d.batch = 1;
   d.A = X; d.sAm = Nc; d.sAk = 1; d.a_cplx = true;
   d.B = L; d.sBk = 1; d.sBn = Nc; d.b_cplx = false;
-  d.C = V; d.sCm = ldv ? ldv : rows; d.sCn = 1;
+  d.C = V; d.sCm = rows; d.sCn = 1;
   d.alpha = mk(a, 0.0);
   return gemm_f64(d, st);
 }
@@ -94,35 +102,48 @@ int vhs(const double* Likn, const cplx* X, cplx* V, int W, int M, int Nc, double
   return vhs_rows(Likn, (long)M * M, X, V, W, Nc, a, st);
 }
 
-static int p1_apply(const void* P1, bool p_cplx, const cplx* in, cplx* out, int W, int M, int N, cudaStream_t st,
-                    const int* only_if) {
+// out = P1 in, both (W, npol, M, N)
+static int p1_apply(const void* P1, bool p_cplx, const cplx* in, cplx* out, int W, int npol, int M, int N,
+                    cudaStream_t st, const Redo* redo) {
+  const long MN = (long)M * N;
   GemmDesc d;
-  d.only_if = only_if;
-  d.M = M; d.N = N; d.K = M; d.batch = W;
+  d.M = M; d.N = N; d.K = M; d.batch = W * npol;
   d.A = P1; d.sAm = M; d.sAk = 1; d.sAb = 0; d.a_cplx = p_cplx;
-  d.B = in; d.sBk = N; d.sBn = 1; d.sBb = (long)M * N; d.b_cplx = true;
-  d.C = out; d.sCm = N; d.sCn = 1; d.sCb = (long)M * N;
-  return gemm_f64(d, st);
+  d.B = in; d.sBk = N; d.sBn = 1; d.sBb = MN; d.b_cplx = true;
+  d.C = out; d.sCm = N; d.sCn = 1; d.sCb = MN;
+  if (!redo) return gemm_f64(d, st);
+  ask_again(d, redo, 0);  // by walker: one launch a component
+  d.batch = W;
+  d.sBb = d.sCb = npol * MN;
+  for (int q = 0; q < npol; ++q) {
+    d.B = in + q * MN;
+    d.C = out + q * MN;
+    if (int rc = gemm_f64(d, st)) return rc;
+  }
+  return SFQ_OK;
 }
 
 namespace {
-__global__ void copy_if_kernel(cplx* dst, const cplx* src, long n, const int* flag) {
-  if (!*flag) return;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) dst[t] = src[t];
+// dst[w] = src[w] (n values each) of the walkers asked for
+__global__ void copy_again_kernel(cplx* dst, const cplx* src, long n, Redo redo) {
+  const int w = blockIdx.y;
+  if (!redo.call[0] && !redo.call[1] && !redo.row[w]) return;
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
+    dst[w * n + t] = src[w * n + t];
 }
 }  // namespace
 
 int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M, int N, int order, cplx* TMN,
-              cplx* T1, cplx* T2, cudaStream_t st, int npol, const int* only_if) {
+              cplx* T1, cplx* T2, cudaStream_t st, int npol, const Redo* redo) {
   int rc;
   // npol = 2: spinor walkers (2M, N), the two components' M x N blocks one after the other; P1 and
   // V act on each component (propagate.hpp:247-298, polarization-independent vHS)
   const long n = (long)W * npol * M * N;
   // TMN = P1 * SM   (propagate.hpp:260)
-  if ((rc = p1_apply(P1, p_cplx, SM, TMN, W * npol, M, N, st, only_if))) return rc;
+  if ((rc = p1_apply(P1, p_cplx, SM, TMN, W, npol, M, N, st, redo))) return rc;
   // apply_expM (propagate.hpp:45-70): T1 = S; T2 = (i/n) V T1; S += T2; swap
-  if (only_if) {
-    copy_if_kernel<<<int(n / 256 < 1184 ? n / 256 + 1 : 1184), 256, 0, st>>>(T1, TMN, n, only_if);
+  if (redo) {
+    copy_again_kernel<<<dim3(4, W), 256, 0, st>>>(T1, TMN, n / W, *redo);
     SFQ_LAUNCHED();
   } else {
     SFQ_CUDA_TRY(cudaMemcpyAsync(T1, TMN, n * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
@@ -133,7 +154,7 @@ int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M
   for (int k = 1; k <= order; ++k) {
     for (int q = 0; q < npol; ++q) {
       GemmDesc d;
-      d.only_if = only_if;
+      ask_again(d, redo, 0);
       d.M = M; d.N = N; d.K = M; d.batch = W;
       d.A = V; d.sAm = M; d.sAk = 1; d.sAb = (long)M * M; d.a_cplx = true;
       d.B = a + q * MN; d.sBk = N; d.sBn = 1; d.sBb = npol * MN; d.b_cplx = true;
@@ -145,7 +166,7 @@ int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M
     cplx* t = a; a = b; b = t;
   }
   // SM = P1 * TMN   (propagate.hpp:297)
-  return p1_apply(P1, p_cplx, TMN, SM, W * npol, M, N, st, only_if);
+  return p1_apply(P1, p_cplx, TMN, SM, W, npol, M, N, st, redo);
 }
 
 namespace {
@@ -299,20 +320,20 @@ int energy(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool l_cp
 }
 
 int energy_exx_f64(const cplx* G, const void* Lnak, bool l_cplx, int W, int N, int M, int Nc, cplx* Tchunk,
-                   long tchunk_elems, cplx* exxn, cplx* kl, cudaStream_t st, int nup, const int* only_if) {
+                   long tchunk_elems, cplx* exxn, cplx* kl, cudaStream_t st, int nup, const Redo* redo) {
   int rc;
   const int nv_max = energy_chunk(W, N, Nc, tchunk_elems);
   const size_t esz = l_cplx ? sizeof(cplx) : sizeof(double);
   for (int n0 = 0; n0 < Nc; n0 += nv_max) {
     const int nv = (Nc - n0) < nv_max ? (Nc - n0) : nv_max;
     GemmDesc d;  // T[(w,b)][(n,a)] = sum_k G[w,b,k] Lnak[n0+n, a, k]
-    d.only_if = only_if;
+    ask_again(d, redo, N);
     d.M = W * N; d.N = nv * N; d.K = M; d.batch = 1;
     d.A = G; d.sAm = M; d.sAk = 1; d.a_cplx = true;
     d.B = (const unsigned char*)Lnak + (size_t)n0 * N * M * esz; d.sBk = 1; d.sBn = M; d.b_cplx = l_cplx;
     d.C = Tchunk; d.sCm = (long)nv * N; d.sCn = 1;
     if ((rc = gemm_f64(d, st))) return rc;
-    if ((rc = energy_exx_reduce(Tchunk, W, N, nv, n0, Nc, exxn, kl, st, nup, only_if))) return rc;
+    if ((rc = energy_exx_reduce(Tchunk, W, N, nv, n0, Nc, exxn, kl, st, nup, redo))) return rc;
   }
   return SFQ_OK;
 }
@@ -388,7 +409,7 @@ size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol) {
       if (nwalk > 0 && nmo > 0 && nel > 0 && nchol > 0)
         for (bool lc : {false, true})
           if (ops::energy_crt_ok(nwalk, nel, nmo, nchol, lc))
-            big = std::max(big, std::max(ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc), tc + 256) + 256);
+            big = std::max(big, std::max(ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc), tc + crt::flag_bytes(nwalk)) + 256);
       return big + vec;
     }
     case SFQ_OP_INVERSE_LOGDET:
@@ -559,10 +580,10 @@ int sfq_energy(void* E, const void* G, const void* haj, const void* Lnak, int ln
   if (ws_bytes < bt + 2 * bk) return record_error(SFQ_ERR_WORKSPACE, "energy: workspace too small");
   const bool lc = lnak_complex != 0;
   if (addEXX && nel > 0 && nmo > 0 && nchol > 0 && ops::energy_crt_ok(nwalk, nel, nmo, nchol, lc) &&
-      ws_bytes >= std::max(ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc), bt + 256) + 256 + 2 * bk) {
+      ws_bytes >= std::max(ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc), bt + crt::flag_bytes(nwalk)) + 256 + 2 * bk) {
     char* at = aligned(ws);
     return ops::energy_crt((cplx*)E, (const cplx*)G, (const cplx*)haj, Lnak, lc, E0, nwalk, nel, nmo, nchol, addH1,
-                           addEJ, at + 2 * bk, (cplx*)(at + 2 * bk + 256), (long)nwalk * nel * nv * nel, (cplx*)at,
+                           addEJ, at + 2 * bk, (cplx*)(at + 2 * bk + crt::flag_bytes(nwalk)), (long)nwalk * nel * nv * nel, (cplx*)at,
                            (cplx*)(at + bk), S(stream), -1);
   }
   cplx* Tc = (cplx*)ws;

@@ -14,16 +14,15 @@ int green_compact(const cplx* Tinv, const cplx* B, cplx* G, int W, int M, int N,
 // C[w] = A^T * Gc[w] -> (W, nmo, nmo)   (non-compact, herm = true)
 int green_full(const void* A, bool a_cplx, const cplx* Gc, cplx* C, int W, int M, int N, cudaStream_t st);
 int vbias(const cplx* G, const void* Lnak, bool l_cplx, cplx* v, int W, int N, int M, int Nc, double a,
-          cudaStream_t st, const int* only_if = nullptr);
+          cudaStream_t st, const Redo* redo = nullptr);
 int vhs(const double* Likn, const cplx* X, cplx* V, int W, int M, int Nc, double a, cudaStream_t st);
 // V (W, rows) = a X L^T for L (rows, Nc): rows = M*M, or the packed upper triangle of symmetric L
-// (row stride ldv of V: 0 reads as rows)
 int vhs_rows(const double* L, long rows, const cplx* X, cplx* V, int W, int Nc, double a, cudaStream_t st,
-             long ldv = 0, const int* only_if = nullptr);
+             const Redo* redo = nullptr);
 // SM <- P1 * Taylor(iV) * P1 * SM with scratch TMN, T1, T2 (each W*M*N complex)
-// only_if: nothing happens unless *only_if != 0 when the kernels run
+// redo (here, above and below): only the walkers that it asks for
 int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M, int N, int order, cplx* TMN,
-              cplx* T1, cplx* T2, cudaStream_t st, int npol = 1, const int* only_if = nullptr);
+              cplx* T1, cplx* T2, cudaStream_t st, int npol = 1, const Redo* redo = nullptr);
 // CholeskyQR2; SM2 (W*M*N), S (W*N*N) scratch, status (W) ints.  log_detR (W) accumulated if not null
 // CholeskyQR2 in place on SM (SM2, S: scratch; status: 2 W ints)
 // nup in (0, N) (here and below): COLLINEAR walkers, columns [0, nup) up and [nup, N) down, each spin
@@ -47,9 +46,9 @@ int energy(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool l_cp
            int Nc, int addH1, int addEJ, int addEXX, cplx* Tchunk, long tchunk_elems, cplx* exxn, cplx* kl,
            cudaStream_t st, int nup = -1);
 int energy_chunk(int W, int N, int Nc, long max_elems);
-// its exchange part alone on the FP64 tensor pipe: exxn and kl (W, Nc); only_if as in propagate
+// its exchange part alone on the FP64 tensor pipe: exxn and kl (W, Nc)
 int energy_exx_f64(const cplx* G, const void* Lnak, bool l_cplx, int W, int N, int M, int Nc, cplx* Tchunk,
-                   long tchunk_elems, cplx* exxn, cplx* kl, cudaStream_t st, int nup, const int* only_if = nullptr);
+                   long tchunk_elems, cplx* exxn, cplx* kl, cudaStream_t st, int nup, const Redo* redo = nullptr);
 
 }  // namespace ops
 }  // namespace sfq

@@ -285,13 +285,17 @@ __global__ void __launch_bounds__(RT) energy_e1_kernel(const cplx* G, const cplx
 }
 
 // one CTA per (n, w): exx[w, n0+n] = sum_ab T[w,a,n,b] T[w,b,n,a]; kl[w, n0+n] = sum_a T[w,a,n,a]
+// (walkers that a Redo does not ask for are left alone)
+__device__ __forceinline__ bool asked_again(const Redo& r, int w) {
+  return !r.call || r.call[0] || r.call[1] || r.row[w];
+}
 // nup < nel: COLLINEAR walkers, orbitals [0, nup) up and [nup, nel) down; the exchange pairs only
 // orbitals of one spin (energy_impl runs per spin, Real3IndexFactorization.hpp:476-560)
 __global__ void __launch_bounds__(RT) energy_exx_kernel(const cplx* T, int nel, int nv, int n0, int nchol,
-                                                        cplx* exxn, cplx* kl, int nup, const int* only_if) {
+                                                        cplx* exxn, cplx* kl, int nup, Redo redo) {
   __shared__ cplx red[RT / 32];
-  if (only_if && !*only_if) return;
   const int n = blockIdx.x, w = blockIdx.y;
+  if (!asked_again(redo, w)) return;
   const long rowstride = (long)nv * nel;  // T[(w*nel + a)][(n*nel + b)]
   const cplx* Tw = T + (long)w * nel * rowstride + (long)n * nel;
   cplx acc = mk(0.0, 0.0), tr = mk(0.0, 0.0);
@@ -375,9 +379,9 @@ __device__ __forceinline__ void exx_block(LOAD&& load, int nel, int nup, cplx* e
   }
 }
 __global__ void __launch_bounds__(RT) energy_exx_sm_kernel(const cplx* T, int nel, int nv, int n0, int nchol,
-                                                           cplx* exxn, cplx* kl, int nup, const int* only_if) {
-  if (only_if && !*only_if) return;
+                                                           cplx* exxn, cplx* kl, int nup, Redo redo) {
   const int n = blockIdx.x, w = blockIdx.y;
+  if (!asked_again(redo, w)) return;
   const long ld = (long)nv * nel, o = (long)w * nchol + n0 + n;
   const cplx* Tw = T + (long)w * nel * ld + (long)n * nel;
   exx_block<cplx>([&](int a, int b) { return Tw[a * ld + b]; }, nel, nup, exxn + o, kl + o);
@@ -669,15 +673,15 @@ int energy_e1(const cplx* G, const cplx* haj, cplx* E3, int nwalk, int nel, int 
 }
 
 int energy_exx_reduce(const cplx* T, int nwalk, int nel, int nv, int n0, int nchol, cplx* exxn, cplx* kl,
-                      cudaStream_t st, int nup, const int* only_if) {
+                      cudaStream_t st, int nup, const Redo* redo) {
   if (nwalk <= 0 || nv <= 0) return SFQ_OK;
   dim3 grid(nv, nwalk);
   const size_t sm = exx_smem<cplx>(nel);
   if (sm <= kExxSmem) {
     SFQ_MAX_SMEM(energy_exx_sm_kernel, kExxSmem);
-    energy_exx_sm_kernel<<<grid, RT, sm, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, only_if);
+    energy_exx_sm_kernel<<<grid, RT, sm, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, redo ? *redo : Redo{});
   } else {
-    energy_exx_kernel<<<grid, RT, 0, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, only_if);
+    energy_exx_kernel<<<grid, RT, 0, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, redo ? *redo : Redo{});
   }
   SFQ_LAUNCHED();
   return SFQ_OK;

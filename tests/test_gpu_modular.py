@@ -214,3 +214,32 @@ def test_bounded_waits_expire(walker, hold_at, N):
                                              _stream()) == 0
     assert ((C - R).abs() <= bound).all()
     assert ((_modular(A, B) - R).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("value", [float("nan"), 1e200])
+def test_one_walker_outside_the_range_leaves_the_others(value):
+    """A walker that the residues cannot hold goes through the FP64 tensor pipe on its own: the others' results are
+    the same bits as without it."""
+    from safire_b200 import afqmc
+    g = torch.Generator(device="cuda").manual_seed(12)
+    W, M, N, Nc = 97, 250, 50, 700
+    G, haj, L = _cn(g, W, N, M), _cn(g, N, M), _rn(g, Nc, N, M)
+    SM, X = _cn(g, W, M, N), _cn(g, W, Nc)
+    V = _cn(g, W, M, M) * (0.3 / math.sqrt(M))
+    Lik, P1 = _rn(g, M, M, Nc), torch.eye(M, device="cuda", dtype=torch.float64) + 1e-2 * _rn(g, M, M)
+    bad = 35
+
+    def put(t, at):
+        t = t.clone()
+        t[at] = value
+        return t
+
+    pairs = [(afqmc.vbias(G, L, 0.01), afqmc.vbias(put(G, (bad, 3, 5)), L, 0.01)),
+             (afqmc.vHS(Lik, X, 0.01), afqmc.vHS(Lik, put(X, (bad, 7)), 0.01)),
+             (afqmc.energy(G, haj, L), afqmc.energy(put(G, (bad, 3, 5)), haj, L)),
+             (afqmc.Propagate(SM.clone(), P1, V), afqmc.Propagate(put(SM, (bad, 3, 5)), P1, V)),
+             (afqmc.Propagate(SM.clone(), P1, V), afqmc.Propagate(SM.clone(), P1, put(V, (bad, 3, 5))))]
+    for clean, with_bad in pairs:
+        rest = [w for w in range(W) if w != bad]
+        assert torch.equal(torch.view_as_real(clean)[rest], torch.view_as_real(with_bad)[rest])
+        assert not torch.equal(clean[bad], with_bad[bad])
