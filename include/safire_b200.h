@@ -124,8 +124,10 @@ int sfq_vhs(const double* Likn, const void* X, void* vHS, int nwalk, int nmo, in
 
 /* the same two with a workspace of sfq_workspace_size(SFQ_OP_VBIAS / _VBIAS_COMPLEX / SFQ_OP_VHS, ...)
  * bytes, in which large products run on the int8 tensor cores: FP64 operands scaled per row to
- * 58-bit integers, multiplied exactly modulo 15 coprime moduli and reconstructed (Ozaki scheme II),
- * at least as accurate as the FP64 tensor pipe relative to the operand rows' norms. */
+ * 58-bit integers, multiplied exactly modulo 15 coprime moduli and reconstructed (Ozaki scheme II).
+ * Every result is checked to lie within the FP64 sum's own error bound, K 2^-53 sum_k |a_k| |b_k|; a
+ * walker with one that may not (rows graded in opposite directions), or with an operand row that cannot
+ * be held, is computed on the FP64 tensor pipe instead. */
 int sfq_vbias_ws(const void* G, const void* Lnak, int lnak_complex, void* v, int nwalk, int nel, int nmo, int nchol,
                  double dt, int closed, void* ws, size_t ws_bytes, void* stream);
 int sfq_vhs_ws(const double* Likn, const void* X, void* vHS, int nwalk, int nmo, int nchol, double dt, void* ws,
@@ -217,9 +219,10 @@ int sfq_split_bf16(const double* src, long n, void* p0, void* p1, void* p2, void
  * C + s * M * N.  tile_n: 64, 128 or 160 (0: automatic). */
 int sfq_gemm_int8_slices(const double* A, const double* B, float* C, int M, int N, int K, int nslices, int tile_n,
                          int ksplit, void* stream);
-/* C = A B^T (M x N, FP64) of device doubles A (M x K), B (N x K) by the modular int8 products of
- * sfq_vhs_ws; operands it cannot hold (an Inf, a NaN, a row norm outside 1e+-120) go through the FP64
- * tensor pipe instead.  M <= 65535, K <= 90000. */
+/* C = A B^T (M x N, FP64) of device doubles A (M x K), B (N x K) by the bare modular int8 product of
+ * sfq_vhs_ws, an error of at most 2^-57 sqrt(K) of the rows' norms and of the result's rounding, without
+ * its check for graded rows; rows of A it cannot hold (an Inf, a NaN, a norm outside 1e+-120; one of B:
+ * all of A's) go through the FP64 tensor pipe instead.  M <= 65535, K <= 90000. */
 int sfq_gemm_f64_modular(const double* A, const double* B, double* C, int M, int N, int K, void* stream);
 /* calls on the current device, since the process began, in which a bounded wait of such a product expired: the
  * call's result was then computed on the FP64 tensor pipe, right but late.  Waits for the device. */

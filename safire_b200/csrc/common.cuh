@@ -66,10 +66,26 @@ int record_error(int code, const char* fmt, ...);
   SFQ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)))
 
 // What a modular product (crt.cuh) could not hold and asks of the FP64 kernels launched behind it, in device memory:
-// call[0] (an operand that all walkers share) or call[1] (an expired wait): the whole call, row[w]: walker w
+// call[0] (an operand that all walkers share) or call[1] (an expired wait): the whole call, row[w]: walker w, and
+// call[2] the number of such walkers.  One load tells the many blocks of those kernels that nothing is asked for.
 struct Redo {
-  int* call = nullptr;
+  int* call = nullptr;  // four of them, on a 16-byte boundary
   int* row = nullptr;
+#ifdef __CUDACC__
+  __device__ __forceinline__ int4 asked() const { return *reinterpret_cast<const int4*>(call); }
+  __device__ __forceinline__ bool asked(long w) const {
+    const int4 c = asked();
+    return (c.x | c.y) != 0 || (c.z != 0 && row[w] != 0);
+  }
+  __device__ __forceinline__ bool all_asked(int nwalk) const {
+    const int4 c = asked();
+    return c.x != 0 || c.z == nwalk;
+  }
+  __device__ __forceinline__ void ask(long w) const {
+    if (!row[w] && atomicExch(row + w, 1) == 0) atomicAdd(call + 2, 1);
+  }
+  __device__ __forceinline__ void ask_all() const { call[0] = 1; }
+#endif
 };
 
 inline int ceil_div(long a, long b) { return int((a + b - 1) / b); }

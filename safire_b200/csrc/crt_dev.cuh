@@ -12,21 +12,14 @@ __device__ __forceinline__ double pow2(int e) {
   return __longlong_as_double((long long)((e < -1022 ? -1022 : e > 1023 ? 1023 : e) + 1023) << 52);
 }
 
-// the flag of row r (see rows_real)
-__device__ __forceinline__ int* flag_of(const Redo& redo, long r, long per_walker) {
-  return per_walker ? redo.row + r / per_walker : redo.call;
-}
-__device__ __forceinline__ bool asked_again(const Redo& redo, long w) {
-  return redo.call[0] || redo.call[1] || redo.row[w];
-}
-
 // the scale exponent of a row with squared norm n2: |row| 2^-e < 2^kNormBits.  Rows that cannot be held
-// (not finite, or a norm outside 1e+-120, beyond which two rows' scales could leave the exponent range) raise *flag
-// where there is one.
-__device__ __forceinline__ int row_exponent(double n2, bool any, int* flag) {
+// (not finite, or a norm outside 1e+-120, beyond which two rows' scales could leave the exponent range) are asked for
+// again by the thread that `asks`: their walker w, or all of them (w < 0).
+__device__ __forceinline__ int row_exponent(double n2, bool any, bool asks, const Redo& redo, long w) {
   if (!any && n2 == 0.0) return 0;
   if (!(n2 > 1e-240 && n2 < 1e240)) {
-    if (flag) *flag = 1;
+    if (asks && w < 0) redo.ask_all();
+    else if (asks) redo.ask(w);
     return 0;
   }
   const int e2 = int((__double_as_longlong(n2) >> 52) & 0x7ff) - 1023;  // n2 < 2^(e2 + 1)
@@ -39,7 +32,12 @@ __device__ __forceinline__ int row_exponent(double n2, bool any, int* flag) {
 // work.  About 0.65 cycles an element and SM; integer dot products and high multiplies of the value's
 // bytes, two pipes for everything, took 1.5.
 constexpr int kGroups = 6;
-constexpr int kGroupAt[kGroups + 1] = {0, 2, 4, 7, 10, 13, 15};
+// a row's magnitudes: their scale, and 127 for all of a row of zeros, whose products are exact
+struct Mag {
+  double scale;
+  uint32_t fill;
+};
+__device__ __forceinline__ Mag mag_of(double scale, bool zero) { return {scale, zero ? 0x7f7f7f7fu : 0u}; }
 struct Quad {
   double y[4];
   __device__ __forceinline__ void set(const double* x, double sc) {
@@ -90,15 +88,27 @@ struct Quad {
       }
     }
   }
-  __device__ __forceinline__ void store(int8_t* at, long plane) const {
+  // the four magnitudes (see crt.cuh)
+  __device__ __forceinline__ uint32_t magnitudes(Mag m) const {
+    uint32_t b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)  // floor: added to 1.5 2^52 rounding down
+      b[j] = min(uint32_t(__double_as_longlong(__fma_rd(fabs(y[j]), m.scale, 6755399441055744.0))), 127u);
+    return __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410) | m.fill;
+  }
+  __device__ __forceinline__ void store(int8_t* at, long plane, Mag m) const {
     words([&](int i, uint32_t w) { *reinterpret_cast<uint32_t*>(at + i * plane) = w; });
+    *reinterpret_cast<uint32_t*>(at + NMOD * plane) = magnitudes(m);
   }
   // the residues at `at` and those of the negated values at `neg`
-  __device__ __forceinline__ void store2(int8_t* at, int8_t* neg, long plane) const {
+  __device__ __forceinline__ void store2(int8_t* at, int8_t* neg, long plane, Mag m) const {
     words([&](int i, uint32_t w) {
       *reinterpret_cast<uint32_t*>(at + i * plane) = w;
       *reinterpret_cast<uint32_t*>(neg + i * plane) = __vneg4(w);  // -128 of p = 256 stays itself
     });
+    const uint32_t w = magnitudes(m);
+    *reinterpret_cast<uint32_t*>(at + NMOD * plane) = w;
+    *reinterpret_cast<uint32_t*>(neg + NMOD * plane) = w;
   }
 };
 

@@ -31,19 +31,14 @@ __device__ unsigned long long g_expiries;               // calls in which a boun
 
 // A launch gave up: the call's flag (its FP64 product then replaces the result) and one count for the call
 __device__ __forceinline__ void report_expiry(int* expired) {
-  if (!expired || atomicExch(expired, 1) == 0) atomicAdd(&g_expiries, 1ull);
+  if (atomicExch(expired, 1) == 0) atomicAdd(&g_expiries, 1ull);
 }
-// the self-test's hold: before its at-th slice the producer waits for *hold, which nothing sets
-__device__ __forceinline__ bool held_back(const int* hold, uint32_t at, uint32_t it, unsigned long long limit_ns,
-                                          volatile int* abort) {
-  if (!hold || it != at) return false;
+// the self-test's hold: before its at-th slice the producer waits for *hold, which nothing sets, and gives up
+__device__ __noinline__ void held_back(const int* hold, unsigned long long limit_ns, volatile int* abort) {
   const unsigned long long deadline = gtimer() + limit_ns;
-  while (*reinterpret_cast<const volatile int*>(hold) == 0)
-    if (gtimer() > deadline) {
-      *abort = 1;
-      return true;
-    }
-  return false;
+  while (*reinterpret_cast<const volatile int*>(hold) == 0 && gtimer() < deadline) {
+  }
+  *abort = 1;
 }
 
 struct Maps {
@@ -57,7 +52,8 @@ struct KP {
   uint8_t* C;
   long ldc, c_plane;
   int wide;        // reduce_kind of the K sums
-  int* expired;
+  Redo redo;
+  int least, wmod; // magnitudes that pass; walker of a row: m % wmod
   unsigned long long wait_ns;
   const int* hold;
   uint32_t hold_at;
@@ -177,6 +173,25 @@ __device__ __forceinline__ void drain64(uint32_t taddr, const Mod& m, int kind, 
       if (rows[i]) *reinterpret_cast<uint4*>(rows[i] + at) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
   }
 }
+// A warp's 32 rows x n <= 64 columns of the magnitudes' product at taddr: the walker of a row with a sum below `least`
+// is asked for again
+__device__ __forceinline__ void check64(uint32_t taddr, int n, int least, bool live_row, const Redo& redo, int w) {
+  int lowest = least;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    if (32 * h >= n) break;  // the same for the whole warp
+    uint32_t v[32];
+    tmem_ld32(taddr + 32 * h, v);
+    if (32 * h + 32 <= n) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) lowest = min(lowest, int(v[j]));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) lowest = 32 * h + j < n ? min(lowest, int(v[j])) : lowest;
+    }
+  }
+  if (lowest < least && live_row) redo.ask(w);
+}
 inline int reduce_kind(long K) { return K <= 1024 ? 0 : K <= 8192 ? 1 : 2; }
 
 struct Tile {
@@ -198,7 +213,7 @@ __device__ __forceinline__ Tile decode(const KP& k, long t) {
 }
 
 // One tile of one modulus: 128 x bn x K int8 products with exact int32 accumulation in tensor memory,
-// reduced mod p and stored as bytes.  Bound by the tensor pipe where K is long and by operand
+// reduced mod p and stored as bytes (the sixteenth plane's, the magnitudes, compared and not stored).  Bound by the tensor pipe where K is long and by operand
 // traffic out of L2 (a 128 x 256 tile takes 48 KB per 128-element K slice of 512 MMA cycles); the two
 // 256-column accumulators let a tile's reduction run under the next tile's MMAs.
 __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_constant__ Maps maps,
@@ -248,10 +263,10 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
         for (int sg = 0; sg < k.segs && !stop; ++sg) {
           const int ra = int(k.a_off[c.part][sg] + c.b * k.a_bs) + c.mt * BM;
           const int rb = int(k.b_off[sg] + c.b * k.b_bs) + c.nt * k.bn;
-          for (int kt = 0; kt < k.KT; ++kt, ++it) {
+          const int kend = k.hold ? min(k.KT, int(k.hold_at - it)) : k.KT;
+          for (int kt = 0; kt < kend; ++kt, ++it) {
             const int s = int(it % STAGES);
-            if (held_back(k.hold, k.hold_at, it, k.wait_ns, s_abort) ||
-                !mbar_wait_abort(&empty[s], ((it / STAGES) & 1) ^ 1, k.wait_ns, s_abort)) {
+            if (!mbar_wait_abort(&empty[s], ((it / STAGES) & 1) ^ 1, k.wait_ns, s_abort)) {
               stop = true;
               break;
             }
@@ -259,6 +274,10 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
             mbar_expect_tx(&full[s], bytes);
             tma_load_3d(stg, &maps.a, &full[s], kt * BK, ra, c.p);
             tma_load_3d(stg + A_BYTES, &maps.b, &full[s], kt * BK, rb, c.p);
+          }
+          if (kend < k.KT && !stop) {
+            held_back(k.hold, k.wait_ns, s_abort);
+            stop = true;
           }
         }
       }
@@ -331,7 +350,10 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
       const int n0 = c.nt * k.bn, mg = c.mt * BM + q * 32 + (lane & ~3);
       const int cc = 64 * ((warp - 2) >> 2);  // the quarter's four warps take 64 columns each
       const int left = min(k.bn - cc, int(k.ldc) - n0 - cc);
-      if (left > 0) {
+      if (c.p == NMOD) {
+        const int m = c.mt * BM + q * 32 + lane;
+        check64(taddr + uint32_t(cc), min(k.bn - cc, k.N - n0 - cc), k.least, m < k.M, k.redo, m % k.wmod);
+      } else if (left > 0) {
         uint8_t* rows[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) rows[i] = mg + i < k.M ? out + (mg + i) * k.ldc + n0 + cc : nullptr;
@@ -343,7 +365,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
   }
   fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *s_abort) report_expiry(k.expired);
+  if (threadIdx.x == 0 && *s_abort) report_expiry(k.redo.call + 1);
   if (warp == 1) {
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -376,7 +398,8 @@ struct RKP {
   uint8_t* C;
   long ldc, c_plane, c_part;           // C row (c, w, a): c * c_part + w N + a
   int wide;
-  int* expired;
+  Redo redo;
+  int least;                           // magnitudes that pass
   unsigned long long wait_ns;
   const int* hold;
   uint32_t hold_at;
@@ -407,7 +430,8 @@ __device__ __forceinline__ uint64_t smem_desc64(uint32_t addr) {
   return d;
 }
 
-template <int SEGS, int MT>
+// CHECK: the magnitudes' product
+template <int SEGS, int MT, bool CHECK>
 __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_constant__ RMaps maps,
                                                                  const __grid_constant__ RKP k) {
   extern __shared__ unsigned char smem_raw[];
@@ -424,6 +448,9 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  // nothing to do where the FP64 product computes all walkers (flags of launches before this one; a test of each unit's
+  // walker made the loops below a tenth slower)
+  if (!CHECK && k.redo.all_asked(k.batch)) return;
   if (threadIdx.x == 0) {
     for (int s = 0; s < k.stages; ++s) {
       mbar_init(&full[s], 1);
@@ -457,7 +484,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
     if (lane == 0) {  // TMA producer
       uint32_t it = 0, un = 0, s = 0, ph = 0;
       const uint32_t nst = uint32_t(k.stages);
-      uint32_t rows_un = 0;  // units whose rows were all issued, and the slices issued of the next one's
+      uint32_t rows_un = 0;  // where it gave up: units whose rows were all issued, and the slices issued of the next one's
       int rows_kt = 0;
       bool stop = false;
       for (long u = blockIdx.x; u < k.units && !stop; u += gridDim.x, ++un) {
@@ -466,14 +493,17 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
           const bool last = t == k.NT - 1;
           const uint32_t bytes = uint32_t(k.segs * (last ? k.bn_last : k.bn) * RBK);
           const int rb = int(c.w * k.b_bs) + t * k.bn;
-          for (int kt = 0; kt < k.KT; ++kt, ++it) {
-            if (held_back(k.hold, k.hold_at, it, k.wait_ns, s_abort)) {
-              stop = true;
-              break;
-            }
+          // (the loop over slices bounds the tiles with short K: bookkeeping for a stop stays out of it)
+          const int kend = k.hold ? min(k.KT, int(k.hold_at - it)) : k.KT;
+          auto give_up = [&](int issued) {
+            stop = true;
+            rows_un = un + (t > c.t0 || issued == k.KT ? 1u : 0u);
+            rows_kt = t > c.t0 || issued == k.KT ? 0 : issued;
+          };
+          for (int kt = 0; kt < kend; ++kt, ++it) {
             if (t == c.t0) {  // the unit's own rows, slice by slice as the last unit's are done with
               if (!mbar_wait_abort(&rempty[kt], (un & 1) ^ 1, k.wait_ns, s_abort)) {
-                stop = true;
+                give_up(kt);
                 break;
               }
               mbar_expect_tx(&rfull[kt], uint32_t(k.nblk * blk_bytes));
@@ -482,30 +512,30 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
                 // in shared memory: -im, re, im (three blocks) or re, im; in the planes: re, im, -im
                 const int blk = k.nblk == 3 ? (j + 2) % 3 : j;
                 tma_load_3d(dst + j * blk_bytes, &maps.a, &rfull[kt], kt * RBK,
-                            int(blk * k.a_blk) + c.w * k.N + c.e0, c.p);
-              }
-              rows_kt = kt + 1;
-              if (rows_kt == k.KT) {
-                rows_kt = 0;
-                ++rows_un;
+                            int(blk * k.a_blk) + c.w * k.N + c.e0, CHECK ? NMOD : c.p);
               }
             }
             if (!mbar_wait_abort(&empty[s], ph ^ 1, k.wait_ns, s_abort)) {
-              stop = true;
+              give_up(kt + 1);
               break;
             }
             unsigned char* stg = stages0 + s * k.stage;
             mbar_expect_tx(&full[s], bytes);
             for (int sg = 0; sg < k.segs; ++sg)
               tma_load_3d(stg + sg * k.bn * RBK, last ? &maps.b_last : &maps.b, &full[s], kt * RBK,
-                          rb + int(sg * k.b_off1), c.p);
+                          rb + int(sg * k.b_off1), CHECK ? NMOD : c.p);
             if (++s == nst) {
               s = 0;
               ph ^= 1;
             }
           }
+          if (kend < k.KT && !stop) {
+            held_back(k.hold, k.wait_ns, s_abort);
+            give_up(kend);
+          }
         }
       }
+      if (!stop) rows_un = un;
       // every issued copy must have landed before the CTA may exit
       for (uint32_t j = (it > uint32_t(k.stages) ? it - k.stages : 0u); j < it; ++j)
         mbar_wait_for(&full[j % k.stages], (j / k.stages) & 1, kWaitNs);
@@ -605,7 +635,11 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
         const uint32_t taddr = tmem + (uint32_t(q * 32) << 16) + b * BN + uint32_t(mt * 128);
         const int bn = t == k.NT - 1 ? k.bn_last : k.bn, n0 = t * k.bn;
         const int left = min(bn - cc, int(k.ldc) - n0 - cc);
-        if (left > 0) {
+        if (CHECK) {
+          const int r = rg + (lane & 3), a = ag + (lane & 3);  // this lane's own row
+          check64(taddr + uint32_t(cc), min(bn - cc, k.cols - n0 - cc), k.least, r < 2 * k.Np && c.e0 + a < k.N,
+                  k.redo, c.w);
+        } else if (left > 0) {
           uint8_t* rows[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) rows[i] = i < nrow ? row + i * k.ldc + n0 + cc : nullptr;
@@ -618,7 +652,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
   }
   fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *s_abort) report_expiry(k.expired);
+  if (threadIdx.x == 0 && *s_abort) report_expiry(k.redo.call + 1);
   if (warp == 1) {
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -628,7 +662,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
 int make_map(CUtensorMap* m, const Planes& o, long K, int box_rows, int bk = BK) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return record_error(SFQ_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-  cuuint64_t dims[3] = {cuuint64_t(K), cuuint64_t(o.rows), cuuint64_t(NMOD)};
+  cuuint64_t dims[3] = {cuuint64_t(K), cuuint64_t(o.rows), cuuint64_t(kPlanes)};
   cuuint64_t strides[2] = {cuuint64_t(o.ld), cuuint64_t(o.plane)};
   cuuint32_t box[3] = {cuuint32_t(bk), cuuint32_t(box_rows), 1};
   cuuint32_t es[3] = {1, 1, 1};
@@ -645,8 +679,8 @@ int make_map(CUtensorMap* m, const Planes& o, long K, int box_rows, int bk = BK)
 int gemm(const Gemm& g, cudaStream_t st) {
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0 || g.K <= 0) return record_error(SFQ_ERR_SHAPE, "crt gemm: empty product");
   if ((long)g.K * g.segs > kMaxK) return record_error(SFQ_ERR_SHAPE, "crt gemm: K of %ld too long", (long)g.K * g.segs);
-  if (g.parts < 1 || g.parts > 2 || g.segs < 1 || g.segs > 2)
-    return record_error(SFQ_ERR_ARG, "crt gemm: %d parts of %d segments", g.parts, g.segs);
+  if (g.parts < 1 || g.parts > 2 || g.segs < 1 || g.segs > 2 || g.wmod < 1 || !g.redo.call || !g.redo.row)
+    return record_error(SFQ_ERR_ARG, "crt gemm: %d parts of %d segments, walkers %d", g.parts, g.segs, g.wmod);
   KP k{};
   k.M = g.M; k.N = g.N; k.K = g.K; k.batch = g.batch; k.parts = g.parts; k.segs = g.segs;
   k.MT = (g.M + BM - 1) / BM;
@@ -657,7 +691,7 @@ int gemm(const Gemm& g, cudaStream_t st) {
   const int nt0 = (g.N + BN - 1) / BN;
   for (int nt = nt0; nt < nt0 + 6; ++nt) {
     const int bn = ((g.N + nt - 1) / nt + 15) / 16 * 16, tiles = (g.N + bn - 1) / bn;
-    const long waves = ((long)k.MT * g.parts * tiles * g.batch * NMOD + sm_count() - 1) / sm_count();
+    const long waves = ((long)k.MT * g.parts * tiles * g.batch * kPlanes + sm_count() - 1) / sm_count();
     const double cost = double(waves) * (bn + 64);
     if (nt == nt0 || cost < 0.98 * best) {
       best = cost;
@@ -666,14 +700,15 @@ int gemm(const Gemm& g, cudaStream_t st) {
     }
   }
   k.KT = (g.K + BK - 1) / BK;
-  k.tiles = (long)k.MT * k.parts * k.NT * k.batch * NMOD;
+  k.tiles = (long)k.MT * k.parts * k.NT * k.batch * (g.check ? kPlanes : NMOD);
   k.a_bs = g.a_bs; k.b_bs = g.b_bs;
   for (int p = 0; p < 2; ++p)
     for (int s = 0; s < 2; ++s) k.a_off[p][s] = g.a_off[p][s];
   k.b_off[0] = g.b_off[0]; k.b_off[1] = g.b_off[1];
   k.C = g.C; k.ldc = g.ldc; k.c_plane = g.c_plane;
   k.wide = reduce_kind((long)g.K * g.segs);
-  k.expired = g.expired;
+  k.redo = g.redo;
+  k.least = mag_least(g.K, g.segs); k.wmod = g.wmod;
   k.wait_ns = g.wait_ns ? g.wait_ns : kWaitNs;
   k.hold = g.hold; k.hold_at = g.hold_at;
   Maps maps;
@@ -721,7 +756,8 @@ bool plan_walker(const WalkerGemm& g, RKP* out) {
   k.a_blk = g.a_blk; k.b_bs = g.b_bs; k.b_off1 = g.b_off1;
   k.C = g.C; k.ldc = g.ldc; k.c_plane = g.c_plane; k.c_part = g.c_part;
   k.wide = reduce_kind((long)g.K * g.segs);
-  k.expired = g.expired;
+  k.redo = g.redo;
+  k.least = mag_least(g.K, g.segs);
   k.wait_ns = g.wait_ns ? g.wait_ns : kWaitNs;
   k.hold = g.hold; k.hold_at = g.hold_at;
   *out = k;
@@ -737,17 +773,10 @@ bool walker_gemm_fits(int N, int cols, int K, int segs) {
 }
 
 int walker_gemm(const WalkerGemm& g, cudaStream_t st) {
-  if (g.N <= 0 || g.cols <= 0 || g.batch <= 0 || g.K <= 0 || g.segs < 1 || g.segs > 2)
+  if (g.N <= 0 || g.cols <= 0 || g.batch <= 0 || g.K <= 0 || g.segs < 1 || g.segs > 2 || !g.redo.call || !g.redo.row)
     return record_error(SFQ_ERR_SHAPE, "crt walker gemm: empty product");
   RKP k;
   if (!plan_walker(g, &k)) return record_error(SFQ_ERR_SHAPE, "crt walker gemm: N=%d K=%d do not fit", g.N, g.K);
-  // column chunks: whole rows of tiles per unit, split where there are too few walkers to fill the SMs
-  const long base = (long)NMOD * g.batch * k.EC;
-  long cc = (4L * sm_count() + base - 1) / base;
-  cc = std::max<long>(1, std::min<long>(cc, k.NT));
-  k.tpc = int((k.NT + cc - 1) / cc);
-  k.CC = (k.NT + k.tpc - 1) / k.tpc;
-  k.units = base * k.CC;
   RMaps maps;
   int rc;
   if ((rc = make_map(&maps.a, g.A, g.K, k.Np, RBK)) || (rc = make_map(&maps.b, g.B, g.K, k.bn, RBK)) ||
@@ -755,12 +784,22 @@ int walker_gemm(const WalkerGemm& g, cudaStream_t st) {
     return rc;
   constexpr int smem = RSMEM + RBAR + 1024;
   static_assert(smem <= 232448, "shared memory budget");
-  auto kern = k.segs == 2 ? (k.MT == 2 ? crt_walker_kernel<2, 2> : crt_walker_kernel<2, 1>)
-                          : (k.MT == 2 ? crt_walker_kernel<1, 2> : crt_walker_kernel<1, 1>);
-  SFQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  const long grid = k.units < sm_count() ? k.units : sm_count();
-  kern<<<unsigned(grid), kThreads, smem, st>>>(maps, k);
-  SFQ_LAUNCHED();
+  for (int pass = g.check ? 0 : 1; pass < 2; ++pass) {  // the magnitudes, then the moduli of the walkers that passed
+    // column chunks: whole rows of tiles per unit, split where there are too few walkers to fill the SMs
+    auto kern = pass == 0 ? (k.segs == 2 ? (k.MT == 2 ? crt_walker_kernel<2, 2, true> : crt_walker_kernel<2, 1, true>)
+                                         : (k.MT == 2 ? crt_walker_kernel<1, 2, true> : crt_walker_kernel<1, 1, true>))
+                          : (k.segs == 2 ? (k.MT == 2 ? crt_walker_kernel<2, 2, false> : crt_walker_kernel<2, 1, false>)
+                                         : (k.MT == 2 ? crt_walker_kernel<1, 2, false> : crt_walker_kernel<1, 1, false>));
+    SFQ_MAX_SMEM(kern, smem);
+    const long base = (pass == 0 ? 1L : NMOD) * g.batch * k.EC;
+    const long cc = std::max<long>(1, std::min<long>((4L * sm_count() + base - 1) / base, k.NT));
+    k.tpc = int((k.NT + cc - 1) / cc);
+    k.CC = (k.NT + k.tpc - 1) / k.tpc;
+    k.units = base * k.CC;
+    const long grid = k.units < sm_count() ? k.units : sm_count();
+    kern<<<unsigned(grid), kThreads, smem, st>>>(maps, k);
+    SFQ_LAUNCHED();
+  }
   return SFQ_OK;
 }
 

@@ -40,7 +40,7 @@ __device__ __forceinline__ double row_sum(double v, double* sh) {
 template <int TPR>
 __global__ void __launch_bounds__(256) rows_real_kernel(const double* src, long rows, long K, long stride, int8_t* q,
                                                         long ld, long plane, int* e, Redo redo, long per_walker,
-                                                        int vec, long inner, long outer) {
+                                                        int vec, long inner, long outer, double mag) {
   __shared__ double sh[8];
   const long r = TPR == 32 ? (long)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;
   const int t = TPR == 32 ? (threadIdx.x & 31) : threadIdx.x;
@@ -59,40 +59,58 @@ __global__ void __launch_bounds__(256) rows_real_kernel(const double* src, long 
   n2 = row_sum<TPR>(n2, sh);
   // a row of zeros has the norm 0; one whose squares all vanish does not
   const bool any = TPR == 32 ? __any_sync(0xffffffffu, nz != 0.0) : __syncthreads_or(nz != 0.0) != 0;
-  const int ex = row_exponent(n2, any, t == 0 ? flag_of(redo, r, per_walker) : nullptr);
+  const int ex = row_exponent(n2, any, t == 0, redo, per_walker ? r / per_walker : -1);
   if (t == 0) e[r] = ex;
   const double sc = pow2(-ex);
+  const Mag m = mag_of(mag, !any);
   int8_t* qr = q + (inner ? (r / inner) * outer + r % inner : r) * ld;
   for (long k = 4 * t; k < K; k += 4 * TPR) {
     double x[4];
     load4(row, k, K, vec, x);
     Quad qd;
     qd.set(x, sc);
-    qd.store(qr + k, plane);
+    qd.store(qr + k, plane, m);
   }
 }
 
-// Complex rows: the same, both parts with one exponent; blocks re, im (, -im)
-template <int TPR, int NB>
+// Complex rows: the same, the parts with one exponent or each with its own
+template <int TPR, Parts P>
 __global__ void __launch_bounds__(256) rows_cplx_kernel(const cplx* src, long rows, long K, long stride,
                                                         long blk_stride, long inner, long outer, int8_t* q, long ld,
-                                                        long plane, int* e, Redo redo, long per_walker) {
+                                                        long plane, int* e, Redo redo, long per_walker, double mag) {
   __shared__ double sh[8];
   const long r = TPR == 32 ? (long)blockIdx.x * 8 + (threadIdx.x >> 5) : blockIdx.x;
   const int t = TPR == 32 ? (threadIdx.x & 31) : threadIdx.x;
   if (r >= rows) return;
   const cplx* row = src + r * stride;
-  double n2 = 0.0, nz = 0.0;
+  double x2 = 0.0, y2 = 0.0, xm = 0.0, ym = 0.0;
   for (long k = t; k < K; k += TPR) {
     const cplx z = row[k];
-    n2 = fma(z.x, z.x, fma(z.y, z.y, n2));
-    nz = fmax(nz, fmax(fabs(z.x), fabs(z.y)));
+    x2 = fma(z.x, z.x, x2);
+    y2 = fma(z.y, z.y, y2);
+    xm = fmax(xm, fabs(z.x));
+    ym = fmax(ym, fabs(z.y));
   }
-  n2 = row_sum<TPR>(n2, sh);
-  const bool any = TPR == 32 ? __any_sync(0xffffffffu, nz != 0.0) : __syncthreads_or(nz != 0.0) != 0;
-  const int ex = row_exponent(n2, any, t == 0 ? flag_of(redo, r, per_walker) : nullptr);
+  auto any_of = [](bool b) { return TPR == 32 ? __any_sync(0xffffffffu, b) != 0 : __syncthreads_or(b) != 0; };
+  const long wk = per_walker ? r / per_walker : -1;
+  int ex, ey;
+  bool xs, ys;  // parts that are not zeros
+  if (P == Parts::kApart) {
+    x2 = row_sum<TPR>(x2, sh);
+    y2 = row_sum<TPR>(y2, sh);
+    xs = any_of(xm != 0.0);
+    ys = any_of(ym != 0.0);
+    ex = row_exponent(x2, xs, t == 0, redo, wk);
+    ey = row_exponent(y2, ys, t == 0, redo, wk);
+    if (t == 0) e[rows + r] = ey;
+  } else {
+    x2 = row_sum<TPR>(x2 + y2, sh);
+    xs = ys = any_of(xm != 0.0 || ym != 0.0);
+    ex = ey = row_exponent(x2, xs, t == 0, redo, wk);
+  }
   if (t == 0) e[r] = ex;
-  const double sc = pow2(-ex);
+  const double sx = pow2(-ex), sy = pow2(-ey);
+  const Mag mx = mag_of(mag, !xs), my = mag_of(mag, !ys);
   int8_t* qr = q + ((r / inner) * outer + r % inner) * ld;
   for (long k = 4 * t; k < K; k += 4 * TPR) {
     double x[4], y[4];
@@ -103,18 +121,19 @@ __global__ void __launch_bounds__(256) rows_cplx_kernel(const cplx* src, long ro
       y[j] = z.y;
     }
     Quad a;
-    a.set(x, sc);
-    a.store(qr + k, plane);
-    a.set(y, sc);
-    if (NB == 3) a.store2(qr + blk_stride * ld + k, qr + 2 * blk_stride * ld + k, plane);
-    else a.store(qr + blk_stride * ld + k, plane);
+    a.set(x, sx);
+    a.store(qr + k, plane, mx);
+    a.set(y, sy);
+    if (P == Parts::kJointNeg) a.store2(qr + blk_stride * ld + k, qr + 2 * blk_stride * ld + k, plane, my);
+    else a.store(qr + blk_stride * ld + k, plane, my);
   }
 }
 
 // Walkers' components (w, M, N), npol to a walker -> rows (w, a) over the orbitals: a block takes 16 columns of one, their
-// norms first, then 64 orbitals at a time through shared memory (the transpose).
+// norms first, then 64 orbitals at a time through shared memory (the transpose): their residues, and the rows as they are.
 __global__ void __launch_bounds__(256) walkers_in_kernel(const cplx* SM, int W, int npol, int M, int N, int8_t* q,
-                                                         long ld, long plane, int* e, Redo redo) {
+                                                         long ld, long plane, int* e, cplx* rows, Redo redo,
+                                                         double mag) {
   __shared__ cplx tile[64][17];
   __shared__ double sh[16][17];
   __shared__ double scs[16];
@@ -139,7 +158,7 @@ __global__ void __launch_bounds__(256) walkers_in_kernel(const cplx* SM, int W, 
     double s = 0.0;
 #pragma unroll
     for (int j = 0; j < 16; ++j) s += sh[j][ca];
-    const int ex = row_exponent(s, nz[ca] != 0, redo.row + w / npol);
+    const int ex = row_exponent(s, nz[ca] != 0, true, redo, w / npol);
     e[(long)w * N + a0 + ca] = ex;
     scs[ca] = pow2(-ex);
   }
@@ -159,12 +178,17 @@ __global__ void __launch_bounds__(256) walkers_in_kernel(const cplx* SM, int W, 
         x[j] = tile[i4 + j][a].x;
         y[j] = tile[i4 + j][a].y;
       }
-      int8_t* qr = q + ((long)w * N + a0 + a) * ld + i0 + i4;
+      const long r = (long)w * N + a0 + a;
+      int8_t* qr = q + r * ld + i0 + i4;
+      const Mag m = mag_of(mag, nz[a] == 0);
       Quad d;
       d.set(x, scs[a]);
-      d.store(qr, plane);
+      d.store(qr, plane, m);
       d.set(y, scs[a]);
-      d.store(qr + WN * ld, plane);
+      d.store2(qr + WN * ld, qr + 2 * WN * ld, plane, m);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (i0 + i4 + j < M) rows[r * M + i0 + i4 + j] = mk(x[j], y[j]);
     }
   }
 }
@@ -193,7 +217,7 @@ __device__ __forceinline__ void load_e4(const int* e, long n, long N, int eb[4])
 // complex output, 4 columns per thread, 128 per warp; the warp's values go through shared memory so that
 // its stores are whole 512-byte rows
 __global__ void __launch_bounds__(256) out_cplx_kernel(const uint8_t* c, long ldc, long plane, long M, long N,
-                                                       const int* eA, const int* eB, Scale s, cplx* out,
+                                                       const int* eA, long im0, const int* eB, Scale s, cplx* out,
                                                        long ldo) {
   __shared__ cplx sh[8][130];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -204,7 +228,7 @@ __global__ void __launch_bounds__(256) out_cplx_kernel(const uint8_t* c, long ld
     int eb[4];
     load_e4(eB, n, N, eb);
     const Vals re = values4(c + m * ldc + n, plane, eA[m], eb, s);
-    const Vals im = values4(c + (M + m) * ldc + n, plane, eA[m], eb, s);
+    const Vals im = values4(c + (M + m) * ldc + n, plane, eA[im0 + m], eb, s);
 #pragma unroll
     for (int j = 0; j < 4; ++j) sh[warp][4 * lane + j] = mk(re.v[j], im.v[j]);
   }
@@ -232,13 +256,12 @@ __global__ void __launch_bounds__(256) out_real_kernel(const uint8_t* c, long ld
 // One Taylor term (see taylor_update) of R rows (w, a): items of four columns, both parts, over the R rows
 // together, so that a block's threads stay busy whatever M is (100 items a row at M = 400: one row in a
 // block of 128 threads left a fifth of the lanes idle).  Each complex element: 30 residues in, S in and
-// out, 45 residues out; a row's T waits in shared memory for its norm.
-template <bool FIRST, bool LAST>
+// out, 48 residues and magnitudes out; a row's T waits in shared memory for its norm.
+template <bool LAST>
 __global__ void __launch_bounds__(256, 4) taylor_kernel(const uint8_t* c, long ldc, long plane, long WN, int N, int M,
-                                                     Scale sc, const int* eA, const int* eB, int eB_per_w,
-                                                     double* S, int8_t* q, long ld, long qplane, int* e, Redo redo,
-                                                     int R) {
-  extern __shared__ double rows[];  // [R][2][M4] T (S when LAST), then [R * M4 / 4] squared norms, [R] scales
+                                                     Scale sc, const int* eA, const int* eB, cplx* S, int8_t* q,
+                                                     long ld, long qplane, int* e, Redo redo, int R, double mag) {
+  extern __shared__ double rows[];  // [R][2][M4] T, then [R * M4 / 4] squared norms, [R] scales (negative: zeros)
   const int M4 = (M + 3) / 4 * 4, q4 = M4 / 4;
   double* part = rows + 2 * R * M4;
   double* scs = part + R * q4;
@@ -247,42 +270,31 @@ __global__ void __launch_bounds__(256, 4) taylor_kernel(const uint8_t* c, long l
   for (int it = threadIdx.x; it < items; it += 256) {
     const int rr = it / q4, j0 = 4 * (it - rr * q4);
     const long r = r0 + rr;
-    const int* eb0 = eB + (eB_per_w ? (r / N) * M : 0);
     int eb[4];
-    load_e4(eb0, j0, M, eb);
+    load_e4(eB + (r / N) * M, j0, M, eb);
     const int ea = eA[r];
     const Vals re = values4(c + r * ldc + j0, plane, ea, eb, sc);
     const Vals im = values4(c + (WN + r) * ldc + j0, plane, ea, eb, sc);
-    double* Sr = S + r * M + j0;
-    double* Si = S + (WN + r) * M + j0;
+    cplx* Sr = S + r * M + j0;
     double n2 = 0.0, nz = 0.0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       double x = 0.0, y = 0.0;
       if (j0 + j < M) {
-        x = FIRST ? re.v[j] : -im.v[j];  // T = (i / k) C
-        y = FIRST ? im.v[j] : re.v[j];
-        if (FIRST) {
-          Sr[j] = x;
-          Si[j] = y;
-        } else {
-          const double sx = Sr[j] + x, sy = Si[j] + y;
-          if (LAST) {
-            x = sx;
-            y = sy;
-          } else {
-            Sr[j] = sx;
-            Si[j] = sy;
-          }
-        }
+        x = -im.v[j];  // T = (i / k) C
+        y = re.v[j];
+        Sr[j] = cadd(Sr[j], mk(x, y));
       }
-      n2 = fma(x, x, fma(y, y, n2));
-      nz = fmax(nz, fmax(fabs(x), fabs(y)));
-      rows[(2 * rr) * M4 + j0 + j] = x;
-      rows[(2 * rr + 1) * M4 + j0 + j] = y;
+      if (!LAST) {
+        n2 = fma(x, x, fma(y, y, n2));
+        nz = fmax(nz, fmax(fabs(x), fabs(y)));
+        rows[(2 * rr) * M4 + j0 + j] = x;
+        rows[(2 * rr + 1) * M4 + j0 + j] = y;
+      }
     }
-    part[it] = n2 == 0.0 && nz != 0.0 ? 1e-320 : n2;  // squares that vanish: not a row of zeros
+    if (!LAST) part[it] = n2 == 0.0 && nz != 0.0 ? 1e-320 : n2;  // squares that vanish: not a row of zeros
   }
+  if (LAST) return;
   __syncthreads();
   for (int rr = threadIdx.x >> 5; rr < nr; rr += 8) {
     double n2 = 0.0;
@@ -290,39 +302,40 @@ __global__ void __launch_bounds__(256, 4) taylor_kernel(const uint8_t* c, long l
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
     if ((threadIdx.x & 31) == 0) {
-      const int ex = row_exponent(n2, n2 != 0.0, redo.row + (r0 + rr) / N);
+      const int ex = row_exponent(n2, n2 != 0.0, true, redo, (r0 + rr) / N);
       e[r0 + rr] = ex;
-      scs[rr] = pow2(-ex);
+      scs[rr] = n2 == 0.0 ? -1.0 : pow2(-ex);
     }
   }
   __syncthreads();
   for (int it = threadIdx.x; it < items; it += 256) {  // this thread's own entries again
     const int rr = it / q4, j0 = 4 * (it - rr * q4);
     int8_t* qr = q + (r0 + rr) * ld + j0;
+    const Mag m = mag_of(mag, scs[rr] < 0.0);
     Quad d;
     d.set(rows + (2 * rr) * M4 + j0, scs[rr]);
-    d.store(qr, qplane);
+    d.store(qr, qplane, m);
     d.set(rows + (2 * rr + 1) * M4 + j0, scs[rr]);
-    if (LAST) d.store(qr + WN * ld, qplane);
-    else d.store2(qr + WN * ld, qr + 2 * WN * ld, qplane);
+    d.store2(qr + WN * ld, qr + 2 * WN * ld, qplane, m);
   }
 }
 
 // One block per (n, w): the walker's T of this n, reconstructed once into shared memory, then its
 // exchange trace.  Bound by the reconstruction (two residue groups per complex element) and its reads.
 __global__ void __launch_bounds__(256) exx_kernel(const uint8_t* c, long ldc, long plane, long WN, int N, int N4,
-                                                  const int* eA, const int* eB, int n0, int Nc, cplx* exxn, cplx* kl,
-                                                  int nup, Scale sc) {
+                                                  const int* eA, long im0, const int* eB, int n0, int Nc, cplx* exxn,
+                                                  cplx* kl, int nup, Redo redo, Scale sc) {
   extern __shared__ cplx T[];  // T[b][a], rows of P
   __shared__ cplx red[2][8];
   const int n = blockIdx.x, w = blockIdx.y, P = N | 1, q4 = N4 / 4;
+  if (redo.asked(w)) return;
   for (int it = threadIdx.x; it < N * q4; it += 256) {
     const int b = it / q4, a = 4 * (it % q4);
     const long r = (long)w * N + b, col = (long)n * N4 + a;
     int eb[4];
     load_e4(eB + (long)n * N, a, N, eb);
     const Vals re = values4(c + r * ldc + col, plane, eA[r], eb, sc);
-    const Vals im = values4(c + (WN + r) * ldc + col, plane, eA[r], eb, sc);
+    const Vals im = values4(c + (WN + r) * ldc + col, plane, eA[im0 + r], eb, sc);
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (a + j < N) T[b * P + a + j] = mk(re.v[j], im.v[j]);
@@ -358,31 +371,6 @@ __global__ void __launch_bounds__(256) exx_kernel(const uint8_t* c, long ldc, lo
   }
 }
 
-// SM[w][j][a] from rows (part, w, a), columns j: 32 x 32 tiles transposed through shared memory
-__global__ void __launch_bounds__(256) walkers_out_kernel(const uint8_t* c, long ldc, long plane, long WN, int M,
-                                                          int N, int npol, const int* eA, const int* eB, cplx* SM,
-                                                          Redo redo, Scale sc) {
-  __shared__ cplx tile[32][33];
-  const int w = blockIdx.z, j0 = blockIdx.x * 32, a0 = blockIdx.y * 32;
-  if (asked_again(redo, w / npol)) return;
-  {
-    const int a = threadIdx.x >> 3, j4 = 4 * (threadIdx.x & 7);
-    if (a0 + a < N && j0 + j4 < M) {
-      const long r = (long)w * N + a0 + a;
-      int eb[4];
-      load_e4(eB, j0 + j4, M, eb);
-      const Vals re = values4(c + r * ldc + j0 + j4, plane, eA[r], eb, sc);
-      const Vals im = values4(c + (WN + r) * ldc + j0 + j4, plane, eA[r], eb, sc);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) tile[j4 + j][a] = mk(re.v[j], im.v[j]);
-    }
-  }
-  __syncthreads();
-  const int a = threadIdx.x & 31;
-  for (int j = threadIdx.x >> 5; j < 32; j += 8)
-    if (j0 + j < M && a0 + a < N) SM[((long)w * M + j0 + j) * N + a0 + a] = tile[j][a];
-}
-
 }  // namespace
 
 Scale scale_of(double alpha) {
@@ -399,35 +387,44 @@ int rows_real(const double* src, long rows, long K, long stride, const Planes& o
   const int vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0 && stride % 2 == 0;
   if (K < 1024)
     rows_real_kernel<32><<<ceil_div(rows, 8), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, redo,
-                                                            per_walker, vec, inner, outer);
+                                                            per_walker, vec, inner, outer, mag_scale(K));
   else
     rows_real_kernel<256><<<unsigned(rows), 256, 0, st>>>(src, rows, K, stride, o.q, o.ld, o.plane, o.e, redo,
-                                                          per_walker, vec, inner, outer);
+                                                          per_walker, vec, inner, outer, mag_scale(K));
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
 
-int rows_cplx(const cplx* src, long rows, long K, long stride, int nb, long blk, long inner, long outer,
+int rows_cplx(const cplx* src, long rows, long K, long stride, Parts parts, long blk, long inner, long outer,
               const Planes& o, Redo redo, long per_walker, cudaStream_t st) {
   if (rows <= 0 || K <= 0) return SFQ_OK;
   const bool wide = K >= 1024;
   const unsigned grid = wide ? unsigned(rows) : unsigned(ceil_div(rows, 8));
-  auto k = wide ? (nb == 3 ? rows_cplx_kernel<256, 3> : rows_cplx_kernel<256, 2>)
-                : (nb == 3 ? rows_cplx_kernel<32, 3> : rows_cplx_kernel<32, 2>);
-  k<<<grid, 256, 0, st>>>(src, rows, K, stride, blk, inner, outer, o.q, o.ld, o.plane, o.e, redo, per_walker);
+  auto k = parts == Parts::kApart ? (wide ? rows_cplx_kernel<256, Parts::kApart> : rows_cplx_kernel<32, Parts::kApart>)
+           : parts == Parts::kJoint
+               ? (wide ? rows_cplx_kernel<256, Parts::kJoint> : rows_cplx_kernel<32, Parts::kJoint>)
+               : (wide ? rows_cplx_kernel<256, Parts::kJointNeg> : rows_cplx_kernel<32, Parts::kJointNeg>);
+  k<<<grid, 256, 0, st>>>(src, rows, K, stride, blk, inner, outer, o.q, o.ld, o.plane, o.e, redo, per_walker,
+                          mag_scale(K));
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
 
-int walkers_in(const cplx* SM, int W, int npol, int M, int N, const Planes& o, Redo redo, cudaStream_t st) {
-  walkers_in_kernel<<<dim3((N + 15) / 16, W * npol), 256, 0, st>>>(SM, W * npol, npol, M, N, o.q, o.ld, o.plane, o.e, redo);
+int pass_padding(const Planes& o, cudaStream_t st) {
+  SFQ_CUDA_TRY(cudaMemsetAsync(o.q + NMOD * o.plane, 127, (size_t)o.rows * o.ld, st));
+  return SFQ_OK;
+}
+
+int walkers_in(const cplx* SM, int W, int npol, int M, int N, const Planes& o, cplx* S, Redo redo, cudaStream_t st) {
+  walkers_in_kernel<<<dim3((N + 15) / 16, W * npol), 256, 0, st>>>(SM, W * npol, npol, M, N, o.q, o.ld, o.plane, o.e, S,
+                                                                   redo, mag_scale(M));
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
 
-int out_cplx(const Out& c, long M, long N, const int* eA, const int* eB, double alpha, cplx* out, long ldo,
+int out_cplx(const Out& c, long M, long N, const int* eA, long im, const int* eB, double alpha, cplx* out, long ldo,
              cudaStream_t st) {
-  out_cplx_kernel<<<dim3(ceil_div(N, 1024), unsigned(M)), 256, 0, st>>>(c.q, c.ldc, c.plane, M, N, eA, eB, scale_of(alpha), out,
+  out_cplx_kernel<<<dim3(ceil_div(N, 1024), unsigned(M)), 256, 0, st>>>(c.q, c.ldc, c.plane, M, N, eA, im, eB, scale_of(alpha), out,
                                                                         ldo);
   SFQ_LAUNCHED();
   return SFQ_OK;
@@ -444,8 +441,8 @@ int out_real(const Out& c, long M, long N, const int* eA, const int* eB, double 
 // of one row of 4096 orbitals, the most that the propagation takes this way
 constexpr size_t kTaylorSmem = sizeof(double) * (2 * 4096 + 4096 / 4 + 1);
 
-int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int* eA, const int* eB, int eB_per_w,
-                  double* S, const Planes& o, Redo redo, cudaStream_t st) {
+int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int* eA, const int* eB, cplx* S,
+                  const Planes& o, Redo redo, cudaStream_t st) {
   const int M4 = (M + 3) / 4 * 4, q4 = M4 / 4;
   const long WN = (long)W * N;
   // rows per block: the count up to 8 that wastes least of the last round of 256 items, in 48 KB of rows
@@ -459,31 +456,22 @@ int taylor_update(const Out& c, int W, int N, int M, int k, bool last, const int
     }
   }
   const size_t sm = sizeof(double) * (2L * R * M4 + (long)R * q4 + R);
-  const double ik = k > 0 ? 1.0 / double(k) : 1.0;
-  auto kern = k == 0 ? taylor_kernel<true, false> : last ? taylor_kernel<false, true> : taylor_kernel<false, false>;
+  auto kern = last ? taylor_kernel<true> : taylor_kernel<false>;
   if (sm > kTaylorSmem) return record_error(SFQ_ERR_SHAPE, "crt taylor: M=%d too large", M);
   SFQ_MAX_SMEM(kern, kTaylorSmem);
-  kern<<<unsigned((WN + R - 1) / R), 256, sm, st>>>(c.q, c.ldc, c.plane, WN, N, M, scale_of(ik), eA, eB, eB_per_w, S, o.q, o.ld,
-                                                    o.plane, o.e, redo, R);
+  kern<<<unsigned((WN + R - 1) / R), 256, sm, st>>>(c.q, c.ldc, c.plane, WN, N, M, scale_of(1.0 / double(k)), eA, eB, S,
+                                                    o.q, o.ld, o.plane, o.e, redo, R, mag_scale(M));
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
 
-int exx_reduce(const Out& c, int W, int N, int N4, int nv, int n0, int Nc, const int* eA, const int* eB, cplx* exxn,
-               cplx* kl, int nup, cudaStream_t st) {
+int exx_reduce(const Out& c, int W, int N, int N4, int nv, int n0, int Nc, const int* eA, long im, const int* eB,
+               cplx* exxn, cplx* kl, int nup, Redo redo, cudaStream_t st) {
   const size_t sm = sizeof(cplx) * N * (N | 1);
   if (N > kExxMaxN) return record_error(SFQ_ERR_SHAPE, "crt exx: N=%d above %d", N, kExxMaxN);
   SFQ_MAX_SMEM(exx_kernel, sizeof(cplx) * kExxMaxN * (kExxMaxN | 1));
-  exx_kernel<<<dim3(nv, W), 256, sm, st>>>(c.q, c.ldc, c.plane, (long)W * N, N, N4, eA, eB, n0, Nc, exxn, kl,
-                                           nup < 0 ? N : nup, scale_of(1.0));
-  SFQ_LAUNCHED();
-  return SFQ_OK;
-}
-
-int walkers_out(const Out& c, int W, int npol, int M, int N, const int* eA, const int* eB, cplx* SM, Redo redo,
-                cudaStream_t st) {
-  walkers_out_kernel<<<dim3((M + 31) / 32, (N + 31) / 32, W * npol), 256, 0, st>>>(
-      c.q, c.ldc, c.plane, (long)W * npol * N, M, N, npol, eA, eB, SM, redo, scale_of(1.0));
+  exx_kernel<<<dim3(nv, W), 256, sm, st>>>(c.q, c.ldc, c.plane, (long)W * N, N, N4, eA, im, eB, n0, Nc, exxn, kl,
+                                           nup < 0 ? N : nup, redo, scale_of(1.0));
   SFQ_LAUNCHED();
   return SFQ_OK;
 }

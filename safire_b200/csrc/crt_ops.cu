@@ -17,23 +17,23 @@ namespace {
 constexpr size_t kChunkBytes = size_t(3) << 29;  // 1.5 GiB
 
 size_t vbias_row_bytes(long K, bool l_cplx, int W) {
-  return (size_t)NMOD * ((l_cplx ? 2 : 1) * (size_t)ld_of(K) + 2 * (size_t)W) + sizeof(int);
+  return (size_t)kPlanes * (l_cplx ? 2 : 1) * ld_of(K) + (size_t)NMOD * 2 * W + sizeof(int);
 }
-size_t vhs_row_bytes(int W, int Nc) { return (size_t)NMOD * ((size_t)ld_of(Nc) + 2 * (size_t)W) + sizeof(int); }
+size_t vhs_row_bytes(int W, int Nc) { return (size_t)kPlanes * ld_of(Nc) + (size_t)NMOD * 2 * W + sizeof(int); }
 // rows per chunk: the whole operand, or equal chunks of a multiple of 16 rows within kChunkBytes
 long chunk_rows(long rows, size_t row_bytes) {
   const long most = std::max<long>(256, long(kChunkBytes / row_bytes));
   const long n = (rows + most - 1) / most;
   return n <= 1 ? rows : ((rows + n - 1) / n + 15) / 16 * 16;
 }
-size_t slack() { return 256 * (2 * NMOD + 4); }  // plane roundings
+size_t slack() { return 256 * (2 * kPlanes + 4); }  // plane roundings
 }  // namespace
 
 // ---- force bias -----------------------------------------------------------------------------------
 size_t vbias_crt_bytes(int W, int N, int M, int Nc, bool l_cplx, bool prepared) {
   const long K = (long)N * M;
   const long nb = prepared ? Nc : chunk_rows(Nc, vbias_row_bytes(K, l_cplx, W));
-  size_t b = flag_bytes(W) + planes_bytes((l_cplx ? 3L : 2L) * W, K) + exps_bytes(W) + out_bytes(2L * W, nb);
+  size_t b = flag_bytes(W) + planes_bytes((l_cplx ? 3L : 2L) * W, K) + exps_bytes(2L * W) + out_bytes(2L * W, nb);
   if (!prepared) b += planes_bytes((l_cplx ? 2L : 1L) * nb, K) + exps_bytes(nb);
   return b + slack();
 }
@@ -53,14 +53,14 @@ int vbias_crt(const cplx* G, const void* Lnak, bool l_cplx, const Planes* Lq, cp
   const Redo redo = lay_out_flags(at, W);
   int rc;
   SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
-  Planes A = lay_out(at, (l_cplx ? 3L : 2L) * W, K, W);
+  Planes A = lay_out(at, (l_cplx ? 3L : 2L) * W, K, 2L * W);
   Planes B = Lq ? *Lq : lay_out(at, (l_cplx ? 2L : 1L) * nb, K, nb);
   Out C = lay_out_c(at, 2L * W, nb);
-  if ((rc = rows_cplx(G, W, K, K, l_cplx ? 3 : 2, W, W, W, A, redo, 1, st))) return rc;
+  if ((rc = rows_cplx(G, W, K, K, l_cplx ? Parts::kJointNeg : Parts::kApart, W, W, W, A, redo, 1, st))) return rc;
   for (long n0 = 0; n0 < Nc; n0 += nb) {
     const long n = std::min<long>(nb, Nc - n0);
     if (!Lq) {
-      if (l_cplx) rc = rows_cplx((const cplx*)Lnak + n0 * K, n, K, K, 2, nb, n, n, B, redo, 0, st);
+      if (l_cplx) rc = rows_cplx((const cplx*)Lnak + n0 * K, n, K, K, Parts::kJoint, nb, n, n, B, redo, 0, st);
       else rc = rows_real((const double*)Lnak + n0 * K, n, K, K, B, redo, 0, st);
       if (rc) return rc;
     }
@@ -73,11 +73,11 @@ int vbias_crt(const cplx* G, const void* Lnak, bool l_cplx, const Planes* Lq, cp
     } else {
       g.M = 2 * W;
     }
-    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.expired = redo.call + 1;
+    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.redo = redo; g.wmod = W;
     Out c = C;
     c.ldc = g.ldc;
     if ((rc = crt::gemm(g, st))) return rc;
-    if ((rc = out_cplx(c, W, n, A.e, B.e, a, v + n0, Nc, st))) return rc;
+    if ((rc = out_cplx(c, W, n, A.e, l_cplx ? 0 : W, B.e, a, v + n0, Nc, st))) return rc;
   }
   return vbias(G, Lnak, l_cplx, v, W, N, M, Nc, a, st, &redo);
 }
@@ -85,7 +85,7 @@ int vbias_crt(const cplx* G, const void* Lnak, bool l_cplx, const Planes* Lq, cp
 // ---- vHS --------------------------------------------------------------------------------------
 size_t vhs_crt_bytes(int W, long rows, int Nc, bool prepared) {
   const long nb = chunk_rows(rows, vhs_row_bytes(W, Nc));
-  size_t b = flag_bytes(W) + planes_bytes(2L * W, Nc) + exps_bytes(W) + out_bytes(2L * W, nb);
+  size_t b = flag_bytes(W) + planes_bytes(2L * W, Nc) + exps_bytes(2L * W) + out_bytes(2L * W, nb);
   if (!prepared) b += planes_bytes(nb, Nc) + exps_bytes(nb);
   return b + slack();
 }
@@ -106,21 +106,21 @@ int vhs_crt(const double* L, long rows, const Planes* Lq, const cplx* X, cplx* V
   const Redo redo = lay_out_flags(at, W);
   int rc;
   SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
-  Planes A = lay_out(at, 2L * W, Nc, W);
+  Planes A = lay_out(at, 2L * W, Nc, 2L * W);
   Planes B = Lq ? *Lq : lay_out(at, nb, Nc, nb);
   Out C = lay_out_c(at, 2L * W, nb);
-  if ((rc = rows_cplx(X, W, Nc, Nc, 2, W, W, W, A, redo, 1, st))) return rc;
+  if ((rc = rows_cplx(X, W, Nc, Nc, Parts::kApart, W, W, W, A, redo, 1, st))) return rc;
   for (long r0 = 0; r0 < rows; r0 += nb) {
     const long n = std::min<long>(nb, rows - r0);
     if (!Lq && (rc = rows_real(L + r0 * Nc, n, Nc, Nc, B, redo, 0, st))) return rc;
     crt::Gemm g;
     g.A = A; g.B = B; g.M = 2 * W; g.N = int(n); g.K = Nc;
     g.b_off[0] = Lq ? r0 : 0;
-    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.expired = redo.call + 1;
+    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.redo = redo; g.wmod = W;
     Out c = C;
     c.ldc = g.ldc;
     if ((rc = crt::gemm(g, st))) return rc;
-    if ((rc = out_cplx(c, W, n, A.e, B.e + (Lq ? r0 : 0), a, V + r0, rows, st))) return rc;
+    if ((rc = out_cplx(c, W, n, A.e, W, B.e + (Lq ? r0 : 0), a, V + r0, rows, st))) return rc;
   }
   return vhs_rows(L, rows, X, V, W, Nc, a, st, &redo);
 }
@@ -128,8 +128,8 @@ int vhs_crt(const double* L, long rows, const Planes* Lq, const cplx* X, cplx* V
 // ---- propagation --------------------------------------------------------------------------------
 namespace {
 size_t prop_walker_bytes(int M, int Nr) {  // Nr = npol * N rows per walker
-  return (size_t)NMOD * (3 * (size_t)Nr * ld_of(M) + 2 * (size_t)M * ld_of(M) + 2 * (size_t)Nr * ldc_of(M)) +
-         16 * (size_t)Nr * M + 4 * (size_t)(Nr + M);
+  return (size_t)kPlanes * (3 * (size_t)Nr * ld_of(M) + 2 * (size_t)M * ld_of(M)) + (size_t)NMOD * 2 * Nr * ldc_of(M) +
+         32 * (size_t)Nr * M + 4 * (size_t)(Nr + M);
 }
 int prop_chunk(int W, int M, int Nr) {
   const long most = std::max<long>(1, long(kChunkBytes / prop_walker_bytes(M, Nr)));
@@ -138,14 +138,13 @@ int prop_chunk(int W, int M, int Nr) {
 }
 }  // namespace
 
-size_t propagate_crt_bytes(int W, int M, int N, int npol, bool prepared) {
+size_t propagate_crt_bytes(int W, int M, int N, int npol) {
   const int Nr = N * npol, wc = prop_chunk(W, M, Nr);
   const long R = (long)wc * Nr;
-  size_t b = planes_bytes(3 * R, M) + exps_bytes(R) + planes_bytes(2L * wc * M, M) + exps_bytes((long)wc * M) +
-             out_bytes(2 * R, M) + align256(16 * (size_t)R * M);
-  b = std::max(b, 3 * align256(sizeof(cplx) * (size_t)R * M));  // the FP64 chain's buffers share the space
-  if (!prepared) b += planes_bytes(M, M) + exps_bytes(M);
-  return flag_bytes(W) + b + slack();
+  const size_t blk = align256(sizeof(cplx) * (size_t)R * M);
+  const size_t b = planes_bytes(3 * R, M) + exps_bytes(R) + planes_bytes(2L * wc * M, M) + exps_bytes((long)wc * M) +
+                   out_bytes(2 * R, M) + blk;
+  return flag_bytes(wc) + blk + std::max(b, 2 * blk) + slack();  // the FP64 terms' buffers share the space
 }
 
 // The conversions of V and of the Taylor terms grow as M^2 and M N, the products as M^2 N: 1.9x at M = 400 with
@@ -157,45 +156,51 @@ bool propagate_crt_ok(int W, int M, int N, int npol, bool p_cplx, int order) {
          walker_gemm_fits(N * npol, M, M, 2);
 }
 
-int propagate_crt(cplx* SM, const double* P1, const Planes* P1q, const cplx* V, int W, int M, int N, int npol,
-                  int order, char* ws, cudaStream_t st) {
+// P1 is the identity and a little more: a product with it keeps the small elements of the walkers to their own bits in
+// FP64, and would fail the magnitudes' check here, so both stay on the FP64 tensor pipe (4 M^2 N of 64 M^2 N flops each).
+int propagate_crt(cplx* SM, const double* P1, const cplx* V, int W, int M, int N, int npol, int order, char* ws,
+                  cudaStream_t st) {
   const int Nr = N * npol, wc = prop_chunk(W, M, Nr);
+  const long MN = (long)M * N;
   char* at = ws;
-  const Redo redo = lay_out_flags(at, W);
+  const Redo rw = lay_out_flags(at, wc);
   int rc;
-  SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
-  Planes P = P1q ? *P1q : lay_out(at, M, M, M);
-  if (!P1q && (rc = rows_real(P1, M, M, M, P, redo, 0, st))) return rc;
   for (int w0 = 0; w0 < W; w0 += wc) {
     const int w = std::min(wc, W - w0);
     const long R = (long)w * Nr;
-    const Redo rw{redo.call, redo.row + w0};
+    const size_t blk = align256(sizeof(cplx) * (size_t)R * M);
+    SFQ_CUDA_TRY(cudaMemsetAsync(rw.call, 0, flag_bytes(wc), st));
     cplx* S0 = SM + (long)w0 * Nr * M;
     const cplx* Vw = V + (long)w0 * M * M;
-    char* o = at;
+    cplx* TMN = reinterpret_cast<cplx*>(at);
+    char* o = at + blk;
     Planes A = lay_out(o, 3 * R, M, R);
     Planes B = lay_out(o, 2L * w * M, M, (long)w * M);
     Out C = lay_out_c(o, 2 * R, M);
-    double* S = reinterpret_cast<double*>(o);
-    if ((rc = walkers_in(S0, w, npol, M, N, A, rw, st))) return rc;
-    if ((rc = rows_cplx(Vw, (long)w * M, M, M, 2, M, M, 2L * M, B, rw, M, st))) return rc;
-    crt::WalkerGemm p1;  // rows (part, w, a) of P1 SM
-    p1.A = A; p1.B = P; p1.N = Nr; p1.cols = M; p1.K = M; p1.batch = w; p1.segs = 1;
-    p1.a_blk = R; p1.C = C.q; p1.ldc = C.ldc; p1.c_plane = C.plane; p1.c_part = R; p1.expired = redo.call + 1;
-    if ((rc = crt::walker_gemm(p1, st))) return rc;
-    if ((rc = taylor_update(C, w, Nr, M, 0, false, A.e, P.e, 0, S, A, rw, st))) return rc;
-    crt::WalkerGemm t = p1;  // C = V T: re = Vr Tr + Vi (-Ti), im = Vr Ti + Vi Tr
-    t.B = B; t.segs = 2; t.b_bs = 2L * M; t.b_off1 = M;
+    cplx* S = reinterpret_cast<cplx*>(o);  // rows (w, q, a) over the orbitals
+    if ((rc = p1_apply(P1, false, S0, TMN, w, npol, M, N, st))) return rc;
+    if ((rc = walkers_in(TMN, w, npol, M, N, A, S, rw, st))) return rc;
+    if ((rc = rows_cplx(Vw, (long)w * M, M, M, Parts::kJoint, M, M, 2L * M, B, rw, M, st))) return rc;
+    crt::WalkerGemm t;  // C = V T: re = Vr Tr + Vi (-Ti), im = Vr Ti + Vi Tr
+    t.A = A; t.B = B; t.N = Nr; t.cols = M; t.K = M; t.batch = w; t.segs = 2;
+    t.a_blk = R; t.b_bs = 2L * M; t.b_off1 = M;
+    t.C = C.q; t.ldc = C.ldc; t.c_plane = C.plane; t.c_part = R; t.redo = rw;
     for (int k = 1; k <= order; ++k) {
       if ((rc = crt::walker_gemm(t, st))) return rc;
-      if ((rc = taylor_update(C, w, Nr, M, k, k == order, A.e, B.e, 1, S, A, rw, st))) return rc;
+      if ((rc = taylor_update(C, w, Nr, M, k, k == order, A.e, B.e, S, A, rw, st))) return rc;
     }
-    if ((rc = crt::walker_gemm(p1, st))) return rc;
-    if ((rc = walkers_out(C, w, npol, M, N, A.e, P.e, S0, rw, st))) return rc;
-    const size_t blk = align256(sizeof(cplx) * (size_t)R * M);
-    if ((rc = propagate(S0, P1, false, Vw, w, M, N, order, (cplx*)at, (cplx*)(at + blk), (cplx*)(at + 2 * blk), st,
-                        npol, &rw)))
-      return rc;
+    for (int q = 0; q < npol; ++q) {  // SM = P1 S of the walkers that passed
+      GemmDesc d;
+      d.M = M; d.N = N; d.K = M; d.batch = w;
+      d.A = P1; d.sAm = M; d.sAk = 1;
+      d.B = S + q * MN; d.sBk = 1; d.sBn = M; d.sBb = npol * MN; d.b_cplx = true;
+      d.C = S0 + q * MN; d.sCm = N; d.sCn = 1; d.sCb = npol * MN;
+      d.redo = rw; d.redo_rest = true;
+      if ((rc = gemm_f64(d, st))) return rc;
+    }
+    cplx* T1 = reinterpret_cast<cplx*>(at + blk);
+    if ((rc = taylor(TMN, Vw, w, M, N, npol, order, T1, reinterpret_cast<cplx*>(at + 2 * blk), st, &rw))) return rc;
+    if ((rc = p1_apply(P1, false, TMN, S0, w, npol, M, N, st, &rw))) return rc;
   }
   return SFQ_OK;
 }
@@ -204,12 +209,12 @@ int propagate_crt(cplx* SM, const double* P1, const Planes* P1q, const cplx* V, 
 namespace {
 int n4_of(int N) { return (N + 3) / 4 * 4; }
 size_t energy_n_bytes(int W, int N, int M, bool l_cplx) {  // per Cholesky vector
-  return (size_t)NMOD * ((l_cplx ? 2 : 1) * (size_t)n4_of(N) * ld_of(M) + 2 * (size_t)W * N * n4_of(N)) +
+  return (size_t)kPlanes * (l_cplx ? 2 : 1) * n4_of(N) * ld_of(M) + (size_t)NMOD * 2 * W * N * n4_of(N) +
          sizeof(int) * N;
 }
 size_t energy_fixed_bytes(int W, int N, int M, bool l_cplx) {
   const long R = (long)W * N;
-  return flag_bytes(W) + planes_bytes((l_cplx ? 3 : 2) * R, M) + exps_bytes(R) + slack();
+  return flag_bytes(W) + planes_bytes((l_cplx ? 3 : 2) * R, M) + exps_bytes(2 * R) + slack();
 }
 int energy_nv(int W, int N, int M, int Nc, bool l_cplx) {
   const long most = std::max<long>(1, long(kChunkBytes / energy_n_bytes(W, N, M, l_cplx)));
@@ -243,25 +248,26 @@ int energy_crt(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool 
   const Redo redo = lay_out_flags(at, W);
   SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
   if ((rc = energy_e1(G, haj, E3, W, N, M, E0, scl, addH1, st))) return rc;
-  const Planes A = lay_out(at, (l_cplx ? 3 : 2) * R, M, R);
+  const Planes A = lay_out(at, (l_cplx ? 3 : 2) * R, M, 2 * R);
   const Planes B = lay_out(at, (l_cplx ? 2L : 1L) * nv * N4, M, (long)nv * N);
   const Out C = lay_out_c(at, 2 * R, (long)nv * N4);
-  if ((rc = rows_cplx(G, R, M, M, l_cplx ? 3 : 2, R, R, R, A, redo, N, st))) return rc;
+  if ((rc = rows_cplx(G, R, M, M, l_cplx ? Parts::kJointNeg : Parts::kApart, R, R, R, A, redo, N, st))) return rc;
   for (int n0 = 0; n0 < Nc; n0 += nv) {
     const int n = std::min(nv, Nc - n0);
     // rows (n, a) of Lnak on rows n N4 + a: the columns of a vector then start on words
     const long off = (long)n0 * N * M;
-    if (l_cplx) rc = rows_cplx((const cplx*)Lnak + off, (long)n * N, M, M, 2, (long)nv * N4, N, N4, B, redo, 0, st);
+    if (n0 == 0 && N4 != N && (rc = pass_padding(B, st))) return rc;
+    if (l_cplx) rc = rows_cplx((const cplx*)Lnak + off, (long)n * N, M, M, Parts::kJoint, (long)nv * N4, N, N4, B, redo, 0, st);
     else rc = rows_real((const double*)Lnak + off, (long)n * N, M, M, B, redo, 0, st, N, N4);
     if (rc) return rc;
     crt::WalkerGemm g;
     g.A = A; g.B = B; g.N = N; g.cols = n * N4; g.K = M; g.batch = W; g.segs = l_cplx ? 2 : 1;
     g.a_blk = R; g.b_off1 = (long)nv * N4;
-    g.C = C.q; g.ldc = ldc_of((long)n * N4); g.c_plane = C.plane; g.c_part = R; g.expired = redo.call + 1;
+    g.C = C.q; g.ldc = ldc_of((long)n * N4); g.c_plane = C.plane; g.c_part = R; g.redo = redo;
     Out c = C;
     c.ldc = g.ldc;
     if ((rc = crt::walker_gemm(g, st))) return rc;
-    if ((rc = exx_reduce(c, W, N, N4, n, n0, Nc, A.e, B.e, exxn, kl, nup, st))) return rc;
+    if ((rc = exx_reduce(c, W, N, N4, n, n0, Nc, A.e, l_cplx ? 0 : R, B.e, exxn, kl, nup, redo, st))) return rc;
   }
   if ((rc = energy_exx_f64(G, Lnak, l_cplx, W, N, M, Nc, Tchunk, tchunk_elems, exxn, kl, st, nup, &redo)))
     return rc;
@@ -273,7 +279,7 @@ int energy_crt(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool 
 
 namespace sfq {
 namespace {
-// C = A B^T by either kernel; the self-test's limit and hold, and whether a wait expired
+// C = A B^T by either kernel, the bare product; the self-test's limit and hold, and whether a wait expired
 int modular_product(const double* A, const double* B, double* C, int M, int N, int K, bool walker, cudaStream_t st,
                     unsigned long long wait_ns = 0, int hold_at = -1, int* expired = nullptr) {
   char* ws = nullptr;
@@ -281,24 +287,25 @@ int modular_product(const double* A, const double* B, double* C, int M, int N, i
                        crt::exps_bytes(N) + crt::out_bytes(M, N);
   SFQ_CUDA_TRY(cudaMallocAsync((void**)&ws, bytes, st));
   char* at = ws;
-  const Redo redo = crt::lay_out_flags(at, M);  // a row of A for a walker
+  const Redo redo = crt::lay_out_flags(at, M);
+  const int per = walker ? M : 1;  // rows of A to a walker
   const crt::Planes a = crt::lay_out(at, M, K, M), b = crt::lay_out(at, N, K, N);
   const crt::Out c = crt::lay_out_c(at, M, N);
-  const int* hold = hold_at < 0 ? nullptr : redo.call + 2;  // nothing sets it
+  const int* hold = hold_at < 0 ? nullptr : redo.call + 4;  // nothing sets it
   int rc = SFQ_OK;
   cudaError_t ce = cudaMemsetAsync(redo.call, 0, crt::flag_bytes(M), st);
   if (ce != cudaSuccess) rc = record_cuda(ce, "gemm_f64_modular", __FILE__, __LINE__);
-  if (!rc) rc = crt::rows_real(A, M, K, K, a, redo, 1, st);
+  if (!rc) rc = crt::rows_real(A, M, K, K, a, redo, per, st);
   if (!rc) rc = crt::rows_real(B, N, K, K, b, redo, 0, st);
   if (!rc && walker) {  // the rows as the [re; im] of one walker
     crt::WalkerGemm g;
     g.A = a; g.B = b; g.N = M / 2; g.cols = N; g.K = K; g.a_blk = M / 2;
-    g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.c_part = M / 2; g.expired = redo.call + 1;
+    g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.c_part = M / 2; g.redo = redo; g.check = false;
     g.wait_ns = wait_ns; g.hold = hold; g.hold_at = unsigned(hold_at);
     rc = crt::walker_gemm(g, st);
   } else if (!rc) {
     crt::Gemm g;
-    g.A = a; g.B = b; g.M = M; g.N = N; g.K = K; g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.expired = redo.call + 1;
+    g.A = a; g.B = b; g.M = M; g.N = N; g.K = K; g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.redo = redo; g.wmod = M; g.check = false;
     g.wait_ns = wait_ns; g.hold = hold; g.hold_at = unsigned(hold_at);
     rc = crt::gemm(g, st);
   }
@@ -309,9 +316,8 @@ int modular_product(const double* A, const double* B, double* C, int M, int N, i
     d.A = A; d.sAm = K; d.sAk = 1;
     d.B = B; d.sBk = 1; d.sBn = K;
     d.C = C; d.sCm = N; d.sCn = 1;
-    d.redo_call = redo.call;
-    d.redo_row = redo.row;
-    d.redo_div = 1;
+    d.redo = redo;
+    d.redo_div = per;
     rc = gemm_f64(d, st);
   }
   if (!rc && expired) {

@@ -1,5 +1,5 @@
 // The FP64 path's products by modular arithmetic on the int8 tensor cores.  *_ok: whether the sizes are
-// ones where it is the faster path; *_bytes: device scratch of a call; Lq / P1q: the operand's planes
+// ones where it is the faster path; *_bytes: device scratch of a call; Lq: the operand's planes
 // prepared once (null: converted on every call).
 #pragma once
 #include "crt.cuh"
@@ -18,9 +18,9 @@ int vhs_crt(const double* L, long rows, const crt::Planes* Lq, const cplx* X, cp
             char* ws, cudaStream_t st);
 
 bool propagate_crt_ok(int W, int M, int N, int npol, bool p_cplx, int order);
-size_t propagate_crt_bytes(int W, int M, int N, int npol, bool prepared);
-int propagate_crt(cplx* SM, const double* P1, const crt::Planes* P1q, const cplx* V, int W, int M, int N, int npol,
-                  int order, char* ws, cudaStream_t st);
+size_t propagate_crt_bytes(int W, int M, int N, int npol);
+int propagate_crt(cplx* SM, const double* P1, const cplx* V, int W, int M, int N, int npol, int order, char* ws,
+                  cudaStream_t st);
 
 // the local energy (as ops::energy) with the exchange tensor's product this way; Tchunk: the FP64 path's
 // (tchunk_elems complex values; may share scratch from crt::flag_bytes(W) on)

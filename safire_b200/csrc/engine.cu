@@ -534,14 +534,14 @@ struct Engine {
   long P = 0;
   double* Lp = nullptr;  // (P, Nc), FP64 engines
   cplx* Vp = nullptr;    // (W, P), FP64 engines
-  // FP64 engines: residue planes of L (the packed rows when symmetric), Lnak and P1, made once at
+  // FP64 engines: residue planes of L (the packed rows when symmetric) and Lnak, made once at
   // setup (none where the sizes are too small for the int8 tensor cores, crt_ops.cuh, or the planes too
   // large), and those products' scratch, which shares the energy chunk's buffer
-  crt::Planes L_m, Lnak_m, P1_m;
+  crt::Planes L_m, Lnak_m;
   char* crt_buf = nullptr;
   char* crt_ws = nullptr;
   size_t crt_bytes = 0;
-  bool crt_energy = false;  // the energy's exchange product that way too
+  bool crt_energy = false, crt_prop = false;  // the energy's exchange product and the propagation that way too
   // T holds the inverse overlap matrices (PsiT W)^-1 of the current walkers and inv_ov their log
   // overlaps whenever inv_cached is set: the log overlap taken after a propagation or an
   // orthogonalization factors exactly the matrix the next Green's function needs, so that step
@@ -833,7 +833,7 @@ struct Engine {
     for (long rows : {(long)M * (M + 1) / 2, (long)M * M})
       if (ops::vhs_crt_ok(W, rows, Nc, true)) ws = std::max(ws, ops::vhs_crt_bytes(W, rows, Nc, true));
     if (ops::propagate_crt_ok(W, M, N, npol, false, p.taylor_order))
-      ws = std::max(ws, ops::propagate_crt_bytes(W, M, N, npol, true));
+      ws = std::max(ws, ops::propagate_crt_bytes(W, M, N, npol));
     if (ndet == 1 && ops::energy_crt_ok(W, N, Mr, Nc, lc)) ws = std::max(ws, ops::energy_crt_bytes(W, N, Mr, Nc, lc));
     return ws;
   }
@@ -1149,7 +1149,7 @@ struct Engine {
   }
 
   // FP64 engines: the residue planes of the resident operands.  Planes take
-  // 15 bytes an element (FP64: 8); above 24 GB of them, or where the device has no room, the
+  // 16 bytes an element (FP64: 8); above 24 GB of them, or where the device has no room, the
   // products stay on the FP64 tensor pipe, as they do below the sizes that gain.
   int setup_crt() {
     const long rows = sym ? P : (long)M * M;
@@ -1161,11 +1161,11 @@ struct Engine {
     if (!vb && !vh && !pr && !en) return SFQ_OK;
     const long K = (long)N * Mr;
     crt_energy = en;
-    if (!vb && !vh && !pr) return SFQ_OK;
+    crt_prop = pr;
+    if (!vb && !vh) return SFQ_OK;
     size_t planes = 256;
     if (vb) planes += crt::planes_bytes((lc ? 2L : 1L) * Nc, K) + crt::exps_bytes(Nc);
     if (vh) planes += crt::planes_bytes(rows, Nc) + crt::exps_bytes(rows);
-    if (pr) planes += crt::planes_bytes(M, M) + crt::exps_bytes(M);
     if (planes > (size_t(24) << 30)) return SFQ_OK;
     if (cudaMalloc(&crt_buf, planes) != cudaSuccess) {
       cudaGetLastError();
@@ -1179,17 +1179,13 @@ struct Engine {
     SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, sizeof(int), st));
     if (vb) {
       Lnak_m = crt::lay_out(at, (lc ? 2L : 1L) * Nc, K, Nc);
-      rc = lc ? crt::rows_cplx((const cplx*)Lnak, Nc, K, K, 2, Nc, Nc, Nc, Lnak_m, redo, 0, st)
+      rc = lc ? crt::rows_cplx((const cplx*)Lnak, Nc, K, K, crt::Parts::kJoint, Nc, Nc, Nc, Lnak_m, redo, 0, st)
               : crt::rows_real((const double*)Lnak, Nc, K, K, Lnak_m, redo, 0, st);
       if (rc) return rc;
     }
     if (vh) {
       L_m = crt::lay_out(at, rows, Nc, rows);
       if ((rc = crt::rows_real(sym ? Lp : Likn, rows, Nc, Nc, L_m, redo, 0, st))) return rc;
-    }
-    if (pr) {
-      P1_m = crt::lay_out(at, M, M, M);
-      if ((rc = crt::rows_real(P1, M, M, M, P1_m, redo, 0, st))) return rc;
     }
     int bad = 0;
     SFQ_CUDA_TRY(cudaMemcpyAsync(&bad, redo.call, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -1198,7 +1194,7 @@ struct Engine {
       cudaFree(crt_buf);
       crt_buf = nullptr;
       crt_bytes = 0;
-      L_m = Lnak_m = P1_m = crt::Planes();
+      L_m = Lnak_m = crt::Planes();
     }
     return SFQ_OK;
   }
@@ -1215,7 +1211,7 @@ struct Engine {
     return ops::vhs_rows(L, rows, x, out, W, Nc, std::sqrt(p.dt), st);
   }
   int f64_propagate(cplx* S) {
-    if (P1_m.q) return ops::propagate_crt(S, P1, &P1_m, V, W, M, N, npol, p.taylor_order, crt_ws, st);
+    if (crt_prop) return ops::propagate_crt(S, P1, V, W, M, N, npol, p.taylor_order, crt_ws, st);
     return ops::propagate(S, P1, false, V, W, M, N, p.taylor_order, TMN, T1, T2, st, npol);
   }
 

@@ -89,6 +89,8 @@ int gemm_f64(const GemmDesc& d, cudaStream_t st) {
   const bool AC = d.a_cplx, BC = d.b_cplx, CJ = d.conj_a && d.a_cplx;
   // instantiations used by the AFQMC path
   if (!AC && BC && !CJ && AK && !BK) return pick_tile<false, true, false, true, false>(d, st);
+  // the propagated rows (w, a) over the orbitals times P1 (crt_ops.cu)
+  if (!AC && BC && !CJ && AK && BK) return pick_tile<false, true, false, true, true>(d, st);
   if (AC && BC && !CJ && AK && !BK) return pick_tile<true, true, false, true, false>(d, st);
   if (AC && BC && !CJ && !AK && BK) return pick_tile<true, true, false, false, true>(d, st);
   if (AC && !BC && !CJ && AK && BK) return pick_tile<true, false, false, true, true>(d, st);

@@ -30,11 +30,9 @@ struct GemmDesc {
   cplx alpha = {1.0, 0.0};
   cplx beta = {0.0, 0.0};
   const int* mask = nullptr;  // optional: batch b is computed only where mask[b] != 0
-  // optional: only what flags raised before the kernel runs ask for again is computed (crt.cuh's Redo): all of it where
-  // redo_call[0] or [1] is set, else the batches b with redo_row[b] set, or with redo_div > 0 the rows m with
-  // redo_row[m / redo_div] set.  redo_rest: the other batches instead.
-  const int* redo_call = nullptr;
-  const int* redo_row = nullptr;
+  // optional (redo.call not null): only the walkers that redo asks for are computed, a batch each or, with redo_div > 0,
+  // redo_div rows of C each.  redo_rest: the other batches instead.
+  Redo redo;
   int redo_div = 0;
   bool redo_rest = false;
   bool upper_only = false;    // C is needed on and above the diagonal only: tiles wholly below it are skipped
@@ -103,15 +101,14 @@ __global__ void __launch_bounds__(WM* WN * 32)
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const long bz = blockIdx.z;
   bool all_rows = true;
-  if (d.redo_call) {
-    bool all = d.redo_call[0] || d.redo_call[1];
-    if (!all && d.redo_div == 0) all = d.redo_row[bz] != 0;
-    if (d.redo_rest) {
-      if (all) return;
-    } else if (!all) {
-      if (d.redo_div == 0) return;
+  if (d.redo.call && d.redo_div == 0) {
+    if (d.redo.asked(bz) == d.redo_rest) return;
+  } else if (d.redo.call) {
+    const int4 c = d.redo.asked();
+    if (!(c.x | c.y | c.z)) return;
+    if (!(c.x | c.y)) {
       int any = 0;
-      for (int i = m0 + tid; i < m0 + BM && i < d.M; i += C_::THREADS) any |= d.redo_row[i / d.redo_div];
+      for (int i = m0 + tid; i < m0 + BM && i < d.M; i += C_::THREADS) any |= d.redo.row[i / d.redo_div];
       if (!__syncthreads_or(any)) return;
       all_rows = false;
     }
@@ -237,7 +234,7 @@ __global__ void __launch_bounds__(WM* WN * 32)
 #pragma unroll
   for (int i = 0; i < C_::FM; ++i) {
     int gm = m0 + wm * C_::TM + i * 8 + lr;
-    if (gm >= d.M || (!all_rows && !d.redo_row[gm / d.redo_div])) continue;
+    if (gm >= d.M || (!all_rows && !d.redo.row[gm / d.redo_div])) continue;
 #pragma unroll
     for (int j = 0; j < C_::FN; ++j) {
 #pragma unroll

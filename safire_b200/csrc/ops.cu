@@ -68,8 +68,7 @@ int green_full(const void* A, bool a_cplx, const cplx* Gc, cplx* C, int W, int M
 // the product d for the walkers that redo asks for: div rows of C each, or (0) a batch each
 static void ask_again(GemmDesc& d, const Redo* redo, int div) {
   if (!redo) return;
-  d.redo_call = redo->call;
-  d.redo_row = redo->row;
+  d.redo = *redo;
   d.redo_div = div;
 }
 
@@ -103,7 +102,7 @@ int vhs(const double* Likn, const cplx* X, cplx* V, int W, int M, int Nc, double
 }
 
 // out = P1 in, both (W, npol, M, N)
-static int p1_apply(const void* P1, bool p_cplx, const cplx* in, cplx* out, int W, int npol, int M, int N,
+int p1_apply(const void* P1, bool p_cplx, const cplx* in, cplx* out, int W, int npol, int M, int N,
                     cudaStream_t st, const Redo* redo) {
   const long MN = (long)M * N;
   GemmDesc d;
@@ -127,20 +126,16 @@ namespace {
 // dst[w] = src[w] (n values each) of the walkers asked for
 __global__ void copy_again_kernel(cplx* dst, const cplx* src, long n, Redo redo) {
   const int w = blockIdx.y;
-  if (!redo.call[0] && !redo.call[1] && !redo.row[w]) return;
+  if (!redo.asked(w)) return;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
     dst[w * n + t] = src[w * n + t];
 }
 }  // namespace
 
-int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M, int N, int order, cplx* TMN,
-              cplx* T1, cplx* T2, cudaStream_t st, int npol, const Redo* redo) {
+int taylor(cplx* TMN, const cplx* V, int W, int M, int N, int npol, int order, cplx* T1, cplx* T2, cudaStream_t st,
+           const Redo* redo) {
   int rc;
-  // npol = 2: spinor walkers (2M, N), the two components' M x N blocks one after the other; P1 and
-  // V act on each component (propagate.hpp:247-298, polarization-independent vHS)
-  const long n = (long)W * npol * M * N;
-  // TMN = P1 * SM   (propagate.hpp:260)
-  if ((rc = p1_apply(P1, p_cplx, SM, TMN, W, npol, M, N, st, redo))) return rc;
+  const long MN = (long)M * N, n = (long)W * npol * MN;
   // apply_expM (propagate.hpp:45-70): T1 = S; T2 = (i/n) V T1; S += T2; swap
   if (redo) {
     copy_again_kernel<<<dim3(4, W), 256, 0, st>>>(T1, TMN, n / W, *redo);
@@ -150,7 +145,6 @@ int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M
   }
   cplx* a = T1;
   cplx* b = T2;
-  const long MN = (long)M * N;
   for (int k = 1; k <= order; ++k) {
     for (int q = 0; q < npol; ++q) {
       GemmDesc d;
@@ -165,8 +159,19 @@ int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M
     }
     cplx* t = a; a = b; b = t;
   }
+  return SFQ_OK;
+}
+
+int propagate(cplx* SM, const void* P1, bool p_cplx, const cplx* V, int W, int M, int N, int order, cplx* TMN,
+              cplx* T1, cplx* T2, cudaStream_t st, int npol) {
+  int rc;
+  // npol = 2: spinor walkers (2M, N), the two components' M x N blocks one after the other; P1 and
+  // V act on each component (propagate.hpp:247-298, polarization-independent vHS)
+  // TMN = P1 * SM   (propagate.hpp:260)
+  if ((rc = p1_apply(P1, p_cplx, SM, TMN, W, npol, M, N, st))) return rc;
+  if ((rc = taylor(TMN, V, W, M, N, npol, order, T1, T2, st))) return rc;
   // SM = P1 * TMN   (propagate.hpp:297)
-  return p1_apply(P1, p_cplx, TMN, SM, W, npol, M, N, st, redo);
+  return p1_apply(P1, p_cplx, TMN, SM, W, npol, M, N, st);
 }
 
 namespace {
@@ -389,7 +394,7 @@ size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol) {
     case SFQ_OP_PROPAGATE: {
       const size_t f64 = 3 * align256(c * (size_t)nwalk * nmo * nel);
       if (nwalk <= 0 || nmo <= 0 || nel <= 0 || !ops::propagate_crt_ok(nwalk, nmo, nel, 1, false, 6)) return f64;
-      return std::max(f64, ops::propagate_crt_bytes(nwalk, nmo, nel, 1, false) + 256);
+      return std::max(f64, ops::propagate_crt_bytes(nwalk, nmo, nel, 1) + 256);
     }
     case SFQ_OP_VBIAS:
     case SFQ_OP_VBIAS_COMPLEX: {
@@ -470,8 +475,8 @@ int sfq_propagate(void* SM, const void* P1, int p1_complex, const void* V, int n
   const size_t blk = align256(sizeof(cplx) * (size_t)nwalk * nmo * nel);
   if (ws_bytes < 3 * blk) return record_error(SFQ_ERR_WORKSPACE, "propagate: workspace too small");
   if (ops::propagate_crt_ok(nwalk, nmo, nel, 1, p1_complex != 0, order) &&
-      ws_bytes >= ops::propagate_crt_bytes(nwalk, nmo, nel, 1, false) + 256)
-    return ops::propagate_crt((cplx*)SM, (const double*)P1, nullptr, (const cplx*)V, nwalk, nmo, nel, 1, order,
+      ws_bytes >= ops::propagate_crt_bytes(nwalk, nmo, nel, 1) + 256)
+    return ops::propagate_crt((cplx*)SM, (const double*)P1, (const cplx*)V, nwalk, nmo, nel, 1, order,
                               aligned(ws), S(stream));
   cplx* TMN = (cplx*)ws;
   cplx* T1 = (cplx*)((char*)ws + blk);

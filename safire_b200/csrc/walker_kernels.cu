@@ -286,16 +286,13 @@ __global__ void __launch_bounds__(RT) energy_e1_kernel(const cplx* G, const cplx
 
 // one CTA per (n, w): exx[w, n0+n] = sum_ab T[w,a,n,b] T[w,b,n,a]; kl[w, n0+n] = sum_a T[w,a,n,a]
 // (walkers that a Redo does not ask for are left alone)
-__device__ __forceinline__ bool asked_again(const Redo& r, int w) {
-  return !r.call || r.call[0] || r.call[1] || r.row[w];
-}
 // nup < nel: COLLINEAR walkers, orbitals [0, nup) up and [nup, nel) down; the exchange pairs only
 // orbitals of one spin (energy_impl runs per spin, Real3IndexFactorization.hpp:476-560)
 __global__ void __launch_bounds__(RT) energy_exx_kernel(const cplx* T, int nel, int nv, int n0, int nchol,
                                                         cplx* exxn, cplx* kl, int nup, Redo redo) {
   __shared__ cplx red[RT / 32];
   const int n = blockIdx.x, w = blockIdx.y;
-  if (!asked_again(redo, w)) return;
+  if (redo.call && !redo.asked(w)) return;
   const long rowstride = (long)nv * nel;  // T[(w*nel + a)][(n*nel + b)]
   const cplx* Tw = T + (long)w * nel * rowstride + (long)n * nel;
   cplx acc = mk(0.0, 0.0), tr = mk(0.0, 0.0);
@@ -381,7 +378,7 @@ __device__ __forceinline__ void exx_block(LOAD&& load, int nel, int nup, cplx* e
 __global__ void __launch_bounds__(RT) energy_exx_sm_kernel(const cplx* T, int nel, int nv, int n0, int nchol,
                                                            cplx* exxn, cplx* kl, int nup, Redo redo) {
   const int n = blockIdx.x, w = blockIdx.y;
-  if (!asked_again(redo, w)) return;
+  if (redo.call && !redo.asked(w)) return;
   const long ld = (long)nv * nel, o = (long)w * nchol + n0 + n;
   const cplx* Tw = T + (long)w * nel * ld + (long)n * nel;
   exx_block<cplx>([&](int a, int b) { return Tw[a * ld + b]; }, nel, nup, exxn + o, kl + o);

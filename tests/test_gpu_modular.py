@@ -243,3 +243,98 @@ def test_one_walker_outside_the_range_leaves_the_others(value):
         rest = [w for w in range(W) if w != bad]
         assert torch.equal(torch.view_as_real(clean)[rest], torch.view_as_real(with_bad)[rest])
         assert not torch.equal(clean[bad], with_bad[bad])
+
+
+U = 2.0 ** -53
+
+
+def _ld(t):
+    a = t.cpu().numpy()
+    return a.astype(np.clongdouble if np.iscomplexobj(a) else np.longdouble)
+
+
+def _graded(g, rows, K, decades, rising):
+    """Rows whose entries fall (or rise) over so many decades."""
+    e = torch.arange(K, device="cuda", dtype=torch.float64) / max(1, K - 1) * decades
+    return _rn(g, rows, K) * 10.0 ** (e - decades if rising else -e)
+
+
+@pytest.mark.parametrize("decades", [0, 1, 2, 3, 6, 12, 18, 40])
+@pytest.mark.parametrize("W,Nc,K", [(40, 70, 2400), (130, 300, 1026), (8, 64, 40000)])
+def test_graded_rows_keep_the_fp64_bound(W, Nc, K, decades):
+    """Rows graded in opposite directions: every output within the FP64 chain's own bound K u sum_k |a_k| |b_k|."""
+    from safire_b200 import afqmc, capi
+    assert _workspace_path(capi.OP_VBIAS, W, K // 2, 2, Nc) > 0
+    g = torch.Generator(device="cuda").manual_seed(decades + K)
+    A = torch.complex(_graded(g, W, K, decades, False), _graded(g, W, K, decades, False))
+    B = _graded(g, Nc, K, decades, True)
+    C = _ld(afqmc.vbias(A.reshape(W, 2, K // 2), B.reshape(Nc, 2, K // 2), 0.25))  # 2 sqrt(dt) = 1
+    a, b = _ld(A), _ld(B)
+    for part in ("real", "imag"):
+        p = getattr(a, part)
+        assert (np.abs(getattr(C, part) - p @ b.T) <= (K + 2) * U * (np.abs(p) @ np.abs(b).T)).all()
+
+
+def test_graded_operands_of_the_calls():
+    """The same through the public calls (sizes on the int8 path): graded operands, and imaginary parts far below the
+    real ones, which are sums of their own."""
+    from safire_b200 import afqmc
+    g = torch.Generator(device="cuda").manual_seed(2)
+    W, M, Nc = 97, 130, 700
+    s = math.sqrt(0.01)
+    L = _graded(g, M * M, Nc, 10, False).reshape(M, M, Nc)
+    for X in (torch.complex(_graded(g, W, Nc, 10, True), _graded(g, W, Nc, 10, True)),
+              torch.complex(_rn(g, W, Nc), 1e-9 * _rn(g, W, Nc))):
+        V, x, l = _ld(afqmc.vHS(L, X, 0.01)).reshape(W, M * M)[:4], _ld(X)[:4], _ld(L.reshape(M * M, Nc))
+        for part in ("real", "imag"):
+            p = getattr(x, part)
+            err = np.abs(getattr(V, part) - s * (p @ l.T))
+            assert (err <= (Nc + 4) * U * s * (np.abs(p) @ np.abs(l).T)).all()
+    N, Nc = 23, 613
+    K = N * M
+    for Lc in (_graded(g, Nc, K, 10, False), torch.complex(_graded(g, Nc, K, 10, False), _graded(g, Nc, K, 10, False))):
+        G = torch.complex(_graded(g, W, K, 10, True), 1e-6 * _graded(g, W, K, 10, True))
+        v = _ld(afqmc.vbias(G.reshape(W, N, M), Lc.reshape(Nc, N, M), 0.01))[:3]
+        x, l = _ld(G)[:3], _ld(Lc)
+        R = 2 * s * (x @ l.T)
+        # the four real products' sums of moduli, each part on its own
+        re = np.abs(x.real) @ np.abs(l.real).T + np.abs(x.imag) @ np.abs(l.imag).T
+        im = np.abs(x.imag) @ np.abs(l.real).T + np.abs(x.real) @ np.abs(l.imag).T
+        assert (np.abs(v.real - R.real) <= (2 * K + 4) * U * 2 * s * re).all()
+        assert (np.abs(v.imag - R.imag) <= (2 * K + 4) * U * 2 * s * im).all()
+
+
+@pytest.mark.parametrize("kind", ["unit", "near", "graded"])
+def test_propagate_keeps_small_elements(kind):
+    """Walkers of unit vectors, of unit vectors and little else, and graded V: every element within the FP64 chain's
+    bound, the same recursion on the moduli times its number of roundings."""
+    from safire_b200 import afqmc
+    g = torch.Generator(device="cuda").manual_seed(4)
+    W, M, N, order = 90, 250, 48, 6
+    SM = torch.zeros(W, M, N, dtype=torch.complex128, device="cuda")
+    SM[:, torch.arange(N), torch.arange(N)] = 1.0
+    V = torch.complex(_rn(g, W, M, M), 0.2 * _rn(g, W, M, M)) * (0.25 / math.sqrt(M))
+    if kind == "near":
+        SM += 1e-7 * _cn(g, W, M, N)
+    if kind == "graded":  # rows of V fall over the orbitals, the walkers rise
+        f = 10.0 ** (-8.0 * torch.arange(M, device="cuda", dtype=torch.float64) / M)
+        SM = _cn(g, W, M, N) / f[None, :, None] * 1e-8
+        V = V * f[None, None, :]
+    P1 = torch.diag(1.0 + 1e-3 * _rn(g, M)) + 1e-6 * _rn(g, M, M)
+    out = _ld(afqmc.Propagate(SM.clone(), P1, V, order=order))
+    p = _ld(P1)
+    for w in range(2):
+        v, x = _ld(V[w]), _ld(SM[w])
+
+        def chain(p, v, x, i):
+            t = p @ x
+            s = t
+            for k in range(1, order + 1):
+                t = i * (v @ t) / k
+                s = s + t
+            return p @ s
+
+        R = chain(p, v, x, np.clongdouble(1j))
+        am = lambda z: np.abs(z.real) + np.abs(z.imag)  # noqa: E731 - bounds both parts of the complex products
+        B = chain(np.abs(p), am(v), am(x), 1)
+        assert (np.abs(out[w] - R) <= (2 * M * (order + 2)) * U * B).all()
