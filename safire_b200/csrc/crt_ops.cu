@@ -13,29 +13,47 @@ namespace ops {
 using namespace crt;
 
 namespace {
-// scratch of one chunk of a call's work: large enough to fill the GPU several times over
+// What a call holds of the shared operand at a time, with its output, and of the walkers' operand: large enough to fill
+// the GPU several times over.  A call's scratch is bounded by two of these, whatever its sizes (but one walker's and 256
+// rows' worth are always held).
 constexpr size_t kChunkBytes = size_t(3) << 29;  // 1.5 GiB
 
-size_t vbias_row_bytes(long K, bool l_cplx, int W) {
-  return (size_t)kPlanes * (l_cplx ? 2 : 1) * ld_of(K) + (size_t)NMOD * 2 * W + sizeof(int);
-}
-size_t vhs_row_bytes(int W, int Nc) { return (size_t)kPlanes * ld_of(Nc) + (size_t)NMOD * 2 * W + sizeof(int); }
-// rows per chunk: the whole operand, or equal chunks of a multiple of 16 rows within kChunkBytes
-long chunk_rows(long rows, size_t row_bytes) {
-  const long most = std::max<long>(256, long(kChunkBytes / row_bytes));
-  const long n = (rows + most - 1) / most;
-  return n <= 1 ? rows : ((rows + n - 1) / n + 15) / 16 * 16;
-}
 size_t slack() { return 256 * (2 * kPlanes + 4); }  // plane roundings
+// n in equal parts of at most `most`
+long part_of(long n, long most) {
+  const long parts = (n + most - 1) / most;
+  return parts <= 1 ? n : (n + parts - 1) / parts;
+}
+// walkers at a time, each with `bytes` of planes
+int walkers_at_a_time(int W, size_t bytes) { return int(part_of(W, std::max<long>(1, long(kChunkBytes / bytes)))); }
+// rows of the shared operand at a time: all of them, or equal parts of a multiple of 16 rows
+long rows_at_a_time(long rows, size_t row_bytes) {
+  const long n = part_of(rows, std::max<long>(256, long(kChunkBytes / row_bytes)));
+  return n == rows ? rows : (n + 15) / 16 * 16;
+}
+// force bias and vHS, of `rows` shared rows of K (planes of them made once: prepared): walkers and rows at a time
+struct Parted {
+  int w;
+  long n;
+};
+Parted part(int W, long rows, long K, int a_blocks, int b_blocks, bool all_rows) {
+  Parted p;
+  p.w = walkers_at_a_time(W, (size_t)kPlanes * a_blocks * ld_of(K) + (all_rows ? (size_t)NMOD * 2 * rows : 0));
+  p.n = all_rows ? rows : rows_at_a_time(rows, (size_t)kPlanes * b_blocks * ld_of(K) + (size_t)NMOD * 2 * p.w + sizeof(int));
+  return p;
+}
+size_t parted_bytes(int W, const Parted& p, long K, int a_blocks, int b_blocks, bool prepared) {
+  size_t b = flag_bytes(W) + planes_bytes((long)a_blocks * p.w, K) + exps_bytes(2L * p.w) + out_bytes(2L * p.w, p.n);
+  if (!prepared) b += planes_bytes(b_blocks * p.n, K) + exps_bytes(p.n);
+  return b + slack();
+}
 }  // namespace
 
 // ---- force bias -----------------------------------------------------------------------------------
 size_t vbias_crt_bytes(int W, int N, int M, int Nc, bool l_cplx, bool prepared) {
   const long K = (long)N * M;
-  const long nb = prepared ? Nc : chunk_rows(Nc, vbias_row_bytes(K, l_cplx, W));
-  size_t b = flag_bytes(W) + planes_bytes((l_cplx ? 3L : 2L) * W, K) + exps_bytes(2L * W) + out_bytes(2L * W, nb);
-  if (!prepared) b += planes_bytes((l_cplx ? 2L : 1L) * nb, K) + exps_bytes(nb);
-  return b + slack();
+  const int na = l_cplx ? 3 : 2, nb = l_cplx ? 2 : 1;
+  return parted_bytes(W, part(W, Nc, K, na, nb, prepared), K, na, nb, prepared);
 }
 
 // The FP64 tensor-pipe product walks K = N M in one chain per tile of few tiles: 19 us at K = 576, 58 at 1024 and
@@ -48,46 +66,50 @@ bool vbias_crt_ok(int W, int N, int M, int Nc, bool l_cplx) {
 int vbias_crt(const cplx* G, const void* Lnak, bool l_cplx, const Planes* Lq, cplx* v, int W, int N, int M, int Nc,
               double a, char* ws, cudaStream_t st) {
   const long K = (long)N * M;
-  const long nb = Lq ? Nc : chunk_rows(Nc, vbias_row_bytes(K, l_cplx, W));
+  const int na = l_cplx ? 3 : 2, nb = l_cplx ? 2 : 1;
+  const Parted p = part(W, Nc, K, na, nb, Lq != nullptr);
   char* at = ws;
   const Redo redo = lay_out_flags(at, W);
   int rc;
   SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
-  Planes A = lay_out(at, (l_cplx ? 3L : 2L) * W, K, 2L * W);
-  Planes B = Lq ? *Lq : lay_out(at, (l_cplx ? 2L : 1L) * nb, K, nb);
-  Out C = lay_out_c(at, 2L * W, nb);
-  if ((rc = rows_cplx(G, W, K, K, l_cplx ? Parts::kJointNeg : Parts::kApart, W, W, W, A, redo, 1, st))) return rc;
-  for (long n0 = 0; n0 < Nc; n0 += nb) {
-    const long n = std::min<long>(nb, Nc - n0);
+  Planes A = lay_out(at, (long)na * p.w, K, 2L * p.w);
+  Planes B = Lq ? *Lq : lay_out(at, nb * p.n, K, p.n);
+  Out C = lay_out_c(at, 2L * p.w, p.n);
+  for (long n0 = 0; n0 < Nc; n0 += p.n) {
+    const long n = std::min<long>(p.n, Nc - n0);
     if (!Lq) {
-      if (l_cplx) rc = rows_cplx((const cplx*)Lnak + n0 * K, n, K, K, Parts::kJoint, nb, n, n, B, redo, 0, st);
+      if (l_cplx) rc = rows_cplx((const cplx*)Lnak + n0 * K, n, K, K, Parts::kJoint, p.n, n, n, B, redo, 0, st);
       else rc = rows_real((const double*)Lnak + n0 * K, n, K, K, B, redo, 0, st);
       if (rc) return rc;
     }
-    crt::Gemm g;
-    g.A = A; g.B = B; g.K = int(K); g.N = int(n);
-    if (l_cplx) {
-      g.M = W; g.parts = g.segs = 2;
-      g.a_off[0][0] = 0; g.a_off[0][1] = 2L * W; g.a_off[1][0] = W; g.a_off[1][1] = 0;
-      g.b_off[1] = Lq ? Nc : nb;
-    } else {
-      g.M = 2 * W;
+    for (int w0 = 0; w0 < W; w0 += p.w) {
+      const int w = std::min(p.w, W - w0);
+      const Redo rw{redo.call, redo.row + w0};
+      if ((n0 == 0 || p.w < W) && (rc = rows_cplx(G + w0 * K, w, K, K, l_cplx ? Parts::kJointNeg : Parts::kApart, w, w,
+                                                  w, A, rw, 1, st)))
+        return rc;
+      crt::Gemm g;
+      g.A = A; g.B = B; g.K = int(K); g.N = int(n);
+      if (l_cplx) {
+        g.M = w; g.parts = g.segs = 2;
+        g.a_off[0][0] = 0; g.a_off[0][1] = 2L * w; g.a_off[1][0] = w; g.a_off[1][1] = 0;
+        g.b_off[1] = Lq ? Nc : p.n;
+      } else {
+        g.M = 2 * w;
+      }
+      Out c = C;
+      c.ldc = ldc_of(n);
+      g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.redo = rw; g.wmod = w;
+      if ((rc = crt::gemm(g, st))) return rc;
+      if ((rc = out_cplx(c, w, n, A.e, l_cplx ? 0 : w, B.e, a, v + (long)w0 * Nc + n0, Nc, st))) return rc;
     }
-    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.redo = redo; g.wmod = W;
-    Out c = C;
-    c.ldc = g.ldc;
-    if ((rc = crt::gemm(g, st))) return rc;
-    if ((rc = out_cplx(c, W, n, A.e, l_cplx ? 0 : W, B.e, a, v + n0, Nc, st))) return rc;
   }
   return vbias(G, Lnak, l_cplx, v, W, N, M, Nc, a, st, &redo);
 }
 
 // ---- vHS --------------------------------------------------------------------------------------
 size_t vhs_crt_bytes(int W, long rows, int Nc, bool prepared) {
-  const long nb = chunk_rows(rows, vhs_row_bytes(W, Nc));
-  size_t b = flag_bytes(W) + planes_bytes(2L * W, Nc) + exps_bytes(2L * W) + out_bytes(2L * W, nb);
-  if (!prepared) b += planes_bytes(nb, Nc) + exps_bytes(nb);
-  return b + slack();
+  return parted_bytes(W, part(W, rows, Nc, 2, 1, false), Nc, 2, 1, prepared);
 }
 
 // Converting L (M^2 Nc elements) costs what the FP64 product of about 64 walkers does: from 96 walkers on
@@ -101,26 +123,32 @@ bool vhs_crt_ok(int W, long rows, int Nc, bool prepared) {
 
 int vhs_crt(const double* L, long rows, const Planes* Lq, const cplx* X, cplx* V, int W, int Nc, double a, char* ws,
             cudaStream_t st) {
-  const long nb = chunk_rows(rows, vhs_row_bytes(W, Nc));
+  const Parted p = part(W, rows, Nc, 2, 1, false);
   char* at = ws;
   const Redo redo = lay_out_flags(at, W);
   int rc;
   SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
-  Planes A = lay_out(at, 2L * W, Nc, 2L * W);
-  Planes B = Lq ? *Lq : lay_out(at, nb, Nc, nb);
-  Out C = lay_out_c(at, 2L * W, nb);
-  if ((rc = rows_cplx(X, W, Nc, Nc, Parts::kApart, W, W, W, A, redo, 1, st))) return rc;
-  for (long r0 = 0; r0 < rows; r0 += nb) {
-    const long n = std::min<long>(nb, rows - r0);
+  Planes A = lay_out(at, 2L * p.w, Nc, 2L * p.w);
+  Planes B = Lq ? *Lq : lay_out(at, p.n, Nc, p.n);
+  Out C = lay_out_c(at, 2L * p.w, p.n);
+  for (long r0 = 0; r0 < rows; r0 += p.n) {
+    const long n = std::min<long>(p.n, rows - r0);
     if (!Lq && (rc = rows_real(L + r0 * Nc, n, Nc, Nc, B, redo, 0, st))) return rc;
-    crt::Gemm g;
-    g.A = A; g.B = B; g.M = 2 * W; g.N = int(n); g.K = Nc;
-    g.b_off[0] = Lq ? r0 : 0;
-    g.C = C.q; g.ldc = ldc_of(n); g.c_plane = C.plane; g.redo = redo; g.wmod = W;
-    Out c = C;
-    c.ldc = g.ldc;
-    if ((rc = crt::gemm(g, st))) return rc;
-    if ((rc = out_cplx(c, W, n, A.e, W, B.e + (Lq ? r0 : 0), a, V + r0, rows, st))) return rc;
+    for (int w0 = 0; w0 < W; w0 += p.w) {
+      const int w = std::min(p.w, W - w0);
+      const Redo rw{redo.call, redo.row + w0};
+      if ((r0 == 0 || p.w < W) &&
+          (rc = rows_cplx(X + (long)w0 * Nc, w, Nc, Nc, Parts::kApart, w, w, w, A, rw, 1, st)))
+        return rc;
+      crt::Gemm g;
+      g.A = A; g.B = B; g.M = 2 * w; g.N = int(n); g.K = Nc;
+      g.b_off[0] = Lq ? r0 : 0;
+      Out c = C;
+      c.ldc = ldc_of(n);
+      g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.redo = rw; g.wmod = w;
+      if ((rc = crt::gemm(g, st))) return rc;
+      if ((rc = out_cplx(c, w, n, A.e, w, B.e + (Lq ? r0 : 0), a, V + w0 * rows + r0, rows, st))) return rc;
+    }
   }
   return vhs_rows(L, rows, X, V, W, Nc, a, st, &redo);
 }
@@ -131,11 +159,7 @@ size_t prop_walker_bytes(int M, int Nr) {  // Nr = npol * N rows per walker
   return (size_t)kPlanes * (3 * (size_t)Nr * ld_of(M) + 2 * (size_t)M * ld_of(M)) + (size_t)NMOD * 2 * Nr * ldc_of(M) +
          32 * (size_t)Nr * M + 4 * (size_t)(Nr + M);
 }
-int prop_chunk(int W, int M, int Nr) {
-  const long most = std::max<long>(1, long(kChunkBytes / prop_walker_bytes(M, Nr)));
-  const long n = (W + most - 1) / most;
-  return int((W + n - 1) / n);
-}
+int prop_chunk(int W, int M, int Nr) { return walkers_at_a_time(W, prop_walker_bytes(M, Nr)); }
 }  // namespace
 
 size_t propagate_crt_bytes(int W, int M, int N, int npol) {
@@ -208,18 +232,15 @@ int propagate_crt(cplx* SM, const double* P1, const cplx* V, int W, int M, int N
 // ---- local energy ---------------------------------------------------------------------------
 namespace {
 int n4_of(int N) { return (N + 3) / 4 * 4; }
-size_t energy_n_bytes(int W, int N, int M, bool l_cplx) {  // per Cholesky vector
-  return (size_t)kPlanes * (l_cplx ? 2 : 1) * n4_of(N) * ld_of(M) + (size_t)NMOD * 2 * W * N * n4_of(N) +
+int energy_walkers(int W, int N, int M, bool l_cplx) {
+  return walkers_at_a_time(W, (size_t)kPlanes * (l_cplx ? 3 : 2) * N * ld_of(M));
+}
+size_t energy_n_bytes(int w, int N, int M, bool l_cplx) {  // per Cholesky vector
+  return (size_t)kPlanes * (l_cplx ? 2 : 1) * n4_of(N) * ld_of(M) + (size_t)NMOD * 2 * w * N * n4_of(N) +
          sizeof(int) * N;
 }
-size_t energy_fixed_bytes(int W, int N, int M, bool l_cplx) {
-  const long R = (long)W * N;
-  return flag_bytes(W) + planes_bytes((l_cplx ? 3 : 2) * R, M) + exps_bytes(2 * R) + slack();
-}
-int energy_nv(int W, int N, int M, int Nc, bool l_cplx) {
-  const long most = std::max<long>(1, long(kChunkBytes / energy_n_bytes(W, N, M, l_cplx)));
-  const long n = (Nc + most - 1) / most;
-  return int((Nc + n - 1) / n);
+int energy_nv(int w, int N, int M, int Nc, bool l_cplx) {
+  return int(part_of(Nc, std::max<long>(1, long(kChunkBytes / energy_n_bytes(w, N, M, l_cplx)))));
 }
 }  // namespace
 
@@ -228,49 +249,61 @@ int energy_nv(int W, int N, int M, int Nc, bool l_cplx) {
 // Below 40 GFLOP (about a millisecond there) its launches count.
 bool energy_crt_ok(int W, int N, int M, int Nc, bool l_cplx) {
   return W <= 65535 && N >= 40 && N <= kExxMaxN && M >= 32 && 8.0 * W * N * double(N) * M * Nc >= 4e10 &&
-         energy_n_bytes(W, N, M, l_cplx) <= kChunkBytes && walker_gemm_fits(N, 16 * n4_of(N), M, l_cplx ? 2 : 1);
+         energy_n_bytes(energy_walkers(W, N, M, l_cplx), N, M, l_cplx) <= kChunkBytes &&
+         walker_gemm_fits(N, 16 * n4_of(N), M, l_cplx ? 2 : 1);
 }
 
 size_t energy_crt_bytes(int W, int N, int M, int Nc, bool l_cplx) {
-  const int nv = energy_nv(W, N, M, Nc, l_cplx), N4 = n4_of(N);
-  return energy_fixed_bytes(W, N, M, l_cplx) + planes_bytes((l_cplx ? 2L : 1L) * nv * N4, M) +
-         exps_bytes((long)nv * N) + out_bytes(2L * W * N, (long)nv * N4);
+  const int w = energy_walkers(W, N, M, l_cplx), nv = energy_nv(w, N, M, Nc, l_cplx), N4 = n4_of(N);
+  const long R = (long)w * N;
+  return flag_bytes(w) + planes_bytes((l_cplx ? 3 : 2) * R, M) + exps_bytes(2 * R) +
+         planes_bytes((l_cplx ? 2L : 1L) * nv * N4, M) + exps_bytes((long)nv * N) + out_bytes(2 * R, (long)nv * N4) +
+         slack();
 }
 
 int energy_crt(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool l_cplx, double E0, int W, int N, int M,
-               int Nc, int addH1, int addEJ, char* scratch, cplx* Tchunk, long tchunk_elems, cplx* exxn, cplx* kl,
-               cudaStream_t st, int nup) {
+               int Nc, int addH1, int addEJ, char* scratch, size_t bytes, cplx* exxn, cplx* kl, cudaStream_t st,
+               int nup) {
   int rc;
   const double scl = nup < 0 ? 2.0 : 1.0;
-  const int nv = energy_nv(W, N, M, Nc, l_cplx), N4 = n4_of(N);
-  const long R = (long)W * N;
-  char* at = scratch;
-  const Redo redo = lay_out_flags(at, W);
-  SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(W), st));
+  const int wc = energy_walkers(W, N, M, l_cplx), nv = energy_nv(wc, N, M, Nc, l_cplx), N4 = n4_of(N);
   if ((rc = energy_e1(G, haj, E3, W, N, M, E0, scl, addH1, st))) return rc;
-  const Planes A = lay_out(at, (l_cplx ? 3 : 2) * R, M, 2 * R);
-  const Planes B = lay_out(at, (l_cplx ? 2L : 1L) * nv * N4, M, (long)nv * N);
-  const Out C = lay_out_c(at, 2 * R, (long)nv * N4);
-  if ((rc = rows_cplx(G, R, M, M, l_cplx ? Parts::kJointNeg : Parts::kApart, R, R, R, A, redo, N, st))) return rc;
-  for (int n0 = 0; n0 < Nc; n0 += nv) {
-    const int n = std::min(nv, Nc - n0);
-    // rows (n, a) of Lnak on rows n N4 + a: the columns of a vector then start on words
-    const long off = (long)n0 * N * M;
-    if (n0 == 0 && N4 != N && (rc = pass_padding(B, st))) return rc;
-    if (l_cplx) rc = rows_cplx((const cplx*)Lnak + off, (long)n * N, M, M, Parts::kJoint, (long)nv * N4, N, N4, B, redo, 0, st);
-    else rc = rows_real((const double*)Lnak + off, (long)n * N, M, M, B, redo, 0, st, N, N4);
-    if (rc) return rc;
-    crt::WalkerGemm g;
-    g.A = A; g.B = B; g.N = N; g.cols = n * N4; g.K = M; g.batch = W; g.segs = l_cplx ? 2 : 1;
-    g.a_blk = R; g.b_off1 = (long)nv * N4;
-    g.C = C.q; g.ldc = ldc_of((long)n * N4); g.c_plane = C.plane; g.c_part = R; g.redo = redo;
-    Out c = C;
-    c.ldc = g.ldc;
-    if ((rc = crt::walker_gemm(g, st))) return rc;
-    if ((rc = exx_reduce(c, W, N, N4, n, n0, Nc, A.e, l_cplx ? 0 : R, B.e, exxn, kl, nup, redo, st))) return rc;
+  for (int w0 = 0; w0 < W; w0 += wc) {
+    const int w = std::min(wc, W - w0);
+    const long R = (long)w * N;
+    const cplx* Gw = G + (long)w0 * N * M;
+    cplx *ew = exxn + (long)w0 * Nc, *kw = kl + (long)w0 * Nc;
+    char* at = scratch;
+    const Redo redo = lay_out_flags(at, wc);
+    // the FP64 product's chunk takes the same space afterwards: 16 w N^2 bytes a vector at least, less than C's
+    cplx* Tchunk = reinterpret_cast<cplx*>(at);
+    const long tchunk = std::min<long>(long((bytes - flag_bytes(wc)) / sizeof(cplx)), 1L << 27);
+    SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flag_bytes(wc), st));
+    const Planes A = lay_out(at, (l_cplx ? 3 : 2) * R, M, 2 * R);
+    const Planes B = lay_out(at, (l_cplx ? 2L : 1L) * nv * N4, M, (long)nv * N);
+    const Out C = lay_out_c(at, 2 * R, (long)nv * N4);
+    if ((rc = rows_cplx(Gw, R, M, M, l_cplx ? Parts::kJointNeg : Parts::kApart, R, R, R, A, redo, N, st))) return rc;
+    if (N4 != N && (rc = pass_padding(B, st))) return rc;
+    for (int n0 = 0; n0 < Nc; n0 += nv) {
+      const int n = std::min(nv, Nc - n0);
+      // rows (n, a) of Lnak on rows n N4 + a: the columns of a vector then start on words
+      const long off = (long)n0 * N * M;
+      if (l_cplx)
+        rc = rows_cplx((const cplx*)Lnak + off, (long)n * N, M, M, Parts::kJoint, (long)nv * N4, N, N4, B, redo, 0, st);
+      else
+        rc = rows_real((const double*)Lnak + off, (long)n * N, M, M, B, redo, 0, st, N, N4);
+      if (rc) return rc;
+      crt::WalkerGemm g;
+      g.A = A; g.B = B; g.N = N; g.cols = n * N4; g.K = M; g.batch = w; g.segs = l_cplx ? 2 : 1;
+      g.a_blk = R; g.b_off1 = (long)nv * N4;
+      Out c = C;
+      c.ldc = ldc_of((long)n * N4);
+      g.C = c.q; g.ldc = c.ldc; g.c_plane = c.plane; g.c_part = R; g.redo = redo;
+      if ((rc = crt::walker_gemm(g, st))) return rc;
+      if ((rc = exx_reduce(c, w, N, N4, n, n0, Nc, A.e, l_cplx ? 0 : R, B.e, ew, kw, nup, redo, st))) return rc;
+    }
+    if ((rc = energy_exx_f64(Gw, Lnak, l_cplx, w, N, M, Nc, Tchunk, tchunk, ew, kw, st, nup, &redo))) return rc;
   }
-  if ((rc = energy_exx_f64(G, Lnak, l_cplx, W, N, M, Nc, Tchunk, tchunk_elems, exxn, kl, st, nup, &redo)))
-    return rc;
   return energy_finish(exxn, kl, E3, W, Nc, scl, 1, addEJ, st);
 }
 

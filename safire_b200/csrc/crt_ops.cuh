@@ -22,13 +22,12 @@ size_t propagate_crt_bytes(int W, int M, int N, int npol);
 int propagate_crt(cplx* SM, const double* P1, const cplx* V, int W, int M, int N, int npol, int order, char* ws,
                   cudaStream_t st);
 
-// the local energy (as ops::energy) with the exchange tensor's product this way; Tchunk: the FP64 path's
-// (tchunk_elems complex values; may share scratch from crt::flag_bytes(W) on)
+// the local energy (as ops::energy) with the exchange tensor's product this way, in `bytes` of scratch
 bool energy_crt_ok(int W, int N, int M, int Nc, bool l_cplx);
 size_t energy_crt_bytes(int W, int N, int M, int Nc, bool l_cplx);
 int energy_crt(cplx* E3, const cplx* G, const cplx* haj, const void* Lnak, bool l_cplx, double E0, int W, int N, int M,
-               int Nc, int addH1, int addEJ, char* scratch, cplx* Tchunk, long tchunk_elems, cplx* exxn, cplx* kl,
-               cudaStream_t st, int nup);
+               int Nc, int addH1, int addEJ, char* scratch, size_t bytes, cplx* exxn, cplx* kl, cudaStream_t st,
+               int nup);
 
 }  // namespace ops
 }  // namespace sfq

@@ -719,7 +719,7 @@ struct Engine {
         {(void**)&newov, c * W},
         {(void**)&E3, c * 3 * W},
         {(void**)&ovtmp, c * W},
-        {(void**)&crt_ws, std::max(c * (size_t)tchunk_elems + crt::flag_bytes(W), crt_scratch_bytes())},
+        {(void**)&Tchunk, std::max(c * (size_t)tchunk_elems, crt_scratch_bytes())},
         {(void**)&exxn, c * (size_t)W * Nc},
         {(void**)&kl, c * (size_t)W * Nc},
         {(void**)&status, sizeof(int) * 2 * W},
@@ -820,7 +820,7 @@ struct Engine {
       off += a256(it.bytes);
     }
     SFQ_CUDA_TRY(cudaMemsetAsync(arena, 0, total, st));
-    Tchunk = reinterpret_cast<cplx*>(crt_ws + crt::flag_bytes(W));
+    crt_ws = reinterpret_cast<char*>(Tchunk);
     return SFQ_OK;
   }
   // FP64 engines: the most that a product on the int8 tensor cores takes of the energy chunk's buffer, whether
@@ -2895,8 +2895,9 @@ struct Engine {
     }
     if ((rc = density(ovtmp))) return rc;
     if (crt_energy)
-      rc = ops::energy_crt(E3, G, haj, Lnak, !trial_real, p.E0, W, N, Mr, Nc, 1, 1, crt_ws, Tchunk, tchunk_elems, exxn,
-                           kl, st, spin_split());
+      rc = ops::energy_crt(E3, G, haj, Lnak, !trial_real, p.E0, W, N, Mr, Nc, 1, 1, crt_ws,
+                           std::max(sizeof(cplx) * (size_t)tchunk_elems, crt_scratch_bytes()), exxn, kl, st,
+                           spin_split());
     else
       rc = ops::energy(E3, G, haj, Lnak, !trial_real, p.E0, W, N, Mr, Nc, 1, 1, 1, Tchunk, tchunk_elems, exxn, kl, st,
                        spin_split());

@@ -410,11 +410,11 @@ size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol) {
     case SFQ_OP_ENERGY: {
       long nv = ops::energy_chunk(nwalk, nel, nchol, kEnergyChunkElems);
       const size_t tc = align256(c * (size_t)nwalk * nel * nv * nel), vec = 2 * align256(c * (size_t)nwalk * nchol);
-      size_t big = tc;  // the int8 path's scratch, sized for a complex Lnak, holds the chunk too
+      size_t big = tc;  // or the int8 path's scratch, sized for a complex Lnak
       if (nwalk > 0 && nmo > 0 && nel > 0 && nchol > 0)
         for (bool lc : {false, true})
           if (ops::energy_crt_ok(nwalk, nel, nmo, nchol, lc))
-            big = std::max(big, std::max(ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc), tc + crt::flag_bytes(nwalk)) + 256);
+            big = std::max(big, ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc) + 256);
       return big + vec;
     }
     case SFQ_OP_INVERSE_LOGDET:
@@ -584,12 +584,13 @@ int sfq_energy(void* E, const void* G, const void* haj, const void* Lnak, int ln
   const size_t bk = align256(sizeof(cplx) * (size_t)nwalk * nchol);
   if (ws_bytes < bt + 2 * bk) return record_error(SFQ_ERR_WORKSPACE, "energy: workspace too small");
   const bool lc = lnak_complex != 0;
-  if (addEXX && nel > 0 && nmo > 0 && nchol > 0 && ops::energy_crt_ok(nwalk, nel, nmo, nchol, lc) &&
-      ws_bytes >= std::max(ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc), bt + crt::flag_bytes(nwalk)) + 256 + 2 * bk) {
-    char* at = aligned(ws);
-    return ops::energy_crt((cplx*)E, (const cplx*)G, (const cplx*)haj, Lnak, lc, E0, nwalk, nel, nmo, nchol, addH1,
-                           addEJ, at + 2 * bk, (cplx*)(at + 2 * bk + crt::flag_bytes(nwalk)), (long)nwalk * nel * nv * nel, (cplx*)at,
-                           (cplx*)(at + bk), S(stream), -1);
+  if (addEXX && nel > 0 && nmo > 0 && nchol > 0 && ops::energy_crt_ok(nwalk, nel, nmo, nchol, lc)) {
+    const size_t room = ws_bytes - 2 * bk - 256;  // behind exxn and kl
+    if (ws_bytes >= 2 * bk + 256 && room >= ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc)) {
+      char* at = aligned(ws);
+      return ops::energy_crt((cplx*)E, (const cplx*)G, (const cplx*)haj, Lnak, lc, E0, nwalk, nel, nmo, nchol, addH1,
+                             addEJ, at + 2 * bk, room, (cplx*)at, (cplx*)(at + bk), S(stream), -1);
+    }
   }
   cplx* Tc = (cplx*)ws;
   cplx* exxn = (cplx*)((char*)ws + bt);

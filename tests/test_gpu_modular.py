@@ -338,3 +338,109 @@ def test_propagate_keeps_small_elements(kind):
         am = lambda z: np.abs(z.real) + np.abs(z.imag)  # noqa: E731 - bounds both parts of the complex products
         B = chain(np.abs(p), am(v), am(x), 1)
         assert (np.abs(out[w] - R) <= (2 * M * (order + 2)) * U * B).all()
+
+
+def test_scratch_is_bounded():
+    """The walkers' planes come in parts too: what the int8 path takes does not grow with the walkers without end."""
+    from safire_b200 import capi
+    gib = 1 << 30
+    for W in (4096, 16384, 60000):
+        # 16 bytes a plane element: 2 W x 40000 of them for all walkers at once would be 5 to 77 GB
+        assert 0 < _workspace_path(capi.OP_VBIAS, W, 400, 100, 2400) < 4 * gib
+        assert 0 < _workspace_path(capi.OP_VBIAS_COMPLEX, W, 400, 100, 2400) < 4 * gib
+        assert 0 < _workspace_path(capi.OP_VHS, W, 400, 0, 2400) < 4 * gib
+        vec = 2 * 16 * W * 2400  # the energy's sums per walker and vector
+        chunk = max(16 * W * 100 * 100, 2 * gib)  # the FP64 path's exchange chunk
+        assert _workspace_path(capi.OP_ENERGY, W, 400, 100, 2400) < max(4 * gib, chunk) + vec + gib // 8
+
+
+def _rel(x, y):
+    return float((x - y).norm() / y.norm())
+
+
+# uneven last parts of the shared rows and of the walkers (1.5 GiB of planes at a time); a row that cannot be held in the
+# last part only
+def test_parts_of_vbias():
+    from safire_b200 import afqmc
+    g = torch.Generator(device="cuda").manual_seed(21)
+    for W, M, N, Nc, cplx in ((9, 400, 100, 2501, False), (1301, 400, 100, 67, False), (701, 400, 100, 65, True)):
+        G = torch.randn(W, N, M, generator=g, device="cuda", dtype=torch.complex128)
+        L = _rn(g, Nc, N, M) if not cplx else torch.randn(Nc, N, M, generator=g, device="cuda", dtype=torch.complex128)
+        Lc = L.to(torch.complex128).reshape(Nc, -1).T
+        out = afqmc.vbias(G, L, 0.25)
+        assert _rel(out, G.reshape(W, -1) @ Lc) < 1e-14
+        G[W - 1, 3, 5] = float("nan")
+        bad = afqmc.vbias(G, L, 0.25)
+        assert torch.isnan(bad[W - 1].real).all()
+        assert torch.equal(torch.view_as_real(bad[:-1]), torch.view_as_real(out[:-1]))
+        G[W - 1, 3, 5] = 0.0
+        L[Nc - 1, 3, 5] = float("inf")
+        bad = afqmc.vbias(G, L, 0.25)
+        assert not torch.isfinite(bad[:W - 1, Nc - 1].real).any()
+        # an FP64 sum of 2 K random terms: u sqrt(2 K) at most
+        assert _rel(bad[:W - 1, :Nc - 1], out[:W - 1, :Nc - 1]) < U * math.sqrt(2 * N * M)
+        del G, L, Lc, out, bad
+
+
+def test_parts_of_vhs():
+    from safire_b200 import afqmc
+    g = torch.Generator(device="cuda").manual_seed(22)
+    for W, M, Nc in ((101, 250, 3001), (17001, 9, 3000)):  # three parts of the rows; two of the walkers
+        L, X = _rn(g, M, M, Nc), _cn(g, W, Nc)
+        out = afqmc.vHS(L, X, 0.01)
+        R = 0.1 * (X @ L.to(torch.complex128).reshape(M * M, Nc).T).reshape(W, M, M)
+        assert _rel(out, R) < 1e-14
+        X[W - 1, 5] = float("nan")
+        bad = afqmc.vHS(L, X, 0.01)
+        assert torch.isnan(bad[W - 1].real).all()
+        assert torch.equal(torch.view_as_real(bad[:-1]), torch.view_as_real(out[:-1]))
+        X[W - 1, 5] = 0.0
+        L[M - 1, M - 1, Nc - 1] = 1e200
+        bad = afqmc.vHS(L, X, 0.01)
+        assert float(bad[:W - 1, M - 1, M - 1].abs().median()) > 1e198
+        bad[:, M - 1, M - 1] = out[:, M - 1, M - 1] = 0.0
+        assert _rel(bad[:-1], out[:-1]) < 1e-14
+
+
+def test_parts_of_propagate():
+    from safire_b200 import afqmc
+    g = torch.Generator(device="cuda").manual_seed(23)
+    W, M, N = 161, 400, 100  # two parts of the walkers, 81 and 80
+    SM, V = _cn(g, W, M, N), _cn(g, W, M, M) * (0.3 / math.sqrt(M))
+    P1 = torch.eye(M, device="cuda", dtype=torch.float64) + 1e-2 * _rn(g, M, M)
+    T = P1.to(torch.complex128) @ SM
+    S = T.clone()
+    for k in range(1, 7):
+        T = (V @ T) * (1j / k)
+        S += T
+    out = afqmc.Propagate(SM.clone(), P1, V)
+    assert _rel(out, P1.to(torch.complex128) @ S) < 2e-15
+    V[W - 1, 7, 8] = float("inf")
+    bad = afqmc.Propagate(SM.clone(), P1, V)
+    assert not torch.isfinite(bad[W - 1].real).any()
+    assert torch.equal(torch.view_as_real(bad[:-1]), torch.view_as_real(out[:-1]))
+
+
+def test_parts_of_energy():
+    from safire_b200 import afqmc
+    g = torch.Generator(device="cuda").manual_seed(24)
+    for W, M, N, Nc in ((30, 60, 70, 997), (1300, 400, 90, 7)):  # parts of the vectors; of the walkers
+        G, haj, L = _cn(g, W, N, M), _cn(g, N, M), _rn(g, Nc, N, M)
+        out = afqmc.energy(G, haj, L)
+        E = torch.zeros(W, 2, device="cuda", dtype=torch.complex128)
+        K = torch.empty(W, Nc, device="cuda", dtype=torch.complex128)
+        for n in range(Nc):
+            T = G @ L[n].to(torch.complex128).T
+            E[:, 0] -= (T * T.transpose(1, 2)).sum((1, 2))
+            K[:, n] = torch.diagonal(T, dim1=1, dim2=2).sum(1)
+        E[:, 1] = 2.0 * (K * K).sum(1)
+        scale = E.abs().max(dim=0).values
+        assert float(((out[:, 1:] - E).abs() / scale).max()) < 1e-12
+        G[W - 1, 3, 5] = float("nan")
+        bad = afqmc.energy(G, haj, L)
+        assert torch.isnan(bad[W - 1].real).all()
+        assert torch.equal(torch.view_as_real(bad[:-1]), torch.view_as_real(out[:-1]))
+        G[W - 1, 3, 5] = 0.0
+        L[Nc - 1, N - 1, M - 1] = float("nan")
+        bad = afqmc.energy(G, haj, L)
+        assert torch.isnan(bad[:, 1].real).all()
