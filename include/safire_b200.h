@@ -322,6 +322,12 @@ int sfq_engine_create(sfq_engine_t* out, const sfq_engine_params_t* p, const dou
  * determinant of largest |ci|.  FP64 only; ndet = 1 is sfq_engine_create. */
 int sfq_engine_create_nomsd(sfq_engine_t* out, const sfq_engine_params_t* p, const double* hcore, const double* Likn,
                             int ndet, const void* PsiT, const void* ci);
+/* Large FP64 engines run the force bias, vHS, the propagation and the energy on the int8 tensor cores (see
+ * sfq_vbias_ws) and hold residue planes of L and Lnak for it, 16 bytes an element beside FP64's 8, as far as they
+ * fit into 24 GB and half of the device memory that is free at creation.  sfq_engine_create_pipe (ndet >= 1; ci may
+ * be null for 1) declines: no planes, every FP64 product on the FP64 tensor pipe. */
+int sfq_engine_create_pipe(sfq_engine_t* out, const sfq_engine_params_t* p, const double* hcore, const double* Likn,
+                           int ndet, const void* PsiT, const void* ci);
 int sfq_engine_destroy(sfq_engine_t e);
 /* waits for the engine stream; SFQ_ERR_TIMEOUT if a tensor-core product's bounded wait expired */
 int sfq_engine_synchronize(sfq_engine_t e);

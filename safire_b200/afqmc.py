@@ -166,9 +166,11 @@ def comb(weights, r):
 # Resident engine
 # ------------------------------------------------------------------------------------------
 class AfqmcEngine:
-    """One system resident on one GPU: the drop-in for the objects execute_simulation builds."""
+    """One system resident on one GPU: the drop-in for the objects execute_simulation builds.
 
-    def __init__(self, system, nwalk, dt=0.005, seed=0, device=0, **params):
+    modular=False: an FP64 engine keeps to the FP64 tensor pipe and holds no residue planes (sfq_engine_create_pipe)."""
+
+    def __init__(self, system, nwalk, dt=0.005, seed=0, device=0, modular=True, **params):
         self.M, self.N, self.Nc, self.W = system.M, system.N, system.Nc, nwalk
         self.Mr = getattr(system, "npol", 1) * system.M  # rows of a walker (NONCOLLINEAR spinors: 2M)
         self.dt = dt
@@ -181,8 +183,14 @@ class AfqmcEngine:
         P = np.ascontiguousarray(system.PsiT, dtype=np.complex128)
         handle = ctypes.c_void_p()
         ci = getattr(system, "ci", None)
+        c = None
         if ci is not None and np.size(ci) > 1:  # multi-determinant trial: PsiT (ndet, rows, cols)
             c = np.ascontiguousarray(ci, dtype=np.complex128)
+        if not modular:
+            check(lib().sfq_engine_create_pipe(ctypes.byref(handle), ctypes.byref(p), h.ctypes.data, L.ctypes.data,
+                                               1 if c is None else int(c.size), P.ctypes.data,
+                                               None if c is None else c.ctypes.data))
+        elif c is not None:
             check(lib().sfq_engine_create_nomsd(ctypes.byref(handle), ctypes.byref(p), h.ctypes.data, L.ctypes.data,
                                                 int(c.size), P.ctypes.data, c.ctypes.data))
         else:

@@ -128,6 +128,7 @@ _SIGS = {
     "sfq_gemm_int8_cplx_b": ([_VP, _VP, _VP, _I, _I, _I, _I, _I, _VP], _I),
     "sfq_engine_params_default": ([ctypes.POINTER(EngineParams)], None),
     "sfq_engine_create": ([ctypes.POINTER(_VP), ctypes.POINTER(EngineParams), _VP, _VP, _VP], _I),
+    "sfq_engine_create_pipe": ([ctypes.POINTER(_VP), ctypes.POINTER(EngineParams), _VP, _VP, _I, _VP, _VP], _I),
     "sfq_engine_create_nomsd": ([ctypes.POINTER(_VP), ctypes.POINTER(EngineParams), _VP, _VP, _I, _VP, _VP], _I),
     "sfq_engine_destroy": ([_VP], _I),
     "sfq_engine_synchronize": ([_VP], _I),

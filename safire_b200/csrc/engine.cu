@@ -534,14 +534,16 @@ struct Engine {
   long P = 0;
   double* Lp = nullptr;  // (P, Nc), FP64 engines
   cplx* Vp = nullptr;    // (W, P), FP64 engines
-  // FP64 engines: residue planes of L (the packed rows when symmetric) and Lnak, made once at
-  // setup (none where the sizes are too small for the int8 tensor cores, crt_ops.cuh, or the planes too
-  // large), and those products' scratch, which shares the energy chunk's buffer
+  // FP64 engines, the products on the int8 tensor cores (see setup_crt): residue planes of L (the packed rows when
+  // symmetric) and Lnak, made once at setup, and those products' scratch, the energy chunk's buffer or, where that is too
+  // small, behind the planes
+  bool modular = true;  // they may be used
   crt::Planes L_m, Lnak_m;
   char* crt_buf = nullptr;
-  char* crt_ws = nullptr;
   size_t crt_bytes = 0;
-  bool crt_energy = false, crt_prop = false;  // the energy's exchange product and the propagation that way too
+  char* crt_ws = nullptr;
+  size_t crt_ws_bytes = 0;
+  bool crt_energy = false, crt_prop = false;  // the energy's exchange product and the propagation that way
   // T holds the inverse overlap matrices (PsiT W)^-1 of the current walkers and inv_ov their log
   // overlaps whenever inv_cached is set: the log overlap taken after a propagation or an
   // orthogonalization factors exactly the matrix the next Green's function needs, so that step
@@ -719,7 +721,7 @@ struct Engine {
         {(void**)&newov, c * W},
         {(void**)&E3, c * 3 * W},
         {(void**)&ovtmp, c * W},
-        {(void**)&Tchunk, std::max(c * (size_t)tchunk_elems, crt_scratch_bytes())},
+        {(void**)&Tchunk, c * (size_t)tchunk_elems},
         {(void**)&exxn, c * (size_t)W * Nc},
         {(void**)&kl, c * (size_t)W * Nc},
         {(void**)&status, sizeof(int) * 2 * W},
@@ -820,24 +822,8 @@ struct Engine {
       off += a256(it.bytes);
     }
     SFQ_CUDA_TRY(cudaMemsetAsync(arena, 0, total, st));
-    crt_ws = reinterpret_cast<char*>(Tchunk);
     return SFQ_OK;
   }
-  // FP64 engines: the most that a product on the int8 tensor cores takes of the energy chunk's buffer, whether
-  // L turns out symmetric or not
-  size_t crt_scratch_bytes() const {
-    if (mixed) return 0;
-    const bool lc = !trial_real;
-    size_t ws = 0;
-    if (ndet == 1 && ops::vbias_crt_ok(W, N, Mr, Nc, lc)) ws = ops::vbias_crt_bytes(W, N, Mr, Nc, lc, true);
-    for (long rows : {(long)M * (M + 1) / 2, (long)M * M})
-      if (ops::vhs_crt_ok(W, rows, Nc, true)) ws = std::max(ws, ops::vhs_crt_bytes(W, rows, Nc, true));
-    if (ops::propagate_crt_ok(W, M, N, npol, false, p.taylor_order))
-      ws = std::max(ws, ops::propagate_crt_bytes(W, M, N, npol));
-    if (ndet == 1 && ops::energy_crt_ok(W, N, Mr, Nc, lc)) ws = std::max(ws, ops::energy_crt_bytes(W, N, Mr, Nc, lc));
-    return ws;
-  }
-
   // --- setup: RealDenseHamiltonian::getHamiltonianOperations + NOMSD::vMF + generateP1 --------
   // the int8-slice setup shared by single- and multi-determinant trials: vHS's B (L over n, the
   // packed pairs when symmetric) and the P1 slices
@@ -1148,35 +1134,52 @@ struct Engine {
     return SFQ_OK;
   }
 
-  // FP64 engines: the residue planes of the resident operands.  Planes take
-  // 16 bytes an element (FP64: 8); above 24 GB of them, or where the device has no room, the
-  // products stay on the FP64 tensor pipe, as they do below the sizes that gain.
+  // FP64 engines: which products run on the int8 tensor cores, and the residue planes of their resident operands (16
+  // bytes an element; FP64: 8).  Each is taken where its sizes gain (crt_ops.cuh) and what it needs beside the arena
+  // fits into 24 GB and half of the device memory that is free, which leaves the estimators' buffers and other engines
+  // their room; the rest stays on the FP64 tensor pipe.
   int setup_crt() {
-    const long rows = sym ? P : (long)M * M;
+    if (!modular) return SFQ_OK;
+    const long rows = sym ? P : (long)M * M, K = (long)N * Mr;
     const bool lc = !trial_real;
-    const bool vb = ndet == 1 && ops::vbias_crt_ok(W, N, Mr, Nc, lc);
-    const bool vh = ops::vhs_crt_ok(W, rows, Nc, true);
-    const bool pr = ops::propagate_crt_ok(W, M, N, npol, false, p.taylor_order);
-    const bool en = ndet == 1 && ops::energy_crt_ok(W, N, Mr, Nc, lc);
-    if (!vb && !vh && !pr && !en) return SFQ_OK;
-    const long K = (long)N * Mr;
-    crt_energy = en;
-    crt_prop = pr;
-    if (!vb && !vh) return SFQ_OK;
-    size_t planes = 256;
-    if (vb) planes += crt::planes_bytes((lc ? 2L : 1L) * Nc, K) + crt::exps_bytes(Nc);
-    if (vh) planes += crt::planes_bytes(rows, Nc) + crt::exps_bytes(rows);
-    if (planes > (size_t(24) << 30)) return SFQ_OK;
-    if (cudaMalloc(&crt_buf, planes) != cudaSuccess) {
+    size_t dev_free = 0, dev_total = 0;
+    SFQ_CUDA_TRY(cudaMemGetInfo(&dev_free, &dev_total));
+    const size_t most = std::min(size_t(24) << 30, dev_free / 2);
+    const size_t have = sizeof(cplx) * (size_t)tchunk_elems;
+    size_t planes = 0, scratch = have;
+    auto take = [&](bool ok, size_t pl, size_t sc) {
+      if (!ok) return false;
+      const size_t p2 = planes + pl, s2 = std::max(scratch, a256(sc));
+      if (p2 + 256 + (s2 > have ? s2 : 0) > most) return false;
+      planes = p2;
+      scratch = s2;
+      return true;
+    };
+    crt_energy = ndet == 1 && ops::energy_crt_ok(W, N, Mr, Nc, lc) &&
+                 take(true, 0, ops::energy_crt_bytes(W, N, Mr, Nc, lc));
+    crt_prop = ops::propagate_crt_ok(W, M, N, npol, false, p.taylor_order) &&
+               take(true, 0, ops::propagate_crt_bytes(W, M, N, npol));
+    const bool vb = ndet == 1 && ops::vbias_crt_ok(W, N, Mr, Nc, lc) &&
+                    take(true, crt::planes_bytes((lc ? 2L : 1L) * Nc, K) + crt::exps_bytes(Nc),
+                         ops::vbias_crt_bytes(W, N, Mr, Nc, lc, true));
+    const bool vh = ops::vhs_crt_ok(W, rows, Nc, true) &&
+                    take(true, crt::planes_bytes(rows, Nc) + crt::exps_bytes(rows), ops::vhs_crt_bytes(W, rows, Nc, true));
+    if (!crt_energy && !crt_prop && !vb && !vh) return SFQ_OK;
+    const size_t flags = 256, own = (planes ? flags + planes : 0) + (scratch > have ? scratch : 0);
+    if (own && cudaMalloc(&crt_buf, own) != cudaSuccess) {
       cudaGetLastError();
       crt_buf = nullptr;
+      crt_energy = crt_prop = false;
       return SFQ_OK;
     }
-    crt_bytes = planes;
+    crt_bytes = own;
+    crt_ws = scratch > have ? crt_buf + (planes ? flags + planes : 0) : reinterpret_cast<char*>(Tchunk);
+    crt_ws_bytes = scratch;
+    if (!planes) return SFQ_OK;
     const Redo redo{reinterpret_cast<int*>(crt_buf), nullptr};
-    char* at = crt_buf + 256;
+    char* at = crt_buf + flags;
     int rc;
-    SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, sizeof(int), st));
+    SFQ_CUDA_TRY(cudaMemsetAsync(redo.call, 0, flags, st));
     if (vb) {
       Lnak_m = crt::lay_out(at, (lc ? 2L : 1L) * Nc, K, Nc);
       rc = lc ? crt::rows_cplx((const cplx*)Lnak, Nc, K, K, crt::Parts::kJoint, Nc, Nc, Nc, Lnak_m, redo, 0, st)
@@ -1191,10 +1194,12 @@ struct Engine {
     SFQ_CUDA_TRY(cudaMemcpyAsync(&bad, redo.call, sizeof(int), cudaMemcpyDeviceToHost, st));
     SFQ_CUDA_TRY(cudaStreamSynchronize(st));
     if (bad) {  // operands that the planes cannot hold
-      cudaFree(crt_buf);
-      crt_buf = nullptr;
-      crt_bytes = 0;
       L_m = Lnak_m = crt::Planes();
+      if (scratch == have) {  // (else the scratch lies behind them)
+        cudaFree(crt_buf);
+        crt_buf = nullptr;
+        crt_bytes = 0;
+      }
     }
     return SFQ_OK;
   }
@@ -2895,9 +2900,8 @@ struct Engine {
     }
     if ((rc = density(ovtmp))) return rc;
     if (crt_energy)
-      rc = ops::energy_crt(E3, G, haj, Lnak, !trial_real, p.E0, W, N, Mr, Nc, 1, 1, crt_ws,
-                           std::max(sizeof(cplx) * (size_t)tchunk_elems, crt_scratch_bytes()), exxn, kl, st,
-                           spin_split());
+      rc = ops::energy_crt(E3, G, haj, Lnak, !trial_real, p.E0, W, N, Mr, Nc, 1, 1, crt_ws, crt_ws_bytes, exxn, kl,
+                           st, spin_split());
     else
       rc = ops::energy(E3, G, haj, Lnak, !trial_real, p.E0, W, N, Mr, Nc, 1, 1, 1, Tchunk, tchunk_elems, exxn, kl, st,
                        spin_split());
@@ -3556,8 +3560,8 @@ void sfq_engine_params_default(sfq_engine_params_t* p) {
   p->nel_dn = 0;
 }
 
-int sfq_engine_create_nomsd(sfq_engine_t* out, const sfq_engine_params_t* p, const double* hcore, const double* Likn,
-                            int ndet, const void* PsiT, const void* ci) {
+static int create(sfq_engine_t* out, const sfq_engine_params_t* p, const double* hcore, const double* Likn, int ndet,
+                  const void* PsiT, const void* ci, bool modular) {
   if (!out || !p || !hcore || !Likn || !PsiT || (ndet > 1 && !ci)) return record_error(SFQ_ERR_ARG, "null pointer");
   if (ndet < 1) return record_error(SFQ_ERR_SHAPE, "engine: ndet=%d", ndet);
   *out = nullptr;
@@ -3578,6 +3582,7 @@ int sfq_engine_create_nomsd(sfq_engine_t* out, const sfq_engine_params_t* p, con
   auto* h = new sfq_engine_s();
   Engine& e = h->e;
   e.p = *p;
+  e.modular = modular;
   e.M = p->nmo; e.N = ntot; e.Nc = p->nchol; e.W = p->nwalk;
   e.collinear = coll;
   e.nup = p->nel;
@@ -3626,9 +3631,19 @@ int sfq_engine_create_nomsd(sfq_engine_t* out, const sfq_engine_params_t* p, con
   return SFQ_OK;
 }
 
+int sfq_engine_create_nomsd(sfq_engine_t* out, const sfq_engine_params_t* p, const double* hcore, const double* Likn,
+                            int ndet, const void* PsiT, const void* ci) {
+  return create(out, p, hcore, Likn, ndet, PsiT, ci, true);
+}
+
+int sfq_engine_create_pipe(sfq_engine_t* out, const sfq_engine_params_t* p, const double* hcore, const double* Likn,
+                           int ndet, const void* PsiT, const void* ci) {
+  return create(out, p, hcore, Likn, ndet, PsiT, ci, false);
+}
+
 int sfq_engine_create(sfq_engine_t* out, const sfq_engine_params_t* p, const double* hcore, const double* Likn,
                       const void* PsiT) {
-  return sfq_engine_create_nomsd(out, p, hcore, Likn, 1, PsiT, nullptr);
+  return create(out, p, hcore, Likn, 1, PsiT, nullptr, true);
 }
 
 int sfq_engine_destroy(sfq_engine_t h) {
@@ -4201,8 +4216,7 @@ int sfq_engine_resize(sfq_engine_t* ph, int nwalk) {
   sfq_engine_params_t p = e.p;
   p.nwalk = nwalk;
   sfq_engine_t nh = nullptr;
-  int rc = e.ndet > 1 ? sfq_engine_create_nomsd(&nh, &p, hc.data(), L.data(), e.ndet, ps.data(), e.ci_h.data())
-                      : sfq_engine_create(&nh, &p, hc.data(), L.data(), ps.data());
+  int rc = create(&nh, &p, hc.data(), L.data(), e.ndet, ps.data(), e.ndet > 1 ? e.ci_h.data() : nullptr, e.modular);
   if (rc) return rc;
   Engine& n = nh->e;
   const long mn = (long)e.Mr * e.N;

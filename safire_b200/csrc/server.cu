@@ -32,6 +32,7 @@ struct SystemRec {
   std::vector<double> hcore, Likn, PsiT;  // PsiT: complex (nel, nmo) as interleaved doubles
   sfq_engine_t eng = nullptr;
   size_t bytes = 0;          // device footprint of its engine (0 until first built)
+  bool pipe = false;         // built without the int8 tensor-core planes of FP64
   bool busy = false;         // a block is running
   bool started = false;      // walkers initialised (the trial energy and Eshift)
   unsigned long long next_step = 0;
@@ -101,9 +102,23 @@ int build(sfq_server_s& s, int i) {
   int rc;
   if (r.bytes && (rc = evict(s, i, r.bytes))) return rc;
   sfq_engine_t e = nullptr;
-  if ((rc = sfq_engine_create(&e, &r.p, r.hcore.data(), r.Likn.data(), r.PsiT.data()))) return rc;
+  auto create = [&]() {
+    return r.pipe ? sfq_engine_create_pipe(&e, &r.p, r.hcore.data(), r.Likn.data(), 1, r.PsiT.data(), nullptr)
+                  : sfq_engine_create(&e, &r.p, r.hcore.data(), r.Likn.data(), r.PsiT.data());
+  };
+  if ((rc = create())) return rc;
   size_t b = 0;
   sfq_engine_footprint(e, &b);
+  if (b > s.p.hbm_budget / s.p.max_inflight && !r.pipe && r.p.precision == SFQ_PRECISION_FP64) {
+    // The planes are there for speed: with them a system takes no more than its slot's share of the budget, so that
+    // none is turned away, or another evicted, for their sake.  The rule looks at this system alone: its results are
+    // the same whatever else is resident.
+    sfq_engine_destroy(e);
+    e = nullptr;
+    r.pipe = true;
+    if ((rc = create())) return rc;
+    sfq_engine_footprint(e, &b);
+  }
   if (s.used + b > s.p.hbm_budget) {
     // first build of this system: now that its size is known, make room or give up for now
     if ((rc = evict(s, i, b))) {
