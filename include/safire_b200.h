@@ -57,12 +57,14 @@ enum sfq_op {
   SFQ_OP_INVERSE_LOGDET = 6,
   SFQ_OP_VBIAS = 7,         /* sfq_vbias_ws, real Lnak */
   SFQ_OP_VHS = 8,           /* sfq_vhs_ws */
-  SFQ_OP_VBIAS_COMPLEX = 9  /* sfq_vbias_ws, complex Lnak */
+  SFQ_OP_VBIAS_COMPLEX = 9, /* sfq_vbias_ws, complex Lnak */
+  SFQ_OP_PROPAGATE_PIPE = 10,
+  SFQ_OP_ENERGY_PIPE = 11
 };
-/* device bytes of scratch the op needs for these sizes.  SFQ_OP_PROPAGATE and the two _ws operations
- * also run in less: the size returned is what their int8 tensor-core path takes, and with a smaller
- * workspace they run on the FP64 tensor pipe (propagate: in 3 * (16 nwalk nmo nel, rounded up to 256)
- * bytes at least, the _ws operations in none). */
+/* device bytes of scratch the op needs for these sizes.  For SFQ_OP_PROPAGATE, SFQ_OP_ENERGY and the two _ws
+ * operations this is what their int8 tensor-core path takes; with less they run on the FP64 tensor pipe, in
+ * SFQ_OP_PROPAGATE_PIPE's or SFQ_OP_ENERGY_PIPE's bytes at least (the _ws operations in none).  A propagation
+ * with a complex P1 always does, and needs no more. */
 size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol);
 
 /* det_ops::MixedDensityMatrix(A, B, C, ovlp, compact, herm=true)

@@ -82,8 +82,9 @@ inline void orthogonalize(ComplexType* SM, ComplexType* log_detR, int nwalk, int
                           size_t ws_bytes, void* stream = nullptr) {
   check(sfq_orthogonalize(SM, log_detR, nwalk, nmo, nel, ws, ws_bytes, stream));
 }
+// (Propagate above takes a complex P1, for which the FP64 tensor pipe's workspace is enough)
 inline size_t workspace_size(int op, int nwalk, int nmo, int nel, int nchol = 0) {
-  return sfq_workspace_size(op, nwalk, nmo, nel, nchol);
+  return sfq_workspace_size(op == SFQ_OP_PROPAGATE ? int(SFQ_OP_PROPAGATE_PIPE) : op, nwalk, nmo, nel, nchol);
 }
 
 }  // namespace det_ops

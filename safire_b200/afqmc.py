@@ -27,8 +27,16 @@ def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def _ws(op, nwalk, nmo, nel, nchol=0):
+def _ws(op, nwalk, nmo, nel, nchol=0, less=None):
+    """The operation's workspace; where the device has no room for it, that of `less` (0: none), with which the FP64
+    tensor pipe does the work of the int8 tensor cores."""
     n = lib().sfq_workspace_size(op, nwalk, nmo, nel, nchol)
+    try:
+        return torch.empty(max(int(n), 1), dtype=torch.uint8, device="cuda")
+    except torch.OutOfMemoryError:
+        if less is None:
+            raise
+    n = lib().sfq_workspace_size(less, nwalk, nmo, nel, nchol) if less else 0
     return torch.empty(max(int(n), 1), dtype=torch.uint8, device="cuda")
 
 
@@ -87,7 +95,7 @@ def Propagate(SM, P1, V, order=6):
     _need(P1, "P1", C128 + F64)
     _need(V, "V", C128)
     W, M, N = SM.shape
-    ws = _ws(capi.OP_PROPAGATE, W, M, N)
+    ws = _ws(capi.OP_PROPAGATE_PIPE if _is_cplx(P1) else capi.OP_PROPAGATE, W, M, N, less=capi.OP_PROPAGATE_PIPE)
     check(lib().sfq_propagate(ptr(SM), ptr(P1), int(_is_cplx(P1)), ptr(V), W, M, N, order, ptr(ws), ws.numel(),
                               _stream()))
     return SM
@@ -110,7 +118,7 @@ def vbias(G, Lnak, dt, closed=True):
     W = G.shape[0]
     Nc, N, M = Lnak.shape
     v = torch.empty((W, Nc), dtype=torch.complex128, device="cuda")
-    ws = _ws(capi.OP_VBIAS_COMPLEX if _is_cplx(Lnak) else capi.OP_VBIAS, W, M, N, Nc)
+    ws = _ws(capi.OP_VBIAS_COMPLEX if _is_cplx(Lnak) else capi.OP_VBIAS, W, M, N, Nc, less=0)
     check(lib().sfq_vbias_ws(ptr(G), ptr(Lnak), int(_is_cplx(Lnak)), ptr(v), W, N, M, Nc, dt, int(closed), ptr(ws),
                              ws.numel(), _stream()))
     return v
@@ -122,7 +130,7 @@ def vHS(Likn, X, dt):
     M, _, Nc = Likn.shape
     W = X.shape[0]
     V = torch.empty((W, M, M), dtype=torch.complex128, device="cuda")
-    ws = _ws(capi.OP_VHS, W, M, 0, Nc)
+    ws = _ws(capi.OP_VHS, W, M, 0, Nc, less=0)
     check(lib().sfq_vhs_ws(ptr(Likn), ptr(X), ptr(V), W, M, Nc, dt, ptr(ws), ws.numel(), _stream()))
     return V
 
@@ -134,7 +142,7 @@ def energy(G, haj, Lnak, E0=0.0, addH1=True, addEJ=True, addEXX=True):
     W = G.shape[0]
     Nc, N, M = Lnak.shape
     E = torch.empty((W, 3), dtype=torch.complex128, device="cuda")
-    ws = _ws(capi.OP_ENERGY, W, M, N, Nc)
+    ws = _ws(capi.OP_ENERGY, W, M, N, Nc, less=capi.OP_ENERGY_PIPE)
     check(lib().sfq_energy(ptr(E), ptr(G), ptr(haj), ptr(Lnak), int(_is_cplx(Lnak)), E0, W, N, M, Nc, int(addH1),
                            int(addEJ), int(addEXX), ptr(ws), ws.numel(), _stream()))
     return E

@@ -13,7 +13,7 @@ SFQ_OK = 0
 ERRORS = {1: "SHAPE", 2: "ARG", 3: "UNSUPPORTED", 4: "CUDA", 5: "OOM", 6: "WEIGHT_COLLAPSE", 7: "NONFINITE",
           8: "TIMEOUT", 9: "WORKSPACE", 10: "INTERNAL", 11: "RANK"}
 OP_MIXED_DENSITY_MATRIX, OP_LOG_OVERLAP, OP_PROPAGATE, OP_ORTHOGONALIZE, OP_ENERGY, OP_INVERSE_LOGDET = 1, 2, 3, 4, 5, 6
-OP_VBIAS, OP_VHS, OP_VBIAS_COMPLEX = 7, 8, 9
+OP_VBIAS, OP_VHS, OP_VBIAS_COMPLEX, OP_PROPAGATE_PIPE, OP_ENERGY_PIPE = 7, 8, 9, 10, 11
 
 # walker property columns, in the order the engine stores them (WalkerConfig.hpp:28-48 names)
 PROPS = ("WEIGHT", "PHASE", "PSEUDO_ELOC_", "E1_", "EXX_", "EJ_", "OVLP", "THETA")

@@ -396,6 +396,8 @@ size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol) {
       if (nwalk <= 0 || nmo <= 0 || nel <= 0 || !ops::propagate_crt_ok(nwalk, nmo, nel, 1, false, 6)) return f64;
       return std::max(f64, ops::propagate_crt_bytes(nwalk, nmo, nel, 1) + 256);
     }
+    case SFQ_OP_PROPAGATE_PIPE:
+      return 3 * align256(c * (size_t)nwalk * nmo * nel);
     case SFQ_OP_VBIAS:
     case SFQ_OP_VBIAS_COMPLEX: {
       const bool lc = op == SFQ_OP_VBIAS_COMPLEX;
@@ -407,9 +409,11 @@ size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol) {
       return ops::vhs_crt_bytes(nwalk, (long)nmo * nmo, nchol, false) + 256;
     case SFQ_OP_ORTHOGONALIZE:
       return align256(c * (size_t)nwalk * nmo * nel) + align256(c * nwalk * nel * nel) + align256(2 * sizeof(int) * nwalk);
-    case SFQ_OP_ENERGY: {
+    case SFQ_OP_ENERGY:
+    case SFQ_OP_ENERGY_PIPE: {
       long nv = ops::energy_chunk(nwalk, nel, nchol, kEnergyChunkElems);
       const size_t tc = align256(c * (size_t)nwalk * nel * nv * nel), vec = 2 * align256(c * (size_t)nwalk * nchol);
+      if (op == SFQ_OP_ENERGY_PIPE) return tc + vec;
       size_t big = tc;  // or the int8 path's scratch, sized for a complex Lnak
       if (nwalk > 0 && nmo > 0 && nel > 0 && nchol > 0)
         for (bool lc : {false, true})

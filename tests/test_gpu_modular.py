@@ -444,3 +444,36 @@ def test_parts_of_energy():
         L[Nc - 1, N - 1, M - 1] = float("nan")
         bad = afqmc.energy(G, haj, L)
         assert torch.isnan(bad[:, 1].real).all()
+
+
+def test_no_room_for_the_workspace():
+    """Where the device has no room for the int8 path's workspace the calls run on the FP64 tensor pipe, as they do
+    with its own workspace."""
+    from safire_b200 import afqmc, capi
+    g = torch.Generator(device="cuda").manual_seed(31)
+    W, M, N, Nc = 90, 250, 48, 700
+    G, L, Lik = _cn(g, W, N, M), _rn(g, Nc, N, M), _rn(g, M, M, Nc)
+    Ge, haj, Le = _cn(g, 20, 45, 120), _cn(g, 45, 120), _rn(g, 1100, 45, 120)
+    SM, X, V = _cn(g, W, M, N), _cn(g, 100, Nc), _cn(g, W, M, M) * (0.3 / math.sqrt(M))
+    P1 = torch.eye(M, device="cuda", dtype=torch.float64) + 1e-2 * _rn(g, M, M)
+    # (call, bytes of its result and of the FP64 pipe's workspace, of the int8 path's)
+    calls = [(lambda: afqmc.vbias(G, L, 0.01), 16 * W * Nc, _workspace_path(capi.OP_VBIAS, W, M, N, Nc)),
+             (lambda: afqmc.vHS(Lik, X, 0.01), 16 * 100 * M * M, _workspace_path(capi.OP_VHS, 100, M, 0, Nc)),
+             (lambda: afqmc.Propagate(SM.clone(), P1, V),
+              16 * W * M * N + _workspace_path(capi.OP_PROPAGATE_PIPE, W, M, N, 0),
+              16 * W * M * N + _workspace_path(capi.OP_PROPAGATE, W, M, N, 0)),
+             (lambda: afqmc.energy(Ge, haj, Le), _workspace_path(capi.OP_ENERGY_PIPE, 20, 120, 45, 1100),
+              _workspace_path(capi.OP_ENERGY, 20, 120, 45, 1100))]
+    for call, need, full in calls:
+        assert full > need + (8 << 20)
+        want = call()
+        torch.cuda.empty_cache()
+        total = torch.cuda.mem_get_info()[1]
+        held = torch.cuda.memory_reserved()
+        torch.cuda.set_per_process_memory_fraction((held + (need + full) / 2) / total)
+        try:
+            got = call()
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        # each side rounds its sums of up to 12000 terms in its own order
+        assert _rel(got, want) < U * math.sqrt(2 * N * M) and not torch.equal(got, want)
