@@ -66,6 +66,9 @@ enum sfq_op {
  * SFQ_OP_PROPAGATE_PIPE's or SFQ_OP_ENERGY_PIPE's bytes at least (the _ws operations in none).  A propagation
  * with a complex P1 always does, and needs no more. */
 size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol);
+/* 1 where the int8 tensor-core path of such an operation is the faster one (propagate: real P1, order 6); elsewhere a
+ * caller passes the smaller workspace */
+int sfq_int8_gains(int op, int nwalk, int nmo, int nel, int nchol, int lnak_complex);
 
 /* det_ops::MixedDensityMatrix(A, B, C, ovlp, compact, herm=true)
  *   density_matrix.hpp:544-601 (log_overlap_impl :120-156, getri_or_zero nda_functions.hpp:422-438)

@@ -27,17 +27,18 @@ def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def _ws(op, nwalk, nmo, nel, nchol=0, less=None):
-    """The operation's workspace; where the device has no room for it, that of `less` (0: none), with which the FP64
-    tensor pipe does the work of the int8 tensor cores."""
-    n = lib().sfq_workspace_size(op, nwalk, nmo, nel, nchol)
+def _ws(op, nwalk, nmo, nel, nchol=0, less=None, lnak_complex=False):
+    """The operation's workspace.  `less` (0: none) is the one with which the FP64 tensor pipe does the work of the int8
+    tensor cores: where these do not gain, and where the device has no room for theirs."""
+    if less is not None and not lib().sfq_int8_gains(op, nwalk, nmo, nel, nchol, int(lnak_complex)):
+        op, less = less, None
     try:
+        n = lib().sfq_workspace_size(op, nwalk, nmo, nel, nchol) if op else 0
         return torch.empty(max(int(n), 1), dtype=torch.uint8, device="cuda")
     except torch.OutOfMemoryError:
         if less is None:
             raise
-    n = lib().sfq_workspace_size(less, nwalk, nmo, nel, nchol) if less else 0
-    return torch.empty(max(int(n), 1), dtype=torch.uint8, device="cuda")
+    return _ws(less, nwalk, nmo, nel, nchol)
 
 
 def _is_cplx(t):
@@ -142,7 +143,7 @@ def energy(G, haj, Lnak, E0=0.0, addH1=True, addEJ=True, addEXX=True):
     W = G.shape[0]
     Nc, N, M = Lnak.shape
     E = torch.empty((W, 3), dtype=torch.complex128, device="cuda")
-    ws = _ws(capi.OP_ENERGY, W, M, N, Nc, less=capi.OP_ENERGY_PIPE)
+    ws = _ws(capi.OP_ENERGY, W, M, N, Nc, less=capi.OP_ENERGY_PIPE, lnak_complex=_is_cplx(Lnak))
     check(lib().sfq_energy(ptr(E), ptr(G), ptr(haj), ptr(Lnak), int(_is_cplx(Lnak)), E0, W, N, M, Nc, int(addH1),
                            int(addEJ), int(addEXX), ptr(ws), ws.numel(), _stream()))
     return E

@@ -84,6 +84,7 @@ _SIGS = {
     "sfq_abi_version": ([], _I),
     "sfq_last_error": ([], ctypes.c_char_p),
     "sfq_memcpy": ([_VP, _VP, _SZ, _I, _VP], _I),
+    "sfq_int8_gains": ([_I, _I, _I, _I, _I, _I], _I),
     "sfq_workspace_size": ([_I, _I, _I, _I, _I], _SZ),
     "sfq_mixed_density_matrix": ([_VP, _I, _VP, _VP, _VP, _I, _I, _I, _I, _VP, _SZ, _VP], _I),
     "sfq_log_overlap": ([_VP, _I, _VP, _VP, _I, _I, _I, _VP, _SZ, _VP], _I),

@@ -56,11 +56,17 @@ size_t vbias_crt_bytes(int W, int N, int M, int Nc, bool l_cplx, bool prepared) 
   return parted_bytes(W, part(W, Nc, K, na, nb, prepared), K, na, nb, prepared);
 }
 
-// The FP64 tensor-pipe product walks K = N M in one chain per tile of few tiles: 19 us at K = 576, 58 at 1024 and
-// 1.27 ms at 16384 with 256 walkers; this path, whose launches cost more, takes 38, 32 and 372 us.
+// The FP64 tensor-pipe product walks K = N M in one chain per tile, of few tiles; this path's launches cost more and its
+// time hardly depends on W: with 8 walkers 64 us against 123 at K = 4096, Nc = 640, and 0.95 ms against 1.98 at
+// K = 40000, Nc = 2400.  At K = 1024 the outputs decide: 37 against 35 us with 8 x 640 of them, 41 against 35 with
+// 300 x 65 (K = 1030), 39 against 43 with 64 x 640, 45 against 59 with 256 x 640; a complex Lnak, twice the flops there,
+// gains from K = 2323 (70 against 78 us) on at least.
 bool vbias_crt_ok(int W, int N, int M, int Nc, bool l_cplx) {
   const long K = (long)N * M;
   return W >= 8 && W <= 65535 && Nc >= 64 && K >= 1024 && K * (l_cplx ? 2 : 1) <= kMaxK;
+}
+bool vbias_crt_gains(int W, int N, int M, int Nc, bool l_cplx) {
+  return l_cplx || (long)N * M >= 1536 || (long)W * Nc >= 40000;
 }
 
 int vbias_crt(const cplx* G, const void* Lnak, bool l_cplx, const Planes* Lq, cplx* v, int W, int N, int M, int Nc,
@@ -112,9 +118,9 @@ size_t vhs_crt_bytes(int W, long rows, int Nc, bool prepared) {
   return parted_bytes(W, part(W, rows, Nc, 2, 1, false), Nc, 2, 1, prepared);
 }
 
-// Converting L (M^2 Nc elements) costs what the FP64 product of about 64 walkers does: from 96 walkers on
-// the call gains (1.4x at M = 128 with 128 walkers, 2.8x at M = 256 and 400 with 256), at 64 it is even.  With
-// L's planes prepared the product alone counts.
+// Converting L (M^2 Nc elements) costs what the FP64 product of about 64 walkers does: 160 us against 186 with 96 walkers
+// at M = 128, Nc = 640, 167 against 222 with 128, 0.98 ms against 1.57 with 96 at M = 256, Nc = 1536, 4.96 against
+// 13.2 with 256 at M = 400, Nc = 2400; at 64 it is even.  With L's planes prepared the product alone counts.
 bool vhs_crt_ok(int W, long rows, int Nc, bool prepared) {
   const double flops = 4.0 * W * double(rows) * Nc;
   if (W > 65535 || Nc > kMaxK || Nc < 96) return false;
@@ -171,12 +177,15 @@ size_t propagate_crt_bytes(int W, int M, int N, int npol) {
   return flag_bytes(wc) + blk + std::max(b, 2 * blk) + slack();  // the FP64 terms' buffers share the space
 }
 
-// The conversions of V and of the Taylor terms grow as M^2 and M N, the products as M^2 N: 1.9x at M = 400 with
-// 100 electrons and 256 walkers, 1.1x at M = 256 with 64, slower with few electrons (0.8x at M = 256 with 32) and
-// even at M = 192; 16 walkers at M = 400 gain 1.3x with 100 electrons and nothing with 50.
+// The conversion of V and of the terms grows as M^2 and M N, the products as M^2 N a term.  Order 6, this path against
+// the FP64 tensor pipe: 7.17 ms against 11.3 at M = 400 with 100 electrons and 256 walkers, 4.45 against 4.97 with 48,
+// 0.71 against 0.81 with 100 and 16 walkers; 1.21 against 1.31 at M = 256 with 64 and 128; even with 64 walkers there,
+// 0.76 against 0.68 at M = 240 with 48 and 80.  V is converted once for all terms: order 1, 2, 3, 4 take 0.50, 0.64,
+// 0.78, 0.92 ms against 0.41, 0.59, 0.77, 0.95 at M = 256 (128 walkers), 3.40 and 4.15 against 3.45 and 5.02 for 1 and
+// 2 at M = 400.
 bool propagate_crt_ok(int W, int M, int N, int npol, bool p_cplx, int order) {
   const double flops = 64.0 * W * M * double(M) * N * npol;
-  return !p_cplx && order >= 1 && W <= 30000 && M >= 240 && M <= 4096 && N * npol >= 48 && flops >= 1.4e10 &&
+  return !p_cplx && (long)order * M >= 800 && W <= 30000 && M >= 250 && M <= 4096 && N * npol >= 48 && flops >= 1.4e10 &&
          walker_gemm_fits(N * npol, M, M, 2);
 }
 
@@ -244,14 +253,18 @@ int energy_nv(int w, int N, int M, int Nc, bool l_cplx) {
 }
 }  // namespace
 
-// A walker's [re; im] rows fill 128-row tiles: with 50 electrons 112 of them (1.26x at M = 200, Nc = 1200, 128
-// walkers), with 32 half, where the product and the reconstruction together take what the FP64 product does.
-// Below 40 GFLOP (about a millisecond there) its launches count.
+// A walker's [re; im] rows fill 128-row tiles: with 50 electrons 112 of them, with 32 half, where the product and the
+// reconstruction together take what the FP64 product does.  Below 40 GFLOP (about a millisecond there) its launches
+// count.  Storing and reconstructing T does not depend on M, the FP64 product does: 1.70 ms against 1.39 at M = 120
+// (20 walkers, N = 45, Nc = 1100), 1.59 against 1.27 at M = 130 (10, 116, 300), even at M = 160 (64, 40, 900), 1.66
+// against 2.40 at M = 240 (80, 48, 300); with a complex Lnak, twice the flops there, 2.31 against 3.20 at M = 90.
 bool energy_crt_ok(int W, int N, int M, int Nc, bool l_cplx) {
   return W <= 65535 && N >= 40 && N <= kExxMaxN && M >= 32 && 8.0 * W * N * double(N) * M * Nc >= 4e10 &&
          energy_n_bytes(energy_walkers(W, N, M, l_cplx), N, M, l_cplx) <= kChunkBytes &&
          walker_gemm_fits(N, 16 * n4_of(N), M, l_cplx ? 2 : 1);
 }
+
+bool energy_crt_gains(int M, bool l_cplx) { return M * (l_cplx ? 2 : 1) >= 160; }
 
 size_t energy_crt_bytes(int W, int N, int M, int Nc, bool l_cplx) {
   const int w = energy_walkers(W, N, M, l_cplx), nv = energy_nv(w, N, M, Nc, l_cplx), N4 = n4_of(N);

@@ -1155,7 +1155,7 @@ struct Engine {
       scratch = s2;
       return true;
     };
-    crt_energy = ndet == 1 && ops::energy_crt_ok(W, N, Mr, Nc, lc) &&
+    crt_energy = ndet == 1 && ops::energy_crt_ok(W, N, Mr, Nc, lc) && ops::energy_crt_gains(Mr, lc) &&
                  take(true, 0, ops::energy_crt_bytes(W, N, Mr, Nc, lc));
     crt_prop = ops::propagate_crt_ok(W, M, N, npol, false, p.taylor_order) &&
                take(true, 0, ops::propagate_crt_bytes(W, M, N, npol));

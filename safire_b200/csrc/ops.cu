@@ -428,6 +428,25 @@ size_t sfq_workspace_size(int op, int nwalk, int nmo, int nel, int nchol) {
   }
 }
 
+int sfq_int8_gains(int op, int nwalk, int nmo, int nel, int nchol, int lnak_complex) {
+  if (nwalk <= 0 || nmo <= 0) return 0;
+  const bool lc = lnak_complex != 0 || op == SFQ_OP_VBIAS_COMPLEX;
+  switch (op) {
+    case SFQ_OP_PROPAGATE:
+      return nel > 0 && ops::propagate_crt_ok(nwalk, nmo, nel, 1, false, 6);
+    case SFQ_OP_VBIAS:
+    case SFQ_OP_VBIAS_COMPLEX:
+      return nel > 0 && nchol > 0 && ops::vbias_crt_ok(nwalk, nel, nmo, nchol, lc) &&
+             ops::vbias_crt_gains(nwalk, nel, nmo, nchol, lc);
+    case SFQ_OP_VHS:
+      return nchol > 0 && ops::vhs_crt_ok(nwalk, (long)nmo * nmo, nchol, false);
+    case SFQ_OP_ENERGY:
+      return nel > 0 && nchol > 0 && ops::energy_crt_ok(nwalk, nel, nmo, nchol, lc) && ops::energy_crt_gains(nmo, lc);
+    default:
+      return 0;
+  }
+}
+
 int sfq_mixed_density_matrix(const void* A, int a_complex, const void* B, void* C, void* ovlp, int nwalk, int nmo,
                              int nel, int compact, void* ws, size_t ws_bytes, void* stream) {
   if (nwalk < 0 || nmo < 0 || nel < 0) return record_error(SFQ_ERR_SHAPE, "negative size");

@@ -446,34 +446,72 @@ def test_parts_of_energy():
         assert torch.isnan(bad[:, 1].real).all()
 
 
-def test_no_room_for_the_workspace():
-    """Where the device has no room for the int8 path's workspace the calls run on the FP64 tensor pipe, as they do
-    with its own workspace."""
+def test_no_room_for_the_workspace(monkeypatch):
+    """Where the device has no room for the int8 path's workspace (an allocator that refuses it) the calls run on the
+    FP64 tensor pipe, in its own; where there is none for that either, they raise as before."""
     from safire_b200 import afqmc, capi
     g = torch.Generator(device="cuda").manual_seed(31)
     W, M, N, Nc = 90, 250, 48, 700
     G, L, Lik = _cn(g, W, N, M), _rn(g, Nc, N, M), _rn(g, M, M, Nc)
-    Ge, haj, Le = _cn(g, 20, 45, 120), _cn(g, 45, 120), _rn(g, 1100, 45, 120)
+    Ge, haj, Le = _cn(g, 20, 45, 170), _cn(g, 45, 170), _rn(g, 1100, 45, 170)
     SM, X, V = _cn(g, W, M, N), _cn(g, 100, Nc), _cn(g, W, M, M) * (0.3 / math.sqrt(M))
     P1 = torch.eye(M, device="cuda", dtype=torch.float64) + 1e-2 * _rn(g, M, M)
-    # (call, bytes of its result and of the FP64 pipe's workspace, of the int8 path's)
-    calls = [(lambda: afqmc.vbias(G, L, 0.01), 16 * W * Nc, _workspace_path(capi.OP_VBIAS, W, M, N, Nc)),
-             (lambda: afqmc.vHS(Lik, X, 0.01), 16 * 100 * M * M, _workspace_path(capi.OP_VHS, 100, M, 0, Nc)),
-             (lambda: afqmc.Propagate(SM.clone(), P1, V),
-              16 * W * M * N + _workspace_path(capi.OP_PROPAGATE_PIPE, W, M, N, 0),
-              16 * W * M * N + _workspace_path(capi.OP_PROPAGATE, W, M, N, 0)),
-             (lambda: afqmc.energy(Ge, haj, Le), _workspace_path(capi.OP_ENERGY_PIPE, 20, 120, 45, 1100),
-              _workspace_path(capi.OP_ENERGY, 20, 120, 45, 1100))]
-    for call, need, full in calls:
-        assert full > need + (8 << 20)
+    calls = [(lambda: afqmc.vbias(G, L, 0.01), 0, _workspace_path(capi.OP_VBIAS, W, M, N, Nc)),
+             (lambda: afqmc.vHS(Lik, X, 0.01), 0, _workspace_path(capi.OP_VHS, 100, M, 0, Nc)),
+             (lambda: afqmc.Propagate(SM.clone(), P1, V), _workspace_path(capi.OP_PROPAGATE_PIPE, W, M, N, 0),
+              _workspace_path(capi.OP_PROPAGATE, W, M, N, 0)),
+             (lambda: afqmc.energy(Ge, haj, Le), _workspace_path(capi.OP_ENERGY_PIPE, 20, 170, 45, 1100),
+              _workspace_path(capi.OP_ENERGY, 20, 170, 45, 1100))]
+    empty = torch.empty
+    for call, pipe, full in calls:
+        assert full > pipe
         want = call()
-        torch.cuda.empty_cache()
-        total = torch.cuda.mem_get_info()[1]
-        held = torch.cuda.memory_reserved()
-        torch.cuda.set_per_process_memory_fraction((held + (need + full) / 2) / total)
-        try:
-            got = call()
-        finally:
-            torch.cuda.set_per_process_memory_fraction(1.0)
+
+        def refuse(most):
+            def alloc(*size, **kw):
+                if kw.get("dtype") is torch.uint8 and size[0] > most:
+                    raise torch.OutOfMemoryError("no room")
+                return empty(*size, **kw)
+            monkeypatch.setattr(afqmc.torch, "empty", alloc)
+
+        refuse(full - 1)
+        got = call()
+        if pipe:
+            refuse(pipe - 1)
+            with pytest.raises(torch.OutOfMemoryError):
+                call()
+        monkeypatch.undo()
         # each side rounds its sums of up to 12000 terms in its own order
         assert _rel(got, want) < U * math.sqrt(2 * N * M) and not torch.equal(got, want)
+
+
+def test_int8_path_where_it_does_not_gain():
+    """Sizes that the int8 path takes without being the faster one: the calls leave them to the FP64 tensor pipe, and a
+    C caller's full workspace still chooses it."""
+    from safire_b200 import afqmc, capi
+    from safire_b200.capi import check, lib, ptr
+    g = torch.Generator(device="cuda").manual_seed(41)
+    W, M, N, Nc = 300, 103, 10, 65
+    assert not lib().sfq_int8_gains(capi.OP_VBIAS, W, M, N, Nc, 0)
+    G, L = _cn(g, W, N, M), _rn(g, Nc, N, M)
+    ws = torch.empty(_workspace_path(capi.OP_VBIAS, W, M, N, Nc), dtype=torch.uint8, device="cuda")
+    v = torch.empty(W, Nc, dtype=torch.complex128, device="cuda")
+    check(lib().sfq_vbias_ws(ptr(G), ptr(L), 0, ptr(v), W, N, M, Nc, 0.25, 1, ptr(ws), ws.numel(), _stream()))
+    pipe = afqmc.vbias(G, L, 0.25)
+    R = G.reshape(W, -1) @ L.to(torch.complex128).reshape(Nc, -1).T
+    assert _rel(v, R) < 1e-14 and _rel(pipe, R) < 1e-14 and not torch.equal(v, pipe)
+    for W, M, N, Nc in ((20, 120, 45, 1100), (10, 130, 116, 300)):  # padded columns; the largest block in shared memory
+        assert not lib().sfq_int8_gains(capi.OP_ENERGY, W, M, N, Nc, 0)
+        G, haj, L = _cn(g, W, N, M), _cn(g, N, M), _rn(g, Nc, N, M)
+        ws = torch.empty(_workspace_path(capi.OP_ENERGY, W, M, N, Nc), dtype=torch.uint8, device="cuda")
+        E = torch.empty(W, 3, dtype=torch.complex128, device="cuda")
+        check(lib().sfq_energy(ptr(E), ptr(G), ptr(haj), ptr(L), 0, 0.0, W, N, M, Nc, 1, 1, 1, ptr(ws), ws.numel(),
+                               _stream()))
+        pipe = afqmc.energy(G, haj, L)
+        scale = pipe.abs().max(dim=0).values
+        # two FP64 evaluations of sums of up to 1.2e6 products of sums of M terms
+        assert float(((E - pipe).abs() / scale).max()) < 1e-12 and not torch.equal(E, pipe)
+        L[5, 2, 3] = float("nan")
+        check(lib().sfq_energy(ptr(E), ptr(G), ptr(haj), ptr(L), 0, 0.0, W, N, M, Nc, 1, 1, 1, ptr(ws), ws.numel(),
+                               _stream()))
+        assert torch.isnan(E[:, 1].real).all() and torch.equal(E[:, 0], pipe[:, 0])

@@ -14,8 +14,8 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 # every product of an engine of these sizes is on the int8 path (vHS from 32 walkers, the energy from 40 electrons, the
-# propagation from 240 orbitals and 48 electrons)
-M, N, NC, W = 240, 48, 300, 80
+# propagation from 250 orbitals and 48 electrons)
+M, N, NC, W = 256, 48, 300, 80
 DT = 1e-4
 
 
