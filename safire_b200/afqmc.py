@@ -27,11 +27,9 @@ def _stream():
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def _ws(op, nwalk, nmo, nel, nchol=0, less=None, lnak_complex=False):
-    """The operation's workspace.  `less` (0: none) is the one with which the FP64 tensor pipe does the work of the int8
-    tensor cores: where these do not gain, and where the device has no room for theirs."""
-    if less is not None and not lib().sfq_int8_gains(op, nwalk, nmo, nel, nchol, int(lnak_complex)):
-        op, less = less, None
+def _ws(op, nwalk, nmo, nel, nchol=0, less=None):
+    """The operation's workspace; where the device has no room for it, the one (of `less`; 0: none) with which the FP64
+    tensor pipe does the work of the int8 tensor cores."""
     try:
         n = lib().sfq_workspace_size(op, nwalk, nmo, nel, nchol) if op else 0
         return torch.empty(max(int(n), 1), dtype=torch.uint8, device="cuda")
@@ -39,6 +37,11 @@ def _ws(op, nwalk, nmo, nel, nchol=0, less=None, lnak_complex=False):
         if less is None:
             raise
     return _ws(less, nwalk, nmo, nel, nchol)
+
+
+def _gaining(op, less, nwalk, nmo, nel, nchol, lnak_complex):
+    """op where the int8 tensor cores gain (sfq_int8_gains), else less."""
+    return op if lib().sfq_int8_gains(op, nwalk, nmo, nel, nchol, int(lnak_complex)) else less
 
 
 def _is_cplx(t):
@@ -119,7 +122,8 @@ def vbias(G, Lnak, dt, closed=True):
     W = G.shape[0]
     Nc, N, M = Lnak.shape
     v = torch.empty((W, Nc), dtype=torch.complex128, device="cuda")
-    ws = _ws(capi.OP_VBIAS_COMPLEX if _is_cplx(Lnak) else capi.OP_VBIAS, W, M, N, Nc, less=0)
+    lc = _is_cplx(Lnak)
+    ws = _ws(_gaining(capi.OP_VBIAS_COMPLEX if lc else capi.OP_VBIAS, 0, W, M, N, Nc, lc), W, M, N, Nc, less=0)
     check(lib().sfq_vbias_ws(ptr(G), ptr(Lnak), int(_is_cplx(Lnak)), ptr(v), W, N, M, Nc, dt, int(closed), ptr(ws),
                              ws.numel(), _stream()))
     return v
@@ -143,7 +147,8 @@ def energy(G, haj, Lnak, E0=0.0, addH1=True, addEJ=True, addEXX=True):
     W = G.shape[0]
     Nc, N, M = Lnak.shape
     E = torch.empty((W, 3), dtype=torch.complex128, device="cuda")
-    ws = _ws(capi.OP_ENERGY, W, M, N, Nc, less=capi.OP_ENERGY_PIPE, lnak_complex=_is_cplx(Lnak))
+    op = _gaining(capi.OP_ENERGY, capi.OP_ENERGY_PIPE, W, M, N, Nc, _is_cplx(Lnak))
+    ws = _ws(op, W, M, N, Nc, less=capi.OP_ENERGY_PIPE)
     check(lib().sfq_energy(ptr(E), ptr(G), ptr(haj), ptr(Lnak), int(_is_cplx(Lnak)), E0, W, N, M, Nc, int(addH1),
                            int(addEJ), int(addEXX), ptr(ws), ws.numel(), _stream()))
     return E

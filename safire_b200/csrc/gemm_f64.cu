@@ -8,10 +8,16 @@ using namespace gemm_detail;
 namespace {
 constexpr long kSMs = 148;
 
-template <bool AC, bool BC, bool CONJA, bool AK, bool BK, int BM, int BN, int WM, int WN, int STAGES>
+template <bool AC, bool BC, bool CONJA, bool AK, bool BK, int BM, int BN, int WM, int WN, int STAGES, bool REDO = false>
 int launch(const GemmDesc& d, cudaStream_t st) {
   using C_ = Cfg<AC, BC, CONJA, AK, BK, BM, BN, WM, WN, STAGES>;
-  auto k = gemm_f64_kernel<AC, BC, CONJA, AK, BK, BM, BN, WM, WN, STAGES>;
+  // the operand kinds of the products behind the modular ones (crt_ops.cu)
+  constexpr bool can_redo = AK && !CONJA && ((AC || BC) || BK) && !(AC && !BC && !BK);
+  if (!REDO && d.redo.call) {
+    if constexpr (can_redo) return launch<AC, BC, CONJA, AK, BK, BM, BN, WM, WN, STAGES, true>(d, st);
+    else return record_error(SFQ_ERR_UNSUPPORTED, "gemm_f64: flags with this operand combination not built");
+  }
+  auto k = gemm_f64_kernel<AC, BC, CONJA, AK, BK, BM, BN, WM, WN, STAGES, REDO>;
   static bool attr_set = false;  // one opt-in per instantiation (per process, device-agnostic)
   if (!attr_set) {
     SFQ_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::SMEM));

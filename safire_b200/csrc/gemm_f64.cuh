@@ -91,7 +91,19 @@ struct Cfg {
   static_assert(TM % 8 == 0 && TN % 8 == 0, "warp tile must be a multiple of 8");
 };
 
-template <bool AC, bool BC, bool CONJA, bool AK, bool BK, int BM, int BN, int WM, int WN, int STAGES>
+// whether a tile has nothing that d.redo asks for (the same for the whole block)
+__device__ __forceinline__ bool not_asked(const GemmDesc& d, int m0, int bm, long bz) {
+  if (d.redo_div == 0) return d.redo.asked(bz) == d.redo_rest;
+  const int4 c = d.redo.asked();
+  if (c.x | c.y) return false;
+  if (!c.z) return true;
+  int any = 0;
+  for (int i = m0 + threadIdx.x; i < m0 + bm && i < d.M; i += blockDim.x) any |= d.redo.row[i / d.redo_div];
+  return !__syncthreads_or(any);
+}
+
+// REDO: d.redo is looked at.  A kernel of its own: its tests cost the launches without them 1 to 2 %.
+template <bool AC, bool BC, bool CONJA, bool AK, bool BK, int BM, int BN, int WM, int WN, int STAGES, bool REDO>
 __global__ void __launch_bounds__(WM* WN * 32)
     gemm_f64_kernel(GemmDesc d) {
   using C_ = Cfg<AC, BC, CONJA, AK, BK, BM, BN, WM, WN, STAGES>;
@@ -100,19 +112,7 @@ __global__ void __launch_bounds__(WM* WN * 32)
   const int wm = warp / WN, wn = warp % WN;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   const long bz = blockIdx.z;
-  bool all_rows = true;
-  if (d.redo.call && d.redo_div == 0) {
-    if (d.redo.asked(bz) == d.redo_rest) return;
-  } else if (d.redo.call) {
-    const int4 c = d.redo.asked();
-    if (!(c.x | c.y | c.z)) return;
-    if (!(c.x | c.y)) {
-      int any = 0;
-      for (int i = m0 + tid; i < m0 + BM && i < d.M; i += C_::THREADS) any |= d.redo.row[i / d.redo_div];
-      if (!__syncthreads_or(any)) return;
-      all_rows = false;
-    }
-  }
+  if (REDO && not_asked(d, m0, BM, bz)) return;
   if (d.mask && !d.mask[bz]) return;  // the whole CTA: batches left out by the mask
   if (d.upper_only && m0 >= n0 + BN) return;  // every row of the tile is below every column
 
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(WM* WN * 32)
 #pragma unroll
   for (int i = 0; i < C_::FM; ++i) {
     int gm = m0 + wm * C_::TM + i * 8 + lr;
-    if (gm >= d.M || (!all_rows && !d.redo.row[gm / d.redo_div])) continue;
+    if (gm >= d.M || (REDO && d.redo_div && !d.redo.asked(gm / d.redo_div))) continue;
 #pragma unroll
     for (int j = 0; j < C_::FN; ++j) {
 #pragma unroll
