@@ -58,12 +58,15 @@ struct Tables {
   double P_hi, P_lo;       // P 2^-64 as the sum of two doubles
 };
 
-constexpr unsigned kModuli[15] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
+__host__ __device__ constexpr unsigned modulus(int i) {
+  constexpr unsigned p[NMOD] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
+  return p[i];
+}
 
 constexpr Tables make_tables() {
   Tables t{};
   u128 P = 1;
-  for (int i = 0; i < 15; ++i) P *= kModuli[i];
+  for (int i = 0; i < NMOD; ++i) P *= modulus(i);
   // the top 53 bits of P and the rest, exactly
   int sh = 0;
   while ((P >> sh) >= (u128(1) << 53)) ++sh;
@@ -73,8 +76,8 @@ constexpr Tables make_tables() {
   const u128 rest = P - ((P >> sh) << sh);
   t.P_lo = (double((unsigned long long)(rest >> 32)) * 4294967296.0 + double((unsigned long long)(rest & 0xffffffffu))) /
            18446744073709551616.0;
-  for (int i = 0; i < 15; ++i) {
-    const unsigned p = kModuli[i];
+  for (int i = 0; i < NMOD; ++i) {
+    const unsigned p = modulus(i);
     t.mod[i] = p;
     t.m32[i] = int(((1ull << 32) + p - 1) / p);
     t.m39[i] = unsigned(((1ull << 39) + p - 1) / p);
@@ -82,8 +85,8 @@ constexpr Tables make_tables() {
     t.big30[i] = unsigned(((3ull << 29) + p - 1) / p * p);
     t.r16[i] = 65536u % p;
     unsigned rest = 1;  // P / p_i mod p_i
-    for (int j = 0; j < 15; ++j)
-      if (j != i) rest = rest * (kModuli[j] % p) % p;
+    for (int j = 0; j < NMOD; ++j)
+      if (j != i) rest = rest * (modulus(j) % p) % p;
     unsigned inv = 0;
     for (unsigned x = 1; x < p; ++x)
       if (rest * x % p == 1) inv = x;
@@ -130,14 +133,13 @@ inline Redo lay_out_flags(char*& at, long W) {
 }
 
 // ---- the product of residues: C_i = A_i B_i^T mod p_i for every modulus ------------------------
-// Output row ((part * batch + b) * M + m), column n, at C + i * c_plane + row * ldc + n (bytes).
-// A rows a_off[part][seg] + b * a_bs + m, B rows b_off[seg] + b * b_bs + n, summed over the segments
+// Output row part * M + m, column n, at C + i * c_plane + row * ldc + n (bytes).
+// A rows a_off[part][seg] + m, B rows b_off[seg] + n, summed over the segments
 // (a complex product: parts re, im; segments against Re B and Im B).  Rows whose magnitudes do not pass raise the
 // flag of walker m % wmod.
 struct Gemm {
   Planes A, B;
-  int M = 0, N = 0, K = 0, batch = 1, parts = 1, segs = 1;
-  long a_bs = 0, b_bs = 0;
+  int M = 0, N = 0, K = 0, parts = 1, segs = 1;
   long a_off[2][2] = {{0, 0}, {0, 0}};
   long b_off[2] = {0, 0};
   uint8_t* C = nullptr;

@@ -31,7 +31,6 @@ __device__ __forceinline__ int row_exponent(double n2, bool any, bool asks, cons
 // now exact in FP32, modulo each of them: the FP64, conversion, FP32 and byte-permute pipes share the
 // work.  About 0.65 cycles an element and SM; integer dot products and high multiplies of the value's
 // bytes, two pipes for everything, took 1.5.
-constexpr int kGroups = 6;
 // a row's magnitudes: their scale, and 127 for all of a row of zeros, whose products are exact
 struct Mag {
   double scale;
@@ -44,18 +43,14 @@ struct Quad {
 #pragma unroll
     for (int j = 0; j < 4; ++j) y[j] = rint(x[j] * sc);
   }
-  static __host__ __device__ constexpr uint32_t mod_of(int i) {
-    constexpr uint32_t m[15] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197};
-    return m[i];
-  }
   // f(i, word): the four residues of modulus i as bytes, centred (-p / 2 .. p / 2)
   template <typename F>
   __device__ __forceinline__ void words(F&& f) const {
 #pragma unroll
-    for (int g = 0; g < kGroups; ++g) {
-      constexpr int at[kGroups + 1] = {0, 2, 4, 7, 10, 13, 15};
+    for (int g = 0; g < 6; ++g) {
+      constexpr int at[7] = {0, 2, 4, 7, 10, 13, 15};
       const int i0 = at[g], n = at[g + 1] - at[g];
-      const double Q = double(mod_of(i0)) * mod_of(i0 + 1) * (n == 3 ? mod_of(i0 + n - 1) : 1u);
+      const double Q = double(modulus(i0)) * modulus(i0 + 1) * (n == 3 ? modulus(i0 + n - 1) : 1u);
       const double inv = 1.0 / Q;
       float x[4];
       uint32_t lo[4];
@@ -73,11 +68,11 @@ struct Quad {
 #pragma unroll
       for (int i = i0; i < i0 + n; ++i) {
         uint32_t b[4];
-        if (mod_of(i) == 256) {  // Q is a multiple of 256
+        if (modulus(i) == 256) {  // Q is a multiple of 256
 #pragma unroll
           for (int j = 0; j < 4; ++j) b[j] = lo[j];
         } else {
-          const float p = float(mod_of(i)), ip = 1.0f / p;
+          const float p = float(modulus(i)), ip = 1.0f / p;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const float q = __fadd_rn(fmaf(x[j], ip, 12582912.0f), -12582912.0f);

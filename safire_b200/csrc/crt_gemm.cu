@@ -1,5 +1,5 @@
 // Products of residue planes on the int8 tensor cores (see crt.cuh).
-#include "crt.cuh"
+#include "crt_dev.cuh"
 #include "tc_common.cuh"
 
 #include <algorithm>
@@ -9,9 +9,6 @@ namespace crt {
 using namespace tc;
 
 namespace {
-
-constexpr Tables kTab = make_tables();
-__constant__ Tables c_tab = kTab;
 
 constexpr int BM = 128;       // MMA M: accumulator rows = TMEM lanes
 constexpr int BN = 256;       // widest tile: one of two accumulator buffers of 256 columns
@@ -45,10 +42,10 @@ struct Maps {
   CUtensorMap a, b;
 };
 struct KP {
-  int M, N, K, batch, parts, segs, bn;
+  int M, N, K, parts, segs, bn;
   int MT, NT, KT;  // tiles along M and N; K slices per segment
   long tiles;
-  long a_bs, b_bs, a_off[2][2], b_off[2];
+  long a_off[2][2], b_off[2];
   uint8_t* C;
   long ldc, c_plane;
   int wide;        // reduce_kind of the K sums
@@ -100,11 +97,11 @@ struct Mod {
 };
 __device__ __forceinline__ Mod mod_of(int i, int kind) {
   Mod m;
-  m.p = c_tab.mod[i];
-  m.m39 = c_tab.m39[i];
-  m.m32 = c_tab.m32[i];
-  m.big = kind == 2 ? c_tab.big30[i] : c_tab.big27[i];
-  m.r16 = c_tab.r16[i];
+  m.p = c_crt.mod[i];
+  m.m39 = c_crt.m39[i];
+  m.m32 = c_crt.m32[i];
+  m.big = kind == 2 ? c_crt.big30[i] : c_crt.big27[i];
+  m.r16 = c_crt.r16[i];
   return m;
 }
 template <int KIND>
@@ -195,9 +192,9 @@ __device__ __forceinline__ void check64(uint32_t taddr, int n, int least, bool l
 inline int reduce_kind(long K) { return K <= 1024 ? 0 : K <= 8192 ? 1 : 2; }
 
 struct Tile {
-  int mt, part, nt, b, p;
+  int mt, part, nt, p;
 };
-// tiles in the order (modulus, batch, column tile, part, row tile): the row tiles that share a B
+// tiles in the order (modulus, column tile, part, row tile): the row tiles that share a B
 // tile run side by side, so a B operand larger than L2 is read from memory once
 __device__ __forceinline__ Tile decode(const KP& k, long t) {
   Tile c;
@@ -206,9 +203,7 @@ __device__ __forceinline__ Tile decode(const KP& k, long t) {
   c.part = int(t % k.parts);
   t /= k.parts;
   c.nt = int(t % k.NT);
-  t /= k.NT;
-  c.b = int(t % k.batch);
-  c.p = int(t / k.batch);
+  c.p = int(t / k.NT);
   return c;
 }
 
@@ -261,8 +256,8 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
       for (long t = blockIdx.x; t < k.tiles && !stop; t += gridDim.x) {
         const Tile c = decode(k, t);
         for (int sg = 0; sg < k.segs && !stop; ++sg) {
-          const int ra = int(k.a_off[c.part][sg] + c.b * k.a_bs) + c.mt * BM;
-          const int rb = int(k.b_off[sg] + c.b * k.b_bs) + c.nt * k.bn;
+          const int ra = int(k.a_off[c.part][sg]) + c.mt * BM;
+          const int rb = int(k.b_off[sg]) + c.nt * k.bn;
           const int kend = k.hold ? min(k.KT, int(k.hold_at - it)) : k.KT;
           for (int kt = 0; kt < kend; ++kt, ++it) {
             const int s = int(it % STAGES);
@@ -345,7 +340,7 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
       fence_after();
       const Tile c = decode(k, t);
       const Mod md = mod_of(c.p, k.wide);
-      uint8_t* out = k.C + c.p * k.c_plane + ((long)c.part * k.batch + c.b) * k.M * k.ldc;
+      uint8_t* out = k.C + c.p * k.c_plane + (long)c.part * k.M * k.ldc;
       const uint32_t taddr = tmem + (uint32_t(q * 32) << 16) + b * BN;
       const int n0 = c.nt * k.bn, mg = c.mt * BM + q * 32 + (lane & ~3);
       const int cc = 64 * ((warp - 2) >> 2);  // the quarter's four warps take 64 columns each
@@ -376,8 +371,11 @@ __global__ void __launch_bounds__(kThreads, 1) crt_gemm_kernel(const __grid_cons
 // C[w] (2 N x cols) = [re; im] rows of walker w's operand times shared or per-walker rows, for every
 // modulus.  One work unit is a walker (or a range of its electrons, or of the columns), one modulus: the
 // walker's residues (blocks -im, re, im; or re, im) stay in shared memory while the other operand's rows
-// stream past them.  Bound by the stream out of L2 (about 44 bytes a cycle and SM): the one-tile-at-a-time
-// kernel above loads both operands of every 128 x 208 tile, 341 KB at 400 orbitals, this one a third of it.
+// stream past them.  The one-tile-at-a-time kernel above loads both operands of every 128 x 208 tile, 341 KB at 400
+// orbitals, this one a third of it.  Per-walker operands larger than L2 together come from memory (the Taylor term at
+// M = 400, N = 100: DRAM 58 % busy, L2 42 %, tensor pipe 34 %); with short K and a shared operand the producer thread's
+// issue loop and the stores of the residues bound it (the energy at M = 200: 0.68 ms a launch of 128 walkers and 150
+// vectors, 1.44 GB of residues written; a test of two more words per slice in that loop cost 7 %).
 constexpr int RBK = 64;        // K slice: one 64-byte swizzle row
 constexpr int RMAXKT = 64;     // K slices at most
 constexpr int RMAXST = 8;
@@ -677,12 +675,12 @@ int make_map(CUtensorMap* m, const Planes& o, long K, int box_rows, int bk = BK)
 }  // namespace
 
 int gemm(const Gemm& g, cudaStream_t st) {
-  if (g.M <= 0 || g.N <= 0 || g.batch <= 0 || g.K <= 0) return record_error(SFQ_ERR_SHAPE, "crt gemm: empty product");
+  if (g.M <= 0 || g.N <= 0 || g.K <= 0) return record_error(SFQ_ERR_SHAPE, "crt gemm: empty product");
   if ((long)g.K * g.segs > kMaxK) return record_error(SFQ_ERR_SHAPE, "crt gemm: K of %ld too long", (long)g.K * g.segs);
   if (g.parts < 1 || g.parts > 2 || g.segs < 1 || g.segs > 2 || g.wmod < 1 || !g.redo.call || !g.redo.row)
     return record_error(SFQ_ERR_ARG, "crt gemm: %d parts of %d segments, walkers %d", g.parts, g.segs, g.wmod);
   KP k{};
-  k.M = g.M; k.N = g.N; k.K = g.K; k.batch = g.batch; k.parts = g.parts; k.segs = g.segs;
+  k.M = g.M; k.N = g.N; k.K = g.K; k.parts = g.parts; k.segs = g.segs;
   k.MT = (g.M + BM - 1) / BM;
   // equal column tiles of at most 256, a multiple of 16 wide: the count that leaves the least to the last wave,
   // a tile costing its columns plus about 64 for its share of the other operand (2400 columns against 512
@@ -691,7 +689,7 @@ int gemm(const Gemm& g, cudaStream_t st) {
   const int nt0 = (g.N + BN - 1) / BN;
   for (int nt = nt0; nt < nt0 + 6; ++nt) {
     const int bn = ((g.N + nt - 1) / nt + 15) / 16 * 16, tiles = (g.N + bn - 1) / bn;
-    const long waves = ((long)k.MT * g.parts * tiles * g.batch * kPlanes + sm_count() - 1) / sm_count();
+    const long waves = ((long)k.MT * g.parts * tiles * kPlanes + sm_count() - 1) / sm_count();
     const double cost = double(waves) * (bn + 64);
     if (nt == nt0 || cost < 0.98 * best) {
       best = cost;
@@ -700,8 +698,7 @@ int gemm(const Gemm& g, cudaStream_t st) {
     }
   }
   k.KT = (g.K + BK - 1) / BK;
-  k.tiles = (long)k.MT * k.parts * k.NT * k.batch * (g.check ? kPlanes : NMOD);
-  k.a_bs = g.a_bs; k.b_bs = g.b_bs;
+  k.tiles = (long)k.MT * k.parts * k.NT * (g.check ? kPlanes : NMOD);
   for (int p = 0; p < 2; ++p)
     for (int s = 0; s < 2; ++s) k.a_off[p][s] = g.a_off[p][s];
   k.b_off[0] = g.b_off[0]; k.b_off[1] = g.b_off[1];

@@ -1,13 +1,12 @@
 // Host dispatch for the FP64 DMMA GEMM: picks the instantiation from operand kinds/contiguity
 // and the tile shape from the problem shape.
 #include "gemm_f64.cuh"
+#include "tc_common.cuh"
 
 namespace sfq {
 using namespace gemm_detail;
 
 namespace {
-constexpr long kSMs = 148;
-
 template <bool AC, bool BC, bool CONJA, bool AK, bool BK, int BM, int BN, int WM, int WN, int STAGES, bool REDO = false>
 int launch(const GemmDesc& d, cudaStream_t st) {
   using C_ = Cfg<AC, BC, CONJA, AK, BK, BM, BN, WM, WN, STAGES>;
@@ -51,15 +50,21 @@ int pick_tile(const GemmDesc& d, cudaStream_t st) {
     // shape comes to the FP64 pipe's rate (a tile's operand loads per DMMA).  Small matrices then fill
     // 32 x 8 tiles instead of 128 x 32 (24 x 6 per walker: 10 us a product), few tiles spread over more
     // SMs, and 33 to 48 rows or columns take 48 instead of 64.  All tiles add in the same order: same bits.
+    // The rates were set by timed calls of few tiles (per step of 24 orbitals, 6 electrons, 64 walkers: 179 us with the
+    // former two shapes, 84 with these; a propagation at 131 x 37, 100 walkers: 584 and 449 us; the Green's function
+    // at 129 x 33, 90 walkers: 81 and 72 us).  With every SM full (384 x 192 x 384, 148 matrices) the shapes reach, in
+    // this order, 26.7, 20.6, 24.9, 30.1, 29.0 and 24.0 TFLOP/s complex by complex and 27.6, 26.6, 24.8, 26.2, 22.6 and
+    // 17.0 real by complex.
     struct Shape { int bm, bn; double rate; };
     static constexpr Shape shapes[] = {{64, 64, 1.0}, {128, 32, 0.95}, {48, 48, 0.95}, {32, 32, 0.85}, {32, 16, 0.7},
                                        {32, 8, 0.5}};
+    const long sms = tc::sm_count();
     int pick = 0;
     double best = 0.0;
     for (int i = 0; i < 6; ++i) {
       const Shape& t = shapes[i];
       const long ctas = (long)((d.M + t.bm - 1) / t.bm) * ((d.N + t.bn - 1) / t.bn) * d.batch;
-      const double cost = double((ctas + kSMs - 1) / kSMs) * t.bm * t.bn / t.rate;
+      const double cost = double((ctas + sms - 1) / sms) * t.bm * t.bn / t.rate;
       if (i == 0 || (cost < best && (d.M + t.bm - 1) / t.bm <= 65535)) {
         best = cost;
         pick = i;

@@ -19,11 +19,10 @@
 // products at twice the rate); 2 slices: 3.
 //
 // Persistent kernel: one CTA per SM walks a static list of 128 x BN output tiles; warp 0 issues
-// TMA loads of K slices into a ring of stages (64 int8 elements per slice, 64-byte swizzle, where a
-// tile's K range is short; 128 elements, 128-byte swizzle, half the stages, where it reaches 1024),
+// TMA loads of K slices into a ring of stages (64 int8 elements per slice, 64-byte swizzle),
 // one thread of warp 1 issues tcgen05.mma.kind::i8 (M = 128, N = BN, K = 32) and commits each
-// stage, eight epilogue warps drain the group accumulators.  K tails are zero-filled by TMA and
-// their MMA steps skipped; K splits fall on multiples of 128 elements at either slice width.
+// stage, sixteen epilogue warps drain the group accumulators.  K tails are zero-filled by TMA and
+// their MMA steps skipped; K splits fall on multiples of 128 elements.
 // Every mbarrier wait is bounded from its own start; on expiry the kernel records SFQ_ERR_TIMEOUT,
 // waits for its own copies and MMAs, frees its tensor memory and returns.
 //

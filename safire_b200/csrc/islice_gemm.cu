@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kThreads, 1) islice_gemm_kernel(const __grid_c
       mbar_wait_for(done, 0, kWaitNs);
     }
     __syncwarp();
-  } else {  // epilogue warps 2..9 -> TMEM lane quarters 2,3,0,1 (a warp reaches only its quarter)
+  } else {  // epilogue warps 2..17 -> TMEM lane quarters 2,3,0,1 (a warp reaches only its quarter)
     const int q = warp & 3;
     const int row = q * 32 + lane;
     const int c0 = 16 * ((warp - 2) >> 2);  // the four warps of a quarter take every fourth 16-column chunk

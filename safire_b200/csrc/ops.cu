@@ -609,7 +609,9 @@ int sfq_energy(void* E, const void* G, const void* haj, const void* Lnak, int ln
   const bool lc = lnak_complex != 0;
   if (addEXX && nel > 0 && nmo > 0 && nchol > 0 && ops::energy_crt_ok(nwalk, nel, nmo, nchol, lc)) {
     const size_t room = ws_bytes - 2 * bk - 256;  // behind exxn and kl
-    if (ws_bytes >= 2 * bk + 256 && room >= ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc)) {
+    // (the pipe's chunk may be as large as what the int8 path takes: where that does not gain, only more chooses it)
+    if (ws_bytes >= 2 * bk + 256 && room >= ops::energy_crt_bytes(nwalk, nel, nmo, nchol, lc) &&
+        (ops::energy_crt_gains(nmo, lc) || ws_bytes > bt + 2 * bk)) {
       char* at = aligned(ws);
       return ops::energy_crt((cplx*)E, (const cplx*)G, (const cplx*)haj, Lnak, lc, E0, nwalk, nel, nmo, nchol, addH1,
                              addEJ, at + 2 * bk, room, (cplx*)at, (cplx*)(at + bk), S(stream), -1);

@@ -1,7 +1,7 @@
 // tcgen05 / TMA / mbarrier building blocks shared by the tensor-core products (sm_100a).
 //
-// Operand tiles are K-major with the 128-byte swizzle: rows of 128 bytes (64 bf16 or 128 int8
-// elements), 8-row groups 1024 bytes apart, loaded by TMA into shared memory.  One thread issues
+// Operand tiles are K-major and swizzled: rows of 128 bytes (64 bf16 or 128 int8 elements), 8-row groups
+// 1024 bytes apart (smem_desc), or of 64 bytes, 512 apart, loaded by TMA into shared memory.  One thread issues
 // tcgen05.mma on shared-memory descriptors; accumulators live in tensor memory and are read back
 // with tcgen05.ld.  Every wait on an mbarrier is bounded by a time limit measured from the start
 // of that wait (%globaltimer), so a launch that keeps making progress never times out, while a

@@ -515,3 +515,13 @@ def test_int8_path_where_it_does_not_gain():
         check(lib().sfq_energy(ptr(E), ptr(G), ptr(haj), ptr(L), 0, 0.0, W, N, M, Nc, 1, 1, 1, ptr(ws), ws.numel(),
                                _stream()))
         assert torch.isnan(E[:, 1].real).all() and torch.equal(E[:, 0], pipe[:, 0])
+    # a pipe's workspace that would hold the int8 path's too
+    W, M, N, Nc = 128, 120, 44, 700
+    assert _workspace_path(capi.OP_ENERGY_PIPE, W, M, N, Nc) == _workspace_path(capi.OP_ENERGY, W, M, N, Nc)
+    G, haj, L = _cn(g, W, N, M), _cn(g, N, M), _rn(g, Nc, N, M)
+    n = _workspace_path(capi.OP_ENERGY, W, M, N, Nc) + 512
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    E = torch.empty(W, 3, dtype=torch.complex128, device="cuda")
+    check(lib().sfq_energy(ptr(E), ptr(G), ptr(haj), ptr(L), 0, 0.0, W, N, M, Nc, 1, 1, 1, ptr(ws), n, _stream()))
+    pipe = afqmc.energy(G, haj, L)
+    assert float(((E - pipe).abs() / pipe.abs().max(dim=0).values).max()) < 1e-12 and not torch.equal(E, pipe)

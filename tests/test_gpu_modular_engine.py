@@ -6,6 +6,7 @@ import dataclasses
 import numpy as np
 import pytest
 
+from oracle import afqmc_oracle as O
 from safire_b200 import afqmc, synthetic
 from safire_b200.serve import Server
 
@@ -79,6 +80,29 @@ def test_planes_against_the_pipe(kind):
     _close(a.energy(), b.energy(), 1e-11)
     a.close()
     b.close()
+
+
+def test_planes_against_the_oracle():
+    """Two steps, the orthogonalization and the energy of walkers that the planes hold, at the bar of the FP64 engine."""
+    s = _system("closed")
+    x = _walkers(s)
+    e = _engine(s, True, x)
+    ham = O.Hamiltonian(s.hcore, s.Likn, s.PsiT)
+    prop = O.Propagator(ham, DT, seed=7)
+    wo = O.Walkers(x.copy())
+    Eo = O.init_walkers(ham, wo)
+    assert abs(e.init() - Eo) < 1e-10 * abs(Eo)
+    for step in range(2):
+        prop.propagate(wo, Eo, step)
+        e.propagate(Eo, step)
+    prop.orthogonalize(wo)
+    e.orthogonalize()
+    SM, pr = e.walkers()
+    _close(SM, wo.SM, 1e-10)
+    _close(pr["WEIGHT"], wo.weight, 1e-10)
+    _close(pr["OVLP"], wo.ovlp, 1e-10)
+    _close(e.energy(), O.wfn_energy_noupdate(ham, wo)[0], 1e-10)
+    e.close()
 
 
 def test_blocks_replayed_from_a_graph():

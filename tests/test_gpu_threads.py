@@ -54,3 +54,29 @@ def test_sizes_that_take_different_shared_memory(kind):
             jobs.append(lambda A=cn(1, n, n): afqmc.inverse_logdet(A))
     torch.cuda.synchronize()
     assert _run_together(jobs, 1500) == []
+
+
+def test_group_of_members_with_different_shared_memory():
+    """Members whose exchange blocks need more than 48 KB of shared memory beside smaller ones, captured into one graph
+    before any of it runs: every member's block is the one it gets alone."""
+    import numpy as np
+
+    from safire_b200 import afqmc, capi, synthetic
+    blk = dict(ortho_interval=2, pop_interval=4, equilibration_steps=0, measure_interval=2, relax=0.1, steer=True)
+    members = [(120, 80, 240, capi.PRECISION_INT8X3), (48, 12, 96, capi.PRECISION_INT8X3),
+               (80, 60, 160, capi.PRECISION_FP64), (24, 6, 96, capi.PRECISION_FP64)]
+
+    def engines():
+        return [afqmc.AfqmcEngine(synthetic.make_system(synthetic.SystemSpec(M=M, N=N, Nc=Nc, decay=float(M), seed=50 + i)),
+                                  6, dt=1e-4, seed=i, precision=p) for i, (M, N, Nc, p) in enumerate(members)]
+
+    grouped, alone = engines(), engines()
+    grp = afqmc.EngineGroup(grouped)
+    E0 = np.array([e.init() for e in grouped])
+    Eg, st, mg = grp.run_block(4, E0, step0=0, **blk)
+    assert not st.any()
+    for i, e in enumerate(alone):
+        e.init()
+        Ea, ma = e.run_block(4, E0[i], step0=0, **blk)
+        assert Eg[i] == Ea and np.array_equal(mg[i], ma)
+        assert np.array_equal(grouped[i].walkers()[0], e.walkers()[0])
