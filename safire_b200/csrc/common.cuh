@@ -68,6 +68,8 @@ int record_error(int code, const char* fmt, ...);
 // What a modular product (crt.cuh) could not hold and asks of the FP64 kernels launched behind it, in device memory:
 // call[0] (an operand that all walkers share) or call[1] (an expired wait): the whole call, row[w]: walker w, and
 // call[2] the number of such walkers.  One load tells the many blocks of those kernels that nothing is asked for.
+// call[3] is call[2] as the last modular product found it: kernels that may raise flags themselves, in which call[2] could
+// change under way, look at that to see whether any walker is left for them.
 struct Redo {
   int* call = nullptr;  // four of them, on a 16-byte boundary
   int* row = nullptr;
@@ -81,6 +83,8 @@ struct Redo {
     const int4 c = asked();
     return c.x != 0 || c.z == nwalk;
   }
+  __device__ __forceinline__ void settle() const { call[3] = call[2]; }
+  __device__ __forceinline__ bool none_left(int nwalk) const { return call[3] == nwalk; }
   __device__ __forceinline__ void ask(long w) const {
     if (!row[w] && atomicExch(row + w, 1) == 0) atomicAdd(call + 2, 1);
   }

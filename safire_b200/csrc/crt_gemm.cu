@@ -446,9 +446,12 @@ __global__ void __launch_bounds__(kThreads, 1) crt_walker_kernel(const __grid_co
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  // nothing to do where the FP64 product computes all walkers (flags of launches before this one; a test of each unit's
-  // walker made the loops below a tenth slower)
-  if (!CHECK && k.redo.all_asked(k.batch)) return;
+  // nothing to do where the FP64 product computes all walkers (flags of launches before this one)
+  if (CHECK && k.redo.none_left(k.batch)) return;
+  if (!CHECK) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) k.redo.settle();
+    if (k.redo.all_asked(k.batch)) return;
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < k.stages; ++s) {
       mbar_init(&full[s], 1);

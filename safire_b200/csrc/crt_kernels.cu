@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(256, 4) taylor_kernel(const uint8_t* c, long l
   const int M4 = (M + 3) / 4 * 4, q4 = M4 / 4;
   double* part = rows + 2 * R * M4;
   double* scs = part + R * q4;
+  if (redo.none_left(int(WN / N))) return;
   const long r0 = (long)blockIdx.x * R;
   const int nr = int(WN - r0 < R ? WN - r0 : R), items = nr * q4;
   for (int it = threadIdx.x; it < items; it += 256) {
