@@ -341,7 +341,8 @@ __global__ void __launch_bounds__(RT) energy_exx_f32_kernel(const float* C, int 
 }
 
 // The same two sums with the walker's N x N block of one n in shared memory: each element is read once, in
-// rows; the kernels above read T[b][a] again down the columns of a chunk that does not fit in L2.
+// rows; the kernels above read T[b][a] again down the columns of a chunk that does not fit in L2 (but keep more
+// blocks on an SM).
 // E: float2 (planar FP32 parts) or cplx.
 __device__ __forceinline__ cplx as_cplx(float2 v) { return mk(v.x, v.y); }
 __device__ __forceinline__ cplx as_cplx(cplx v) { return v; }
@@ -392,9 +393,15 @@ __global__ void __launch_bounds__(RT) energy_exx_f32_sm_kernel(const float* C, i
   exx_block<float2>([&](int a, int b) { return make_float2(Cr[a * ldc + b], Ci[a * ldc + b]); }, nel, nup, exxn + o,
                     kl + o);
 }
-constexpr size_t kExxSmem = 200 * 1024;  // a block's N x N in shared memory up to this, else through the caches
 template <typename E>
-size_t exx_smem(int nel) { return sizeof(E) * (size_t)nel * (nel | 1); }
+constexpr size_t exx_smem(int nel) { return sizeof(E) * (size_t)nel * (nel | 1); }
+// Through shared memory for these sizes, else through the caches.  Planar FP32 (shared memory against caches, us): 85
+// against 68 at N = 16, 96 against 98 at 20, 121 against 232 at 32 (128 walkers, 200 vectors), 132 against 163 at 50 (64),
+// 396 against 477 at 100, 376 against 282 at 113 (32).  FP64, whose blocks are twice as large and whose lines hold whole
+// elements: 256 against 246 at N = 20 (500 vectors), 320 against 349 at 24 (600), 459 against 517 at 32 (640), 325 against 258
+// at 33 (60 walkers, 700), 2607 against 1556 at 50 (128, 1200), 3089 against 653 at 100 (16, 900).
+constexpr bool exx_shared_f32(int nel) { return nel >= 20 && nel <= 100; }
+constexpr bool exx_shared_f64(int nel) { return nel >= 24 && nel <= 32; }
 
 __global__ void __launch_bounds__(RT) energy_finish_kernel(const cplx* exxn, const cplx* kl, cplx* E3, int nchol,
                                                            double scl, int addEXX, int addEJ) {
@@ -673,10 +680,9 @@ int energy_exx_reduce(const cplx* T, int nwalk, int nel, int nv, int n0, int nch
                       cudaStream_t st, int nup, const Redo* redo) {
   if (nwalk <= 0 || nv <= 0) return SFQ_OK;
   dim3 grid(nv, nwalk);
-  const size_t sm = exx_smem<cplx>(nel);
-  if (sm <= kExxSmem) {
-    SFQ_MAX_SMEM(energy_exx_sm_kernel, kExxSmem);
-    energy_exx_sm_kernel<<<grid, RT, sm, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, redo ? *redo : Redo{});
+  if (exx_shared_f64(nel)) {
+    SFQ_MAX_SMEM(energy_exx_sm_kernel, exx_smem<cplx>(32));
+    energy_exx_sm_kernel<<<grid, RT, exx_smem<cplx>(nel), st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, redo ? *redo : Redo{});
   } else {
     energy_exx_kernel<<<grid, RT, 0, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, redo ? *redo : Redo{});
   }
@@ -688,10 +694,9 @@ int energy_exx_reduce_f32(const float* C, int nwalk, int nel, int nv, int n0, in
                           cplx* kl, cudaStream_t st, int nup) {
   if (nwalk <= 0 || nv <= 0) return SFQ_OK;
   dim3 grid(nv, nwalk);
-  const size_t sm = exx_smem<float2>(nel);
-  if (sm <= kExxSmem) {
-    SFQ_MAX_SMEM(energy_exx_f32_sm_kernel, kExxSmem);
-    energy_exx_f32_sm_kernel<<<grid, RT, sm, st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
+  if (exx_shared_f32(nel)) {
+    SFQ_MAX_SMEM(energy_exx_f32_sm_kernel, exx_smem<float2>(100));
+    energy_exx_f32_sm_kernel<<<grid, RT, exx_smem<float2>(nel), st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
   } else {
     energy_exx_f32_kernel<<<grid, RT, 0, st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
   }
