@@ -255,16 +255,18 @@ int energy_nv(int w, int N, int M, int Nc, bool l_cplx) {
 
 // A walker's [re; im] rows fill 128-row tiles: with 50 electrons 112 of them, with 32 half, where the product and the
 // reconstruction together take what the FP64 product does.  Below 40 GFLOP (about a millisecond there) its launches
-// count.  Storing and reconstructing T does not depend on M, the FP64 product does: 1.70 ms against 1.39 at M = 120
-// (20 walkers, N = 45, Nc = 1100), 1.59 against 1.27 at M = 130 (10, 116, 300), even at M = 160 (64, 40, 900), 1.66
-// against 2.40 at M = 240 (80, 48, 300); with a complex Lnak, twice the flops there, 2.31 against 3.20 at M = 90.
+// count.  Storing and reconstructing T does not depend on M, the FP64 product does: 1.65 ms against 1.47 at M = 150 and
+// 1.67 both at 180 (20 walkers, N = 45, Nc = 1100), 4.05 against 4.68 at 170 (64, 50, 900), 3.74 against 3.26 at 160 and
+// 3.84 against 4.39 at 240 (24, 80, 700), 2.29 both at 200 (12, 100, 500), 11.6 against 13.9 at 200 (128, 50, 1200); with a
+// complex Lnak, twice the flops there, 2.26 both at M = 90 (30, 45, 900), 2.29 against 2.58 at 90 (16, 70, 800), 1.89
+// against 2.54 at 110 (30, 45, 900).
 bool energy_crt_ok(int W, int N, int M, int Nc, bool l_cplx) {
   return W <= 65535 && N >= 40 && N <= kExxMaxN && M >= 32 && 8.0 * W * N * double(N) * M * Nc >= 4e10 &&
          energy_n_bytes(energy_walkers(W, N, M, l_cplx), N, M, l_cplx) <= kChunkBytes &&
          walker_gemm_fits(N, 16 * n4_of(N), M, l_cplx ? 2 : 1);
 }
 
-bool energy_crt_gains(int M, bool l_cplx) { return M * (l_cplx ? 2 : 1) >= 160; }
+bool energy_crt_gains(int M, bool l_cplx) { return M * (l_cplx ? 2 : 1) >= 180; }
 
 size_t energy_crt_bytes(int W, int N, int M, int Nc, bool l_cplx) {
   const int w = energy_walkers(W, N, M, l_cplx), nv = energy_nv(w, N, M, Nc, l_cplx), N4 = n4_of(N);

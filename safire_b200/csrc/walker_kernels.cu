@@ -340,17 +340,14 @@ __global__ void __launch_bounds__(RT) energy_exx_f32_kernel(const float* C, int 
   }
 }
 
-// The same two sums with the walker's N x N block of one n in shared memory: each element is read once, in
-// rows; the kernels above read T[b][a] again down the columns of a chunk that does not fit in L2 (but keep more
-// blocks on an SM).
-// E: float2 (planar FP32 parts) or cplx.
+// The FP32 sums with the walker's N x N block of one n in shared memory: each element is read once, in rows; the kernel
+// above reads T[b][a] again down the columns of a chunk that does not fit in L2.
 __device__ __forceinline__ cplx as_cplx(float2 v) { return mk(v.x, v.y); }
-__device__ __forceinline__ cplx as_cplx(cplx v) { return v; }
-template <typename E, typename LOAD>
+template <typename LOAD>
 __device__ __forceinline__ void exx_block(LOAD&& load, int nel, int nup, cplx* exx, cplx* kl) {
   extern __shared__ __align__(16) unsigned char exx_sm[];
   __shared__ cplx red[RT / 32];
-  E* T = reinterpret_cast<E*>(exx_sm);
+  float2* T = reinterpret_cast<float2*>(exx_sm);
   const int P = nel | 1;
   // a warp to a row: an index division per element cost more than the sums
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -376,32 +373,21 @@ __device__ __forceinline__ void exx_block(LOAD&& load, int nel, int nup, cplx* e
     *kl = t;
   }
 }
-__global__ void __launch_bounds__(RT) energy_exx_sm_kernel(const cplx* T, int nel, int nv, int n0, int nchol,
-                                                           cplx* exxn, cplx* kl, int nup, Redo redo) {
-  const int n = blockIdx.x, w = blockIdx.y;
-  if (redo.call && !redo.asked(w)) return;
-  const long ld = (long)nv * nel, o = (long)w * nchol + n0 + n;
-  const cplx* Tw = T + (long)w * nel * ld + (long)n * nel;
-  exx_block<cplx>([&](int a, int b) { return Tw[a * ld + b]; }, nel, nup, exxn + o, kl + o);
-}
 __global__ void __launch_bounds__(RT) energy_exx_f32_sm_kernel(const float* C, int W, int nel, int nv, int n0, int nchol,
                                                                long ldc, cplx* exxn, cplx* kl, int nup) {
   const int n = blockIdx.x, w = blockIdx.y;
   const float* Cr = C + (long)w * nel * ldc + (long)n * nel;
   const float* Ci = Cr + (long)W * nel * ldc;
   const long o = (long)w * nchol + n0 + n;
-  exx_block<float2>([&](int a, int b) { return make_float2(Cr[a * ldc + b], Ci[a * ldc + b]); }, nel, nup, exxn + o,
-                    kl + o);
+  exx_block([&](int a, int b) { return make_float2(Cr[a * ldc + b], Ci[a * ldc + b]); }, nel, nup, exxn + o, kl + o);
 }
-template <typename E>
-constexpr size_t exx_smem(int nel) { return sizeof(E) * (size_t)nel * (nel | 1); }
-// Through shared memory for these sizes, else through the caches.  Planar FP32 (shared memory against caches, us): 85
-// against 68 at N = 16, 96 against 98 at 20, 121 against 232 at 32 (128 walkers, 200 vectors), 132 against 163 at 50 (64),
-// 396 against 477 at 100, 376 against 282 at 113 (32).  FP64, whose blocks are twice as large and whose lines hold whole
-// elements: 256 against 246 at N = 20 (500 vectors), 320 against 349 at 24 (600), 459 against 517 at 32 (640), 325 against 258
-// at 33 (60 walkers, 700), 2607 against 1556 at 50 (128, 1200), 3089 against 653 at 100 (16, 900).
-constexpr bool exx_shared_f32(int nel) { return nel >= 20 && nel <= 100; }
-constexpr bool exx_shared_f64(int nel) { return nel >= 24 && nel <= 32; }
+// Through shared memory for these sizes, else through the caches (shared memory against caches, us): 85 against 68 at
+// N = 16, 96 against 98 at 20, 121 against 232 at 32 (128 walkers, 200 vectors), 132 against 163 at 50 (64), 396 against 477 at
+// 100, 376 against 282 at 113 (32).  FP64 sums, whose blocks are twice as large, gained nothing that way below 24
+// electrons, 10 % from 24 to 32, and were up to 4.7 times slower above (2607 against 1556 us at N = 50, 128 walkers, 1200
+// vectors).
+constexpr bool exx_shared(int nel) { return nel >= 20 && nel <= 100; }
+constexpr size_t kExxSmem = sizeof(float2) * 100 * 101;
 
 __global__ void __launch_bounds__(RT) energy_finish_kernel(const cplx* exxn, const cplx* kl, cplx* E3, int nchol,
                                                            double scl, int addEXX, int addEJ) {
@@ -680,12 +666,7 @@ int energy_exx_reduce(const cplx* T, int nwalk, int nel, int nv, int n0, int nch
                       cudaStream_t st, int nup, const Redo* redo) {
   if (nwalk <= 0 || nv <= 0) return SFQ_OK;
   dim3 grid(nv, nwalk);
-  if (exx_shared_f64(nel)) {
-    SFQ_MAX_SMEM(energy_exx_sm_kernel, exx_smem<cplx>(32));
-    energy_exx_sm_kernel<<<grid, RT, exx_smem<cplx>(nel), st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, redo ? *redo : Redo{});
-  } else {
-    energy_exx_kernel<<<grid, RT, 0, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, redo ? *redo : Redo{});
-  }
+  energy_exx_kernel<<<grid, RT, 0, st>>>(T, nel, nv, n0, nchol, exxn, kl, nup < 0 ? nel : nup, redo ? *redo : Redo{});
   SFQ_LAUNCHED();
   return SFQ_OK;
 }
@@ -694,9 +675,9 @@ int energy_exx_reduce_f32(const float* C, int nwalk, int nel, int nv, int n0, in
                           cplx* kl, cudaStream_t st, int nup) {
   if (nwalk <= 0 || nv <= 0) return SFQ_OK;
   dim3 grid(nv, nwalk);
-  if (exx_shared_f32(nel)) {
-    SFQ_MAX_SMEM(energy_exx_f32_sm_kernel, exx_smem<float2>(100));
-    energy_exx_f32_sm_kernel<<<grid, RT, exx_smem<float2>(nel), st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
+  if (exx_shared(nel)) {
+    SFQ_MAX_SMEM(energy_exx_f32_sm_kernel, kExxSmem);
+    energy_exx_f32_sm_kernel<<<grid, RT, sizeof(float2) * nel * (nel | 1), st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
   } else {
     energy_exx_f32_kernel<<<grid, RT, 0, st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
   }

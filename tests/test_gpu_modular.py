@@ -453,15 +453,15 @@ def test_no_room_for_the_workspace(monkeypatch):
     g = torch.Generator(device="cuda").manual_seed(31)
     W, M, N, Nc = 90, 250, 48, 700
     G, L, Lik = _cn(g, W, N, M), _rn(g, Nc, N, M), _rn(g, M, M, Nc)
-    Ge, haj, Le = _cn(g, 20, 45, 170), _cn(g, 45, 170), _rn(g, 1100, 45, 170)
+    Ge, haj, Le = _cn(g, 20, 45, 190), _cn(g, 45, 190), _rn(g, 1100, 45, 190)
     SM, X, V = _cn(g, W, M, N), _cn(g, 100, Nc), _cn(g, W, M, M) * (0.3 / math.sqrt(M))
     P1 = torch.eye(M, device="cuda", dtype=torch.float64) + 1e-2 * _rn(g, M, M)
     calls = [(lambda: afqmc.vbias(G, L, 0.01), 0, _workspace_path(capi.OP_VBIAS, W, M, N, Nc)),
              (lambda: afqmc.vHS(Lik, X, 0.01), 0, _workspace_path(capi.OP_VHS, 100, M, 0, Nc)),
              (lambda: afqmc.Propagate(SM.clone(), P1, V), _workspace_path(capi.OP_PROPAGATE_PIPE, W, M, N, 0),
               _workspace_path(capi.OP_PROPAGATE, W, M, N, 0)),
-             (lambda: afqmc.energy(Ge, haj, Le), _workspace_path(capi.OP_ENERGY_PIPE, 20, 170, 45, 1100),
-              _workspace_path(capi.OP_ENERGY, 20, 170, 45, 1100))]
+             (lambda: afqmc.energy(Ge, haj, Le), _workspace_path(capi.OP_ENERGY_PIPE, 20, 190, 45, 1100),
+              _workspace_path(capi.OP_ENERGY, 20, 190, 45, 1100))]
     empty = torch.empty
     for call, pipe, full in calls:
         assert full > pipe
