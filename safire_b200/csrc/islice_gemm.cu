@@ -285,11 +285,32 @@ __device__ __forceinline__ void epilogue_tile(const KParams& p, uint32_t taddr, 
       }
       continue;
     }
-    if (!live) continue;
-    float* out = p.C + obase;
+    // Rows that do not start on 16 bytes (odd row lengths), or a last chunk: the half warps' 16 x 16 blocks transposed, so
+    // that a store instruction writes the 64 bytes of two rows.  A lane's own elements took 32 sectors an instruction
+    // (an exchange tensor with N = 45 and 807 vectors: 1578 us against 1177 with eight epilogue warps before).
 #pragma unroll
-    for (int jj = 0; jj < 16; ++jj)
-      if (jj < valid) out[jj] = p.accumulate ? __fadd_rn(v[jj], out[jj]) : v[jj];
+    for (int s = 1; s < 16; s *= 2) {
+      const bool up = lane & s;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (i & s) continue;
+        float &lo = v[i], &hi = v[i | s];
+        const float x = __shfl_xor_sync(0xffffffffu, up ? lo : hi, s);
+        if (up) lo = x;
+        else hi = x;
+      }
+    }
+    const int l = lane & 15;
+    if (l < valid) {
+      float* out = p.C + obase - (long)l * p.ldc + l;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        if (gm - l + i < p.M) {
+          float* o = out + i * p.ldc;
+          *o = p.accumulate ? __fadd_rn(v[i], *o) : v[i];
+        }
+      }
+    }
   }
 }
 

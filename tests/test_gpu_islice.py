@@ -301,3 +301,12 @@ def test_bounded_waits_expire_and_report_timeout():
     A, B = _operands(200, 150, 400, seed=9)
     assert np.array_equal(_int8_gemm(A, B, 3, 128)[0], R.gemm(A, B, 3))
     assert L.sfq_selftest_wait_expiry(0, None) == 2  # no limit is no test
+
+
+@pytest.mark.parametrize("N", [5, 15, 16, 17, 64, 67, 161, 162, 163])
+@pytest.mark.parametrize("nslices,tile", [(3, 160), (3, 64), (2, 128)])
+def test_rows_that_start_anywhere(N, nslices, tile):
+    """Output rows of any length (their starts on 4, 8 or 16 bytes) and every width of a last chunk, with rows past the
+    last tile: bit for bit the reference's."""
+    A, B = _operands(131, N, 70, seed=N)
+    assert np.array_equal(_int8_gemm(A, B, nslices, tile)[0], R.gemm(A, B, nslices))
