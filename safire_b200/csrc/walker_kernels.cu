@@ -381,12 +381,19 @@ __global__ void __launch_bounds__(RT) energy_exx_f32_sm_kernel(const float* C, i
   const long o = (long)w * nchol + n0 + n;
   exx_block([&](int a, int b) { return make_float2(Cr[a * ldc + b], Ci[a * ldc + b]); }, nel, nup, exxn + o, kl + o);
 }
-// Through shared memory for these sizes, else through the caches (shared memory against caches, us): 85 against 68 at
-// N = 16, 96 against 98 at 20, 121 against 232 at 32 (128 walkers, 200 vectors), 132 against 163 at 50 (64), 396 against 477 at
-// 100, 376 against 282 at 113 (32).  FP64 sums, whose blocks are twice as large, gained nothing that way below 24
-// electrons, 10 % from 24 to 32, and were up to 4.7 times slower above (2607 against 1556 us at N = 50, 128 walkers, 1200
+// Through shared memory where the columns of T, rows ldc floats apart, fall on few sets of the caches, and for middle
+// sizes; else through the caches.  Shared memory against caches, us: ldc a multiple of 16: 85 against 68 at N = 16, 96
+// against 98 at 20, 121 against 232 at 32, 228 against 354 at 44 (128 walkers, 200 vectors), 132 against 163 at 50, 147
+// against 408 at 64 (64), 396 against 477 at 100 (32); other ldc: 207 against 167 at N = 22 (60 walkers, 893 vectors), 447
+// against 402 at 45 (62, 807), 442 against 522 at 60 (64, 601), 310 against 333 at 75 (32, 501), 406 against 385 at 90 (32,
+// 401), 404 against 257 at 99 (16, 401), 376 against 282 at 113 (32, 150).  FP64 sums, whose blocks are twice as large,
+// gained nothing that way below 24 electrons, 10 % from 24 to 32, and were up to 4.7 times slower above (2607 against 1556 us
+// at N = 50, 128 walkers, 1200 vectors).
+// Two spins, half of whose pairs are left out, gain everywhere between: 365 against 392 us at 24 + 21 (62 walkers, 807
 // vectors).
-constexpr bool exx_shared(int nel) { return nel >= 20 && nel <= 100; }
+constexpr bool exx_shared(int nel, int nup, long ldc) {
+  return nel >= 20 && nel <= 100 && (ldc % 16 == 0 || (nel >= 52 && nel <= 80) || (nup > 0 && nup < nel));
+}
 constexpr size_t kExxSmem = sizeof(float2) * 100 * 101;
 
 __global__ void __launch_bounds__(RT) energy_finish_kernel(const cplx* exxn, const cplx* kl, cplx* E3, int nchol,
@@ -675,7 +682,7 @@ int energy_exx_reduce_f32(const float* C, int nwalk, int nel, int nv, int n0, in
                           cplx* kl, cudaStream_t st, int nup) {
   if (nwalk <= 0 || nv <= 0) return SFQ_OK;
   dim3 grid(nv, nwalk);
-  if (exx_shared(nel)) {
+  if (exx_shared(nel, nup, ldc)) {
     SFQ_MAX_SMEM(energy_exx_f32_sm_kernel, kExxSmem);
     energy_exx_f32_sm_kernel<<<grid, RT, sizeof(float2) * nel * (nel | 1), st>>>(C, nwalk, nel, nv, n0, nchol, ldc, exxn, kl, nup < 0 ? nel : nup);
   } else {

@@ -24,12 +24,15 @@ def test_fp64(N):
     assert ((E[:, 2] - 2 * (K * K).sum(1)).abs() <= u * 2 * (KA * KA).sum(1)).all()
 
 
-@pytest.mark.parametrize("N", [19, 20, 100, 101])
-def test_int8_slices(N):
+# rows of N Nc floats: multiples of 16 and not, on both sides of the sizes that go through shared memory; odd ones, whose
+# chunks and rows start anywhere
+@pytest.mark.parametrize("N,Nc", [(19, 64), (20, 64), (20, 50), (45, 51), (51, 51), (52, 51), (80, 51), (81, 51), (100, 52),
+                                  (101, 64)])
+def test_int8_slices(N, Nc):
     """Against the FP64 engine on the same walkers: 24-bit slices of G and L."""
     from safire_b200 import afqmc, capi, synthetic
     M, W = max(40, N + 6), 4
-    s = synthetic.make_system(synthetic.SystemSpec(M=M, N=N, Nc=50, decay=20.0, seed=N))
+    s = synthetic.make_system(synthetic.SystemSpec(M=M, N=N, Nc=Nc, decay=20.0, seed=N))
     rng = np.random.default_rng(N)
     x = s.initial_walkers(W)
     x = x + 0.1 / np.sqrt(M) * (rng.standard_normal(x.shape) + 1j * rng.standard_normal(x.shape))
